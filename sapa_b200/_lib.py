@@ -13,6 +13,8 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 # SAPA_B200_LIB points at another build of the same library (for example one compiled with extra flags)
 LIB_PATH = os.environ.get("SAPA_B200_LIB") or os.path.join(_HERE, "libsapa_b200.so")
 
+HOST_PATH = os.path.join(_HERE, "_host.so")
+
 SAPA_F32, SAPA_F16, SAPA_BF16, SAPA_F64 = 0, 1, 2, 3
 _DTYPE_CODE = {torch.float32: SAPA_F32, torch.float16: SAPA_F16, torch.bfloat16: SAPA_BF16, torch.float64: SAPA_F64}
 SAPA_ERR_UNSUPPORTED = -5
@@ -61,7 +63,7 @@ def lib() -> ctypes.CDLL:
     global _lib
     if _lib is not None:
         return _lib
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(HOST_PATH):
         try:
             from . import build as _build
             _build.build()
@@ -99,6 +101,24 @@ def lib() -> ctypes.CDLL:
         raise RuntimeError("libsapa_b200.so has a different ABI version than this Python package; rebuild it")
     _lib = handle
     return _lib
+
+
+host = None      # the native host path (csrc/host.cpp), loaded by the first op
+
+
+def load_host():
+    """Load the native host path and bind it to the library ``lib()`` uses."""
+    global host
+    if host is None:
+        lib()
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise RuntimeError("the native host path sapa_b200/_host.so is missing or does not fit this torch; run "
+                               f"`python -m sapa_b200.build` ({exc})") from exc
+        _host.bind(LIB_PATH)
+        host = _host
+    return host
 
 
 def dtype_code(t: torch.Tensor) -> int:

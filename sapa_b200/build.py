@@ -1,4 +1,5 @@
-"""Build recipe of ``libsapa_b200.so``: nvcc, sm_100a only, no torch headers (seconds per file).
+"""Build recipe of ``libsapa_b200.so`` (nvcc, sm_100a only, no torch headers: seconds per file) and of ``_host.so``, the
+native host path (g++ with the torch headers; calls the library through its C ABI).
 
     python -m sapa_b200.build [--force]
 
@@ -18,6 +19,9 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libsapa_b200.so")
 SOURCES = ["api.cu", "sapa_b.cu", "sapa_mma.cu", "sapa_tma.cu", "sapa_gath_mma.cu", "sapa_d.cu", "sapa_proj.cu", "sapa_nhwc.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "tma_util.cuh"), os.path.join(INCLUDE, "sapa_b200.h")]
+
+HOST = os.path.join(HERE, "_host.so")
+HOST_SOURCES = [os.path.join(CSRC, f) for f in ("host.cpp", "host_sapa.inc", "host_deform.inc", "host_module.inc")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -40,10 +44,41 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _build_host() -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    include = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    libs = cpp_extension.library_paths()
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in include), HOST_SOURCES[0], "-o", HOST,
+           *(f"-L{p}" for p in libs), *(f"-Wl,-rpath,{p}" for p in libs), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           "-ltorch_cuda", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host.cpp:\n{r.stdout}\n{r.stderr}")
+
+
+def _host_stale() -> bool:
+    deps = HOST_SOURCES + [HEADERS[-1], os.path.abspath(__file__)]
+    return not os.path.exists(HOST) or any(os.path.getmtime(d) > os.path.getmtime(HOST) for d in deps)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every CUDA source for sm_100a and link the shared library; returns its path."""
+    """Compile every CUDA source for sm_100a and link the shared library, and the host path; returns the library's path."""
+    with ThreadPoolExecutor(max_workers=1) as ex:
+        host = ex.submit(_build_host) if force or _host_stale() else None
+        _build_lib(force, verbose)
+        if host is not None:
+            host.result()
+    return LIB
+
+
+def _build_lib(force: bool, verbose: bool) -> None:
     if not force and not _stale():
-        return LIB
+        return
     nvcc = _nvcc()
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
@@ -65,7 +100,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run([nvcc, "-shared", "-o", LIB, *objs, "-lcudart"], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    return LIB
 
 
 if __name__ == "__main__":

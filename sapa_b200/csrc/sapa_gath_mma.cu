@@ -335,16 +335,8 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    const cudaError_t e = cudaFuncSetAttribute(sapa_gath_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
-    if (e != cudaSuccess) {
-        set_error("%s: cudaFuncSetAttribute failed: %s", name, cudaGetErrorString(e));
-        return SAPA_ERR_LAUNCH;
-    }
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-        set_error("%s: cannot query the SM count", name);
-        return SAPA_ERR_LAUNCH;
-    }
+    int sms = 0;
+    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_gath_mma_kernel<T>), G::SMEM_BYTES, name, sms)) return e;
     const long long resident = (long long)CTAS_PER_SM * sms;
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);

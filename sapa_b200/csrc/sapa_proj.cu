@@ -521,17 +521,8 @@ static int run_project(const Plan &p, const void *x, const void *gamma, const vo
     a.kblocks = (C + KCH - 1) / KCH;
     a.nx = p.nx; a.no = p.no; a.tmem_cols = p.tmem_cols; a.wide = p.wide;
     const size_t smem = p.smem;
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    if (cudaFuncSetAttribute(sapa_proj_umma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        set_error("sapa_project_forward: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(cudaGetLastError()));
-        return SAPA_ERR_LAUNCH;
-    }
+    int sms = 0;
+    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_proj_umma_kernel<T>), SMEM_LIMIT, "sapa_proj_umma_kernel", sms)) return e;
     sapa_proj_umma_kernel<T><<<std::min(a.total_tiles, sms), THREADS, smem, st>>>(a);
     return check_launch("sapa_proj_umma_kernel");
 }

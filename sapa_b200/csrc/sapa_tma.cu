@@ -844,16 +844,8 @@ static int launch_persistent(Kernel kernel, const char *name, int threads, int s
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-        set_error("%s: cudaFuncSetAttribute failed: %s", name, cudaGetErrorString(e));
-        return SAPA_ERR_LAUNCH;
-    }
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-        set_error("%s: cannot query the SM count", name);
-        return SAPA_ERR_LAUNCH;
-    }
+    int sms = 0;
+    if (int e = prepare_launch(reinterpret_cast<const void *>(kernel), smem, name, sms)) return e;
     const long long resident = (long long)ctas_per_sm * sms;
     // persistent grid with dynamic tile claiming (static striding left SMs with 6 to 8 tiles instead of ~6.9)
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);

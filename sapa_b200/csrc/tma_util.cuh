@@ -104,6 +104,32 @@ inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
+// Opts `kernel` in to `smem` bytes of dynamic shared memory on the current device (always the same number for one kernel)
+// and reports the device's SM count.  What was already done is remembered per thread: the runtime calls cost a microsecond
+// per launch otherwise.
+inline int prepare_launch(const void *kernel, int smem, const char *name, int &sms) {
+    constexpr int MAX_ENTRIES = 64, MAX_DEVICES = 64;
+    struct Entry { const void *kernel; int dev; };
+    static thread_local Entry done[MAX_ENTRIES];
+    static thread_local int used = 0, counts[MAX_DEVICES] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES ||
+        (counts[dev] == 0 && (cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || counts[dev] <= 0))) {
+        set_error("%s: cannot query the SM count", name);
+        return SAPA_ERR_LAUNCH;
+    }
+    sms = counts[dev];
+    for (int i = 0; i < used; ++i)
+        if (done[i].kernel == kernel && done[i].dev == dev) return SAPA_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+        set_error("%s: cudaFuncSetAttribute failed: %s", name, cudaGetErrorString(e));
+        return SAPA_ERR_LAUNCH;
+    }
+    if (used < MAX_ENTRIES) done[used++] = Entry{kernel, dev};
+    return SAPA_OK;
+}
+
 // Scheduler pair for the next launch on `st`.  A launch recorded into a CUDA graph keeps its pair for every replay,
 // so captured launches draw from a range of their own that the round-robin of ordinary launches never enters:
 // a replay can then never share a pair with an ordinary launch in flight on another stream.  (Two replays of graphs

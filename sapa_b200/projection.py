@@ -23,29 +23,11 @@ def project_supported(x: torch.Tensor, norm, conv: nn.Conv2d) -> bool:
         return False
     if norm is not None and not norm.affine:
         return False
-    b, c, h, w = x.shape
-    groups = norm.num_groups if norm is not None else 0
-    return int(_lib.lib().sapa_project_workspace(b, c, h * w, conv.out_channels, groups, _lib.dtype_code(x))) != 0
+    return _lib.load_host().project_workspace(x, norm.num_groups if norm is not None else 0, conv.weight) != 0
 
 
 def project(x: torch.Tensor, norm, conv: nn.Conv2d) -> torch.Tensor:
     """``conv(norm(x))`` for a 1x1 ``conv`` and a GroupNorm (or ``None``) ``norm``; ``x`` [B, C, H, W] -> [B, d, H, W]."""
-    b, c, h, w = x.shape
-    d = conv.out_channels
-    x = _lib.aligned(x.contiguous())
-    dt = x.dtype
-    weight = conv.weight.detach().reshape(d, c).to(dt).contiguous()
-    bias = conv.bias.detach().to(dt).contiguous() if conv.bias is not None else None
-    groups = norm.num_groups if norm is not None else 0
-    gamma = norm.weight.detach().to(dt).contiguous() if norm is not None else None
-    beta = norm.bias.detach().to(dt).contiguous() if norm is not None else None
-    eps = float(norm.eps) if norm is not None else 0.0
-    code = _lib.dtype_code(x)
-    nbytes = int(_lib.lib().sapa_project_workspace(b, c, h * w, d, groups, code))
-    if nbytes == 0:
-        raise NotImplementedError("sapa_project_forward does not take this shape / dtype (see project_supported)")
-    workspace = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-    out = torch.empty((b, d, h, w), dtype=dt, device=x.device)
-    _lib.call("sapa_project_forward", x.device, x, gamma, beta, weight, bias, out, workspace, workspace.numel(),
-              b, c, h * w, d, groups, eps, code)
-    return out
+    if norm is None:
+        return _lib.load_host().project(x, None, None, 0, 0.0, conv.weight, conv.bias)
+    return _lib.load_host().project(x, norm.weight, norm.bias, norm.num_groups, norm.eps, conv.weight, conv.bias)
