@@ -25,6 +25,8 @@
 
 namespace sapa {
 
+bool gath_mma_supported(int W, int dtype);
+
 namespace gmma {
 
 using namespace tmau;
@@ -41,13 +43,18 @@ __device__ int g_wait_timeout = 0;
 __device__ unsigned g_next_tile[SCHED_SLOTS];
 __device__ unsigned g_ctas_done[SCHED_SLOTS];
 
+constexpr int PT = 4 * 32;                 // threads of the four producer warps of the ragged form
+constexpr int NT_RAGGED = NW * 32 + PT;
+
 struct Args {
+    const void *hi;        // [B, C, 2H, 2W]: read by the ragged form, which has no tensor map
     const void *wt;        // [B, 25, 2H, 2W] window weights (attention map or logit gradients)
     void *out;             // [B, C, top + H + bottom, W]
     int B, C, H, W;        // H = low-res rows covered by the high-res inputs
     int top, Hout;         // row-slab form: the output has `top` extra rows above and Hout = top + H + bottom rows in all
                            // (the cells of the neighbouring slabs that this slab's pixels reach); 0 and H otherwise
     int tiles_x, tiles_y;
+    int csplit, stages;    // work items per tile, each with `stages` channel stages: few tiles are spread over more CTAs
     int sched_slot;
 };
 
@@ -74,8 +81,11 @@ template <typename T> __device__ __forceinline__ int px_off(int px, int ch) {
     else                          return ((((px >> 3) ^ (ch >> 1)) & 3) << 4) | ((px & 7) << 1);             // 64-byte swizzle
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT, CTAS_PER_SM)
+// RAGGED: high-res rows that are not multiples of 16 bytes (or low-res rows of odd length) - no tensor map, PW producer
+// warps copy the pixel pairs a fragment can reach (box pixels 4 .. 27; a pair is always on its own boundary because
+// high-res rows have an even length), static tile order, single-element stores where W is odd.
+template <typename T, bool RAGGED>
+__global__ void __launch_bounds__(RAGGED ? NT_RAGGED : NT, RAGGED ? 1 : CTAS_PER_SM)
 sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     using G = Geo<T>;
     constexpr bool F32 = sizeof(T) == 4;
@@ -96,13 +106,13 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     const int g = lane >> 2, t = lane & 3;
     const int sH = 2 * a.H, sW = 2 * a.W;
     const size_t hi_plane = (size_t)sH * sW;
-    const int nst = (a.C + NCH - 1) / NCH;         // stages per tile
-    const int ntiles = a.B * a.tiles_x * a.tiles_y;
+    const int nst = a.stages;                      // stages per work item
+    const int ntiles = a.B * a.tiles_x * a.tiles_y * a.csplit;     // work items
 
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < NSTAGE; ++i) {
-            mbar_init(full_addr + 8 * i, 1);
+            mbar_init(full_addr + 8 * i, RAGGED ? PT : 1);
             mbar_init(empty_addr + 8 * i, NW);
         }
 #pragma unroll
@@ -111,8 +121,44 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     }
     __syncthreads();
 
+    if constexpr (RAGGED) {
+        if (warp >= NW) {
+            const int ptid = tid - NW * 32, pair = ptid & 15;       // pairs 2 .. 13 of a box row
+            int slot = 0, phase = 0;
+            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+                int t_ = tile / a.csplit;
+                const int vb = tile % a.csplit * nst;
+                const int x0 = (t_ % a.tiles_x) * COLS; t_ /= a.tiles_x;
+                const int y0 = (t_ % a.tiles_y) * ROWS, n = t_ / a.tiles_y;
+                const T *img = static_cast<const T *>(a.hi) + (size_t)n * a.C * hi_plane;
+                const int px = 2 * x0 - 8 + 2 * pair, py = 2 * (y0 - a.top - 2);
+                const bool x_ok = px >= 0 && px < sW;
+                for (int it = 0; it < nst; ++it) {
+                    if (!mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) { atomicExch(&g_wait_timeout, 1); return; }
+                    const unsigned dst = ring_addr + slot * G::BOX_BYTES;
+                    const int c0 = (vb + it) * NCH;
+                    if (pair >= 2 && pair < 14) {
+#pragma unroll 8
+                        for (int i = 0; i < HR * NCH * 16 / PT; ++i) {
+                            const int rc = i * (PT / 16) + (ptid >> 4), ch = rc % NCH, row = rc / NCH;
+                            const bool ok = x_ok && c0 + ch < a.C && py + row >= 0 && py + row < sH;
+                            const T *src = ok ? img + (size_t)(c0 + ch) * hi_plane + (size_t)(py + row) * sW + px : img;
+                            const unsigned at = dst + row * (NCH * G::ROWB) + ch * G::ROWB + px_off<T>(2 * pair, ch);
+                            if constexpr (F32) cp_async8(at, src, ok);
+                            else cp_async4(at, src, ok);
+                        }
+                    }
+                    cp_async_arrive(full_addr + 8 * slot);
+                    if (++slot == NSTAGE) { slot = 0; phase ^= 1; }
+                }
+            }
+            asm volatile("cp.async.wait_all;\n" ::: "memory");      // no copy outlives the thread
+            return;
+        }
+    }
+
     // ---- producer state (lane 0 of the producer warp): the stages of successive tiles form one stream through the ring
-    int p_issued = 0, p_slot = 0, p_phase = 0, p_it = 0, p_ti = 0, p_n = 0, p_x0 = 0, p_y0 = 0;
+    int p_issued = 0, p_slot = 0, p_phase = 0, p_it = 0, p_ti = 0, p_n = 0, p_x0 = 0, p_y0 = 0, p_vb = 0;
     bool p_done = false;
     auto produce = [&](int need) {
         while (!p_done) {
@@ -140,12 +186,13 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                     p_done = true;
                     return;
                 }
+                p_vb = claimed % a.csplit * nst; claimed /= a.csplit;
                 p_x0 = (claimed % a.tiles_x) * COLS; claimed /= a.tiles_x;
                 p_y0 = (claimed % a.tiles_y) * ROWS; claimed /= a.tiles_y;
                 p_n = claimed;
             }
             mbar_expect_tx(bar, G::BOX_BYTES);
-            tma_load_4d(ring_addr + p_slot * G::BOX_BYTES, &xmap, bar, 2 * p_x0 - 8, p_it * NCH, 2 * (p_y0 - a.top - 2), p_n);
+            tma_load_4d(ring_addr + p_slot * G::BOX_BYTES, &xmap, bar, 2 * p_x0 - 8, (p_vb + p_it) * NCH, 2 * (p_y0 - a.top - 2), p_n);
             ++p_issued;
             if (++p_it == nst) { p_it = 0; ++p_ti; }
             if (++p_slot == NSTAGE) { p_slot = 0; p_phase ^= 1; }
@@ -154,7 +201,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
 
     // The producer is a warp of its own (one lane works): inside a consumer warp it took a quarter of that warp's time
     // and the other warps waited a third of theirs for stages it had not issued yet.
-    if (warp == NW) {
+    if (!RAGGED && warp == NW) {
         if (lane == 0) produce(0x7fffffff);
         return;
     }
@@ -179,17 +226,19 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     unsigned bw[5][3][F32 ? 2 : 1];
 
     int slot = 0, phase = 0, it = 0, ti = 0, gs = 0;
-    int n = 0, x0 = 0, y = 0;
+    int n = 0, x0 = 0, y = 0, vb = 0;
     T *o_ptr = nullptr;
     bool store_ok = false;
     for (;; ++gs) {
+        if (RAGGED && it == 0 && (int)blockIdx.x + ti * (int)gridDim.x >= ntiles) break;
         if (!mbar_wait_bounded(full_addr + 8 * slot, phase)) {
             atomicExch(&g_wait_timeout, 1);
             return;
         }
         if (it == 0) {
-            int tile = tile_ids[ti & 7];      // published by the producer before the barrier's phase completed
+            int tile = RAGGED ? (int)blockIdx.x + ti * (int)gridDim.x : tile_ids[ti & 7];      // published by the producer before the barrier's phase completed
             if (tile < 0) break;
+            vb = tile % a.csplit * nst; tile /= a.csplit;
             x0 = (tile % a.tiles_x) * COLS; tile /= a.tiles_x;
             const int y0 = (tile % a.tiles_y) * ROWS; tile /= a.tiles_y;
             n = tile;
@@ -224,7 +273,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                 }
             }
         }
-        const unsigned stage = ring_addr + slot * G::BOX_BYTES + (2 * wy + r) * (NCH * G::ROWB);
+        const unsigned stage = fresh(ring_addr + slot * G::BOX_BYTES + (2 * wy + r) * (NCH * G::ROWB));
 
         // one accumulator per parent row and m block: five (ten) independent MMA chains
         float acc[NB][5][4];
@@ -289,7 +338,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
             __syncwarp();
             if (lane == 0) mbar_arrive(empty_addr + 8 * slot);
             // D fragment: d0,d1 = G[ch g][cols 2t, 2t+1], d2,d3 = G[ch g+8][same]
-            const int c0 = it * NCH;
+            const int c0 = (vb + it) * NCH;
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 if (store_ok) {
@@ -298,7 +347,10 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                     for (int half = 0; half < 2; ++half)
                         if (c0 + 16 * b + 8 * half + g < a.C) {
                             T *oh = o + (size_t)(8 * half) * a.Hout * a.W;
-                            if constexpr (F32) *reinterpret_cast<float2 *>(oh) = make_float2(acc[b][0][2 * half], acc[b][0][2 * half + 1]);
+                            if (RAGGED && (a.W & 1)) {
+                                oh[0] = from_acc<T>(acc[b][0][2 * half]);
+                                if (x0 + 2 * t + 1 < a.W) oh[1] = from_acc<T>(acc[b][0][2 * half + 1]);
+                            } else if constexpr (F32) *reinterpret_cast<float2 *>(oh) = make_float2(acc[b][0][2 * half], acc[b][0][2 * half + 1]);
                             else *reinterpret_cast<unsigned *>(oh) = pack_pair(T(), acc[b][0][2 * half], acc[b][0][2 * half + 1]);
                         }
                 }
@@ -314,33 +366,42 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
 static std::atomic<unsigned> g_next_sched_slot{0}, g_next_captured_slot{0};
 
 template <typename T>
-static int launch(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, cudaStream_t st) {
+static int launch(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype, cudaStream_t st) {
     using G = Geo<T>;
-    const char *name = "sapa_gath_mma_kernel";
-    CUtensorMap xmap;
+    // rows a tensor map can describe and paired stores: the TMA form
+    const bool ragged = !gath_mma_supported(W, dtype);
+    const char *name = ragged ? "sapa_gath_kernel" : "sapa_gath_mma_kernel";
+    CUtensorMap xmap{};
     const CUtensorMapDataType ty = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const CUtensorMapSwizzle sw = sizeof(T) == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-    if (encode_tiled_fn() == nullptr) return SAPA_ERR_UNSUPPORTED;
-    if (!make_nchw_map(&xmap, hi, 2 * W, 2 * H, C, B, BPX, G::NCH, HR, ty, G::ES, sw)) {
+    if (!ragged && !make_nchw_map(&xmap, hi, 2 * W, 2 * H, C, B, BPX, G::NCH, HR, ty, G::ES, sw)) {
         set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
         return SAPA_ERR_UNSUPPORTED;
     }
     Args a{};
-    a.wt = wt; a.out = out; a.B = B; a.C = C; a.H = H; a.W = W; a.top = top; a.Hout = top + H + bottom;
+    a.hi = hi; a.wt = wt; a.out = out; a.B = B; a.C = C; a.H = H; a.W = W; a.top = top; a.Hout = top + H + bottom;
     a.tiles_x = ceil_div(W, COLS);
     a.tiles_y = ceil_div(a.Hout, ROWS);
-    const long long nblocks = (long long)B * a.tiles_x * a.tiles_y;
+    a.csplit = 1; a.stages = ceil_div(C, G::NCH);
+    long long nblocks = (long long)B * a.tiles_x * a.tiles_y;
     if (nblocks > 0x7fffffffLL) {
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
     int sms = 0;
-    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_gath_mma_kernel<T>), G::SMEM_BYTES, name, sms)) return e;
-    const long long resident = (long long)CTAS_PER_SM * sms;
+    const void *kernel = ragged ? reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, true>) : reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, false>);
+    if (int e = prepare_launch(kernel, G::SMEM_BYTES, name, sms)) return e;
+    const long long resident = (long long)(ragged ? 1 : CTAS_PER_SM) * sms;
+    while (a.stages % 2 == 0 && 2 * nblocks <= resident) {      // every channel is independent: halve the items while all run at once
+        a.stages /= 2;
+        a.csplit *= 2;
+        nblocks *= 2;
+    }
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
-    sapa_gath_mma_kernel<T><<<grid, NT, G::SMEM_BYTES, st>>>(xmap, a);
+    if (ragged) sapa_gath_mma_kernel<T, true><<<grid, NT_RAGGED, G::SMEM_BYTES, st>>>(xmap, a);
+    else sapa_gath_mma_kernel<T, false><<<grid, NT, G::SMEM_BYTES, st>>>(xmap, a);
     return check_launch(name);
 }
 
@@ -358,9 +419,9 @@ bool gath_mma_supported(int W, int dtype) {
 // `top` / `bottom`: extra output rows above / below the H rows under the inputs (row-slab backward), 0 otherwise.
 int launch_gath_mma(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype,
                     cudaStream_t st) {
-    if (dtype == SAPA_F32) return gmma::launch<float>(hi, wt, out, B, C, H, W, top, bottom, st);
-    if (dtype == SAPA_F16) return gmma::launch<__half>(hi, wt, out, B, C, H, W, top, bottom, st);
-    if (dtype == SAPA_BF16) return gmma::launch<__nv_bfloat16>(hi, wt, out, B, C, H, W, top, bottom, st);
+    if (dtype == SAPA_F32) return gmma::launch<float>(hi, wt, out, B, C, H, W, top, bottom, dtype, st);
+    if (dtype == SAPA_F16) return gmma::launch<__half>(hi, wt, out, B, C, H, W, top, bottom, dtype, st);
+    if (dtype == SAPA_BF16) return gmma::launch<__nv_bfloat16>(hi, wt, out, B, C, H, W, top, bottom, dtype, st);
     return SAPA_ERR_UNSUPPORTED;
 }
 

@@ -57,12 +57,15 @@ constexpr int MODE_SIM = 2;    // logits only: attn (output) = sim(query, key); 
 constexpr int MODE_AGG = 3;    // aggregation only: out = atn(attn (input weights), value); no key stages
 
 struct Args {
+    const void *q, *k, *v; // the inputs themselves: read by the ragged kernels, which have no tensor maps
     void *out, *attn;      // attn: forward = optional output (softmax), backward = input (saved softmax)
     void *ws;              // backward only: logit gradients [B, 25, 2H, 2W], written for the key-gradient gather
     int B, d, C, H, W;
     int rows, ytop0;
     int y_begin, y_end;    // low-res output rows produced by this launch (a band of [0, H); the whole image except in row-slab calls)
     int tiles_x, tiles_y;  // tiles_y covers the band only
+    int csplit, vstages;   // work items per tile, each with `vstages` value stages (its own share of the channels): a problem
+                           // with few tiles is spread over more CTAs, which all compute the tile's weights
     int sched_slot;        // index into g_next_tile / g_ctas_done
     int slots_f32;         // 16-bit kernel, MODE_SIM: the logits are written as float32
 };
@@ -78,12 +81,42 @@ __device__ __forceinline__ int swz(int col, int channel) { return ((((col >> 2) 
 //              "value" map is the key tensor and the output is grad_query = agg(dS, key).
 // MODE_SIM / MODE_AGG: the logit half / the aggregation half alone (sapa_qk_forward, sapa_av_forward and the halves of
 //              the separate backward ops); the weights of MODE_AGG are read where MODE_BWD reads the attention map.
-template <int MODE>
-__global__ void __launch_bounds__(NT, CTAS_PER_SM)
+// RAGGED: rows that are not multiples of 16 bytes - no tensor maps: RAGGED_PT producer threads copy the boxes element by
+//              element (static tile order), the output leaves from registers; everything behind the ring is the same.
+constexpr int RAGGED_PT = 4 * 32;
+
+// producer threads of the ragged float32 kernel: the columns 2 .. 13 of a key / value box (what a window can reach), and a
+// query box
+template <int NCH>
+__device__ __forceinline__ void ragged_lo_box_f32(unsigned dst, const float *base, int c0, int C, int rows, int W, int y0, int x0, int ptid) {
+    const int col = ptid & 15, x = x0 - 4 + col;
+    const bool x_ok = x >= 0 && x < W;
+    const size_t plane = (size_t)rows * W;
+    if (col < 2 || col > 13) return;
+#pragma unroll
+    for (int i = 0; i < HH * NCH * 16 / RAGGED_PT; ++i) {
+        const int rc = i * (RAGGED_PT / 16) + (ptid >> 4), ch = rc % NCH, row = rc / NCH, y = y0 - 2 + row;
+        const bool ok = x_ok && c0 + ch < C && y >= 0 && y < rows;
+        cp_async4(dst + row * (NCH * ROWB) + ch * ROWB + swz(col, ch), ok ? base + (size_t)(c0 + ch) * plane + (size_t)y * W + x : base, ok);
+    }
+}
+__device__ __forceinline__ void ragged_hi_box_f32(unsigned dst, const float *base, int c0, int C, int H, int W, int y0, int x0, int ptid) {
+    const int pair = ptid & 7, sW = 2 * W;
+    const size_t plane = (size_t)(2 * H) * sW;
+#pragma unroll
+    for (int i = 0; i < 2 * ROWS * F_KCH * 8 / RAGGED_PT; ++i) {
+        const int rc = i * (RAGGED_PT / 8) + (ptid >> 3), ch = rc % F_KCH, row = rc / F_KCH;
+        const bool ok = x0 + pair < W && c0 + ch < C && 2 * y0 + row < 2 * H;
+        cp_async8(dst + row * (F_KCH * ROWB) + ch * ROWB + swz(2 * pair, ch), ok ? base + (size_t)(c0 + ch) * plane + (size_t)(2 * y0 + row) * sW + 2 * (x0 + pair) : base, ok);
+    }
+}
+
+template <int MODE, bool RAGGED>
+__global__ void __launch_bounds__(RAGGED ? NT + RAGGED_PT : NT, RAGGED ? 1 : CTAS_PER_SM)
 sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                           const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap omap, const Args a) {
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ __align__(8) unsigned long long full_bar[NSTAGE];
+    __shared__ __align__(8) unsigned long long full_bar[2 * NSTAGE];       // full, then (ragged form only) empty
     // the swizzle pattern is a function of the absolute shared-memory address: align the ring to 1024 bytes
     const unsigned ring_addr = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u;
     const unsigned bar_addr = (unsigned)__cvta_generic_to_shared(full_bar);
@@ -94,27 +127,57 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
     const int g = lane >> 2, t = lane & 3;
     const int sW = 2 * a.W;
     const size_t hi_plane = (size_t)(2 * a.H) * sW;
-    const int nk = (a.d + F_KCH - 1) / F_KCH, nv = (a.C + F_VCH - 1) / F_VCH, total = nk + nv;
+    const int nk = (a.d + F_KCH - 1) / F_KCH, nv = a.vstages, total = nk + nv;
     // Persistent CTA: its first tile is blockIdx.x, further tiles come from a global counter.  The stages of
     // successive tiles form one continuous stream through the ring, so the first stages of the next tile are in
     // flight while the current tile finishes.  tile_ids[ti & 3] = tile of the ti-th tile of this CTA, -1 = none.
-    const int ntiles = a.B * a.tiles_x * a.tiles_y;
+    const int ntiles = a.B * a.tiles_x * a.tiles_y * a.csplit;     // work items
     __shared__ int tile_ids[4];
 
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < NSTAGE; ++i) {
-            mbar_init(bar_addr + 8 * i, 1);
+            mbar_init(bar_addr + 8 * i, RAGGED ? RAGGED_PT : 1);
+            if (RAGGED) mbar_init(bar_addr + 8 * (NSTAGE + i), 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
 
+    if constexpr (RAGGED) {
+        if (tid >= NT) {
+            const int ptid = tid - NT;
+            const float *qp = static_cast<const float *>(a.q), *kp = static_cast<const float *>(a.k), *vp = static_cast<const float *>(a.v);
+            const size_t lo_plane = (size_t)a.rows * a.W;
+            int slot = 0, phase = 0;
+            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+                int t_ = tile / a.csplit;
+                const int vb = tile % a.csplit * nv;
+                const int x0 = (t_ % a.tiles_x) * COLS; t_ /= a.tiles_x;
+                const int y0 = a.y_begin + (t_ % a.tiles_y) * ROWS, n = t_ / a.tiles_y;
+                for (int it = 0; it < total; ++it) {
+                    if (!mbar_wait_bounded(bar_addr + 8 * (NSTAGE + slot), phase ^ 1)) { atomicExch(&g_wait_timeout, 1); return; }
+                    const unsigned dst = ring_addr + slot * SLOT_BYTES;
+                    if (it < nk) {
+                        ragged_lo_box_f32<F_KCH>(dst, kp + (size_t)n * a.d * lo_plane, it * F_KCH, a.d, a.rows, a.W, a.ytop0 + y0, x0, ptid);
+                        ragged_hi_box_f32(dst + K_BYTES, qp + (size_t)n * a.d * hi_plane, it * F_KCH, a.d, a.H, a.W, y0, x0, ptid);
+                    } else {
+                        ragged_lo_box_f32<F_VCH>(dst, vp + (size_t)n * a.C * lo_plane, (vb + it - nk) * F_VCH, a.C, a.rows, a.W, a.ytop0 + y0, x0, ptid);
+                    }
+                    cp_async_arrive(bar_addr + 8 * slot);
+                    if (++slot == NSTAGE) { slot = 0; phase ^= 1; }
+                }
+            }
+            asm volatile("cp.async.wait_all;\n" ::: "memory");      // no copy outlives the thread
+            return;
+        }
+    }
+
     // Stages are issued in stream order (stage gs goes to slot gs % NSTAGE) by thread 0 only.  The producer keeps its
     // position incrementally: per stage it costs a handful of instructions, which matters because the other seven
     // warps wait for warp 0 at the next barrier.
     bool exhausted = false;
-    int p_it = 0, p_ti = 0, p_slot = 0, p_n = 0, p_x0 = 0, p_y0 = 0;
+    int p_it = 0, p_ti = 0, p_slot = 0, p_n = 0, p_x0 = 0, p_y0 = 0, p_vb = 0;
     auto issue = [&](int) {
         if (exhausted) return;
         if (p_it == 0) {     // first stage of a tile: claim the tile
@@ -123,6 +186,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             if (claimed >= ntiles) claimed = -1;
             tile_ids[p_ti & 3] = claimed;
             if (claimed < 0) { exhausted = true; return; }
+            p_vb = claimed % a.csplit * nv; claimed /= a.csplit;
             p_x0 = (claimed % a.tiles_x) * COLS; claimed /= a.tiles_x;
             p_y0 = a.y_begin + (claimed % a.tiles_y) * ROWS; claimed /= a.tiles_y;
             p_n = claimed;
@@ -134,12 +198,12 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             tma_load_4d(slot + K_BYTES, &qmap, bar, 2 * p_x0, p_it * F_KCH, 2 * p_y0, p_n);
         } else {
             mbar_expect_tx(bar, V_BYTES);
-            tma_load_4d(slot, &vmap, bar, p_x0 - 4, (p_it - nk) * F_VCH, a.ytop0 + p_y0 - 2, p_n);
+            tma_load_4d(slot, &vmap, bar, p_x0 - 4, (p_vb + p_it - nk) * F_VCH, a.ytop0 + p_y0 - 2, p_n);
         }
         if (++p_it == total) { p_it = 0; ++p_ti; }
         p_slot = (p_slot + 1) % NSTAGE;
     };
-    if (tid == 0) {
+    if (!RAGGED && tid == 0) {
 #pragma unroll
         for (int i = 0; i < NSTAGE - 1; ++i) issue(i);
     }
@@ -185,8 +249,9 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
     int gs = 0;
     for (int ti = 0;; ++ti) {
     // written by thread 0 at least one barrier earlier (tile 0 is known to everybody)
-    int tile = ti == 0 ? (int)blockIdx.x : tile_ids[ti & 3];
-    if (tile < 0) break;
+    int tile = RAGGED ? (int)blockIdx.x + ti * (int)gridDim.x : ti == 0 ? (int)blockIdx.x : tile_ids[ti & 3];
+    if (tile < 0 || (RAGGED && tile >= ntiles)) break;
+    const int vb = tile % a.csplit * nv; tile /= a.csplit;
     const int bx = tile % a.tiles_x; tile /= a.tiles_x;
     const int by = tile % a.tiles_y; tile /= a.tiles_y;
     const int n = tile;
@@ -211,10 +276,16 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
     }
 
     for (int it = 0; it < total; ++it, ++gs) {
-        __syncthreads();     // everyone is done with the slot that is refilled next and has written its output fragment
-        if (tid == 0) {
+        // everyone is done with the slot that is refilled next and has written its output fragment
+        if constexpr (RAGGED) {
+            asm volatile("bar.sync 1, %0;\n" ::"n"(NT) : "memory");
+            if (tid == 0 && gs > 0) mbar_arrive(bar_addr + 8 * (NSTAGE + (gs - 1) % NSTAGE));
+        } else {
+            __syncthreads();
+        }
+        if (!RAGGED && tid == 0) {
             if (it > nk) {   // the previous stage was a value stage: its output tile is complete in shared memory
-                tma_store_4d(&omap, obuf_addr + ((it - nk - 1) & 1) * O_BYTES, 2 * x0, (it - nk - 1) * F_VCH, 2 * y0, n);
+                tma_store_4d(&omap, obuf_addr + ((it - nk - 1) & 1) * O_BYTES, 2 * x0, (vb + it - nk - 1) * F_VCH, 2 * y0, n);
                 asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
             }
             issue(gs + NSTAGE - 1);
@@ -223,7 +294,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             atomicExch(&g_wait_timeout, 1);
             return;
         }
-        const unsigned stage = ring_addr + (gs % NSTAGE) * SLOT_BYTES;
+        const unsigned stage = fresh(ring_addr + (gs % NSTAGE) * SLOT_BYTES);
 
         if (it < nk) {
             // ------------------------------------------------------------- logits: S[16 px][8 cells] += Qt[16 px][8 ch] K[8 ch][8 cells]
@@ -311,7 +382,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 }
             }
             if (it == nk - 1 && (MODE == MODE_FWD || MODE == MODE_SIM)) {      // probabilities, or the raw logits of MODE_SIM
-                if (a.attn != nullptr && y < a.y_end && x0 + 4 * h + l < a.W) {
+                if (a.attn != nullptr && vb == 0 && y < a.y_end && x0 + 4 * h + l < a.W) {
                     float *an = static_cast<float *>(a.attn) + (size_t)n * 25 * hi_plane + (size_t)(2 * y) * sW + 2 * (x0 + 4 * h) + g;
 #pragma unroll
                     for (int dy = 0; dy < 5; ++dy)
@@ -325,7 +396,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             if (it == nk - 1 && MODE != MODE_SIM) realign();
         } else {
             // ------------------------------------------------------------- aggregation: Out[16 ch][8 px] += V[16 ch][8 cells] P[8 cells][8 px]
-            const unsigned vb = stage + wrow * (F_VCH * ROWB);
+            const unsigned vbox = stage + wrow * (F_VCH * ROWB);
             float acc[F_VCH / 16][2][4];
 #pragma unroll
             for (int b = 0; b < F_VCH / 16; ++b)
@@ -337,7 +408,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
             auto load_row = [&](int dy) {
 #pragma unroll
                 for (int b = 0; b < F_VCH / 16; ++b) {
-                    const unsigned p = vb + dy * (F_VCH * ROWB) + b * 16 * ROWB;
+                    const unsigned p = vbox + dy * (F_VCH * ROWB) + b * 16 * ROWB;
                     an[b][0] = lds32(p + v_offa);                 // V[ch g][cell t]
                     an[b][1] = lds32(p + 8 * ROWB + v_offa);      // V[ch g+8][cell t]
                     an[b][2] = lds32(p + v_offb);                 // V[ch g][cell t+4]
@@ -370,6 +441,21 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 #pragma unroll
                     for (int r = 0; r < 2; ++r) mma_tf32(acc[b][r], ah[b], tf32_lo(phi[r][dy][0]), tf32_lo(phi[r][dy][1]));
             }
+            if constexpr (RAGGED) {       // pixel pairs straight to memory (rows start on 8 bytes)
+                if (y < a.y_end && x0 + 4 * h + t < a.W) {
+                    float *o = static_cast<float *>(a.out) + ((size_t)n * a.C + (vb + it - nk) * F_VCH + g) * hi_plane + (size_t)(2 * y) * sW + 2 * (x0 + 4 * h + t);
+#pragma unroll
+                    for (int b = 0; b < F_VCH / 16; ++b)
+#pragma unroll
+                        for (int half = 0; half < 2; ++half)
+                            if ((vb + it - nk) * F_VCH + 16 * b + 8 * half + g < a.C)
+#pragma unroll
+                                for (int r = 0; r < 2; ++r)
+                                    __stcs(reinterpret_cast<float2 *>(o + (size_t)(16 * b + 8 * half) * hi_plane + (size_t)r * sW),
+                                           make_float2(acc[b][r][2 * half], acc[b][r][2 * half + 1]));
+                }
+                continue;
+            }
             // D fragment: d0,d1 = Out[ch g][px 2t, 2t+1], d2,d3 = Out[ch g+8][px 2t, 2t+1] -> staging buffer laid out
             // as the output box [hi row][channel][16 hi cols] (64-byte swizzle), stored by TMA after the next barrier
             {
@@ -388,14 +474,14 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         }
     }
     // the tile's last output block
-    __syncthreads();
-    if (tid == 0 && MODE != MODE_SIM) {
-        tma_store_4d(&omap, obuf_addr + ((nv - 1) & 1) * O_BYTES, 2 * x0, (nv - 1) * F_VCH, 2 * y0, n);
+    if (!RAGGED) __syncthreads();
+    if (!RAGGED && tid == 0 && MODE != MODE_SIM) {
+        tma_store_4d(&omap, obuf_addr + ((nv - 1) & 1) * O_BYTES, 2 * x0, (vb + nv - 1) * F_VCH, 2 * y0, n);
         asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
     }
     }
-    if (tid == 0) {
+    if (!RAGGED && tid == 0) {
         asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");   // all output tiles are written
         if (atomicAdd(&g_ctas_done[a.sched_slot], 1u) == gridDim.x - 1) {   // last CTA out: reset the scheduler slot
             g_next_tile[a.sched_slot] = 0u;
@@ -424,6 +510,8 @@ constexpr int COLS = 8;                         // low-res columns of a CTA tile
 constexpr int NSTAGE = 4;                       // ring slots of 20 KB
 constexpr int NW = 2 * ROWS;                    // 8 consumer warps
 constexpr int NT = (NW + 1) * 32;               // + one producer warp
+constexpr int PT = 4 * 32;                      // threads of the four producer warps of the ragged form
+constexpr int NT_RAGGED = NW * 32 + PT;
 constexpr int CTAS_PER_SM = 2;                  // resident CTAs per SM the register budget is tuned for
 constexpr int KCH = 32;                         // key / query channels per stage (k steps of 16 for m16n8k16)
 constexpr int VCH = 32;                         // value channels per stage (multiple of 16)
@@ -477,8 +565,73 @@ __device__ __forceinline__ float ex2_ftz(float x) {
     return y;
 }
 
-template <typename T, int MODE>     // modes: see the float32 kernel
-__global__ void __launch_bounds__(h16::NT, h16::CTAS_PER_SM)
+// Producer warps of the ragged 16-bit kernel: fill one ring slot with the boxes that TMA would put there (the columns of a
+// key / value box that a window can reach: box columns 6 .. 17; the others stay zero from the start of the kernel).  Eight
+// threads (six of them working) per box row, one pixel pair each.
+// Even W: low-res rows start on 4 bytes: asynchronous 4-byte copies.  Odd W: they start on any 2 bytes: two loads into
+// registers one stage ahead (OddBox::load), one shared store per pair (OddBox::store).  High-res rows have an even length
+// always.
+constexpr int LO_ITEMS = HH * 32 * 8 / h16::PT;
+template <typename T>
+__device__ __forceinline__ void ragged_lo_box_16(unsigned dst, const T *base /* plane 0 of the image */, int c0, int C, int rows, int W, int y0, int x0, int ptid) {
+    const int pair = ptid & 7, x = x0 - 2 + 2 * pair;
+    const bool x_ok = pair < 6 && x >= 0 && x < W;
+    const size_t plane = (size_t)rows * W;
+    if (pair >= 6) return;
+#pragma unroll
+    for (int i = 0; i < LO_ITEMS; ++i) {
+        const int rc = i * (h16::PT / 8) + (ptid >> 3), ch = rc & 31, row = rc >> 5, y = y0 - 2 + row;
+        const bool ok = x_ok && c0 + ch < C && y >= 0 && y < rows;
+        cp_async4(dst + row * (32 * h16::KROW) + ch * h16::KROW + 12 + 4 * pair, ok ? base + (size_t)(c0 + ch) * plane + (size_t)y * W + x : base, ok);
+    }
+}
+struct OddBox {
+    unsigned short lo[LO_ITEMS], hi[LO_ITEMS];
+    template <typename T>
+    __device__ __forceinline__ void load(const T *base, int c0, int C, int rows, int W, int y0, int x0, int ptid) {
+        const int pair = ptid & 7, x = x0 - 2 + 2 * pair;
+        const bool lo_ok = pair < 6 && x >= 0 && x < W, hi_ok = pair < 6 && x + 1 >= 0 && x + 1 < W;
+        const size_t plane = (size_t)rows * W;
+        const unsigned short *b16 = reinterpret_cast<const unsigned short *>(base);
+#pragma unroll
+        for (int i = 0; i < LO_ITEMS; ++i) {
+            const int rc = i * (h16::PT / 8) + (ptid >> 3), ch = rc & 31, row = rc >> 5, y = y0 - 2 + row;
+            const bool ok = c0 + ch < C && y >= 0 && y < rows;
+            const unsigned short *p = b16 + (size_t)(c0 + ch) * plane + (size_t)y * W + x;
+            lo[i] = ok && lo_ok ? __ldg(p) : (unsigned short)0;
+            hi[i] = ok && hi_ok ? __ldg(p + 1) : (unsigned short)0;
+        }
+    }
+    __device__ __forceinline__ void store(unsigned dst, int ptid) const {
+        const int pair = ptid & 7;
+        if (pair >= 6) return;
+#pragma unroll
+        for (int i = 0; i < LO_ITEMS; ++i) {
+            const int rc = i * (h16::PT / 8) + (ptid >> 3), ch = rc & 31, row = rc >> 5;
+            sts32(dst + row * (32 * h16::KROW) + ch * h16::KROW + 12 + 4 * pair, (unsigned)lo[i] | ((unsigned)hi[i] << 16));
+        }
+    }
+};
+template <typename T>
+__device__ __forceinline__ void ragged_hi_box_16(unsigned dst, const T *base, int c0, int C, int H, int W, int y0, int x0, int ptid) {
+    const int pair = ptid & 7, sW = 2 * W;
+    const bool x_ok = x0 + pair < W;
+    const size_t plane = (size_t)(2 * H) * sW;
+#pragma unroll
+    for (int i = 0; i < 2 * ROWS * 32 * 8 / h16::PT; ++i) {
+        const int rc = i * (h16::PT / 8) + (ptid >> 3), ch = rc & 31, row = rc >> 5;
+        const bool ok = x_ok && c0 + ch < C && 2 * y0 + row < 2 * H;
+        cp_async4(dst + row * (32 * h16::QROW) + ch * h16::QROW + ((((pair >> 2) ^ (ch >> 2)) & 1) << 4) + 4 * (pair & 3),
+                  ok ? base + (size_t)(c0 + ch) * plane + (size_t)(2 * y0 + row) * sW + 2 * (x0 + pair) : base, ok);
+    }
+}
+
+// modes: see the float32 kernel.  RAGGED: rows that are not multiples of 16 bytes - no tensor maps, four producer warps copy
+// the boxes (static tile order); everything behind the ring is the same.  The FP32-pipe kernels it replaced walked all
+// channels in one CTA per 4 x 32 tile: backward of B=2, C=256, d=32, 25x42 -> 50x84 in bfloat16 438 -> 60 us.  At large
+// sizes the copies bound it: 1.7 - 2x the time of the neighbouring aligned width (8 x 256 x 64x65: 110 us, 64x64: 56 us).
+template <typename T, int MODE, bool RAGGED>
+__global__ void __launch_bounds__(RAGGED ? h16::NT_RAGGED : h16::NT, RAGGED ? 1 : h16::CTAS_PER_SM)
 sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                          const __grid_constant__ CUtensorMap vmap, const Args a) {
     using namespace h16;
@@ -493,22 +646,89 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
     const int g = lane >> 2, t = lane & 3;
     const int sW = 2 * a.W;
     const size_t hi_plane = (size_t)(2 * a.H) * sW;
-    const int nk = (a.d + KCH - 1) / KCH, nv = (a.C + VCH - 1) / VCH, total = nk + nv;
-    const int ntiles = a.B * a.tiles_x * a.tiles_y;
+    const int nk = (a.d + KCH - 1) / KCH, nv = a.vstages, total = nk + nv;
+    const int ntiles = a.B * a.tiles_x * a.tiles_y * a.csplit;     // work items
 
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < h16::NSTAGE; ++i) {
-            mbar_init(full_addr + 8 * i, 1);
+            mbar_init(full_addr + 8 * i, RAGGED ? (a.W & 1 ? 2 * PT : PT) : 1);
             mbar_init(empty_addr + 8 * i, NW);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    if constexpr (RAGGED)       // box columns that are never copied must read as zero
+        for (int i = tid; i < h16::NSTAGE * h16::SLOT_BYTES / 4; i += h16::NT_RAGGED) sts32(ring_addr + 4 * i, 0u);
     __syncthreads();
+
+    if constexpr (RAGGED) {
+        if (warp >= NW) {
+            const int ptid = tid - NW * 32;
+            const T *qp = static_cast<const T *>(a.q), *kp = static_cast<const T *>(a.k), *vp = static_cast<const T *>(a.v);
+            const size_t lo_plane = (size_t)a.rows * a.W;
+            // position of a stage: its low-res box is read one stage ahead when W is odd
+            struct Pos { int tile, it, x0, y0, n, vb; };
+            const auto locate = [&](Pos &p) {
+                int t_ = p.tile / a.csplit;
+                p.vb = p.tile % a.csplit * nv;
+                p.x0 = (t_ % a.tiles_x) * h16::COLS; t_ /= a.tiles_x;
+                p.y0 = a.y_begin + (t_ % a.tiles_y) * ROWS; p.n = t_ / a.tiles_y;
+            };
+            const auto advance = [&](Pos &p) {
+                if (++p.it < total) return;
+                p.it = 0;
+                p.tile += gridDim.x;
+                if (p.tile < ntiles) locate(p);
+            };
+            Pos cur{(int)blockIdx.x, 0, 0, 0, 0, 0};
+            locate(cur);
+            int slot = 0, phase = 0;
+            const auto claim = [&]() {
+                if (mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) return true;
+                atomicExch(&g_wait_timeout, 1);
+                return false;
+            };
+            const auto next_slot = [&]() { if (++slot == h16::NSTAGE) { slot = 0; phase ^= 1; } };
+            if (a.W & 1) {
+                OddBox box;
+                const auto load = [&](const Pos &p) {
+                    const bool key = p.it < nk;
+                    box.load(key ? kp + (size_t)p.n * a.d * lo_plane : vp + (size_t)p.n * a.C * lo_plane, key ? p.it * KCH : (p.vb + p.it - nk) * VCH,
+                             key ? a.d : a.C, a.rows, a.W, a.ytop0 + p.y0, p.x0, ptid);
+                };
+                load(cur);
+                while (cur.tile < ntiles) {
+                    if (!claim()) return;
+                    const unsigned dst = ring_addr + slot * h16::SLOT_BYTES, bar = full_addr + 8 * slot;
+                    if (cur.it < nk) ragged_hi_box_16<T>(dst + h16::K_BYTES, qp + (size_t)cur.n * a.d * hi_plane, cur.it * KCH, a.d, a.H, a.W, cur.y0, cur.x0, ptid);
+                    box.store(dst, ptid);
+                    cp_async_arrive(bar);        // the query copies, and ...
+                    mbar_arrive(bar);            // ... the shared stores (two arrivals per thread)
+                    next_slot();
+                    advance(cur);
+                    if (cur.tile < ntiles) load(cur);
+                }
+            } else {
+                while (cur.tile < ntiles) {
+                    if (!claim()) return;
+                    const unsigned dst = ring_addr + slot * h16::SLOT_BYTES;
+                    const bool key = cur.it < nk;
+                    ragged_lo_box_16<T>(dst, key ? kp + (size_t)cur.n * a.d * lo_plane : vp + (size_t)cur.n * a.C * lo_plane,
+                                        key ? cur.it * KCH : (cur.vb + cur.it - nk) * VCH, key ? a.d : a.C, a.rows, a.W, a.ytop0 + cur.y0, cur.x0, ptid);
+                    if (key) ragged_hi_box_16<T>(dst + h16::K_BYTES, qp + (size_t)cur.n * a.d * hi_plane, cur.it * KCH, a.d, a.H, a.W, cur.y0, cur.x0, ptid);
+                    cp_async_arrive(full_addr + 8 * slot);
+                    next_slot();
+                    advance(cur);
+                }
+            }
+            asm volatile("cp.async.wait_all;\n" ::: "memory");      // no copy outlives the thread
+            return;
+        }
+    }
 
     // ---- producer state (lane 0 of the producer warp).  The stages of successive tiles form one continuous stream through
     // the ring; the first tile of a CTA is blockIdx.x, further tiles come from a global counter.
-    int p_issued = 0, p_slot = 0, p_phase = 0, p_it = 0, p_ti = 0, p_n = 0, p_x0 = 0, p_y0 = 0;
+    int p_issued = 0, p_slot = 0, p_phase = 0, p_it = 0, p_ti = 0, p_n = 0, p_x0 = 0, p_y0 = 0, p_vb = 0;
     bool p_done = false;
     // Issues every stage whose slot is free; when the stage `need` (the one the warp is about to wait for) has not
     // been issued yet it waits for that slot.  A slot is free when all NW warps have released its previous use; on
@@ -539,6 +759,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                     p_done = true;
                     return;
                 }
+                p_vb = claimed % a.csplit * nv; claimed /= a.csplit;
                 p_x0 = (claimed % a.tiles_x) * h16::COLS; claimed /= a.tiles_x;
                 p_y0 = a.y_begin + (claimed % a.tiles_y) * ROWS; claimed /= a.tiles_y;
                 p_n = claimed;
@@ -550,7 +771,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 tma_load_4d(dst + h16::K_BYTES, &qmap, bar, 2 * p_x0, p_it * KCH, 2 * p_y0, p_n);
             } else {
                 mbar_expect_tx(bar, h16::V_BYTES);
-                tma_load_4d(dst, &vmap, bar, p_x0 - 8, (p_it - nk) * VCH, a.ytop0 + p_y0 - 2, p_n);
+                tma_load_4d(dst, &vmap, bar, p_x0 - 8, (p_vb + p_it - nk) * VCH, a.ytop0 + p_y0 - 2, p_n);
             }
             ++p_issued;
             if (++p_it == total) { p_it = 0; ++p_ti; }
@@ -560,7 +781,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 
     // The producer is a warp of its own (one lane works): inside a consumer warp it sat on that warp's critical path -
     // 40 % of the warp's time at config 2 - and the other warps waited for the stages it had not issued yet.
-    if (warp == NW) {
+    if (!RAGGED && warp == NW) {
         if (lane == 0) produce(0x7fffffff);
         return;
     }
@@ -598,25 +819,28 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 
     int slot = 0, phase = 0, it = 0, ti = 0, gs = 0;
     int n = 0, x0 = 0, y = 0;
+    int c0 = 0;                   // first channel of the current value stage
     // kernel-wide strides in 32-bit words of the 16-bit output / attention tensors (two elements per word)
     const size_t plane_w = hi_plane >> 1;
-    const int C = a.C, Wlo = a.W, Hlo = a.H;
+    const int C = a.C, Wlo = a.W;
     unsigned *o_ptr = nullptr;            // this lane's output word for the first channel of the current value stage
     bool row_ok = false, col_ok0 = false, col_ok1 = false;
     constexpr float LOG2E = 1.4426950408889634f;
     for (;; ++gs) {
+        if (RAGGED && it == 0 && (int)blockIdx.x + ti * (int)gridDim.x >= ntiles) break;
         if (!mbar_wait_bounded(full_addr + 8 * slot, phase)) {
             atomicExch(&g_wait_timeout, 1);
             return;
         }
         if (it == 0) {
-            int tile = tile_ids[ti & 3];      // published by the producer before the barrier's phase completed
+            int tile = RAGGED ? (int)blockIdx.x + ti * (int)gridDim.x : tile_ids[ti & 3];      // published by the producer before the barrier's phase completed
             if (tile < 0) break;
+            c0 = tile % a.csplit * nv * VCH; tile /= a.csplit;
             x0 = (tile % a.tiles_x) * h16::COLS; tile /= a.tiles_x;
             y = a.y_begin + (tile % a.tiles_y) * ROWS + wrow; tile /= a.tiles_y;
             n = tile;
             row_ok = y < a.y_end; col_ok0 = x0 + t < Wlo; col_ok1 = x0 + 4 + t < Wlo;
-            o_ptr = reinterpret_cast<unsigned *>(static_cast<T *>(a.out) + ((size_t)n * C + g) * hi_plane +
+            o_ptr = reinterpret_cast<unsigned *>(static_cast<T *>(a.out) + ((size_t)n * C + c0 + g) * hi_plane +
                                                  (size_t)(2 * y + r) * sW + 2 * x0 + 2 * t);
 #pragma unroll
             for (int p = 0; p < 2; ++p)
@@ -641,7 +865,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 }
             }
         }
-        const unsigned stage = ring_addr + slot * h16::SLOT_BYTES;
+        const unsigned stage = fresh(ring_addr + slot * h16::SLOT_BYTES);
 
         if (it < nk) {
             // ------------------------------------------------------------- logits
@@ -760,7 +984,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                         }
                 }
             } else if (it == nk - 1 && (MODE == MODE_FWD || MODE == MODE_SIM)) {
-                if (a.attn != nullptr && row_ok) {
+                if (a.attn != nullptr && c0 == 0 && row_ok) {
                     // the two pixels of a pair are neighbours in memory: one 32-bit store per (window slot, pair)
                     unsigned *an = reinterpret_cast<unsigned *>(static_cast<T *>(a.attn) + (size_t)n * 25 * hi_plane +
                                                                 (size_t)(2 * y + r) * sW + 2 * x0 + 2 * t);
@@ -810,7 +1034,6 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
             // D fragment of group p: d0,d1 = Out[ch g][px 8p+2t, +1], d2,d3 = Out[ch g+8][same].  Neighbouring lanes swap one
             // pair so that even lanes hold pixels 2t .. 2t+3 of the left group and odd lanes 2(t-1) .. 2(t-1)+3 of the right
             // group: a quad then writes one full 32-byte sector per store instruction (half sectors cost an L1 tag cycle each).
-            const int c0 = (it - nk) * VCH;
             unsigned *o = o_ptr + ((t & 1) ? 3 : 0);
             o_ptr += (size_t)VCH * plane_w;
             if (row_ok) {          // warp-uniform; columns are always inside (W is a multiple of the tile width here)
@@ -819,11 +1042,21 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 for (int j = 0; j < VCH / 8; ++j) {       // channel g + 8j: block j/2, half j%2
                     const unsigned v0 = pack_pair(T(), acc[j >> 1][0][2 * (j & 1)], acc[j >> 1][0][2 * (j & 1) + 1]);
                     const unsigned v1 = pack_pair(T(), acc[j >> 1][1][2 * (j & 1)], acc[j >> 1][1][2 * (j & 1) + 1]);
+                    if constexpr (RAGGED) {       // rows on 4-byte boundaries, columns to be checked: one pair per store
+                        unsigned *oc = o - (odd ? 3 : 0);
+                        if (c0 + 8 * j + g < C) {
+                            if (col_ok0) oc[0] = v0;
+                            if (col_ok1) oc[4] = v1;
+                        }
+                        o += 8 * plane_w;
+                        continue;
+                    }
                     const unsigned got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
                     if (c0 + 8 * j + g < C) __stcs(reinterpret_cast<uint2 *>(o), odd ? make_uint2(got, v1) : make_uint2(v0, got));
                     o += 8 * plane_w;
                 }
             }
+            c0 += VCH;
         }
         if (++slot == h16::NSTAGE) { slot = 0; phase ^= 1; }
         if (++it == total) { it = 0; ++ti; }
@@ -837,9 +1070,9 @@ static std::atomic<unsigned> g_next_sched_slot{0}, g_next_captured_slot{0};
 
 // Opts in to the dynamic shared memory, sizes the persistent grid, picks a scheduler slot and launches.
 template <typename Kernel, typename... Maps>
-static int launch_persistent(Kernel kernel, const char *name, int threads, int smem, int ctas_per_sm, Args &a, cudaStream_t st,
+static int launch_persistent(Kernel kernel, const char *name, int threads, int smem, int ctas_per_sm, bool split, Args &a, cudaStream_t st,
                              const Maps &...maps) {
-    const long long nblocks = (long long)a.B * a.tiles_x * a.tiles_y;
+    long long nblocks = (long long)a.B * a.tiles_x * a.tiles_y;
     if (nblocks > 0x7fffffffLL) {
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
@@ -847,6 +1080,13 @@ static int launch_persistent(Kernel kernel, const char *name, int threads, int s
     int sms = 0;
     if (int e = prepare_launch(reinterpret_cast<const void *>(kernel), smem, name, sms)) return e;
     const long long resident = (long long)ctas_per_sm * sms;
+    // halve the channels of an item as long as all items still run at once (stage 1 of the backward writes its logit
+    // gradients and has one or two value stages: not split)
+    while (split && a.vstages >= 2 && a.vstages % 2 == 0 && 2 * nblocks <= resident) {
+        a.vstages /= 2;
+        a.csplit *= 2;
+        nblocks *= 2;
+    }
     // persistent grid with dynamic tile claiming (static striding left SMs with 6 to 8 tiles instead of ~6.9)
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
@@ -856,7 +1096,7 @@ static int launch_persistent(Kernel kernel, const char *name, int threads, int s
 
 }  // namespace tma
 
-// K = 5, s = 2 and every row of every tensor on a 16-byte boundary
+// K = 5, s = 2 and every row of every tensor on a 16-byte boundary; other widths take the ragged form of the kernels
 bool fused_tma_supported(int W, int dtype) {
     if (tma::encode_tiled_fn() == nullptr) return false;
     if (dtype == SAPA_F32) return W % 4 == 0;
@@ -891,9 +1131,11 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     if (mode == MODE_SIM) C = 0;
     if (mode == MODE_AGG) d = 0;
     const bool use_qk = mode != MODE_AGG, use_v = mode != MODE_SIM;
-    CUtensorMap qmap, kmap, vmap, omap;
+    CUtensorMap qmap{}, kmap{}, vmap{}, omap{};
+    const bool ragged = !fused_tma_supported(W, dtype);
     bool ok = true;
-    if (dtype == SAPA_F32) {
+    if (ragged) {
+    } else if (dtype == SAPA_F32) {
         const auto ty = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
         const auto sw = CU_TENSOR_MAP_SWIZZLE_64B;
         if (use_qk) ok = ok && make_nchw_map(&qmap, q, 2 * W, 2 * H, d, B, HC, F_KCH, HH, ty, 4, sw) && make_nchw_map(&kmap, k, W, rows, d, B, HC, F_KCH, HH, ty, 4, sw);
@@ -914,9 +1156,12 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     if (!use_v) { vmap = kmap; omap = kmap; }
     if (dtype != SAPA_F32) omap = vmap;
     Args a{};
+    a.q = q; a.k = k; a.v = v;
     a.out = out; a.attn = attn; a.ws = ws;
     a.B = B; a.d = d; a.C = C; a.H = H; a.W = W; a.rows = rows; a.ytop0 = ytop0;
     a.slots_f32 = slots_f32 ? 1 : 0;
+    static_assert(F_VCH == h16::VCH, "both kernels take the same number of value channels per stage");
+    a.csplit = 1; a.vstages = ceil_div(C, F_VCH);
     static_assert(h16::COLS == COLS, "both kernels use the same tile");
     a.y_begin = y_begin; a.y_end = y_end;
     a.tiles_x = ceil_div(W, COLS);
@@ -927,31 +1172,24 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     static const char *const names16[4] = {"sapa_tma_fused_16_kernel<fwd>", "sapa_tma_fused_16_kernel<bwd>",
                                            "sapa_tma_fused_16_kernel<sim>", "sapa_tma_fused_16_kernel<agg>"};
     const char *n32 = names32[mode & 3], *n16 = names16[mode & 3];
-#define SAPA_TMA_LAUNCH32(M) launch_persistent(sapa_tma_fused_f32_kernel<M>, n32, NT, smem32, CTAS_PER_SM, a, st, qmap, kmap, vmap, omap)
-#define SAPA_TMA_LAUNCH16(T, M) \
-    launch_persistent(sapa_tma_fused_16_kernel<T, M>, n16, h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, a, st, qmap, kmap, vmap)
-    if (dtype == SAPA_F32) {
-        switch (mode) {
-            case MODE_FWD: return SAPA_TMA_LAUNCH32(MODE_FWD);
-            case MODE_BWD: return SAPA_TMA_LAUNCH32(MODE_BWD);
-            case MODE_SIM: return SAPA_TMA_LAUNCH32(MODE_SIM);
-            default: return SAPA_TMA_LAUNCH32(MODE_AGG);
-        }
-    }
-    if (dtype == SAPA_F16) {
-        switch (mode) {
-            case MODE_FWD: return SAPA_TMA_LAUNCH16(__half, MODE_FWD);
-            case MODE_BWD: return SAPA_TMA_LAUNCH16(__half, MODE_BWD);
-            case MODE_SIM: return SAPA_TMA_LAUNCH16(__half, MODE_SIM);
-            default: return SAPA_TMA_LAUNCH16(__half, MODE_AGG);
-        }
-    }
-    switch (mode) {
-        case MODE_FWD: return SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_FWD);
-        case MODE_BWD: return SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_BWD);
-        case MODE_SIM: return SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_SIM);
-        default: return SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_AGG);
-    }
+    // how the ragged launches are recorded: the kernels that serve rows of any length
+    static const char *const names_ragged[4] = {"sapa_tile_kernel<fused>", "sapa_tile_kernel<bwd>", "sapa_tile_kernel<sim>", "sapa_tile_kernel<agg>"};
+    const char *nr = names_ragged[mode & 3];
+#define SAPA_TMA_LAUNCH32(M)                                                                                                             \
+    case M:                                                                                                                              \
+        return ragged ? launch_persistent(sapa_tma_fused_f32_kernel<M, true>, nr, NT + RAGGED_PT, smem32, 1, M != MODE_BWD, a, st, qmap, kmap, vmap, omap) \
+                      : launch_persistent(sapa_tma_fused_f32_kernel<M, false>, n32, NT, smem32, CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap, omap);
+#define SAPA_TMA_LAUNCH16(T, M)                                                                                                          \
+    case M:                                                                                                                              \
+        return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, nr, h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
+                      : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, n16, h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
+    if (dtype == SAPA_F32) switch (mode) { SAPA_TMA_LAUNCH32(MODE_FWD) SAPA_TMA_LAUNCH32(MODE_BWD) SAPA_TMA_LAUNCH32(MODE_SIM) SAPA_TMA_LAUNCH32(MODE_AGG) }
+    if (dtype == SAPA_F16)
+        switch (mode) { SAPA_TMA_LAUNCH16(__half, MODE_FWD) SAPA_TMA_LAUNCH16(__half, MODE_BWD) SAPA_TMA_LAUNCH16(__half, MODE_SIM) SAPA_TMA_LAUNCH16(__half, MODE_AGG) }
+    if (dtype == SAPA_BF16)
+        switch (mode) { SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_FWD) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_BWD) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_SIM) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_AGG) }
+    set_error("sapa_tma_fused: unknown mode %d or dtype code %d", mode, dtype);
+    return SAPA_ERR_ARGUMENT;
 #undef SAPA_TMA_LAUNCH32
 #undef SAPA_TMA_LAUNCH16
 }

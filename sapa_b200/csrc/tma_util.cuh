@@ -56,6 +56,25 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, unsigned sr
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n"
                  ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
+// Per-lane asynchronous copies for rows that a tensor map cannot describe (not a multiple of 16 bytes): 4 or 8 bytes, zeros
+// where `valid` is false; cp_async_arrive makes the barrier (initialised with one count per copying thread) receive this
+// thread's arrival once all its copies so far have landed.
+__device__ __forceinline__ void cp_async4(unsigned dst, const void *src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(unsigned dst, const void *src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(unsigned bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void sts32(unsigned addr, unsigned v) { asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(addr), "r"(v) : "memory"); }
+// An address the compiler must take as new from here on: lds32 is a pure function of its address to the compiler, so a load
+// from a ring slot has to depend on something that follows the wait for the slot.
+__device__ __forceinline__ unsigned fresh(unsigned addr) {
+    asm volatile("" : "+r"(addr) : : "memory");
+    return addr;
+}
 // 32-bit load from a shared-memory address (state-space address, so the compiler emits LDS with an immediate
 // offset instead of a generic load with 64-bit address arithmetic)
 __device__ __forceinline__ unsigned lds32(unsigned addr) {

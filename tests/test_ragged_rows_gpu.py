@@ -1,0 +1,39 @@
+"""Rows that are not multiples of 16 bytes: the ragged form of the tensor-core kernels (no tensor maps, boxes copied by
+producer warps), at the widths and channel counts where its boxes, stores and work items end."""
+import pytest
+import torch
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# B, d, C, H, W: odd and even widths around the 8-column tile, one column, a channel tail, several items per tile (few tiles
+# and many channels), several tiles per CTA
+SHAPES = [(2, 16, 24, 7, 9), (1, 5, 7, 3, 1), (1, 40, 33, 5, 15), (1, 32, 256, 9, 18), (3, 16, 40, 33, 50)]
+
+
+@pytest.mark.parametrize("dtype,tol,tol_grad", [(torch.float32, 1e-5, 2e-5), (torch.bfloat16, 1e-2, 3e-2), (torch.float16, 2e-3, 4e-3)])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "B%d_d%d_C%d_%dx%d" % s)
+def test_ragged_rows_vs_oracle(oracle, shape, dtype, tol, tol_grad):
+    import sapa_b200 as sp
+    from sapa_b200 import _lib
+    B, d, C, H, W = shape
+    g = torch.Generator().manual_seed(3)
+    q, k, v, go = (torch.randn(*s, generator=g).to(dtype) for s in ((B, d, 2 * H, 2 * W), (B, d, H, W), (B, C, H, W), (B, C, 2 * H, 2 * W)))
+    q, k = (0.5 * q).to(dtype), (0.5 * k).to(dtype)
+    n = [t.double().numpy() for t in (q, k, v)]
+    want = oracle.sapa_forward(*n, 5, 2)
+    want_g = oracle.sapa_backward(go.double().numpy(), *n, 5, 2)
+    t = [x.to(DEV).requires_grad_() for x in (q, k, v)]
+    fused = sp.sapa_fused(*t, 5, 2)
+    got = torch.autograd.grad(fused, t, go.to(DEV))
+    assert _lib.last_kernels()[0] == "sapa_tile_kernel<bwd>"
+    sep = sp.av(torch.softmax(sp.qk(t[0], t[1], 5, 2), dim=1), t[2], 5, 2)
+    got_sep = torch.autograd.grad(sep, t, go.to(DEV))
+    # the separate ops round the logits and the attention map too: twice the forward's bound
+    for out, grads, f in ((fused, got, 1), (sep, got_sep, 2)):
+        assert rel_err(out.detach().double().cpu().numpy(), want) < f * tol
+        for a, b in zip(grads, want_g):
+            assert rel_err(a.double().cpu().numpy(), b) < f * tol_grad
+    assert _lib.wait_timeout_flags(DEV) == 0
