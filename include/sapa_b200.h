@@ -307,6 +307,52 @@ int sapa_project_forward(const void *x, const void *gamma, const void *beta, con
                          void *workspace, size_t workspace_bytes, int B, int C, int HW, int d, int groups, float eps,
                          int dtype, void *stream);
 
+/* sapa_project_forward for any multiple of 16 up to 1024 rows (in launches of up to 256).  `out` has out_dtype: the call's
+ * dtype, or SAPA_F16 / SAPA_BF16 for a float32 product (mixed precision).  shuffle_width > 0: the d rows are written as
+ * torch.pixel_shuffle(., 2) would place them, out = [B, d/4, 2 HW/width, 2 width] (the offsets of SAPA-D,
+ * sapa_deform.py:43-46).  Workspace: sapa_project_rows_workspace() bytes (0: not supported), 256-byte aligned. */
+size_t sapa_project_rows_workspace(int B, int C, int HW, int d, int groups, int dtype);
+int sapa_project_rows_forward(const void *x, const void *gamma, const void *beta, const void *weight, const void *bias, void *out,
+                              int shuffle_width, void *workspace, size_t workspace_bytes, int B, int C, int HW, int d, int groups,
+                              float eps, int dtype, int out_dtype, void *stream);
+
+/* One projection: out = weight (GroupNorm(x)) + bias; x [B, C, HW], weight [d, C], out [B, d, HW].  groups = 0: no norm
+ * (gamma, beta unused).  bias may be NULL.  `stats` (or NULL): float pairs [B, groups] = mean and reciprocal standard
+ * deviation, kept for sapa_projections_backward. */
+typedef struct sapa_projection {
+    const void *x, *gamma, *beta, *weight, *bias;
+    void *out, *stats;
+    int B, C, HW, d, groups;
+    float eps;
+} sapa_projection;
+
+/* Up to three projections in two launches, for rows of any length and any d; x and parameters have `dtype`, the outputs
+ * out_dtype (the same, or 16 bits of float32: then operands, product and biased sum are rounded as a 16-bit convolution of a
+ * float32 GroupNorm rounds them).  Workspace: sapa_projections_workspace() bytes (0: not supported), 256-byte aligned. */
+size_t sapa_projections_workspace(const sapa_projection *p, int count);
+int sapa_projections_forward(const sapa_projection *p, int count, void *workspace, size_t workspace_bytes, int dtype,
+                             int out_dtype, void *stream);
+
+/* One projection to differentiate, and optionally a second weight with d2 more rows on the same input (weight2, grad_out2, ...;
+ * d2 = 0 and NULL otherwise).  x, the parameters, grad_x and the parameter gradients share one dtype, grad_out, grad_out2 and
+ * `add` have the other one.  groups = 0: no norm (gamma, beta, stats, grad_gamma, grad_beta unused).  Any of grad_bias,
+ * grad_bias2, grad_x, add may be NULL. */
+typedef struct sapa_projection_grad {
+    const void *x, *grad_out, *grad_out2, *weight, *weight2, *gamma, *beta;
+    const void *stats;              /* from sapa_projections_forward */
+    const void *add;                /* one more gradient of x, [B, C, HW], added to grad_x */
+    void *grad_x, *grad_weight, *grad_weight2, *grad_bias, *grad_bias2, *grad_gamma, *grad_beta;
+    int B, C, HW, d, d2, groups;
+} sapa_projection_grad;
+
+/* Gradients of up to three projections with respect to x and every parameter, in three launches (four when some have a norm
+ * and some do not).  (dtype, grad_dtype): equal, or SAPA_F32 with a 16-bit grad_dtype.  Deterministic.  Behind a norm:
+ * d + d2 <= 64 and at most 256 channels per group.  Workspace: sapa_projections_backward_workspace() bytes (0: not supported),
+ * 256-byte aligned.  The reference leaves this to torch (sapa_base.py:27-34). */
+size_t sapa_projections_backward_workspace(const sapa_projection_grad *p, int count);
+int sapa_projections_backward(const sapa_projection_grad *p, int count, void *workspace, size_t workspace_bytes, int dtype,
+                              int grad_dtype, void *stream);
+
 /* Gradients of sapa_deform_fused_forward with respect to query, key, value and offset from grad_out and the
  * attention map it saved, in one kernel: the chain DeformAVBackward -> softmax backward over the points ->
  * DeformQKBackward of the reference (deform_av_cuda_kernel.cu:230-292, sapa_deform.py:52, deform_qk_cuda_kernel.cu:

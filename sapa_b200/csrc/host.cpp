@@ -34,7 +34,9 @@ struct Api {
     SAPA_FN(sapa_deform_av_forward_dense) SAPA_FN(sapa_deform_av_backward_dense) SAPA_FN(sapa_deform_fused_forward_dense) \
     SAPA_FN(sapa_deform_fused_backward_dense) SAPA_FN(sapa_deform_fused_forward_workspace)                                \
     SAPA_FN(sapa_deform_fused_backward_workspace) SAPA_FN(sapa_deform_fused_backward_scatter_bytes)                       \
-    SAPA_FN(sapa_project_workspace) SAPA_FN(sapa_project_forward)
+    SAPA_FN(sapa_project_workspace) SAPA_FN(sapa_project_forward) SAPA_FN(sapa_project_rows_workspace)                    \
+    SAPA_FN(sapa_project_rows_forward) SAPA_FN(sapa_projections_workspace) SAPA_FN(sapa_projections_forward)              \
+    SAPA_FN(sapa_projections_backward_workspace) SAPA_FN(sapa_projections_backward)
     SAPA_FNS
 #undef SAPA_FN
 };
@@ -130,6 +132,9 @@ PYBIND11_MODULE(_host, m) {
     m.def("deform_qk", &deform_qk);
     m.def("deform_av", &deform_av);
     m.def("deform_sapa_fused", &deform_fused);
+    m.def("sapa_module", &sapa_module);
+    m.def("deform_module", &deform_module);
+    m.def("project_module", &project_module);
     m.def("project", &project);
     m.def("project_workspace", &project_workspace);
 }

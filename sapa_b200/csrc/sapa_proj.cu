@@ -41,6 +41,7 @@
 #include <type_traits>
 
 namespace sapa {
+
 namespace proj {
 
 using namespace tmau;
@@ -60,7 +61,10 @@ struct Args {
     CUtensorMap x_map;              // (pixel, channel, 1, image), box = one 128-byte pixel row x (128 B / esize) channels
     CUtensorMap whi_map, wlo_map;   // (channel, output channel, 1, image), box = 128 bytes of channels x d rows
     const float *bias;              // folded bias [images or 1][d]
-    void *out;                      // [B][d][HW]
+    void *out;                      // first of the d rows of image 0; images are out_rows rows of HW elements apart
+    int out_rows;
+    int shuffle_w;                  // > 0: the rows are sub-pixels, written as torch.pixel_shuffle(., 2) would place them (row
+                                    // 4o + 2i + j of an image of this width = pixels (2y + i, 2x + j) of channel o)
     int B, C, HW, d, w_per_image, tiles_per_image, total_tiles, kblocks, nx, no, tmem_cols;
     int wide;                       // float32: hi*hi and hi*lo in ONE instruction of N = 2d (W' hi and lo blocks are adjacent rows)
 };
@@ -130,7 +134,8 @@ __device__ __forceinline__ void store_out(__nv_bfloat16 *p, float v) { *p = __fl
 // the tensor core reads the activations straight from their ring slot and an operand slot holds only the W' block.
 // float32: an operand slot holds the split activations (hi, lo) and the W' blocks (hi, lo); the split warps move a
 // landed slot into it and hand the ring slot back at once, so the loads in flight do not wait for the MMAs.
-template <typename T>
+// TO = type of the output (that of x, or 16 bits of a float32 product)
+template <typename T, typename TO>
 __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid_constant__ Args a) {
     constexpr bool F32 = sizeof(T) == 4;
     constexpr int KCH = 128 / (int)sizeof(T);        // channels per stage = one 128-byte row of the weight block
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
         }
     } else {        // epilogue warps: warp w owns accumulator lanes 32w .. 32w+31 = pixels px0 + 32w + lane
         unsigned ti = 0;
-        T *out = static_cast<T *>(a.out);
+        TO *out = static_cast<TO *>(a.out);
         for (int tile = blockIdx.x; tile < a.total_tiles && ok; tile += gridDim.x, ++ti) {
             const unsigned buf = ti & 1u, tph = (ti >> 1) & 1u;
             const int bi = tile / tpi, b = a.B - 1 - bi, px = (tile - bi * tpi) * TILE_PX + warp * 32 + lane, wb = a.w_per_image ? b : 0;
@@ -304,7 +309,11 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
             tc_fence_after();
             const unsigned taddr = tmem_base + ((unsigned)(warp * 32) << 16) + buf * acc_cols;
             const float *bias = a.bias + (size_t)wb * d;
-            T *op = out + (size_t)b * d * a.HW + px;
+            TO *op = out + (size_t)b * a.out_rows * a.HW + px;
+            if (a.shuffle_w > 0) {
+                const int y = px / a.shuffle_w, x = px - y * a.shuffle_w;
+                op = out + (size_t)b * a.out_rows * a.HW + (size_t)(4 * y) * a.shuffle_w + 2 * x;
+            }
             for (int c0 = 0; c0 < d; c0 += 16) {
                 unsigned r[16];
                 tc_ld16(taddr + (unsigned)c0, r);
@@ -320,7 +329,12 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
                     tc_fence_before();
                     mbar_arrive(tempty0 + 8 * buf);
                 }
-                if (px < a.HW) {
+                if (px < a.HW && a.shuffle_w > 0) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2)
+                        store_pair<TO>(op + (size_t)(c0 + (j & ~3)) * a.HW + (j & 2) * a.shuffle_w, __uint_as_float(r[j]) + __ldg(bias + c0 + j),
+                                       __uint_as_float(r[j + 1]) + __ldg(bias + c0 + j + 1));
+                } else if (px < a.HW) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) store_out(op + (size_t)(c0 + j) * a.HW, __uint_as_float(r[j]) + __ldg(bias + c0 + j));
                 }
@@ -487,17 +501,18 @@ static bool make_plan(Plan &p, int B, int C, int HW, int d, int groups, int dtyp
     return true;
 }
 
-template <typename T>
-static int run_project(const Plan &p, const void *x, const void *gamma, const void *beta, const void *weight, const void *bias,
-                       void *out, unsigned char *ws, int B, int C, int HW, int d, int groups, float eps, cudaStream_t st) {
+// `first`: the statistics are still to be taken (false for the second half of a projection with more than 256 rows)
+template <typename T, typename TO>
+static int run_project(const Plan &p, const void *x, const void *gamma, const void *beta, const void *weight, const void *bias, void *out, int out_rows,
+                       int shuffle_w, unsigned char *ws, int B, int C, int HW, int d, int groups, float eps, bool first, cudaStream_t st) {
     constexpr int KCH = 128 / (int)sizeof(T);
     constexpr CUtensorMapDataType type = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                          : std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    double2 *partial = reinterpret_cast<double2 *>(ws + p.partial_ofs);
     T *whi = reinterpret_cast<T *>(ws + p.whi_ofs), *wlo = reinterpret_cast<T *>(ws + p.wlo_ofs);
     float *bias_out = reinterpret_cast<float *>(ws + p.bias_ofs);
+    double2 *partial = reinterpret_cast<double2 *>(ws + p.partial_ofs);
     const long long n = groups > 0 ? (long long)(C / groups) * HW : 0;
-    if (groups > 0) {
+    if (groups > 0 && first) {
         gn_partial_kernel<T><<<dim3(p.nsplit, B * groups), STAT_THREADS, 0, st>>>(static_cast<const T *>(x), partial, n, p.nsplit);
         if (int e = check_launch("gn_partial_kernel")) return e;
     }
@@ -514,17 +529,39 @@ static int run_project(const Plan &p, const void *x, const void *gamma, const vo
         set_error("sapa_project_forward: tensor map creation failed (CUresult %d)", last_encode_result());
         return SAPA_ERR_UNSUPPORTED;
     }
-    a.bias = bias_out; a.out = out;
+    a.bias = bias_out; a.out = out; a.out_rows = out_rows; a.shuffle_w = shuffle_w;
     a.B = B; a.C = C; a.HW = HW; a.d = d; a.w_per_image = groups > 0 ? 1 : 0;
     a.tiles_per_image = (HW + TILE_PX - 1) / TILE_PX;
     a.total_tiles = a.tiles_per_image * B;
     a.kblocks = (C + KCH - 1) / KCH;
     a.nx = p.nx; a.no = p.no; a.tmem_cols = p.tmem_cols; a.wide = p.wide;
-    const size_t smem = p.smem;
     int sms = 0;
-    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_proj_umma_kernel<T>), SMEM_LIMIT, "sapa_proj_umma_kernel", sms)) return e;
-    sapa_proj_umma_kernel<T><<<std::min(a.total_tiles, sms), THREADS, smem, st>>>(a);
+    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_proj_umma_kernel<T, TO>), SMEM_LIMIT, "sapa_proj_umma_kernel", sms)) return e;
+    sapa_proj_umma_kernel<T, TO><<<std::min(a.total_tiles, sms), THREADS, p.smem, st>>>(a);
     return check_launch("sapa_proj_umma_kernel");
+}
+
+// rows of one GEMM launch for d output rows: all of them up to 256, else equal parts of whole 16-row blocks
+static int gemm_rows(int d) {
+    for (int parts = 1; parts <= 4; ++parts)
+        if (d % (16 * parts) == 0 && d / parts <= 256) return d / parts;
+    return d;
+}
+
+// plan for d rows in launches of gemm_rows(d)
+static bool make_rows_plan(Plan &p, int B, int C, int HW, int d, int groups, int dtype) {
+    return d > 0 && make_plan(p, B, C, HW, gemm_rows(d), groups, dtype);
+}
+
+template <typename T, typename TO>
+static int run_rows(const Plan &p, const void *x, const void *gamma, const void *beta, const void *weight, const void *bias, void *out, int shuffle_w,
+                    unsigned char *ws, int B, int C, int HW, int d, int groups, float eps, cudaStream_t st) {
+    const int rows = gemm_rows(d);
+    for (int r = 0; r < d; r += rows)
+        if (int e = run_project<T, TO>(p, x, gamma, beta, static_cast<const T *>(weight) + (size_t)r * C, bias != nullptr ? static_cast<const T *>(bias) + r : nullptr,
+                                       static_cast<TO *>(out) + (size_t)r * HW, d, shuffle_w, ws, B, C, HW, rows, groups, eps, r == 0, st))
+            return e;
+    return SAPA_OK;
 }
 
 }  // namespace proj
@@ -568,10 +605,42 @@ int sapa_project_forward(const void *x, const void *gamma, const void *beta, con
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     switch (dtype) {
-        case SAPA_F32: return proj::run_project<float>(p, x, gamma, beta, weight, bias, out, ws, B, C, HW, d, groups, eps, st);
-        case SAPA_F16: return proj::run_project<__half>(p, x, gamma, beta, weight, bias, out, ws, B, C, HW, d, groups, eps, st);
-        default: return proj::run_project<__nv_bfloat16>(p, x, gamma, beta, weight, bias, out, ws, B, C, HW, d, groups, eps, st);
+        case SAPA_F32: return proj::run_project<float, float>(p, x, gamma, beta, weight, bias, out, d, 0, ws, B, C, HW, d, groups, eps, true, st);
+        case SAPA_F16: return proj::run_project<__half, __half>(p, x, gamma, beta, weight, bias, out, d, 0, ws, B, C, HW, d, groups, eps, true, st);
+        default: return proj::run_project<__nv_bfloat16, __nv_bfloat16>(p, x, gamma, beta, weight, bias, out, d, 0, ws, B, C, HW, d, groups, eps, true, st);
     }
+}
+
+size_t sapa_project_rows_workspace(int B, int C, int HW, int d, int groups, int dtype) {
+    proj::Plan p;
+    return proj::make_rows_plan(p, B, C, HW, d, groups, dtype) ? p.total : 0;
+}
+
+int sapa_project_rows_forward(const void *x, const void *gamma, const void *beta, const void *weight, const void *bias, void *out, int shuffle_width,
+                              void *workspace, size_t workspace_bytes, int B, int C, int HW, int d, int groups, float eps, int dtype, int out_dtype,
+                              void *stream) {
+    const char *fn = "sapa_project_rows_forward";
+    trace_reset();
+    proj::Plan p;
+    SAPA_REQUIRE(dtype_size(dtype) != 0, SAPA_ERR_DTYPE, "%s: unknown dtype code %d", fn, dtype);
+    SAPA_REQUIRE(proj::make_rows_plan(p, B, C, HW, d, groups, dtype) && (out_dtype == dtype || (dtype == SAPA_F32 && (out_dtype == SAPA_F16 || out_dtype == SAPA_BF16))),
+                 SAPA_ERR_UNSUPPORTED, "%s: needs float32 / float16 / bfloat16 (output of the same type, or 16 bits of float32), d a multiple of 16 up to 1024, rows of HW "
+                 "and C elements that are multiples of 16 bytes and C divisible by groups", fn);
+    SAPA_CHECK_PTR(fn, x); SAPA_CHECK_PTR(fn, weight);
+    if (groups > 0) { SAPA_CHECK_PTR(fn, gamma); SAPA_CHECK_PTR(fn, beta); }
+    SAPA_REQUIRE(out != nullptr && all_aligned16(x, out), SAPA_ERR_ALIGNMENT, "%s: x and out must be 16-byte aligned", fn);
+    SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= p.total && reinterpret_cast<uintptr_t>(workspace) % 256 == 0,
+                 SAPA_ERR_WORKSPACE, "%s: a 256-byte aligned workspace of %zu bytes is required, got %zu", fn, p.total, workspace_bytes);
+    SAPA_REQUIRE(shuffle_width >= 0 && (shuffle_width == 0 || HW % shuffle_width == 0), SAPA_ERR_ARGUMENT, "%s: bad shuffle width", fn);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    unsigned char *ws = static_cast<unsigned char *>(workspace);
+#define SAPA_ROWS(T, TO) return proj::run_rows<T, TO>(p, x, gamma, beta, weight, bias, out, shuffle_width, ws, B, C, HW, d, groups, eps, st)
+    if (dtype == SAPA_F16) SAPA_ROWS(__half, __half);
+    if (dtype == SAPA_BF16) SAPA_ROWS(__nv_bfloat16, __nv_bfloat16);
+    if (out_dtype == SAPA_F16) SAPA_ROWS(float, __half);
+    if (out_dtype == SAPA_BF16) SAPA_ROWS(float, __nv_bfloat16);
+    SAPA_ROWS(float, float);
+#undef SAPA_ROWS
 }
 
 }  // extern "C"

@@ -11,9 +11,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _lib
 from .deform_functions import deform_av, deform_qk, deform_sapa_fused
 from .functions import av, qk, sapa_fused
-from .projection import project, project_supported
 
 
 def _init_projection(module: nn.Module) -> None:
@@ -41,19 +41,50 @@ def _common_dtype(*tensors):
     return tensors
 
 
+_NO_NORM = (None, None, 0, 0.0)
+
+
+def _norm_args(norm):
+    """(gamma, beta, groups, eps) of a GroupNorm (or of none) for the native module path, None when it is something else."""
+    if norm is None:
+        return _NO_NORM
+    if type(norm) is not nn.GroupNorm or norm.weight is None or norm._forward_hooks or norm._forward_pre_hooks:
+        return None
+    return norm.weight, norm.bias, norm.num_groups, norm.eps
+
+
+def _is_projection(conv):
+    """A 1x1 convolution with nothing around it that only calling the module would run."""
+    return (type(conv) is nn.Conv2d and conv.kernel_size == (1, 1) and conv.stride == (1, 1) and conv.padding == (0, 0) and
+            conv.groups == 1 and not conv._forward_hooks and not conv._forward_pre_hooks and not conv._backward_hooks)
+
+
+def _autocast_dtype():
+    return torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled() else None
+
+
 def _projected(x, norm, conv, fuse):
-    """``conv(norm(x))``.  With ``fuse`` and no gradient to record, GroupNorm and the 1x1 convolution run as one
-    tensor-core GEMM (``sapa_project_forward``); training, CPU tensors and shapes that kernel does not take use the torch
-    modules."""
+    """``conv(norm(x))``: with ``fuse`` GroupNorm and the 1x1 convolution run on this library's GEMM kernels, forward and
+    backward; otherwise, and for what those do not take, on the torch modules."""
     if fuse and x.is_cuda:
-        needs_grad = torch.is_grad_enabled() and (x.requires_grad or conv.weight.requires_grad or
-                                                  (norm is not None and norm.weight.requires_grad))
-        if not needs_grad:
-            if torch.is_autocast_enabled():
-                x = x.to(torch.get_autocast_dtype("cuda"))
-            if project_supported(x, norm, conv):
-                return project(x, norm, conv)
+        args = _norm_args(norm)
+        if args is not None and _is_projection(conv):
+            out = (_lib.host or _lib.load_host()).project_module(x, *args, conv.weight, conv.bias, _autocast_dtype())
+            if out is not None:
+                return out
     return conv(norm(x)) if norm is not None else conv(x)
+
+
+def _native_module(module, y, x, convs, *args):
+    """The whole module in one call (``csrc/host_module.inc``): its projections and the attention.  None where that does not
+    apply: another type or shape than the kernels take, replaced or hooked submodules, parameters of another type than the
+    input in training."""
+    norms = (_norm_args(module.norm_y), _norm_args(module.norm_x)) if module.norm else (_NO_NORM, _NO_NORM)
+    if None in norms or not all(_is_projection(c) for c in convs):
+        return None
+    host = _lib.host or _lib.load_host()
+    call = host.sapa_module if len(convs) == 2 else host.deform_module
+    return call(y, x, *norms[0], *norms[1], *(p for c in convs for p in (c.weight, c.bias)), *args, _autocast_dtype())
 
 
 class SAPA(nn.Module):
@@ -65,7 +96,7 @@ class SAPA(nn.Module):
         dim_x = dim_y if dim_x is None else dim_x
         self.up_factor, self.up_kernel_size, self.embedding_dim = up_factor, up_kernel_size, embedding_dim
         self.norm, self.impl = norm, _check_impl(impl)
-        self.fuse_projection = impl == "fused"      # set to False to keep torch's GroupNorm + convolution at inference too
+        self.fuse_projection = impl == "fused"      # set to False to keep torch's GroupNorm + convolution
         if norm:
             self.norm_y = nn.GroupNorm(32, dim_y)
             self.norm_x = nn.GroupNorm(32, dim_x)
@@ -75,6 +106,10 @@ class SAPA(nn.Module):
 
     def forward(self, y, x):
         # the value is the un-normalised x; only the key is computed from the normalised one
+        if self.fuse_projection and self.impl == "fused" and x.is_cuda:
+            out = _native_module(self, y, x, (self.q, self.k), self.up_kernel_size, self.up_factor)
+            if out is not None:
+                return out
         q = _projected(y, self.norm_y if self.norm else None, self.q, self.fuse_projection)
         k = _projected(x, self.norm_x if self.norm else None, self.k, self.fuse_projection)
         return self.attention(q, k, x)
@@ -108,6 +143,10 @@ class SAPADeform(nn.Module):
         self.apply(_init_projection)
 
     def forward(self, y, x):
+        if self.fuse_projection and self.impl == "fused" and x.is_cuda:
+            out = _native_module(self, y, x, (self.q, self.k, self.offset), self.high_offset, self.num_point, self.up_factor, self.groups)
+            if out is not None:
+                return out
         q = _projected(y, self.norm_y if self.norm else None, self.q, self.fuse_projection)
         k = _projected(x, self.norm_x if self.norm else None, self.k, self.fuse_projection)
         raw = self.offset(self.norm_x(x) if self.norm else x)
