@@ -526,45 +526,6 @@ constexpr int SMEM_BYTES = NSTAGE * SLOT_BYTES + 1024;
 static_assert(K_BYTES % 256 == 0 && SLOT_BYTES % 256 == 0, "the swizzled query box needs 256-byte alignment");
 }  // namespace h16
 
-__device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2(unsigned (&r)[2], unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2_trans(unsigned (&r)[2], unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], unsigned addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-// 8x8 transpose of a matrix of 16-bit elements held one row-pair per lane
-__device__ __forceinline__ unsigned movmatrix_trans(unsigned v) {
-    unsigned r;
-    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(r) : "r"(v));
-    return r;
-}
-template <typename T>
-__device__ __forceinline__ void mma_h16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    if constexpr (std::is_same<T, __half>::value)
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ float2 unpack_pair(__half, unsigned u) { return __half22float2(*reinterpret_cast<const __half2 *>(&u)); }
-__device__ __forceinline__ float2 unpack_pair(__nv_bfloat16, unsigned u) {
-    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u));
-}
-__device__ __forceinline__ float ex2_ftz(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Producer warps of the ragged 16-bit kernel: fill one ring slot with the boxes that TMA would put there (the columns of a
 // key / value box that a window can reach: box columns 6 .. 17; the others stay zero from the start of the kernel).  Eight
 // threads (six of them working) per box row, one pixel pair each.
@@ -1063,6 +1024,8 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
     }
 }
 
+#include "sapa_wide16.cuh"
+
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for every kernel of this file: they all share g_next_tile / g_ctas_done, so two launches that
 // may be in flight together (different streams, different kernels) must never get the same slot
@@ -1108,6 +1071,15 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
                            cudaStream_t st);
 
+// 16-bit: tiles of 4 x 32 instead of 4 x 8 pixels where at least three quarters of their columns are inside the image (below that
+// idle warps cost what the loads save) and nearly every SM gets one.
+// us, 4 x 8 -> 4 x 32: bfloat16 forward 8 x 256 x 64x64 55.7 -> 41.9, 64 x 256 x 128x128 1540 -> 1060, 1 x 256 x 1024x1024 2520 -> 1630;
+// logits 20.8 -> 14.6 and aggregation 50.7 -> 35.1 at 8 x 256 x 64x64.
+static bool wide16_pays(int W, int tiles_y, int B) {
+    const int tiles_x = ceil_div(W, tma::w16::COLS);
+    return 4 * W >= 3 * tiles_x * tma::w16::COLS && (long long)B * tiles_x * tiles_y >= 128;
+}
+
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
 // mode 0 (forward): out = atn(softmax(sim(q, k)), v), attn = optional output.
 // mode 1 (backward stage 1): q = grad_out [B,d,2H,2W], k = value [B,d,H,W] (d = value channels), v = key [B,C,H,W]
@@ -1133,6 +1105,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     const bool use_qk = mode != MODE_AGG, use_v = mode != MODE_SIM;
     CUtensorMap qmap{}, kmap{}, vmap{}, omap{};
     const bool ragged = !fused_tma_supported(W, dtype);
+    const bool wide = !ragged && dtype != SAPA_F32 && wide16_pays(W, ceil_div(y_end - y_begin, ROWS), B);
     bool ok = true;
     if (ragged) {
     } else if (dtype == SAPA_F32) {
@@ -1140,6 +1113,11 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         const auto sw = CU_TENSOR_MAP_SWIZZLE_64B;
         if (use_qk) ok = ok && make_nchw_map(&qmap, q, 2 * W, 2 * H, d, B, HC, F_KCH, HH, ty, 4, sw) && make_nchw_map(&kmap, k, W, rows, d, B, HC, F_KCH, HH, ty, 4, sw);
         if (use_v) ok = ok && make_nchw_map(&vmap, v, W, rows, C, B, HC, F_VCH, HH, ty, 4, sw) && make_nchw_map(&omap, out, 2 * W, 2 * H, C, B, HC, F_VCH, HH, ty, 4, sw);
+    } else if (wide) {
+        const auto ty = dtype == SAPA_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+        const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
+        if (use_qk) ok = ok && make_nchw_map(&qmap, q, 2 * W, 2 * H, d, B, w16::BC, w16::KCH, HH, ty, 2, sw) && make_nchw_map(&kmap, k, W, rows, d, B, w16::BC, w16::KCH, HH, ty, 2, sw);
+        if (use_v) ok = ok && make_nchw_map(&vmap, v, W, rows, C, B, w16::BC, w16::VCH, HH, ty, 2, sw);
     } else {
         const auto ty = dtype == SAPA_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
         if (use_qk) ok = ok && make_nchw_map(&qmap, q, 2 * W, 2 * H, d, B, 16, h16::KCH, HH, ty, 2, CU_TENSOR_MAP_SWIZZLE_32B) &&
@@ -1164,7 +1142,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     a.csplit = 1; a.vstages = ceil_div(C, F_VCH);
     static_assert(h16::COLS == COLS, "both kernels use the same tile");
     a.y_begin = y_begin; a.y_end = y_end;
-    a.tiles_x = ceil_div(W, COLS);
+    a.tiles_x = ceil_div(W, wide ? w16::COLS : COLS);
     a.tiles_y = ceil_div(y_end - y_begin, ROWS);
     constexpr int smem32 = NSTAGE * SLOT_BYTES + 2 * O_BYTES + 1024;
     static const char *const names32[4] = {"sapa_tma_fused_f32_kernel<fwd>", "sapa_tma_fused_f32_kernel<bwd>",
@@ -1182,6 +1160,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
 #define SAPA_TMA_LAUNCH16(T, M)                                                                                                          \
     case M:                                                                                                                              \
         return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, nr, h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
+               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, n16, w16::NT, w16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap)   \
                       : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, n16, h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
     if (dtype == SAPA_F32) switch (mode) { SAPA_TMA_LAUNCH32(MODE_FWD) SAPA_TMA_LAUNCH32(MODE_BWD) SAPA_TMA_LAUNCH32(MODE_SIM) SAPA_TMA_LAUNCH32(MODE_AGG) }
     if (dtype == SAPA_F16)
