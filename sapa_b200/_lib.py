@@ -8,6 +8,7 @@ import ctypes
 import os
 
 import torch
+from torch.autograd import forward_ad
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # SAPA_B200_LIB points at another build of the same library (for example one compiled with extra flags)
@@ -129,6 +130,13 @@ def load_host():
         _host.bind(LIB_PATH)
         host = _host
     return host
+
+
+def transformed() -> bool:
+    """True while torch.jit.trace records, under a torch.func transform and inside forward-mode differentiation.  An op is then a
+    ``torch.autograd.Function``: it appears in a trace as itself, and raises where it has no rule.  The native nodes do neither."""
+    return (torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active() or
+            forward_ad._current_level >= 0)
 
 
 def dtype_code(t: torch.Tensor) -> int:

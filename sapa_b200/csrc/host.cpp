@@ -129,6 +129,14 @@ PYBIND11_MODULE(_host, m) {
     m.def("av", &av);
     m.def("sapa_fused", &sapa_fused);
     m.def("fused_forward_raw", &fused_forward_raw);
+    m.def("qk_backward", &qk_bwd);
+    m.def("av_backward", &av_bwd);
+    m.def("sapa_fused_forward", &fused_forward_with_map);
+    m.def("sapa_fused_backward", &fused_bwd);
+    m.def("deform_qk_backward", &deform_qk_bwd);
+    m.def("deform_av_backward", &deform_av_bwd);
+    m.def("deform_fused_forward", &deform_fused_forward);
+    m.def("deform_fused_backward", &deform_fused_bwd);
     m.def("deform_qk", &deform_qk);
     m.def("deform_av", &deform_av);
     m.def("deform_sapa_fused", &deform_fused);

@@ -4,7 +4,8 @@
 ``QKFunction`` / ``AVFunction`` (sapa/sapa/sapa_func.py:9-96): AssertionError on inconsistent shapes,
 NotImplementedError for CPU tensors, RuntimeError for non-contiguous tensors, ``None`` gradients for the
 two integers.  Checks, allocation and the autograd nodes are native (``csrc/host.cpp``): the Python layer of a call is one
-function call.
+function call.  The ``Function`` classes run the same native code for traces and transforms (``_lib.transformed``), and for
+callers who use them by name.
 """
 from __future__ import annotations
 
@@ -16,11 +17,15 @@ from . import _lib
 
 def qk(query, key, kernel_size, scale_factor):
     """Local similarity: out[n, dy*K+dx, ph, pw] = <query[n,:,ph,pw], key[n,:,ph/s-r+dy, pw/s-r+dx]>."""
+    if _lib.transformed():
+        return QKFunction.apply(query, key, kernel_size, scale_factor)
     return (_lib.host or _lib.load_host()).qk(query, key, kernel_size, scale_factor)
 
 
 def av(attn, value, kernel_size, scale_factor):
     """Aggregation: out[n, c, ph, pw] = sum_k attn[n, k, ph, pw] * value[n, c, window_k(ph, pw)]."""
+    if _lib.transformed():
+        return AVFunction.apply(attn, value, kernel_size, scale_factor)
     return (_lib.host or _lib.load_host()).av(attn, value, kernel_size, scale_factor)
 
 
@@ -30,21 +35,51 @@ def sapa_fused(query, key, value, kernel_size=5, scale_factor=2):
 
     With a fused kernel available the attention map stays in registers (it is written once, for the backward
     pass, only when a gradient is required); otherwise the three separate kernels run."""
+    if _lib.transformed():
+        return SapaFusedFunction.apply(query, key, value, kernel_size, scale_factor)
     return (_lib.host or _lib.load_host()).sapa_fused(query, key, value, kernel_size, scale_factor)
 
 
-class QKFunction:
-    """The name under which the reference exposes ``qk``."""
-    apply = staticmethod(qk)
+class QKFunction(Function):
+    """``qk`` under the name that the reference exposes."""
+
+    @staticmethod
+    def forward(ctx, query, key, kernel_size, scale_factor):
+        ctx.window = (kernel_size, scale_factor)
+        ctx.save_for_backward(query, key)
+        return _lib.load_host().qk(query, key, kernel_size, scale_factor)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return (*_lib.load_host().qk_backward(grad_output, *ctx.saved_tensors, *ctx.window), None, None)
 
 
-class AVFunction:
-    """The name under which the reference exposes ``av``."""
-    apply = staticmethod(av)
+class AVFunction(Function):
+    """``av`` under the name that the reference exposes."""
+
+    @staticmethod
+    def forward(ctx, attn, value, kernel_size, scale_factor):
+        ctx.window = (kernel_size, scale_factor)
+        ctx.save_for_backward(attn, value)
+        return _lib.load_host().av(attn, value, kernel_size, scale_factor)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return (*_lib.load_host().av_backward(grad_output, *ctx.saved_tensors, *ctx.window), None, None)
 
 
-class SapaFusedFunction:
-    apply = staticmethod(sapa_fused)
+class SapaFusedFunction(Function):
+    @staticmethod
+    def forward(ctx, query, key, value, kernel_size, scale_factor):
+        ctx.window = (kernel_size, scale_factor)
+        out, attn = _lib.load_host().sapa_fused_forward(query, key, value, kernel_size, scale_factor, any(ctx.needs_input_grad[:3]))
+        if attn is not None:
+            ctx.save_for_backward(query, key, value, attn)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return (*_lib.load_host().sapa_fused_backward(grad_output, *ctx.saved_tensors, *ctx.window), None, None)
 
 
 def fused_supported(kernel_size: int, scale_factor: int, dtype: torch.dtype) -> bool:

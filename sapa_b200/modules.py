@@ -10,6 +10,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _lib
 from .deform_functions import deform_av, deform_qk, deform_sapa_fused
@@ -44,19 +45,30 @@ def _common_dtype(*tensors):
 _NO_NORM = (None, None, 0, 0.0)
 
 
+def _plain(module, cls):
+    """A ``cls`` with nothing around it that only calling it would run: no hooks, no ``forward`` of its own."""
+    return type(module) is cls and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or
+                                        module._backward_pre_hooks or "forward" in module.__dict__)
+
+
 def _norm_args(norm):
     """(gamma, beta, groups, eps) of a GroupNorm (or of none) for the native module path, None when it is something else."""
     if norm is None:
         return _NO_NORM
-    if type(norm) is not nn.GroupNorm or norm.weight is None or norm._forward_hooks or norm._forward_pre_hooks:
+    if not _plain(norm, nn.GroupNorm) or norm.weight is None:
         return None
     return norm.weight, norm.bias, norm.num_groups, norm.eps
 
 
 def _is_projection(conv):
-    """A 1x1 convolution with nothing around it that only calling the module would run."""
-    return (type(conv) is nn.Conv2d and conv.kernel_size == (1, 1) and conv.stride == (1, 1) and conv.padding == (0, 0) and
-            conv.groups == 1 and not conv._forward_hooks and not conv._forward_pre_hooks and not conv._backward_hooks)
+    return (_plain(conv, nn.Conv2d) and conv.kernel_size == (1, 1) and conv.stride == (1, 1) and conv.padding == (0, 0) and
+            conv.groups == 1)
+
+
+def _native(x):
+    """Whether the native module path may run at all: not for the CPU, nor where only torch's own ops are seen (traces, transforms,
+    hooks on every module)."""
+    return x.is_cuda and not _lib.transformed() and not _has_any_global_hook()
 
 
 def _autocast_dtype():
@@ -66,7 +78,7 @@ def _autocast_dtype():
 def _projected(x, norm, conv, fuse):
     """``conv(norm(x))``: with ``fuse`` GroupNorm and the 1x1 convolution run on this library's GEMM kernels, forward and
     backward; otherwise, and for what those do not take, on the torch modules."""
-    if fuse and x.is_cuda:
+    if fuse and _native(x):
         args = _norm_args(norm)
         if args is not None and _is_projection(conv):
             out = (_lib.host or _lib.load_host()).project_module(x, *args, conv.weight, conv.bias, _autocast_dtype())
@@ -77,8 +89,10 @@ def _projected(x, norm, conv, fuse):
 
 def _native_module(module, y, x, convs, *args):
     """The whole module in one call (``csrc/host_module.inc``): its projections and the attention.  None where that does not
-    apply: another type or shape than the kernels take, replaced or hooked submodules, parameters of another type than the
-    input in training."""
+    apply: another type or shape than the kernels take, replaced or hooked submodules, another ``attention`` than the class's,
+    parameters of another type than the input in training."""
+    if not _native(x) or getattr(module.attention, "__func__", None) not in _ATTENTIONS:
+        return None
     norms = (_norm_args(module.norm_y), _norm_args(module.norm_x)) if module.norm else (_NO_NORM, _NO_NORM)
     if None in norms or not all(_is_projection(c) for c in convs):
         return None
@@ -106,7 +120,7 @@ class SAPA(nn.Module):
 
     def forward(self, y, x):
         # the value is the un-normalised x; only the key is computed from the normalised one
-        if self.fuse_projection and self.impl == "fused" and x.is_cuda:
+        if self.fuse_projection and self.impl == "fused":
             out = _native_module(self, y, x, (self.q, self.k), self.up_kernel_size, self.up_factor)
             if out is not None:
                 return out
@@ -143,7 +157,7 @@ class SAPADeform(nn.Module):
         self.apply(_init_projection)
 
     def forward(self, y, x):
-        if self.fuse_projection and self.impl == "fused" and x.is_cuda:
+        if self.fuse_projection and self.impl == "fused":
             out = _native_module(self, y, x, (self.q, self.k, self.offset), self.high_offset, self.num_point, self.up_factor, self.groups)
             if out is not None:
                 return out
@@ -163,3 +177,6 @@ class SAPADeform(nn.Module):
                                      self.num_point, self.up_factor, self.groups)
         attn = F.softmax(deform_qk(q, k, offset, self.num_point, self.up_factor, self.groups), dim=2)
         return deform_av(attn, x, offset, self.num_point, self.up_factor, self.groups)
+
+
+_ATTENTIONS = (SAPA.attention, SAPADeform.attention)      # what the native module path stands for
