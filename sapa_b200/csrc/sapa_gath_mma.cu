@@ -361,38 +361,62 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     }
 }
 
+#include "sapa_gath_wide16.cuh"
+
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for all element types: they share g_next_tile / g_ctas_done
 static std::atomic<unsigned> g_next_sched_slot{0}, g_next_captured_slot{0};
 
+// 16-bit: tiles of 4 x 32 where at least three quarters of their columns are inside the image (below that idle warps cost what the
+// loads save).  us for both gradients of av in bfloat16, 4 x 8 -> 4 x 32: 8 x 256 x 64x64 112 -> 79, 2 x 512 x 16x32 40 -> 30,
+// 4 x 128 x 32x32 and 1 x 32 x 24x24 the same.
+static bool wide16_pays(int W) {
+    const int cols = ceil_div(W, gw16::COLS) * gw16::COLS;
+    return W % 8 == 0 && 4 * W >= 3 * cols;
+}
+
+// One form of the kernel: its tile, the channels of a stage and the launch.
+struct Form { int rows, cols, nch, threads, smem, ctas_per_sm; };
+
 template <typename T>
 static int launch(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype, cudaStream_t st) {
     using G = Geo<T>;
-    // rows a tensor map can describe and paired stores: the TMA form
-    const bool ragged = !gath_mma_supported(W, dtype);
+    constexpr bool F32 = sizeof(T) == 4;
+    // rows a tensor map can describe and paired stores: the TMA forms
+    const bool ragged = !gath_mma_supported(W, dtype), wide = !F32 && !ragged && wide16_pays(W);
     const char *name = ragged ? "sapa_gath_kernel" : "sapa_gath_mma_kernel";
-    CUtensorMap xmap{};
-    const CUtensorMapDataType ty = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+    const Form f = ragged ? Form{ROWS, COLS, G::NCH, NT_RAGGED, G::SMEM_BYTES, 1}
+                   : wide ? Form{ROWS, gw16::COLS, gw16::NCH, gw16::NT, gw16::SMEM_BYTES, 1}
+                          : Form{ROWS, COLS, G::NCH, NT, G::SMEM_BYTES, CTAS_PER_SM};
+    CUtensorMap xmap{}, bmap{};
+    const CUtensorMapDataType ty = F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const CUtensorMapSwizzle sw = sizeof(T) == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-    if (!ragged && !make_nchw_map(&xmap, hi, 2 * W, 2 * H, C, B, BPX, G::NCH, HR, ty, G::ES, sw)) {
+    bool mapped = true;
+    if (wide)
+        mapped = make_nchw_map(&xmap, hi, 2 * W, 2 * H, C, B, 64, gw16::NCH, HR, ty, G::ES, CU_TENSOR_MAP_SWIZZLE_128B) &&
+                 make_nchw_map(&bmap, hi, 2 * W, 2 * H, C, B, 16, gw16::NCH, HR, ty, G::ES, CU_TENSOR_MAP_SWIZZLE_32B);
+    else if (!ragged)
+        mapped = make_nchw_map(&xmap, hi, 2 * W, 2 * H, C, B, BPX, f.nch, HR, ty, G::ES, F32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+    if (!mapped) {
         set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
         return SAPA_ERR_UNSUPPORTED;
     }
     Args a{};
     a.hi = hi; a.wt = wt; a.out = out; a.B = B; a.C = C; a.H = H; a.W = W; a.top = top; a.Hout = top + H + bottom;
-    a.tiles_x = ceil_div(W, COLS);
-    a.tiles_y = ceil_div(a.Hout, ROWS);
-    a.csplit = 1; a.stages = ceil_div(C, G::NCH);
+    a.tiles_x = ceil_div(W, f.cols);
+    a.tiles_y = ceil_div(a.Hout, f.rows);
+    a.csplit = 1; a.stages = ceil_div(C, f.nch);
     long long nblocks = (long long)B * a.tiles_x * a.tiles_y;
     if (nblocks > 0x7fffffffLL) {
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    int sms = 0;
     const void *kernel = ragged ? reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, true>) : reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, false>);
-    if (int e = prepare_launch(kernel, G::SMEM_BYTES, name, sms)) return e;
-    const long long resident = (long long)(ragged ? 1 : CTAS_PER_SM) * sms;
+    if constexpr (!F32)
+        if (wide) kernel = reinterpret_cast<const void *>(sapa_gath_wide_16_kernel<T>);
+    int sms = 0;
+    if (int e = prepare_launch(kernel, f.smem, name, sms)) return e;
+    const long long resident = (long long)f.ctas_per_sm * sms;
     while (a.stages % 2 == 0 && 2 * nblocks <= resident) {      // every channel is independent: halve the items while all run at once
         a.stages /= 2;
         a.csplit *= 2;
@@ -400,8 +424,13 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     }
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
-    if (ragged) sapa_gath_mma_kernel<T, true><<<grid, NT_RAGGED, G::SMEM_BYTES, st>>>(xmap, a);
-    else sapa_gath_mma_kernel<T, false><<<grid, NT, G::SMEM_BYTES, st>>>(xmap, a);
+    if constexpr (!F32)
+        if (wide) {
+            sapa_gath_wide_16_kernel<T><<<grid, f.threads, f.smem, st>>>(xmap, bmap, a);
+            return check_launch(name);
+        }
+    if (ragged) sapa_gath_mma_kernel<T, true><<<grid, f.threads, f.smem, st>>>(xmap, a);
+    else sapa_gath_mma_kernel<T, false><<<grid, f.threads, f.smem, st>>>(xmap, a);
     return check_launch(name);
 }
 
