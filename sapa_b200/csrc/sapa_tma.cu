@@ -1117,7 +1117,8 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         const auto ty = dtype == SAPA_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
         const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
         if (use_qk) ok = ok && make_nchw_map(&qmap, q, 2 * W, 2 * H, d, B, w16::BC, w16::KCH, HH, ty, 2, sw) && make_nchw_map(&kmap, k, W, rows, d, B, w16::BC, w16::KCH, HH, ty, 2, sw);
-        if (use_v) ok = ok && make_nchw_map(&vmap, v, W, rows, C, B, w16::BC, w16::VCH, HH, ty, 2, sw);
+        if (use_v) ok = ok && make_nchw_map(&vmap, v, W, rows, C, B, w16::BC, w16::VCH, HH, ty, 2, sw) &&
+                        make_nchw_map(&omap, out, 2 * W, 2 * H, C, B, 2 * w16::COLS, w16::VCH, 2, ty, 2, sw);
     } else {
         const auto ty = dtype == SAPA_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
         if (use_qk) ok = ok && make_nchw_map(&qmap, q, 2 * W, 2 * H, d, B, 16, h16::KCH, HH, ty, 2, CU_TENSOR_MAP_SWIZZLE_32B) &&
@@ -1132,7 +1133,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     // maps a mode never touches still travel as kernel parameters: give them defined contents
     if (!use_qk) { qmap = vmap; kmap = vmap; }
     if (!use_v) { vmap = kmap; omap = kmap; }
-    if (dtype != SAPA_F32) omap = vmap;
+    if (dtype != SAPA_F32 && !(wide && use_v)) omap = vmap;
     Args a{};
     a.q = q; a.k = k; a.v = v;
     a.out = out; a.attn = attn; a.ws = ws;
@@ -1160,7 +1161,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
 #define SAPA_TMA_LAUNCH16(T, M)                                                                                                          \
     case M:                                                                                                                              \
         return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, nr, h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
-               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, n16, w16::NT, w16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap)   \
+               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, n16, w16::NT, w16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap, omap) \
                       : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, n16, h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
     if (dtype == SAPA_F32) switch (mode) { SAPA_TMA_LAUNCH32(MODE_FWD) SAPA_TMA_LAUNCH32(MODE_BWD) SAPA_TMA_LAUNCH32(MODE_SIM) SAPA_TMA_LAUNCH32(MODE_AGG) }
     if (dtype == SAPA_F16)

@@ -5,6 +5,10 @@
 // tensor memory accelerator needs two clocks for a 48-byte row as for a 128-byte one), its fragment loads and its stores:
 //   * boxes are 64 columns wide (128-byte rows, 128-byte swizzle, from x0 - 16: a 32-byte boundary), so a row of loads serves
 //     four times as many pixels and touches a page of a large plane a quarter as often;
+//   * outputs go through shared memory and leave as boxes with rows of 128 bytes (one lane of a spare warp issues them): a store
+//     from registers writes eight channels, 32 bytes each, which costs the load / store unit eight cycles (it was 70 % busy, and
+//     what the kernel waited for) and an address translation per channel: 64 x 256 x 128x128 1058 -> 829 us, 1 x 256 x 1024x1024,
+//     whose channels are 8 MB apart, 1666 -> 854;
 //   * a warp owns 8 low-res columns of one low-res row and BOTH of its high-res rows: a key or value fragment is loaded once for
 //     four products instead of twice for two each.
 // Fragments, accumulation order and roundings are those of the 4 x 8 kernel (the 24 columns that a warp reads are the same
@@ -22,20 +26,23 @@ constexpr int K_BYTES = HH * KCH * ROWB;        // 16 KB
 constexpr int Q_BYTES = 2 * ROWS * KCH * ROWB;  // 16 KB
 constexpr int V_BYTES = HH * VCH * ROWB;        // 32 KB
 constexpr int SLOT_BYTES = V_BYTES;
-constexpr int NSTAGE = 6;
-constexpr int SMEM_BYTES = NSTAGE * SLOT_BYTES + 1024;
+constexpr int NSTAGE = 5;
+constexpr int O_BYTES = 2 * ROWS * VCH * ROWB;  // 32 KB: output box [8 high-res rows][32 channels][64 pixels], two of them behind the ring
+constexpr int SMEM_BYTES = NSTAGE * SLOT_BYTES + 2 * O_BYTES + 1024;
 static_assert(K_BYTES + Q_BYTES <= SLOT_BYTES && SMEM_BYTES <= 227 * 1024, "ring");
 }  // namespace w16
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(w16::NT, 1)
-sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const Args a) {
+sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
+                    const __grid_constant__ CUtensorMap omap, const Args a) {
     using namespace w16;
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ __align__(8) unsigned long long bars[2 * w16::NSTAGE];      // full[NSTAGE], empty[NSTAGE]
+    __shared__ __align__(8) unsigned long long bars[2 * w16::NSTAGE + 4];  // full[NSTAGE], empty[NSTAGE]; written[2], free[2] of the output boxes
     __shared__ int tile_ids[8];       // tile_ids[ti & 7] = item of the ti-th turn of this CTA, -1 = no more (the producer is at most NSTAGE turns ahead)
     const unsigned ring_addr = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u;
     const unsigned full_addr = (unsigned)__cvta_generic_to_shared(bars), empty_addr = full_addr + 8 * w16::NSTAGE;
+    const unsigned written_addr = empty_addr + 8 * w16::NSTAGE, free_addr = written_addr + 16, obuf_addr = ring_addr + w16::NSTAGE * w16::SLOT_BYTES;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wrow = warp & 3, wcol = warp >> 2;
@@ -51,12 +58,41 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
             mbar_init(full_addr + 8 * i, 1);
             mbar_init(empty_addr + 8 * i, w16::NW);
         }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(written_addr + 8 * i, w16::NW);
+            mbar_init(free_addr + 8 * i, 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
 
     if (warp >= w16::NW) {            // producer: one lane; the stages of successive items form one stream through the ring
         asm volatile("setmaxnreg.dec.sync.aligned.u32 24;\n");
+        if (MODE != MODE_SIM && tid == (w16::NW + 1) * 32) {
+            // output: one lane of another warp of the group stores the boxes that the consumers have written
+            int buf = 0, par = 0;
+            for (int ti = 0;; ++ti) {
+                for (int it = 0; it < nv; ++it) {
+                    const bool ok = mbar_wait_bounded(written_addr + 8 * buf, par);
+                    if (!ok) atomicExch(&g_wait_timeout, 1);
+                    int u = ok ? tile_ids[ti & 7] : -1;     // as the consumers read it, at most two stages ago
+                    if (u < 0) {
+                        asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+                        return;
+                    }
+                    const int c0 = (u % a.csplit * nv + it) * w16::VCH; u /= a.csplit;
+                    const int x0 = (u % a.tiles_x) * w16::COLS; u /= a.tiles_x;
+                    const int y0 = a.y_begin + (u % a.tiles_y) * ROWS, n = u / a.tiles_y;
+                    for (int row = 0; row < ROWS && y0 + row < a.y_end; ++row)       // pixels and channels beyond the tensor are cut off
+                        tma_store_4d(&omap, obuf_addr + buf * w16::O_BYTES + row * (w16::O_BYTES / ROWS), 2 * x0, c0, 2 * (y0 + row), n);
+                    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                    asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+                    mbar_arrive(free_addr + 8 * buf);
+                    if (++buf == 2) { buf = 0; par ^= 1; }
+                }
+            }
+        }
         if (tid != w16::NW * 32) return;
         int slot = 0, phase = 0;
         for (int ti = 0;; ++ti) {
@@ -105,6 +141,7 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     const int k_off = wrow * (w16::KCH * w16::ROWB) + row_t * w16::ROWB + (((wcol + 1 + chunk_t) ^ sw) << 4);
     const int k_off2 = wrow * (w16::KCH * w16::ROWB) + row_a * w16::ROWB + (((wcol + 3) ^ sw) << 4);
     const int v_off = wrow * (w16::VCH * w16::ROWB) + row_a * w16::ROWB + (((wcol + 1 + chunk_a) ^ sw) << 4);
+    const int o_off = 2 * wrow * (w16::VCH * w16::ROWB) + g * w16::ROWB + (((2 * wcol) ^ g) << 4) + 4 * t;      // output: chunk 2 wcol, the right group's is that ^ 1
     const int v_off2 = wrow * (w16::VCH * w16::ROWB) + row_a * w16::ROWB + (((wcol + 3) ^ sw) << 4);
     bool ok_lo[2], ok_hi[2];
     int dx_lo[2];                 // window column of the lo cell (hi = lo + 8)
@@ -118,11 +155,17 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     const size_t plane_w = hi_plane >> 1;         // strides in 32-bit words (two elements)
     const int row_w = sW >> 1;
     constexpr float LOG2E = 1.4426950408889634f;
-    int slot = 0, phase = 0;
+    int slot = 0, phase = 0, obuf = 0, opar = 0;
     for (int ti = 0;; ++ti) {
         if (!mbar_wait_bounded(full_addr + 8 * slot, phase)) { atomicExch(&g_wait_timeout, 1); return; }
         int item = tile_ids[ti & 7];              // published by the producer before the barrier's phase completed
-        if (item < 0) break;
+        if (item < 0) {
+            if (MODE != MODE_SIM) {               // the storing lane reads -1 and stops
+                if (!mbar_wait_bounded(free_addr + 8 * obuf, opar ^ 1)) atomicExch(&g_wait_timeout, 1);
+                else if (lane == 0) mbar_arrive(written_addr + 8 * obuf);
+            }
+            break;
+        }
         int c0 = item % a.csplit * nv * w16::VCH; item /= a.csplit;
         const int x0 = (item % a.tiles_x) * w16::COLS + 8 * wcol; item /= a.tiles_x;      // first column of this warp
         const int y = a.y_begin + (item % a.tiles_y) * ROWS + wrow, n = item / a.tiles_y;
@@ -296,8 +339,7 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         }
         if (MODE == MODE_SIM) continue;
         // ------------------------------------------------------------- aggregation
-        unsigned *o_ptr = static_cast<unsigned *>(a.out) + ((size_t)n * a.C + c0 + g) * plane_w + pix_w + ((t & 1) ? 3 : 0);
-        for (int it = 0; it < nv; ++it, c0 += w16::VCH, o_ptr += (size_t)w16::VCH * plane_w) {
+        for (int it = 0; it < nv; ++it) {
             if ((MODE != MODE_AGG || it > 0) && !mbar_wait_bounded(full_addr + 8 * slot, phase)) { atomicExch(&g_wait_timeout, 1); return; }
             const unsigned stage = ring_addr + slot * w16::SLOT_BYTES;
             float acc[2][2][2][4];                // [16 channels][high-res row][group]
@@ -327,20 +369,21 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(empty_addr + 8 * slot);
             if (++slot == w16::NSTAGE) { slot = 0; phase ^= 1; }
-            if (live) {
-                // neighbouring lanes swap one pair so that a quad writes one full 32-byte sector of a channel's row per store
-                const bool odd = t & 1;
+            // D fragments -> output box, 128-byte swizzle: the 32 lanes of a store hit 32 banks
+            if (!mbar_wait_bounded(free_addr + 8 * obuf, opar ^ 1)) { atomicExch(&g_wait_timeout, 1); return; }
+            const unsigned ob = obuf_addr + obuf * w16::O_BYTES + o_off;
 #pragma unroll
-                for (int r = 0; r < 2; ++r)
+            for (int r = 0; r < 2; ++r)
 #pragma unroll
-                    for (int j = 0; j < w16::VCH / 8; ++j) {       // channel g + 8j: block j/2, half j%2
-                        const unsigned v0 = pack_pair(T(), acc[j >> 1][r][0][2 * (j & 1)], acc[j >> 1][r][0][2 * (j & 1) + 1]);
-                        const unsigned v1 = pack_pair(T(), acc[j >> 1][r][1][2 * (j & 1)], acc[j >> 1][r][1][2 * (j & 1) + 1]);
-                        const unsigned got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-                        if (c0 + 8 * j + g < a.C)
-                            __stcs(reinterpret_cast<uint2 *>(o_ptr + (size_t)(8 * j) * plane_w + r * row_w), odd ? make_uint2(got, v1) : make_uint2(v0, got));
-                    }
-            }
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int j = 0; j < w16::VCH / 8; ++j)         // channel g + 8j: block j/2, half j%2
+                        sts32((ob ^ (p << 4)) + r * (w16::VCH * w16::ROWB) + 8 * j * w16::ROWB,
+                              pack_pair(T(), acc[j >> 1][r][p][2 * (j & 1)], acc[j >> 1][r][p][2 * (j & 1) + 1]));
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(written_addr + 8 * obuf);
+            if (++obuf == 2) { obuf = 0; opar ^= 1; }
         }
     }
 }
