@@ -14,8 +14,9 @@
 // image read as zero.  All backward kernels are gathers: no atomics, bit-reproducible.
 //
 // Two families:
-//   * tiled kernels for (K, s) = (3,2), f32/f16/bf16 (K = 5 runs on the tensor-core kernels of the other files, rows of any
-//     length): one thread per LOW-res pixel, i.e. per
+//   * tiled kernels for (K, s) = (3,2), f32/f16/bf16, and for (5,2) in float32 with rows that no tensor map describes (the rest of
+//     K = 5 runs on the tensor-core kernels of the other files; float32 as three tf32 products has 1.3e-6 of error where this has
+//     2.4e-7): one thread per LOW-res pixel, i.e. per
 //     s x s group of high-res pixels that share one K x K window; the window weights of the whole group
 //     (K*K*s*s values) live in registers, the low-res halo tile of L is staged in shared memory, and HBM is
 //     touched once per element with vector loads/stores.  The fused kernel runs sim -> softmax -> agg
@@ -555,8 +556,11 @@ bool gath_mma_supported(int W, int dtype);
 int launch_gath_mma(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype,
                     cudaStream_t st);
 
-// (K, s) with kernels that work on tiles: the tensor-core kernels for K = 5 (rows of any length), the tiled kernels of this
-// file for K = 3
+// K = 5, s = 2 on the tensor-core kernels: 16-bit rows of any length, float32 where a tensor map describes the rows
+static bool tensor_core_rows(int W, int dtype) { return dtype == SAPA_F32 ? fused_tma_supported(W, dtype) : dtype != SAPA_F64; }
+static bool tensor_core_gath(int W, int dtype) { return dtype == SAPA_F32 ? gath_mma_supported(W, dtype) : dtype != SAPA_F64; }
+
+// (K, s) with kernels that work on tiles: the tensor-core kernels or the tiled kernels of this file
 static bool tiled_supported(int K, int s, int dtype) {
     return dtype != SAPA_F64 && s == 2 && (K == 5 || K == 3);
 }
@@ -579,17 +583,24 @@ static int launch_tile(TileArgs a, cudaStream_t st) {
 }
 
 template <typename T, int MODE>
-static int launch_tile_ks(const TileArgs &a, cudaStream_t st) {
+static int launch_tile_ks(const TileArgs &a, int K, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4 && MODE != MODE_FUSED)
+        if (K == 5) return launch_tile<T, 5, 2, MODE>(a, st);
     return launch_tile<T, 3, 2, MODE>(a, st);
 }
 
 template <typename T>
-static int launch_gath(const T *hi, const T *wt, T *out, int B, int Cc, int H, int W, cudaStream_t st) {
-    using Shape = TileShape<3, 2, 4, 32, 1>;
-    const int tiles_x = ceil_div(W, Shape::TW), tiles_y = ceil_div(H, Shape::TH);
-    const long long blocks = (long long)B * tiles_x * tiles_y;
-    sapa_gath_kernel<T, Shape><<<(unsigned)blocks, Shape::NT, 0, st>>>(hi, wt, out, B, Cc, H, W, tiles_x, tiles_y);
-    return check_launch("sapa_gath_kernel");
+static int launch_gath(const T *hi, const T *wt, T *out, int B, int Cc, int H, int W, int K, cudaStream_t st) {
+    auto go = [&](auto shape) -> int {
+        using Shape = decltype(shape);
+        const int tiles_x = ceil_div(W, Shape::TW), tiles_y = ceil_div(H, Shape::TH);
+        const long long blocks = (long long)B * tiles_x * tiles_y;
+        sapa_gath_kernel<T, Shape><<<(unsigned)blocks, Shape::NT, 0, st>>>(hi, wt, out, B, Cc, H, W, tiles_x, tiles_y);
+        return check_launch("sapa_gath_kernel");
+    };
+    if constexpr (sizeof(T) == 4)
+        if (K == 5) return go(TileShape<5, 2, 4, 32, 1>{});
+    return go(TileShape<3, 2, 4, 32, 1>{});
 }
 
 static int check_common(const char *fn, int B, int C, int H, int W, int K, int s, int dtype) {
@@ -610,15 +621,15 @@ static int check_common(const char *fn, int B, int C, int H, int W, int K, int s
 int run_sim_slab(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s,
                  int dtype, cudaStream_t st) {
     const bool al = all_aligned16(hi, lo, out);     // misaligned views take the scalar generic kernels
-    if (al && K == 5 && s == 2 && dtype != SAPA_F64) {     // logit half of the tensor-core kernel
+    if (al && K == 5 && s == 2 && tensor_core_rows(W, dtype)) {     // logit half of the tensor-core kernel
         const int e = launch_fused_tma(2, hi, lo, nullptr, nullptr, out, nullptr, B, Cc, 0, H, W, rows, top, 0, H, dtype, st);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
-    if (al && K == 3 && tiled_supported(K, s, dtype)) {
+    if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {
         TileArgs a{};
         a.hi = hi; a.lo1 = lo; a.out_slots = out;
         a.B = B; a.C1 = Cc; a.C2 = 0; a.H = H; a.W = W; a.rows = rows; a.ytop0 = top;
-        return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_SIM>(a, st); });
+        return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_SIM>(a, K, st); });
     }
     if (rows != H || top != 0) {
         set_error("run_sim_slab: a padded slab needs 16-byte aligned tensors and a tiled (K, s)");
@@ -650,16 +661,16 @@ int run_sim(const void *hi, const void *lo, void *out, int B, int Cc, int H, int
 int run_agg_slab(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s,
                  int dtype, cudaStream_t st) {
     const bool al = all_aligned16(wt, lo, out);
-    if (al && K == 5 && s == 2 && dtype != SAPA_F64) {     // aggregation half of the tensor-core kernel
+    if (al && K == 5 && s == 2 && tensor_core_rows(W, dtype)) {     // aggregation half of the tensor-core kernel
         const int e = launch_fused_tma(3, nullptr, nullptr, lo, out, const_cast<void *>(wt), nullptr, B, 0, Cc, H, W, rows, top, 0, H,
                                        dtype, st);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
-    if (al && K == 3 && tiled_supported(K, s, dtype)) {
+    if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {
         TileArgs a{};
         a.slots_in = wt; a.lo2 = lo; a.out_hi = out;
         a.B = B; a.C1 = 0; a.C2 = Cc; a.H = H; a.W = W; a.rows = rows; a.ytop0 = top;
-        return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_AGG>(a, st); });
+        return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_AGG>(a, K, st); });
     }
     if (rows != H || top != 0) {
         set_error("run_agg_slab: a padded slab needs 16-byte aligned tensors and a tiled (K, s)");
@@ -680,14 +691,14 @@ int run_agg(const void *wt, const void *lo, void *out, int B, int Cc, int H, int
 int run_gath(const void *hi, const void *wt, void *out, int B, int Cc, int H, int W, int K, int s, int dtype,
              cudaStream_t st) {
     const bool al = all_aligned16(hi, wt, out);
-    if (al && K == 5 && s == 2 && dtype != SAPA_F64) {
+    if (al && K == 5 && s == 2 && tensor_core_gath(W, dtype)) {
         const int e = launch_gath_mma(hi, wt, out, B, Cc, H, W, 0, 0, dtype, st);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
-    if (al && K == 3 && tiled_supported(K, s, dtype)) {
+    if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {
         return SAPA_DISPATCH_FAST(dtype, [&] {
             return launch_gath<scalar_t>(static_cast<const scalar_t *>(hi), static_cast<const scalar_t *>(wt),
-                                         static_cast<scalar_t *>(out), B, Cc, H, W, st);
+                                         static_cast<scalar_t *>(out), B, Cc, H, W, K, st);
         });
     }
     return SAPA_DISPATCH_ALL(dtype, [&] {
@@ -789,7 +800,7 @@ int sapa_fused_forward_slab_rows(const void *query, const void *key, const void 
         return launch_fused_mma(query, key, value, out, attn, B, d, C, H, W, a.rows, a.ytop0, dtype, st);
     if (K == 5)      // 16-bit rows of odd length
         return launch_fused_tma(0, query, key, value, out, attn, nullptr, B, d, C, H, W, a.rows, a.ytop0, 0, H, dtype, st);
-    return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_FUSED>(a, st); });
+    return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_FUSED>(a, K, st); });
 }
 
 int sapa_fused_forward_slab(const void *query, const void *key, const void *value, void *out, void *attn, int B, int d,
@@ -826,7 +837,7 @@ int sapa_fused_backward(const void *grad_out, const void *query, const void *key
     bool stage1_done = false;
     // misaligned views (a storage offset that is not a multiple of 16 bytes) take the chain of scalar generic kernels
     const bool al = all_aligned16(grad_out, query, key, value, attn, grad_query, grad_key, grad_value);
-    if (al && K == 5 && s == 2 && dtype != SAPA_F64) {
+    if (al && K == 5 && s == 2 && tensor_core_rows(W, dtype)) {
         // tensor-core kernel (the fused forward's data flow with the softmax backward in the middle)
         const int e = launch_fused_tma(1, grad_out, value, key, grad_query, const_cast<void *>(attn), dS, B, C, d, H, W, H, 0,
                                        0, H, dtype, st);
@@ -834,12 +845,12 @@ int sapa_fused_backward(const void *grad_out, const void *query, const void *key
         stage1_done = e == SAPA_OK;
     }
     if (stage1_done) {
-    } else if (al && K == 3 && tiled_supported(K, s, dtype)) {
+    } else if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {
         // one kernel: dA = sim(dOut, V) -> softmax backward with the saved A -> dS (workspace), dQ = agg(dS, Key)
         TileArgs a{};
         a.hi = grad_out; a.lo1 = value; a.slots_in = attn; a.lo2 = key; a.out_slots = dS; a.out_hi = grad_query;
         a.B = B; a.C1 = C; a.C2 = d; a.H = H; a.W = W; a.rows = H; a.ytop0 = 0;
-        if (int e = SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_BWD>(a, st); })) return e;
+        if (int e = SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_BWD>(a, K, st); })) return e;
     } else {
         // dA goes to the workspace, then dS overwrites it in place
         if (int e = run_sim(grad_out, value, dS, B, C, H, W, K, s, dtype, st)) return e;

@@ -993,8 +993,9 @@ extern "C" {
 
 size_t sapa_deform_fused_forward_workspace(int B, int H, int W, int P, int s, int G, int dtype) {
     if (B <= 0 || H <= 0 || W <= 0 || P <= 0 || G <= 0 || s != 2) return 0;
-    // 16-bit tensors: the mixed modes of the tensor-core kernels (16-bit operands, float32 windows)
-    if (dtype != SAPA_F32 && dtype != SAPA_F16 && dtype != SAPA_BF16) return 0;
+    // 16-bit tensors: the mixed modes of the tensor-core kernels (16-bit operands, float32 windows).  Rows that are not multiples of 16 bytes run the
+    // float32 chain on widened tensors, or the gather kernels, with float32 weights
+    if (dtype != SAPA_F32 && !((dtype == SAPA_F16 || dtype == SAPA_BF16) && W % 8 == 0)) return 0;
     const size_t hi = (size_t)s * H * s * W;
     if ((size_t)B * G * hi >= 0xffffffffull) return 0;       // the outlier list indexes (image, group, pixel) with 32 bits
     // dense similarity + window weights (float32 whatever the tensors' type), the outlier list (worst case: every
@@ -1015,7 +1016,7 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     SAPA_CHECK_PTR(fn, out);
     const size_t need = sapa_deform_fused_forward_workspace(B, H, W, P, s, G, dtype);
     SAPA_REQUIRE(s == 2 && P <= MAXP && need != 0, SAPA_ERR_UNSUPPORTED,
-                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, float16 or bfloat16 "
+                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, or float16 / bfloat16 with rows of 16 bytes "
                  "(use sapa_deform_fused_forward)", fn, MAXP);
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && aligned16(workspace), SAPA_ERR_WORKSPACE,
                  "%s: a 16-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);
@@ -1084,7 +1085,7 @@ int sapa_deform_qk_forward_dense(const void *query, const void *key, const void 
     SAPA_CHECK_PTR(fn, query); SAPA_CHECK_PTR(fn, key); SAPA_CHECK_PTR(fn, offset); SAPA_CHECK_PTR(fn, out);
     const size_t need = sapa_deform_fused_forward_workspace(B, H, W, P, s, G, dtype);
     SAPA_REQUIRE(s == 2 && P <= MAXP && need != 0, SAPA_ERR_UNSUPPORTED,
-                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, float16 or bfloat16 "
+                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, or float16 / bfloat16 with rows of 16 bytes "
                  "(use sapa_deform_qk_forward)", fn, MAXP);
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && aligned16(workspace), SAPA_ERR_WORKSPACE,
                  "%s: a 16-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);
@@ -1118,7 +1119,7 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
     SAPA_CHECK_PTR(fn, attn); SAPA_CHECK_PTR(fn, value); SAPA_CHECK_PTR(fn, offset); SAPA_CHECK_PTR(fn, out);
     const size_t need = sapa_deform_fused_forward_workspace(B, H, W, P, s, G, dtype);
     SAPA_REQUIRE(s == 2 && P <= MAXP && need != 0, SAPA_ERR_UNSUPPORTED,
-                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, float16 or bfloat16 "
+                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, or float16 / bfloat16 with rows of 16 bytes "
                  "(use sapa_deform_av_forward)", fn, MAXP);
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && aligned16(workspace), SAPA_ERR_WORKSPACE,
                  "%s: a 16-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);
@@ -1156,8 +1157,9 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
 
 size_t sapa_deform_fused_backward_workspace(int B, int H, int W, int P, int s, int G, int dtype) {
     if (B <= 0 || H <= 0 || W <= 0 || P <= 0 || G <= 0 || s != 2) return 0;
-    // 16-bit tensors: 16-bit operands in the tensor-core kernels, float32 similarities between them
-    if (dtype != SAPA_F32 && dtype != SAPA_F16 && dtype != SAPA_BF16) return 0;
+    // 16-bit tensors: 16-bit operands in the tensor-core kernels, float32 similarities between them.  Rows that are not multiples of 16 bytes run the
+    // float32 chain on widened tensors, or the gather kernels, with float32 weights
+    if (dtype != SAPA_F32 && !((dtype == SAPA_F16 || dtype == SAPA_BF16) && W % 8 == 0)) return 0;
     const size_t hi = (size_t)s * H * s * W;
     if ((size_t)B * G * P >= 0xffffffffull || hi >= 0xffffffffull) return 0;
     // D, dWd (float32), dD, Wd (the tensors' type; sized for float32), the outlier list (worst case: every point) and
@@ -1185,7 +1187,7 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     const size_t side_off = (base + 15) & ~(size_t)15;          // the side buffers of the 16-bit path start here
     const size_t need = side_off + sapa_deform_fused_backward_scatter_bytes(B, Cq, C, H, W, dtype);
     SAPA_REQUIRE(s == 2 && P <= MAXP && base != 0, SAPA_ERR_UNSUPPORTED,
-                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, float16 or bfloat16 "
+                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, or float16 / bfloat16 with rows of 16 bytes "
                  "(use sapa_deform_fused_backward)", fn, MAXP);
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && aligned16(workspace), SAPA_ERR_WORKSPACE,
                  "%s: a 16-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);
@@ -1269,7 +1271,7 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     const size_t side_off = (base + 15) & ~(size_t)15;
     const size_t need = side_off + sapa_deform_fused_backward_scatter_bytes(B, 0, C, H, W, dtype);
     SAPA_REQUIRE(s == 2 && P <= MAXP && base != 0, SAPA_ERR_UNSUPPORTED,
-                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, float16 or bfloat16 "
+                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, or float16 / bfloat16 with rows of 16 bytes "
                  "(use sapa_deform_av_backward)", fn, MAXP);
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && aligned16(workspace), SAPA_ERR_WORKSPACE,
                  "%s: a 16-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);
@@ -1337,7 +1339,7 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     const size_t side_off = (base + 15) & ~(size_t)15;
     const size_t need = side_off + sapa_deform_fused_backward_scatter_bytes(B, Cq, 0, H, W, dtype);
     SAPA_REQUIRE(s == 2 && P <= MAXP && base != 0, SAPA_ERR_UNSUPPORTED,
-                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, float16 or bfloat16 "
+                 "%s: the dense-window path needs s = 2, num_point <= %d and float32, or float16 / bfloat16 with rows of 16 bytes "
                  "(use sapa_deform_qk_backward)", fn, MAXP);
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && aligned16(workspace), SAPA_ERR_WORKSPACE,
                  "%s: a 16-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);

@@ -81,7 +81,7 @@ template <typename T> __device__ __forceinline__ int px_off(int px, int ch) {
     else                          return ((((px >> 3) ^ (ch >> 1)) & 3) << 4) | ((px & 7) << 1);             // 64-byte swizzle
 }
 
-// RAGGED: high-res rows that are not multiples of 16 bytes (or low-res rows of odd length) - no tensor map, PW producer
+// RAGGED (16-bit): high-res rows that are not multiples of 16 bytes (or low-res rows of odd length) - no tensor map, PW producer
 // warps copy the pixel pairs a fragment can reach (box pixels 4 .. 27; a pair is always on its own boundary because
 // high-res rows have an even length), static tile order, single-element stores where W is odd.
 template <typename T, bool RAGGED>
@@ -137,15 +137,25 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                     if (!mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) { atomicExch(&g_wait_timeout, 1); return; }
                     const unsigned dst = ring_addr + slot * G::BOX_BYTES;
                     const int c0 = (vb + it) * NCH;
-                    if (pair >= 2 && pair < 14) {
+                    if (!(a.W & 1)) {             // rows start on 8 bytes: quads 1 .. 6 of a box row
+                        const int quad = ptid & 7, qx = 2 * x0 - 8 + 4 * quad;
+                        if (quad >= 1 && quad < 7) {
+#pragma unroll 8
+                            for (int i = 0; i < HR * NCH * 8 / PT; ++i) {
+                                const int rc = i * (PT / 8) + (ptid >> 3), ch = rc % NCH, row = rc / NCH;
+                                const bool ok = qx >= 0 && qx < sW && c0 + ch < a.C && py + row >= 0 && py + row < sH;
+                                cp_async8(dst + row * (NCH * G::ROWB) + ch * G::ROWB + px_off<T>(4 * quad, ch),
+                                          ok ? img + (size_t)(c0 + ch) * hi_plane + (size_t)(py + row) * sW + qx : img, ok);
+                            }
+                        }
+                    } else if (pair >= 2 && pair < 14) {
 #pragma unroll 8
                         for (int i = 0; i < HR * NCH * 16 / PT; ++i) {
                             const int rc = i * (PT / 16) + (ptid >> 4), ch = rc % NCH, row = rc / NCH;
                             const bool ok = x_ok && c0 + ch < a.C && py + row >= 0 && py + row < sH;
                             const T *src = ok ? img + (size_t)(c0 + ch) * hi_plane + (size_t)(py + row) * sW + px : img;
                             const unsigned at = dst + row * (NCH * G::ROWB) + ch * G::ROWB + px_off<T>(2 * pair, ch);
-                            if constexpr (F32) cp_async8(at, src, ok);
-                            else cp_async4(at, src, ok);
+                            cp_async4(at, src, ok);
                         }
                     }
                     cp_async_arrive(full_addr + 8 * slot);
@@ -385,6 +395,10 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     // rows a tensor map can describe and paired stores: the TMA forms
     const bool ragged = !gath_mma_supported(W, dtype), wide = !F32 && !ragged && wide16_pays(W);
     const char *name = ragged ? "sapa_gath_kernel" : "sapa_gath_mma_kernel";
+    if (F32 && ragged) {
+        set_error("%s: float32 rows have to be of even length", name);
+        return SAPA_ERR_UNSUPPORTED;
+    }
     const Form f = ragged ? Form{ROWS, COLS, G::NCH, NT_RAGGED, G::SMEM_BYTES, 1}
                    : wide ? Form{ROWS, gw16::COLS, gw16::NCH, gw16::NT, gw16::SMEM_BYTES, 1}
                           : Form{ROWS, COLS, G::NCH, NT, G::SMEM_BYTES, CTAS_PER_SM};
@@ -411,9 +425,10 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    const void *kernel = ragged ? reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, true>) : reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, false>);
+    const void *kernel = reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, false>);
     if constexpr (!F32)
-        if (wide) kernel = reinterpret_cast<const void *>(sapa_gath_wide_16_kernel<T>);
+        if (ragged) kernel = reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, true>);
+        else if (wide) kernel = reinterpret_cast<const void *>(sapa_gath_wide_16_kernel<T>);
     int sms = 0;
     if (int e = prepare_launch(kernel, f.smem, name, sms)) return e;
     const long long resident = (long long)f.ctas_per_sm * sms;
@@ -425,12 +440,12 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
     if constexpr (!F32)
-        if (wide) {
-            sapa_gath_wide_16_kernel<T><<<grid, f.threads, f.smem, st>>>(xmap, bmap, a);
+        if (ragged || wide) {
+            if (ragged) sapa_gath_mma_kernel<T, true><<<grid, f.threads, f.smem, st>>>(xmap, a);
+            else sapa_gath_wide_16_kernel<T><<<grid, f.threads, f.smem, st>>>(xmap, bmap, a);
             return check_launch(name);
         }
-    if (ragged) sapa_gath_mma_kernel<T, true><<<grid, f.threads, f.smem, st>>>(xmap, a);
-    else sapa_gath_mma_kernel<T, false><<<grid, f.threads, f.smem, st>>>(xmap, a);
+    sapa_gath_mma_kernel<T, false><<<grid, f.threads, f.smem, st>>>(xmap, a);
     return check_launch(name);
 }
 

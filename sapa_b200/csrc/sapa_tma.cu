@@ -81,42 +81,12 @@ __device__ __forceinline__ int swz(int col, int channel) { return ((((col >> 2) 
 //              "value" map is the key tensor and the output is grad_query = agg(dS, key).
 // MODE_SIM / MODE_AGG: the logit half / the aggregation half alone (sapa_qk_forward, sapa_av_forward and the halves of
 //              the separate backward ops); the weights of MODE_AGG are read where MODE_BWD reads the attention map.
-// RAGGED: rows that are not multiples of 16 bytes - no tensor maps: RAGGED_PT producer threads copy the boxes element by
-//              element (static tile order), the output leaves from registers; everything behind the ring is the same.
-constexpr int RAGGED_PT = 4 * 32;
-
-// producer threads of the ragged float32 kernel: the columns 2 .. 13 of a key / value box (what a window can reach), and a
-// query box
-template <int NCH>
-__device__ __forceinline__ void ragged_lo_box_f32(unsigned dst, const float *base, int c0, int C, int rows, int W, int y0, int x0, int ptid) {
-    const int col = ptid & 15, x = x0 - 4 + col;
-    const bool x_ok = x >= 0 && x < W;
-    const size_t plane = (size_t)rows * W;
-    if (col < 2 || col > 13) return;
-#pragma unroll
-    for (int i = 0; i < HH * NCH * 16 / RAGGED_PT; ++i) {
-        const int rc = i * (RAGGED_PT / 16) + (ptid >> 4), ch = rc % NCH, row = rc / NCH, y = y0 - 2 + row;
-        const bool ok = x_ok && c0 + ch < C && y >= 0 && y < rows;
-        cp_async4(dst + row * (NCH * ROWB) + ch * ROWB + swz(col, ch), ok ? base + (size_t)(c0 + ch) * plane + (size_t)y * W + x : base, ok);
-    }
-}
-__device__ __forceinline__ void ragged_hi_box_f32(unsigned dst, const float *base, int c0, int C, int H, int W, int y0, int x0, int ptid) {
-    const int pair = ptid & 7, sW = 2 * W;
-    const size_t plane = (size_t)(2 * H) * sW;
-#pragma unroll
-    for (int i = 0; i < 2 * ROWS * F_KCH * 8 / RAGGED_PT; ++i) {
-        const int rc = i * (RAGGED_PT / 8) + (ptid >> 3), ch = rc % F_KCH, row = rc / F_KCH;
-        const bool ok = x0 + pair < W && c0 + ch < C && 2 * y0 + row < 2 * H;
-        cp_async8(dst + row * (F_KCH * ROWB) + ch * ROWB + swz(2 * pair, ch), ok ? base + (size_t)(c0 + ch) * plane + (size_t)(2 * y0 + row) * sW + 2 * (x0 + pair) : base, ok);
-    }
-}
-
-template <int MODE, bool RAGGED>
-__global__ void __launch_bounds__(RAGGED ? NT + RAGGED_PT : NT, RAGGED ? 1 : CTAS_PER_SM)
+template <int MODE>
+__global__ void __launch_bounds__(NT, CTAS_PER_SM)
 sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                           const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap omap, const Args a) {
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ __align__(8) unsigned long long full_bar[2 * NSTAGE];       // full, then (ragged form only) empty
+    __shared__ __align__(8) unsigned long long full_bar[NSTAGE];
     // the swizzle pattern is a function of the absolute shared-memory address: align the ring to 1024 bytes
     const unsigned ring_addr = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u;
     const unsigned bar_addr = (unsigned)__cvta_generic_to_shared(full_bar);
@@ -136,42 +106,10 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < NSTAGE; ++i) {
-            mbar_init(bar_addr + 8 * i, RAGGED ? RAGGED_PT : 1);
-            if (RAGGED) mbar_init(bar_addr + 8 * (NSTAGE + i), 1);
-        }
+        for (int i = 0; i < NSTAGE; ++i) mbar_init(bar_addr + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
-
-    if constexpr (RAGGED) {
-        if (tid >= NT) {
-            const int ptid = tid - NT;
-            const float *qp = static_cast<const float *>(a.q), *kp = static_cast<const float *>(a.k), *vp = static_cast<const float *>(a.v);
-            const size_t lo_plane = (size_t)a.rows * a.W;
-            int slot = 0, phase = 0;
-            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-                int t_ = tile / a.csplit;
-                const int vb = tile % a.csplit * nv;
-                const int x0 = (t_ % a.tiles_x) * COLS; t_ /= a.tiles_x;
-                const int y0 = a.y_begin + (t_ % a.tiles_y) * ROWS, n = t_ / a.tiles_y;
-                for (int it = 0; it < total; ++it) {
-                    if (!mbar_wait_bounded(bar_addr + 8 * (NSTAGE + slot), phase ^ 1)) { atomicExch(&g_wait_timeout, 1); return; }
-                    const unsigned dst = ring_addr + slot * SLOT_BYTES;
-                    if (it < nk) {
-                        ragged_lo_box_f32<F_KCH>(dst, kp + (size_t)n * a.d * lo_plane, it * F_KCH, a.d, a.rows, a.W, a.ytop0 + y0, x0, ptid);
-                        ragged_hi_box_f32(dst + K_BYTES, qp + (size_t)n * a.d * hi_plane, it * F_KCH, a.d, a.H, a.W, y0, x0, ptid);
-                    } else {
-                        ragged_lo_box_f32<F_VCH>(dst, vp + (size_t)n * a.C * lo_plane, (vb + it - nk) * F_VCH, a.C, a.rows, a.W, a.ytop0 + y0, x0, ptid);
-                    }
-                    cp_async_arrive(bar_addr + 8 * slot);
-                    if (++slot == NSTAGE) { slot = 0; phase ^= 1; }
-                }
-            }
-            asm volatile("cp.async.wait_all;\n" ::: "memory");      // no copy outlives the thread
-            return;
-        }
-    }
 
     // Stages are issued in stream order (stage gs goes to slot gs % NSTAGE) by thread 0 only.  The producer keeps its
     // position incrementally: per stage it costs a handful of instructions, which matters because the other seven
@@ -203,7 +141,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         if (++p_it == total) { p_it = 0; ++p_ti; }
         p_slot = (p_slot + 1) % NSTAGE;
     };
-    if (!RAGGED && tid == 0) {
+    if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < NSTAGE - 1; ++i) issue(i);
     }
@@ -249,8 +187,8 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
     int gs = 0;
     for (int ti = 0;; ++ti) {
     // written by thread 0 at least one barrier earlier (tile 0 is known to everybody)
-    int tile = RAGGED ? (int)blockIdx.x + ti * (int)gridDim.x : ti == 0 ? (int)blockIdx.x : tile_ids[ti & 3];
-    if (tile < 0 || (RAGGED && tile >= ntiles)) break;
+    int tile = ti == 0 ? (int)blockIdx.x : tile_ids[ti & 3];
+    if (tile < 0) break;
     const int vb = tile % a.csplit * nv; tile /= a.csplit;
     const int bx = tile % a.tiles_x; tile /= a.tiles_x;
     const int by = tile % a.tiles_y; tile /= a.tiles_y;
@@ -277,13 +215,8 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 
     for (int it = 0; it < total; ++it, ++gs) {
         // everyone is done with the slot that is refilled next and has written its output fragment
-        if constexpr (RAGGED) {
-            asm volatile("bar.sync 1, %0;\n" ::"n"(NT) : "memory");
-            if (tid == 0 && gs > 0) mbar_arrive(bar_addr + 8 * (NSTAGE + (gs - 1) % NSTAGE));
-        } else {
-            __syncthreads();
-        }
-        if (!RAGGED && tid == 0) {
+        __syncthreads();
+        if (tid == 0) {
             if (it > nk) {   // the previous stage was a value stage: its output tile is complete in shared memory
                 tma_store_4d(&omap, obuf_addr + ((it - nk - 1) & 1) * O_BYTES, 2 * x0, (vb + it - nk - 1) * F_VCH, 2 * y0, n);
                 asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
@@ -441,21 +374,6 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 #pragma unroll
                     for (int r = 0; r < 2; ++r) mma_tf32(acc[b][r], ah[b], tf32_lo(phi[r][dy][0]), tf32_lo(phi[r][dy][1]));
             }
-            if constexpr (RAGGED) {       // pixel pairs straight to memory (rows start on 8 bytes)
-                if (y < a.y_end && x0 + 4 * h + t < a.W) {
-                    float *o = static_cast<float *>(a.out) + ((size_t)n * a.C + (vb + it - nk) * F_VCH + g) * hi_plane + (size_t)(2 * y) * sW + 2 * (x0 + 4 * h + t);
-#pragma unroll
-                    for (int b = 0; b < F_VCH / 16; ++b)
-#pragma unroll
-                        for (int half = 0; half < 2; ++half)
-                            if ((vb + it - nk) * F_VCH + 16 * b + 8 * half + g < a.C)
-#pragma unroll
-                                for (int r = 0; r < 2; ++r)
-                                    __stcs(reinterpret_cast<float2 *>(o + (size_t)(16 * b + 8 * half) * hi_plane + (size_t)r * sW),
-                                           make_float2(acc[b][r][2 * half], acc[b][r][2 * half + 1]));
-                }
-                continue;
-            }
             // D fragment: d0,d1 = Out[ch g][px 2t, 2t+1], d2,d3 = Out[ch g+8][px 2t, 2t+1] -> staging buffer laid out
             // as the output box [hi row][channel][16 hi cols] (64-byte swizzle), stored by TMA after the next barrier
             {
@@ -474,14 +392,14 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         }
     }
     // the tile's last output block
-    if (!RAGGED) __syncthreads();
-    if (!RAGGED && tid == 0 && MODE != MODE_SIM) {
+    __syncthreads();
+    if (tid == 0 && MODE != MODE_SIM) {
         tma_store_4d(&omap, obuf_addr + ((nv - 1) & 1) * O_BYTES, 2 * x0, (vb + nv - 1) * F_VCH, 2 * y0, n);
         asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
     }
     }
-    if (!RAGGED && tid == 0) {
+    if (tid == 0) {
         asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");   // all output tiles are written
         if (atomicAdd(&g_ctas_done[a.sched_slot], 1u) == gridDim.x - 1) {   // last CTA out: reset the scheduler slot
             g_next_tile[a.sched_slot] = 0u;
@@ -575,9 +493,21 @@ struct OddBox {
 };
 template <typename T>
 __device__ __forceinline__ void ragged_hi_box_16(unsigned dst, const T *base, int c0, int C, int H, int W, int y0, int x0, int ptid) {
-    const int pair = ptid & 7, sW = 2 * W;
-    const bool x_ok = x0 + pair < W;
+    const int sW = 2 * W;
     const size_t plane = (size_t)(2 * H) * sW;
+    if (!(W & 1)) {               // high-res rows start on 8 bytes: four pixels per copy
+        const int quad = ptid & 3;
+#pragma unroll
+        for (int i = 0; i < 2 * ROWS * 32 * 4 / h16::PT; ++i) {
+            const int rc = i * (h16::PT / 4) + (ptid >> 2), ch = rc & 31, row = rc >> 5;
+            const bool ok = x0 + 2 * quad < W && c0 + ch < C && 2 * y0 + row < 2 * H;
+            cp_async8(dst + row * (32 * h16::QROW) + ch * h16::QROW + ((((quad >> 1) ^ (ch >> 2)) & 1) << 4) + 8 * (quad & 1),
+                      ok ? base + (size_t)(c0 + ch) * plane + (size_t)(2 * y0 + row) * sW + 2 * x0 + 4 * quad : base, ok);
+        }
+        return;
+    }
+    const int pair = ptid & 7;
+    const bool x_ok = x0 + pair < W;
 #pragma unroll
     for (int i = 0; i < 2 * ROWS * 32 * 8 / h16::PT; ++i) {
         const int rc = i * (h16::PT / 8) + (ptid >> 3), ch = rc & 31, row = rc >> 5;
@@ -777,6 +707,17 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 
     float s[2][5][4];             // logits, then probabilities: [group][dy][(lo,px0) (lo,px1) (hi,px0) (hi,px1)]
     unsigned pb[2][5][2];         // B fragments of the aggregation
+    // Rows of any length: the FP32-pipe kernels that served them kept the weights in float32, so here they are two terms (pb + pl, 16
+    // bits of a bfloat16 pair, 22 of a float16 one).  Logit gradients have no fixed range: each pixel's are scaled by a power of
+    // two to [1, 2) before they are split, its outputs are scaled back.
+    constexpr bool TWO = RAGGED && (MODE == MODE_FWD || MODE == MODE_BWD);
+    unsigned pl[TWO ? 2 : 1][5][2];
+    float back[2][2] = {{1.f, 1.f}, {1.f, 1.f}};
+    const auto two_terms = [&](float x, float y, unsigned &hi, unsigned &lo) {
+        hi = pack_pair(T(), x, y);
+        const float2 f = unpack_pair(T(), hi);
+        lo = pack_pair(T(), x - f.x, y - f.y);
+    };
 
     int slot = 0, phase = 0, it = 0, ti = 0, gs = 0;
     int n = 0, x0 = 0, y = 0;
@@ -879,6 +820,29 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                         if (pix && ok_lo[p]) wp[(size_t)(dy * 5 + dx_lo[p]) * plane_w + 4 * p] = pb[p][dy][0];
                         if (pix && ok_hi[p]) wp[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + 4 * p] = pb[p][dy][1];
                     }
+                    if constexpr (TWO) {
+                        float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+                        for (int dy = 0; dy < 5; ++dy) {
+                            av[dy][0] *= s[p][dy][0] - d0; av[dy][1] *= s[p][dy][1] - d1;
+                            av[dy][2] *= s[p][dy][2] - d0; av[dy][3] *= s[p][dy][3] - d1;
+                            m0 = fmaxf(m0, fmaxf(fabsf(av[dy][0]), fabsf(av[dy][2])));
+                            m1 = fmaxf(m1, fmaxf(fabsf(av[dy][1]), fabsf(av[dy][3])));
+                        }
+#pragma unroll
+                        for (int sh = 4; sh < 32; sh <<= 1) {
+                            m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, sh));
+                            m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, sh));
+                        }
+                        const int e0 = min(max(254 - (int)(__float_as_uint(m0) >> 23), 1), 253), e1 = min(max(254 - (int)(__float_as_uint(m1) >> 23), 1), 253);
+                        const float f0 = __uint_as_float(e0 << 23), f1 = __uint_as_float(e1 << 23);
+                        back[p][0] = __uint_as_float((254 - e0) << 23); back[p][1] = __uint_as_float((254 - e1) << 23);
+#pragma unroll
+                        for (int dy = 0; dy < 5; ++dy) {
+                            two_terms(av[dy][0] * f0, av[dy][1] * f1, pb[p][dy][0], pl[p][dy][0]);
+                            two_terms(av[dy][2] * f0, av[dy][3] * f1, pb[p][dy][1], pl[p][dy][1]);
+                        }
+                    }
                 }
             }
             if (it == nk - 1 && MODE == MODE_FWD) {
@@ -916,8 +880,13 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                     const float i0 = __frcp_rn(z0), i1 = __frcp_rn(z1);
 #pragma unroll
                     for (int dy = 0; dy < 5; ++dy) {
-                        pb[p][dy][0] = pack_pair(T(), s[p][dy][0] * i0, s[p][dy][1] * i1);
-                        pb[p][dy][1] = pack_pair(T(), s[p][dy][2] * i0, s[p][dy][3] * i1);
+                        if constexpr (TWO) {
+                            two_terms(s[p][dy][0] * i0, s[p][dy][1] * i1, pb[p][dy][0], pl[p][dy][0]);
+                            two_terms(s[p][dy][2] * i0, s[p][dy][3] * i1, pb[p][dy][1], pl[p][dy][1]);
+                        } else {
+                            pb[p][dy][0] = pack_pair(T(), s[p][dy][0] * i0, s[p][dy][1] * i1);
+                            pb[p][dy][1] = pack_pair(T(), s[p][dy][2] * i0, s[p][dy][3] * i1);
+                        }
                     }
                 }
             }
@@ -968,6 +937,10 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                     for (int dy = 0; dy < 5; ++dy) {
                         pb[p][dy][0] = movmatrix_trans(pb[p][dy][0]);
                         pb[p][dy][1] = movmatrix_trans(pb[p][dy][1]);
+                        if constexpr (TWO) {
+                            pl[p][dy][0] = movmatrix_trans(pl[p][dy][0]);
+                            pl[p][dy][1] = movmatrix_trans(pl[p][dy][1]);
+                        }
                     }
             }
         } else {
@@ -989,6 +962,10 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                     ldsm_x2(vc, vc_addr + dy * (VCH * KROW) + b * 16 * KROW);
                     mma_h16<T>(acc[b][0], va[0], va[1], va[2], va[3], pb[0][dy][0], pb[0][dy][1]);
                     mma_h16<T>(acc[b][1], va[2], va[3], vc[0], vc[1], pb[1][dy][0], pb[1][dy][1]);
+                    if constexpr (TWO) {
+                        mma_h16<T>(acc[b][0], va[0], va[1], va[2], va[3], pl[0][dy][0], pl[0][dy][1]);
+                        mma_h16<T>(acc[b][1], va[2], va[3], vc[0], vc[1], pl[1][dy][0], pl[1][dy][1]);
+                    }
                 }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty_addr + 8 * slot);
@@ -1001,6 +978,12 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 const bool odd = t & 1;
 #pragma unroll
                 for (int j = 0; j < VCH / 8; ++j) {       // channel g + 8j: block j/2, half j%2
+                    if constexpr (TWO && MODE == MODE_BWD)
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) {
+                            acc[j >> 1][p][2 * (j & 1)] *= back[p][0];
+                            acc[j >> 1][p][2 * (j & 1) + 1] *= back[p][1];
+                        }
                     const unsigned v0 = pack_pair(T(), acc[j >> 1][0][2 * (j & 1)], acc[j >> 1][0][2 * (j & 1) + 1]);
                     const unsigned v1 = pack_pair(T(), acc[j >> 1][1][2 * (j & 1)], acc[j >> 1][1][2 * (j & 1) + 1]);
                     if constexpr (RAGGED) {       // rows on 4-byte boundaries, columns to be checked: one pair per store
@@ -1105,6 +1088,10 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     const bool use_qk = mode != MODE_AGG, use_v = mode != MODE_SIM;
     CUtensorMap qmap{}, kmap{}, vmap{}, omap{};
     const bool ragged = !fused_tma_supported(W, dtype);
+    if (ragged && dtype == SAPA_F32) {
+        set_error("sapa_tma_fused: float32 rows have to be multiples of 16 bytes");
+        return SAPA_ERR_UNSUPPORTED;
+    }
     const bool wide = !ragged && dtype != SAPA_F32 && wide16_pays(W, ceil_div(y_end - y_begin, ROWS), B);
     bool ok = true;
     if (ragged) {
@@ -1156,8 +1143,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     const char *nr = names_ragged[mode & 3];
 #define SAPA_TMA_LAUNCH32(M)                                                                                                             \
     case M:                                                                                                                              \
-        return ragged ? launch_persistent(sapa_tma_fused_f32_kernel<M, true>, nr, NT + RAGGED_PT, smem32, 1, M != MODE_BWD, a, st, qmap, kmap, vmap, omap) \
-                      : launch_persistent(sapa_tma_fused_f32_kernel<M, false>, n32, NT, smem32, CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap, omap);
+        return launch_persistent(sapa_tma_fused_f32_kernel<M>, n32, NT, smem32, CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap, omap);
 #define SAPA_TMA_LAUNCH16(T, M)                                                                                                          \
     case M:                                                                                                                              \
         return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, nr, h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
