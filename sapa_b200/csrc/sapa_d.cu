@@ -428,21 +428,20 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
     }
 }
 
-// Adds a_p * bilinear(value_c) of the listed outlier points to the output.  Eight threads per listed pixel: each takes
-// every eighth channel of the group, four channels at a time in registers, walks the pixel's outlier points for them
+// Adds a_p * bilinear(value_c) of the listed outlier points to the output.  SUB threads per listed pixel: each takes
+// every SUB-th channel of the group, CH channels at a time in registers, walks the pixel's outlier points for them
 // and then updates the output elements once, read-modify-write without atomics (a listed pixel of a group belongs to
 // exactly one thread group, and the aggregation kernel that wrote the output has finished): the forward pass is
 // deterministic and a 16-bit output is rounded once more, not once per point.
-template <typename T>
-__global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const unsigned int *__restrict__ tap_count,
-                                      const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ out,
-                                      int C, int H, int W, int P, int G, int rows, int ytop) {
-    constexpr int CH = 4;
+template <int SUB, int CH, typename T>
+__device__ __forceinline__ void outlier_pixels(const OutlierTap *__restrict__ taps, unsigned int n, const T *__restrict__ value,
+                                               const T *__restrict__ offset, T *__restrict__ out, int C, int H, int W, int P, int G, int rows, int ytop) {
     const int sW = 2 * W, gc = C / G;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)rows * W;
-    const unsigned int n = *tap_count;
-    const int sub = threadIdx.x & 7;
-    for (unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; e < n; e += (gridDim.x * blockDim.x) >> 3) {
+    const int sub = threadIdx.x % SUB;
+    // entries of a short list are spread over the blocks, those of a long one stay next to their neighbours
+    const unsigned int first = SUB == 32 ? threadIdx.x / SUB * gridDim.x + blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) / SUB;
+    for (unsigned int e = first; e < n; e += gridDim.x * blockDim.x / SUB) {
         const OutlierTap *t = taps + e;
         const unsigned int idx = __ldg(&t->idx), mask = __ldg(&t->mask);
         const size_t bg = idx / hi, pix = idx % hi;
@@ -450,10 +449,13 @@ __global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const
         const T *offp = offset + bg * P * 2 * hi + pix;
         const T *vp = value + bg * gc * lo;
         T *op = out + bg * gc * hi + pix;
-        for (int c0 = sub; c0 < gc; c0 += 8 * CH) {
-            float acc[CH];
+        for (int c0 = sub; c0 < gc; c0 += SUB * CH) {
+            float acc[CH], old[CH];
 #pragma unroll
-            for (int j = 0; j < CH; ++j) acc[j] = 0.f;
+            for (int j = 0; j < CH; ++j) {
+                acc[j] = 0.f;
+                old[j] = c0 + SUB * j < gc ? to_acc(op[(size_t)(c0 + SUB * j) * hi]) : 0.f;
+            }
             for (unsigned int m = mask; m != 0; m &= m - 1) {
                 const int p = __ffs(m) - 1;
                 const float w = float(px) + to_acc(__ldg(offp + (size_t)(2 * p) * hi));
@@ -463,17 +465,28 @@ __global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const
                 bl.setup(h, w, rows, W);
 #pragma unroll
                 for (int j = 0; j < CH; ++j) {
-                    const int c = c0 + 8 * j;
+                    const int c = c0 + SUB * j;
                     if (c < gc) acc[j] += a * bl.sample(vp + (size_t)c * lo);
                 }
             }
 #pragma unroll
             for (int j = 0; j < CH; ++j) {
-                const int c = c0 + 8 * j;
-                if (c < gc) op[(size_t)c * hi] = from_acc<T>(to_acc(op[(size_t)c * hi]) + acc[j]);
+                const int c = c0 + SUB * j;
+                if (c < gc) op[(size_t)c * hi] = from_acc<T>(old[j] + acc[j]);
             }
         }
     }
+}
+// A short list (learned offsets: a few hundred entries) is a chain of dependent loads per entry: a warp per entry and every channel
+// in flight at once (20 -> OUTFWD us for 600 pixels of 64 channels).  A long one is bound by its sectors, which neighbouring pixels
+// share when eight threads serve each.
+template <typename T>
+__global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const unsigned int *__restrict__ tap_count,
+                                      const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ out,
+                                      int C, int H, int W, int P, int G, int rows, int ytop) {
+    const unsigned int n = *tap_count;
+    if (n <= gridDim.x * (blockDim.x / 32)) outlier_pixels<32, 2>(taps, n, value, offset, out, C, H, W, P, G, rows, ytop);
+    else outlier_pixels<8, 4>(taps, n, value, offset, out, C, H, W, P, G, rows, ytop);
 }
 
 // ---------------------------------------------------------------------------------- backward, dense-window path
@@ -640,23 +653,24 @@ deform_window_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ v
     }
 }
 
-// Gradients of the listed outlier points: eight threads per point share its sampling set-up and take every eighth
+// Gradients of the listed outlier points: SUB threads per point share its sampling set-up and take every SUB-th
 // channel; dQ, dKey and dV are added to what the SAPA-B kernels wrote (atomics), the point's offset gradient is written.
 // TA = type of the scatter targets grad_key / grad_value: T itself in float32; float for 16-bit tensors, where they are
 // zeroed side buffers that deform_add_scatter_kernel folds into the 16-bit gradients afterwards (a 16-bit atomic per
 // corner and channel was 2x slower than the whole float32 pass and rounds at every addition).
-template <typename T, typename TA>
-__global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count,
+template <int SUB, typename T, typename TA>
+__device__ __forceinline__ void outlier_points_bwd(const OutlierGrad *__restrict__ taps, unsigned int n,
                                           const T *__restrict__ grad_out, const T *__restrict__ query, const T *__restrict__ key,
                                           const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ grad_query,
                                           TA *__restrict__ grad_key, TA *__restrict__ grad_value, T *__restrict__ grad_offset,
                                           int Cq, int C, int H, int W, int P, int G) {
     const int sW = 2 * W, gq = Cq / G, gc = C / G;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)H * W;
-    const unsigned int n = *tap_count;
-    const int lane = threadIdx.x & 31, sub = lane & 7;
-    const unsigned int group_mask = 0xffu << (lane & ~7);
-    for (unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; e < n; e += (gridDim.x * blockDim.x) >> 3) {
+    const int lane = threadIdx.x & 31, sub = lane % SUB;
+    const unsigned int group_mask = SUB == 32 ? 0xffffffffu : 0xffu << (lane & ~7);
+    // entries of a short list are spread over the blocks, those of a long one stay next to their neighbours
+    const unsigned int first = SUB == 32 ? threadIdx.x / SUB * gridDim.x + blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) / SUB;
+    for (unsigned int e = first; e < n; e += gridDim.x * blockDim.x / SUB) {
         const OutlierGrad t = taps[e];
         const size_t pix = t.pix;
         const int px = (int)(pix % sW) >> 1, py = (int)(pix / sW) >> 1;
@@ -667,7 +681,7 @@ __global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, 
         const float hh = 1.f - bl.lh, hw = 1.f - bl.lw;
         const size_t bg = t.k / (unsigned int)P;
         float g_w = 0.f, g_h = 0.f;
-        for (int c = sub; c < gc && grad_value != nullptr; c += 8) {      // aggregation: dV scatter and its offset gradient
+        for (int c = sub; c < gc && grad_value != nullptr; c += SUB) {      // aggregation: dV scatter and its offset gradient
             float v00, v01, v10, v11;
             bl.corners(value + (bg * gc + c) * lo, v00, v01, v10, v11);
             const float tw = to_acc(grad_out[(bg * gc + c) * hi + pix]) * t.a;
@@ -679,7 +693,7 @@ __global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, 
             g_w += (-hh * v00 + hh * v01 - bl.lh * v10 + bl.lh * v11) * tw;
             g_h += (-hw * v00 - bl.lw * v01 + hw * v10 + bl.lw * v11) * tw;
         }
-        for (int c = sub; c < gq && grad_query != nullptr; c += 8) {      // similarity: dQ, dKey scatter and its offset gradient
+        for (int c = sub; c < gq && grad_query != nullptr; c += SUB) {      // similarity: dQ, dKey scatter and its offset gradient
             float v00, v01, v10, v11;
             bl.corners(key + (bg * gq + c) * lo, v00, v01, v10, v11);
             atomicAdd(grad_query + (bg * gq + c) * hi + pix, from_acc<T>(t.ds * (bl.w00 * v00 + bl.w01 * v01 + bl.w10 * v10 + bl.w11 * v11)));
@@ -693,7 +707,7 @@ __global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, 
             g_h += (-hw * v00 - bl.lw * v01 + hw * v10 + bl.lw * v11) * tw;
         }
 #pragma unroll
-        for (int sh = 1; sh < 8; sh <<= 1) {
+        for (int sh = 1; sh < SUB; sh <<= 1) {
             g_w += __shfl_xor_sync(group_mask, g_w, sh);
             g_h += __shfl_xor_sync(group_mask, g_h, sh);
         }
@@ -704,17 +718,76 @@ __global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, 
     }
 }
 
-// dst[i] += side[i] for the 16-bit gradients whose outlier contributions were collected in float32; nothing to do (and
-// nothing read) when the list was empty.
+template <typename T, typename TA>      // a warp per entry of a short list, as in the forward pass
+__global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count,
+                                          const T *__restrict__ grad_out, const T *__restrict__ query, const T *__restrict__ key,
+                                          const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ grad_query,
+                                          TA *__restrict__ grad_key, TA *__restrict__ grad_value, T *__restrict__ grad_offset,
+                                          int Cq, int C, int H, int W, int P, int G) {
+    const unsigned int n = *tap_count;
+    if (n <= gridDim.x * (blockDim.x / 32))
+        outlier_points_bwd<32>(taps, n, grad_out, query, key, value, offset, grad_query, grad_key, grad_value, grad_offset, Cq, C, H, W, P, G);
+    else
+        outlier_points_bwd<8>(taps, n, grad_out, query, key, value, offset, grad_query, grad_key, grad_value, grad_offset, Cq, C, H, W, P, G);
+}
+
+// The float32 side buffers of the 16-bit gradients: zeroed before the list kernel, added to the gradients after it (one rounding per
+// element).  A short list touches a few thousand of the buffers' cells: those alone are zeroed, and taken back by an exchange that
+// gives each cell's whole sum to one of the points that share it.  A long list goes over the buffers (42 MB, 8 + 25 us, at 8 images
+// of 320 channels, 64 x 64; the short form: SHORT us).
+struct Scatter { float *key, *value; size_t n_key, n_value; int gq, gc; };      // the value buffer lies behind the key buffer
+
+// f(cell index of the key buffer or of the value buffer, which) for the four corners of every listed point and all channels of its
+// group; a warp per corner
+template <typename T, typename F>
+__device__ __forceinline__ void for_scattered(const OutlierGrad *__restrict__ taps, unsigned int n, const T *__restrict__ offset, const Scatter &sc, int H, int W,
+                                              int P, F f) {
+    const int sW = 2 * W;
+    const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)H * W;
+    for (unsigned int e = threadIdx.x / 32 * gridDim.x + blockIdx.x; e < 4 * n; e += gridDim.x * (blockDim.x / 32)) {
+        const OutlierGrad t = taps[e >> 2];
+        const size_t pix = t.pix, bg = t.k / (unsigned int)P;
+        const int px = (int)(pix % sW) >> 1, py = (int)(pix / sW) >> 1;
+        const float w = float(px) + to_acc(__ldg(offset + (size_t)t.k * 2 * hi + pix)), h = float(py) + to_acc(__ldg(offset + (size_t)t.k * 2 * hi + hi + pix));
+        Bilinear<float> bl;
+        bl.setup(h, w, H, W);
+        const int at = (e & 2) != 0 ? ((e & 1) != 0 ? bl.i11 : bl.i10) : (e & 1) != 0 ? bl.i01 : bl.i00;
+        if (at < 0) continue;
+        for (int c = threadIdx.x & 31; c < sc.gq + sc.gc; c += 32) {
+            const bool key = c < sc.gq;
+            f((key ? bg * sc.gq + c : bg * sc.gc + (c - sc.gq)) * lo + at, key);
+        }
+    }
+}
+
 template <typename T>
-__global__ void deform_add_scatter_kernel(const unsigned int *__restrict__ tap_count, T *__restrict__ dst_a,
-                                          const float *__restrict__ side_a, size_t n_a, T *__restrict__ dst_b,
-                                          const float *__restrict__ side_b, size_t n_b) {
-    if (*tap_count == 0) return;
+__global__ void deform_zero_scatter_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count, const T *__restrict__ offset,
+                                           const Scatter sc, int H, int W, int P) {
+    const unsigned int n = *tap_count;
+    if (n <= gridDim.x * (blockDim.x / 32)) {
+        for_scattered(taps, n, offset, sc, H, W, P, [&](size_t i, bool key) { (key ? sc.key : sc.value)[i] = 0.f; });
+        return;
+    }
+    float *base = sc.n_key != 0 ? sc.key : sc.value;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < sc.n_key + sc.n_value; i += (size_t)gridDim.x * blockDim.x) base[i] = 0.f;
+}
+
+template <typename T>
+__global__ void deform_add_scatter_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count, const T *__restrict__ offset,
+                                          const Scatter sc, T *__restrict__ grad_key, T *__restrict__ grad_value, int H, int W, int P) {
+    const unsigned int n = *tap_count;
+    if (n <= gridDim.x * (blockDim.x / 32)) {
+        for_scattered(taps, n, offset, sc, H, W, P, [&](size_t i, bool key) {
+            const float v = atomicExch((key ? sc.key : sc.value) + i, 0.f);
+            T *dst = (key ? grad_key : grad_value) + i;
+            if (v != 0.f) *dst = from_acc<T>(to_acc(*dst) + v);
+        });
+        return;
+    }
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_a + n_b; i += stride) {
-        if (i < n_a) dst_a[i] = from_acc<T>(to_acc(dst_a[i]) + side_a[i]);
-        else dst_b[i - n_a] = from_acc<T>(to_acc(dst_b[i - n_a]) + side_b[i - n_a]);
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < sc.n_key + sc.n_value; i += stride) {
+        if (i < sc.n_key) grad_key[i] = from_acc<T>(to_acc(grad_key[i]) + sc.key[i]);
+        else grad_value[i - sc.n_key] = from_acc<T>(to_acc(grad_value[i - sc.n_key]) + sc.value[i - sc.n_key]);
     }
 }
 
@@ -1244,15 +1317,17 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     }
     const size_t n_k = (size_t)B * Cq * H * W, n_v = (size_t)B * C * H * W;
     float *side_k = reinterpret_cast<float *>(static_cast<char *>(workspace) + side_off), *side_v = side_k + n_k;
-    if (int e = memset_async(side_k, (n_k + n_v) * sizeof(float), st, fn)) return e;
+    const Scatter sc{side_k, side_v, n_k, n_v, Cq / G, C / G};
     return SAPA_DISPATCH_FAST(dtype, [&] {
+        deform_zero_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
+        if (int e = check_launch("deform_zero_scatter_kernel")) return e;
         deform_outlier_bwd_kernel<scalar_t, float><<<148 * 8, 256, 0, st>>>(
             taps, tap_count, static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(query),
             static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
             static_cast<scalar_t *>(grad_query), side_k, side_v, static_cast<scalar_t *>(grad_offset), Cq, C, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
-        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(tap_count, static_cast<scalar_t *>(grad_key), side_k, n_k,
-                                                                    static_cast<scalar_t *>(grad_value), side_v, n_v);
+        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(grad_key),
+                                                                     static_cast<scalar_t *>(grad_value), H, W, P);
         return check_launch("deform_add_scatter_kernel");
     });
 }
@@ -1315,14 +1390,16 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     }
     const size_t n_v = (size_t)B * C * H * W;
     float *side_v = reinterpret_cast<float *>(static_cast<char *>(workspace) + side_off);
-    if (int e = memset_async(side_v, n_v * sizeof(float), st, fn)) return e;
+    const Scatter sc{nullptr, side_v, 0, n_v, 0, C / G};
     return SAPA_DISPATCH_FAST(dtype, [&] {
+        deform_zero_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
+        if (int e = check_launch("deform_zero_scatter_kernel")) return e;
         deform_outlier_bwd_kernel<scalar_t, float><<<148 * 8, 256, 0, st>>>(
             taps, tap_count, static_cast<const scalar_t *>(grad_out), nullptr, nullptr, static_cast<const scalar_t *>(value),
             static_cast<const scalar_t *>(offset), nullptr, nullptr, side_v, static_cast<scalar_t *>(grad_offset), C, C, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
-        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(tap_count, static_cast<scalar_t *>(grad_value), side_v, n_v,
-                                                                    static_cast<scalar_t *>(nullptr), nullptr, 0);
+        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(nullptr),
+                                                                     static_cast<scalar_t *>(grad_value), H, W, P);
         return check_launch("deform_add_scatter_kernel");
     });
 }
@@ -1383,15 +1460,17 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     }
     const size_t n_k = (size_t)B * Cq * H * W;
     float *side_k = reinterpret_cast<float *>(static_cast<char *>(workspace) + side_off);
-    if (int e = memset_async(side_k, n_k * sizeof(float), st, fn)) return e;
+    const Scatter sc{side_k, nullptr, n_k, 0, Cq / G, 0};
     return SAPA_DISPATCH_FAST(dtype, [&] {
+        deform_zero_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
+        if (int e = check_launch("deform_zero_scatter_kernel")) return e;
         deform_outlier_bwd_kernel<scalar_t, float><<<148 * 8, 256, 0, st>>>(
             taps, tap_count, nullptr, static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), nullptr,
             static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(grad_query), side_k, nullptr,
             static_cast<scalar_t *>(grad_offset), Cq, Cq, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
-        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(tap_count, static_cast<scalar_t *>(grad_key), side_k, n_k,
-                                                                    static_cast<scalar_t *>(nullptr), nullptr, 0);
+        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(grad_key),
+                                                                     static_cast<scalar_t *>(nullptr), H, W, P);
         return check_launch("deform_add_scatter_kernel");
     });
 }
