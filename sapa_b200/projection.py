@@ -1,8 +1,7 @@
 """GroupNorm + 1x1 projection in front of the attention (``self.q(self.norm_y(y))`` / ``self.k(self.norm_x(x))`` of the
 reference modules, sapa_base.py:27-34, sapa_deform.py:35-42) as one tensor-core GEMM: ``sapa_project_forward`` of the C ABI.
 
-Forward only.  The modules use it when no gradient is needed (inference); training keeps torch's GroupNorm and
-convolution, whose backward autograd already provides.
+Forward only; the modules reach this kernel, and the ones that are differentiable, through their native path.
 """
 from __future__ import annotations
 
