@@ -37,3 +37,15 @@ def test_ragged_rows_vs_oracle(oracle, shape, dtype, tol, tol_grad):
         for a, b in zip(grads, want_g):
             assert rel_err(a.double().cpu().numpy(), b) < f * tol_grad
     assert _lib.wait_timeout_flags(DEV) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_odd_rows_keep_float32_weights(dtype):
+    """The attention weights of rows of odd length are two terms: what the output is off by is its own rounding and little more
+    (weights of one 16-bit term would add 0.9 of that rounding)."""
+    import sapa_b200 as sp
+    g = torch.Generator().manual_seed(8)
+    q, k, v = ((torch.randn(*s, generator=g) * f).to(dtype).to(DEV) for s, f in (((2, 32, 40, 82), 0.5), ((2, 32, 20, 41), 0.5), ((2, 64, 20, 41), 1.0)))
+    want = sp.sapa_fused(q.double(), k.double(), v.double(), 5, 2)
+    off = [float((t.double() - want).norm()) for t in (sp.sapa_fused(q, k, v, 5, 2), want.to(dtype))]
+    assert off[0] <= 1.1 * off[1]
