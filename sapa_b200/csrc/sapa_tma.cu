@@ -1055,12 +1055,13 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
                            cudaStream_t st);
 
 // 16-bit: tiles of 4 x 32 instead of 4 x 8 pixels where at least three quarters of their columns are inside the image (below that
-// idle warps cost what the loads save) and nearly every SM gets one.
-// us, 4 x 8 -> 4 x 32: bfloat16 forward 8 x 256 x 64x64 55.7 -> 41.9, 64 x 256 x 128x128 1540 -> 1060, 1 x 256 x 1024x1024 2520 -> 1630;
-// logits 20.8 -> 14.6 and aggregation 50.7 -> 35.1 at 8 x 256 x 64x64.
+// idle warps cost what the loads save) and two thirds of the SMs get one.
+// us, 4 x 8 -> 4 x 32: bfloat16 forward 8 x 256 x 64x64 55.7 -> 40.9, 64 x 256 x 128x128 1540 -> 830, 1 x 256 x 1024x1024 2520 -> 854;
+// float16 forward 4 x 128 x 56x56 (112 tiles) 24.6 -> 19.4; with fewer tiles the 4 x 8 ones use more SMs: module training at
+// 8 x 256 x 32x32 (64 tiles) 252 -> 264, forward of 1 x 64 x 64x64 (32 tiles) 13.2 -> 14.3.
 static bool wide16_pays(int W, int tiles_y, int B) {
     const int tiles_x = ceil_div(W, tma::w16::COLS);
-    return 4 * W >= 3 * tiles_x * tma::w16::COLS && (long long)B * tiles_x * tiles_y >= 128;
+    return 4 * W >= 3 * tiles_x * tma::w16::COLS && (long long)B * tiles_x * tiles_y >= 100;
 }
 
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
