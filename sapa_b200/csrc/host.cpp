@@ -8,6 +8,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include <dlfcn.h>
@@ -60,6 +61,20 @@ void bind(const std::string &path) {
 }
 #define PY_ASSERT(cond) do { if (!(cond)) raise(PyExc_AssertionError, #cond); } while (0)
 
+// The ops mean the same inside torch.autocast as outside (the modules are given its type as an argument): the torch ops on their
+// way must not cast.  softmax and sum come out in float32 there, and the kernels would read that as 16-bit elements.
+struct NoAutocast {
+    c10::impl::ExcludeDispatchKeyGuard off{c10::autocast_dispatch_keyset};
+};
+// an entry point as Python calls it
+template <typename R, typename... A>
+auto native(R (*f)(A...)) {
+    return [f](A... a) -> R {
+        const NoAutocast no_autocast;
+        return f(a...);
+    };
+}
+
 void need_cuda(const Tensor &t) {
     if (!t.is_cuda()) raise(PyExc_NotImplementedError, "");
 }
@@ -77,6 +92,11 @@ void check_tensors(std::initializer_list<Named> named) {
                     first.scalar_type(), " (all tensors of a call share one dtype)");
         TORCH_CHECK(t.device() == first.device(), n.name, " is on ", t.device(), ", expected ", first.device());
     }
+}
+
+// an intermediate that the kernels read as elements of `like`'s type
+void same_type(const Tensor &t, const Tensor &like, const char *name) {
+    TORCH_CHECK(t.scalar_type() == like.scalar_type(), name, " has dtype ", t.scalar_type(), ", expected ", like.scalar_type());
 }
 
 int dtype_code(const Tensor &t) {
@@ -125,24 +145,24 @@ void check_window(int64_t K, int64_t s) {
 
 PYBIND11_MODULE(_host, m) {
     m.def("bind", &bind);
-    m.def("qk", &qk);
-    m.def("av", &av);
-    m.def("sapa_fused", &sapa_fused);
-    m.def("fused_forward_raw", &fused_forward_raw);
-    m.def("qk_backward", &qk_bwd);
-    m.def("av_backward", &av_bwd);
-    m.def("sapa_fused_forward", &fused_forward_with_map);
-    m.def("sapa_fused_backward", &fused_bwd);
-    m.def("deform_qk_backward", &deform_qk_bwd);
-    m.def("deform_av_backward", &deform_av_bwd);
-    m.def("deform_fused_forward", &deform_fused_forward);
-    m.def("deform_fused_backward", &deform_fused_bwd);
-    m.def("deform_qk", &deform_qk);
-    m.def("deform_av", &deform_av);
-    m.def("deform_sapa_fused", &deform_fused);
-    m.def("sapa_module", &sapa_module);
-    m.def("deform_module", &deform_module);
-    m.def("project_module", &project_module);
-    m.def("project", &project);
-    m.def("project_workspace", &project_workspace);
+    m.def("qk", native(&qk));
+    m.def("av", native(&av));
+    m.def("sapa_fused", native(&sapa_fused));
+    m.def("fused_forward_raw", native(&fused_forward_raw));
+    m.def("qk_backward", native(&qk_bwd));
+    m.def("av_backward", native(&av_bwd));
+    m.def("sapa_fused_forward", native(&fused_forward_with_map));
+    m.def("sapa_fused_backward", native(&fused_bwd));
+    m.def("deform_qk_backward", native(&deform_qk_bwd));
+    m.def("deform_av_backward", native(&deform_av_bwd));
+    m.def("deform_fused_forward", native(&deform_fused_forward));
+    m.def("deform_fused_backward", native(&deform_fused_bwd));
+    m.def("deform_qk", native(&deform_qk));
+    m.def("deform_av", native(&deform_av));
+    m.def("deform_sapa_fused", native(&deform_fused));
+    m.def("sapa_module", native(&sapa_module));
+    m.def("deform_module", native(&deform_module));
+    m.def("project_module", native(&project_module));
+    m.def("project", native(&project));
+    m.def("project_workspace", native(&project_workspace));
 }
