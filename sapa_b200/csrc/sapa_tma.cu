@@ -517,6 +517,54 @@ __device__ __forceinline__ void ragged_hi_box_16(unsigned dst, const T *base, in
     }
 }
 
+// The sums of a value stage over the 25 cells of every pixel alone, for a warp with a sum that is not finite.  The matrix product
+// also takes the other cells of its 16 columns, with weights of zero, and 0 * inf would reach pixels whose window has no
+// infinity; of a weight in two terms the second may be negative, and inf - inf would take the place of an infinity inside it.
+// WEIGHTS_POSITIVE: softmax weights, of which none is zero however small its 16-bit terms are.
+template <typename T, bool TWO, bool WEIGHTS_POSITIVE, int N>
+__device__ __forceinline__ void window_sums(float (&acc)[h16::VCH / 16][2][4], const unsigned (&pb)[2][5][2], const unsigned (&pl)[N][5][2], unsigned rows,
+                                            int lane) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        float sum[h16::VCH / 16][4] = {};
+#pragma unroll
+        for (int dy = 0; dy < 5; ++dy)
+#pragma unroll 1
+            for (int dx = 0; dx < 5; ++dx) {
+                // cell k of the 16 lies in the fragment of lane (pixel, (k & 7) / 2), register k / 8, half k & 1
+                const int k = 6 + t - 4 * p + dx;
+                float w[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int src = 4 * (2 * t + j) + ((k & 7) >> 1);
+                    const auto term = [&](unsigned left, unsigned right) {
+                        const unsigned l = __shfl_sync(0xffffffffu, left, src), r = __shfl_sync(0xffffffffu, right, src);
+                        const float2 f = unpack_pair(T(), k & 8 ? r : l);
+                        return k & 1 ? f.y : f.x;
+                    };
+                    w[j] = term(pb[p][dy][0], pb[p][dy][1]);
+                    if constexpr (TWO) {
+                        const float second = term(pl[p][dy][0], pl[p][dy][1]);
+                        if (fabsf(w[j]) <= FLT_MAX) w[j] += second;
+                    }
+                    if (WEIGHTS_POSITIVE && w[j] == 0.f) w[j] = FLT_MIN;
+                }
+                const unsigned cell = rows + (dy * h16::VCH + g) * h16::KROW + 2 * (8 * p + k);
+#pragma unroll
+                for (int i = 0; i < h16::VCH / 8; ++i) {       // channel g + 8i: block i/2, half i%2
+                    const float v = lds_16(T(), cell + 8 * i * h16::KROW);
+                    sum[i >> 1][2 * (i & 1)] = fmaf(w[0], v, sum[i >> 1][2 * (i & 1)]);
+                    sum[i >> 1][2 * (i & 1) + 1] = fmaf(w[1], v, sum[i >> 1][2 * (i & 1) + 1]);
+                }
+            }
+#pragma unroll
+        for (int b = 0; b < h16::VCH / 16; ++b)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[b][p][i] = sum[b][i];
+    }
+}
+
 // modes: see the float32 kernel.  RAGGED: rows that are not multiples of 16 bytes - no tensor maps, four producer warps copy
 // the boxes (static tile order); everything behind the ring is the same.  The FP32-pipe kernels it replaced walked all
 // channels in one CTA per 4 x 32 tile: backward of B=2, C=256, d=32, 25x42 -> 50x84 in bfloat16 438 -> 60 us.  At large
@@ -796,6 +844,12 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
                     const bool pix = row_ok && (p == 0 ? col_ok0 : col_ok1);
+                    if constexpr (RAGGED)          // cells outside the window may hold an infinity: 0 * inf in the sums below
+#pragma unroll
+                        for (int dy = 0; dy < 5; ++dy) {
+                            if (!ok_lo[p]) s[p][dy][0] = s[p][dy][1] = 0.f;
+                            if (!ok_hi[p]) s[p][dy][2] = s[p][dy][3] = 0.f;
+                        }
                     float av[5][4];
                     float d0 = 0.f, d1 = 0.f;
 #pragma unroll
@@ -967,6 +1021,17 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                         mma_h16<T>(acc[b][1], va[2], va[3], vc[0], vc[1], pl[1][dy][0], pl[1][dy][1]);
                     }
                 }
+            if constexpr (RAGGED) {
+                float zero = 0.f;
+#pragma unroll
+                for (int b = 0; b < VCH / 16; ++b)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) zero = fmaf(acc[b][p][i], 0.f, zero);
+                if (__any_sync(0xffffffffu, !(zero == 0.f)))
+                    window_sums<T, TWO, MODE == MODE_FWD>(acc, pb, pl, stage + wrow * (VCH * KROW), lane);
+            }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty_addr + 8 * slot);
             // D fragment of group p: d0,d1 = Out[ch g][px 8p+2t, +1], d2,d3 = Out[ch g+8][same].  Neighbouring lanes swap one

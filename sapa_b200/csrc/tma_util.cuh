@@ -7,6 +7,7 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <cfloat>
 #include <type_traits>
 
 namespace sapa {
@@ -138,6 +139,12 @@ __device__ __forceinline__ void mma_h16(float (&d)[4], unsigned a0, unsigned a1,
 __device__ __forceinline__ float2 unpack_pair(__half, unsigned u) { return __half22float2(*reinterpret_cast<const __half2 *>(&u)); }
 __device__ __forceinline__ float2 unpack_pair(__nv_bfloat16, unsigned u) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u));
+}
+// one 16-bit element from a shared-memory address
+template <typename T> __device__ __forceinline__ float lds_16(T, unsigned addr) {
+    unsigned short u;
+    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(u) : "r"(addr));
+    return unpack_pair(T(), u).x;
 }
 __device__ __forceinline__ float ex2_ftz(float x) {
     float y;

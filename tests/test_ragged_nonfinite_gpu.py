@@ -1,0 +1,85 @@
+"""Rows that are not multiples of 16 bytes, 16-bit types: an infinity or a NaN reaches the pixels (cells) whose window holds it and no
+other, as in sums over the window alone - the tensor-core kernels multiply whole fragments, with weights of zero beside it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+INF, NAN = float("inf"), float("nan")
+
+# (image, channel, row, column, value) of a low-resolution tensor: inside a tile, at its edges and at the image's, two of one window
+SPOTS = [(0, 3, 7, 9, INF), (0, 5, 11, 15, NAN), (1, 0, 0, 0, -INF), (1, 7, 12, 16, INF), (1, 7, 13, 17, INF), (1, 9, 5, 24, INF)]
+
+
+def _rand(*shape, scale=1.0, dtype):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(sum(shape))) * scale).to(dtype).to(DEV)
+
+
+def _planted(t):
+    bad = t.clone()
+    for n, c, y, x, v in SPOTS:
+        bad[n, c, y, x] = v
+    return bad
+
+
+def _near(mask):
+    """Low-resolution cells with a marked one in their 5 x 5 neighbourhood."""
+    return torch.nn.functional.max_pool2d(mask.float(), 5, 1, 2) > 0
+
+
+def _up(mask):
+    return mask.repeat_interleave(2, 2).repeat_interleave(2, 3)
+
+
+def _same_elsewhere(got, clean, reached, dtype):
+    """Where nothing reaches, the result of the clean input (sums in another order, one rounding: two ulps); where something does, no
+    finite number."""
+    assert not torch.isfinite(got[reached]).any()
+    a, b = got[~reached].float(), clean[~reached].float()
+    assert bool(((a - b).abs() <= 2 * torch.finfo(dtype).eps * b.abs() + 1e-6 * float(b.abs().max())).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("W", [25, 42])
+def test_values(W, dtype):
+    import sapa_b200 as sp
+    H, C = 17, 40
+    value = _rand(2, C, H, W, dtype=dtype)
+    bad = _planted(value)
+    attn = (torch.rand(2, 25, 2 * H, 2 * W, generator=torch.Generator().manual_seed(1)) + 0.1).to(dtype).to(DEV)
+    reached = _up(_near(~torch.isfinite(bad)))
+    got = sp.av(attn, bad, 5, 2)
+    _same_elsewhere(got, sp.av(attn, value, 5, 2), reached, dtype)
+    only_inf = _up(_near(bad == INF) & ~_near((bad != bad) | (bad == -INF)))
+    assert bool((got[only_inf] == INF).all())
+    if W % 2:      # the fused kernel of odd rows: weights in two terms of both signs, some below the smallest 16-bit number
+        for scale in (0.5, 3.0):
+            q, k = _rand(2, 8, 2 * H, 2 * W, scale=scale, dtype=dtype), _rand(2, 8, H, W, scale=scale, dtype=dtype)
+            got = sp.sapa_fused(q, k, bad, 5, 2)
+            _same_elsewhere(got, sp.sapa_fused(q, k, value, 5, 2), reached, dtype)
+            assert bool((got[only_inf] == INF).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("W", [25, 42])
+def test_query_gradient(W, dtype):
+    """Stage 1 of the backward: its query gradient, with infinities among the values."""
+    import sapa_b200 as sp
+    H, C = 17, 40
+    q, k, value = (_rand(*s, dtype=dtype) for s in ((2, 8, 2 * H, 2 * W), (2, 8, H, W), (2, C, H, W)))
+    go = _rand(2, C, 2 * H, 2 * W, dtype=dtype)
+    bad = _planted(value)
+    reached = _up(_near(~torch.isfinite(bad))).any(1, keepdim=True).expand(-1, 8, -1, -1)
+
+    def grad(v):
+        t = q.clone().requires_grad_()
+        return torch.autograd.grad(sp.sapa_fused(t, k, v, 5, 2), t, go)[0]
+    _same_elsewhere(grad(bad), grad(value), reached, dtype)
+    # the separate op: logit gradients are given, keys hold the infinities
+    ds = _rand(2, 25, 2 * H, 2 * W, dtype=dtype)
+    key = _rand(2, 40, H, W, dtype=dtype)
+
+    def grad_qk(kk):
+        t = _rand(2, 40, 2 * H, 2 * W, dtype=dtype).requires_grad_()
+        return torch.autograd.grad(sp.qk(t, kk, 5, 2), t, ds)[0]
+    _same_elsewhere(grad_qk(_planted(key)), grad_qk(key), _up(_near(~torch.isfinite(_planted(key)))), dtype)
