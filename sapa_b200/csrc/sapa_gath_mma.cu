@@ -81,6 +81,31 @@ template <typename T> __device__ __forceinline__ int px_off(int px, int ch) {
     else                          return ((((px >> 3) ^ (ch >> 1)) & 3) << 4) | ((px & 7) << 1);             // 64-byte swizzle
 }
 
+// A lane's outputs again, columns x and x + 1 of every eighth channel, as sums over the pixels of a cell's own parents alone; for a
+// lane with a sum that is not finite.  The matrix product also takes the other pixels of its fragments, with weights of zero, and
+// 0 * inf would reach cells that no infinity reaches.
+template <typename T>
+__device__ __forceinline__ void store_cell_sums(const Args &a, int n, int c0, int count, int y, int x0) {
+    const int sW = 2 * a.W;
+    const size_t hi_plane = (size_t)(2 * a.H) * sW;
+#pragma unroll 1
+    for (int i = 0; i < 2 * count; ++i) {
+        const int c = c0 + 8 * (i >> 1), x = x0 + (i & 1);
+        if (c >= a.C || x >= a.W) continue;
+        float s = 0.f;
+#pragma unroll 1
+        for (int cell = 0; cell < 25; ++cell) {       // window cell of the parent that reaches (y, x) through it
+            const int yp = y - a.top + 2 - cell / 5, xp = x + 2 - cell % 5;
+            if (yp < 0 || yp >= a.H || xp < 0 || xp >= a.W) continue;
+            const size_t at = (size_t)(2 * yp) * sW + 2 * xp;
+            const T *w = static_cast<const T *>(a.wt) + ((size_t)n * 25 + cell) * hi_plane + at, *h = static_cast<const T *>(a.hi) + ((size_t)n * a.C + c) * hi_plane + at;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s = fmaf(to_acc(w[(e >> 1) * sW + (e & 1)]), to_acc(h[(e >> 1) * sW + (e & 1)]), s);
+        }
+        static_cast<T *>(a.out)[(((size_t)n * a.C + c) * a.Hout + y) * a.W + x] = from_acc<T>(s);
+    }
+}
+
 // RAGGED (16-bit): high-res rows that are not multiples of 16 bytes (or low-res rows of odd length) - no tensor map, PW producer
 // warps copy the pixel pairs a fragment can reach (box pixels 4 .. 27; a pair is always on its own boundary because
 // high-res rows have an even length), static tile order, single-element stores where W is odd.
@@ -364,6 +389,14 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                             else *reinterpret_cast<unsigned *>(oh) = pack_pair(T(), acc[b][0][2 * half], acc[b][0][2 * half + 1]);
                         }
                 }
+            }
+            if constexpr (RAGGED) {
+                float zero = 0.f;
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) zero = fmaf(acc[b][0][i], 0.f, zero);
+                if (store_ok && !(zero == 0.f)) store_cell_sums<T>(a, n, c0 + g, NB * 2, y, x0 + 2 * t);
             }
         }
         if (++slot == NSTAGE) { slot = 0; phase ^= 1; }

@@ -166,6 +166,7 @@ sapa_gath_wide_16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
                 for (int i = 0; i < 4; ++i) s[i] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
                 if (c0 + g < a.C) *reinterpret_cast<unsigned *>(o) = pack_pair(T(), s[0], s[1]);
                 if (c0 + 8 + g < a.C) *reinterpret_cast<unsigned *>(o + 8 * out_plane) = pack_pair(T(), s[2], s[3]);
+                if (!((s[0] + s[1] + s[2] + s[3]) * 0.f == 0.f)) store_cell_sums<T>(a, n, c0 + g, 2, y, x0 + 2 * t);
             }
         }
     }

@@ -1,5 +1,6 @@
-"""Rows that are not multiples of 16 bytes, 16-bit types: an infinity or a NaN reaches the pixels (cells) whose window holds it and no
-other, as in sums over the window alone - the tensor-core kernels multiply whole fragments, with weights of zero beside it."""
+"""Rows that are not multiples of 16 bytes, and gradients gathered on 4 x 32 tiles, in 16 bits: an infinity or a NaN reaches the pixels
+(cells) whose window holds it and no other, as in sums over the window alone - the tensor-core kernels multiply whole fragments,
+with weights of zero beside it."""
 import pytest
 import torch
 
@@ -83,3 +84,30 @@ def test_query_gradient(W, dtype):
         t = _rand(2, 40, 2 * H, 2 * W, dtype=dtype).requires_grad_()
         return torch.autograd.grad(sp.qk(t, kk, 5, 2), t, ds)[0]
     _same_elsewhere(grad_qk(_planted(key)), grad_qk(key), _up(_near(~torch.isfinite(_planted(key)))), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("W", [25, 42, 64])      # 64: tiles of 4 x 32 cells, whose fragments are wider than a tile's reach
+def test_gathered_gradients(W, dtype):
+    """Value gradient of av and key gradient of qk, with infinities among the high-resolution gradients (queries)."""
+    import sapa_b200 as sp
+    H, C = 17, 40
+    hi = _rand(2, C, 2 * H, 2 * W, dtype=dtype)
+    bad = hi.clone()
+    for n, c, y, x, v in SPOTS:
+        bad[n, c, 2 * y + x % 2, 2 * x + y % 2] = v
+    bad[0, 8, 16, 21] = INF      # a pixel that the next tile's fragments hold beside those that reach it
+    marked = ~torch.isfinite(bad)
+    reached = _near(torch.nn.functional.max_pool2d(marked.float(), 2) > 0)
+    slots = (torch.rand(2, 25, 2 * H, 2 * W, generator=torch.Generator().manual_seed(1)) + 0.1).to(dtype).to(DEV)
+    low = _rand(2, C, H, W, dtype=dtype)
+
+    def value_grad(go):
+        t = low.clone().requires_grad_()
+        return torch.autograd.grad(sp.av(slots, t, 5, 2), t, go)[0]
+
+    def key_grad(q):
+        t = low.clone().requires_grad_()
+        return torch.autograd.grad(sp.qk(q, t, 5, 2), t, slots)[0]
+    for grad in (value_grad, key_grad):
+        _same_elsewhere(grad(bad), grad(hi), reached, dtype)
