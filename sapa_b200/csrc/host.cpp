@@ -66,10 +66,12 @@ void bind(const std::string &path) {
 struct NoAutocast {
     c10::impl::ExcludeDispatchKeyGuard off{c10::autocast_dispatch_keyset};
 };
-// an entry point as Python calls it
+// An entry point as Python calls it: without the interpreter lock, which other threads may need while a launch waits for room in
+// the queue or an allocation for the device.
 template <typename R, typename... A>
 auto native(R (*f)(A...)) {
     return [f](A... a) -> R {
+        const pybind11::gil_scoped_release no_lock;
         const NoAutocast no_autocast;
         return f(a...);
     };
