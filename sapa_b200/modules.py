@@ -11,6 +11,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 from torch.nn.modules.module import _has_any_global_hook
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _lib
 from .deform_functions import deform_av, deform_qk, deform_sapa_fused
@@ -42,6 +44,7 @@ def _common_dtype(*tensors):
     return tensors
 
 
+_PLAIN = (torch.Tensor, nn.Parameter, type(None))
 _NO_NORM = (None, None, 0, 0.0)
 
 
@@ -65,10 +68,14 @@ def _is_projection(conv):
             conv.groups == 1)
 
 
-def _native(x):
-    """Whether the native module path may run at all: not for the CPU, nor where only torch's own ops are seen (traces, transforms,
-    hooks on every module)."""
-    return x.is_cuda and not _lib.transformed() and not _has_any_global_hook()
+def _native(*tensors):
+    """Whether the native module path may run at all for these inputs and parameters (or None): not for the CPU, nor where only
+    torch's own ops are seen - traces, transforms, hooks on every module, torch-function and torch-dispatch modes (a default
+    device aside) - nor for subclasses of Tensor, whose elements may lie anywhere."""
+    return (tensors[0].is_cuda and not _lib.transformed() and not _has_any_global_hook() and
+            torch._C._len_torch_dispatch_stack() == 0 and
+            (torch._C._len_torch_function_stack() == 0 or all(type(m) is DeviceContext for m in _get_current_function_mode_stack())) and
+            all(type(t) in _PLAIN for t in tensors))
 
 
 def _autocast_dtype():
@@ -78,9 +85,9 @@ def _autocast_dtype():
 def _projected(x, norm, conv, fuse):
     """``conv(norm(x))``: with ``fuse`` GroupNorm and the 1x1 convolution run on this library's GEMM kernels, forward and
     backward; otherwise, and for what those do not take, on the torch modules."""
-    if fuse and _native(x):
+    if fuse and x.is_cuda:
         args = _norm_args(norm)
-        if args is not None and _is_projection(conv):
+        if args is not None and _is_projection(conv) and _native(x, *args[:2], conv.weight, conv.bias):
             out = (_lib.host or _lib.load_host()).project_module(x, *args, conv.weight, conv.bias, _autocast_dtype())
             if out is not None:
                 return out
@@ -91,14 +98,17 @@ def _native_module(module, y, x, convs, *args):
     """The whole module in one call (``csrc/host_module.inc``): its projections and the attention.  None where that does not
     apply: another type or shape than the kernels take, replaced or hooked submodules, another ``attention`` than the class's,
     parameters of another type than the input in training."""
-    if not _native(x) or getattr(module.attention, "__func__", None) not in _ATTENTIONS:
+    if not x.is_cuda or getattr(module.attention, "__func__", None) not in _ATTENTIONS:
         return None
     norms = (_norm_args(module.norm_y), _norm_args(module.norm_x)) if module.norm else (_NO_NORM, _NO_NORM)
     if None in norms or not all(_is_projection(c) for c in convs):
         return None
+    params = [p for c in convs for p in (c.weight, c.bias)]
+    if not _native(x, y, *norms[0][:2], *norms[1][:2], *params):
+        return None
     host = _lib.host or _lib.load_host()
     call = host.sapa_module if len(convs) == 2 else host.deform_module
-    return call(y, x, *norms[0], *norms[1], *(p for c in convs for p in (c.weight, c.bias)), *args, _autocast_dtype())
+    return call(y, x, *norms[0], *norms[1], *params, *args, _autocast_dtype())
 
 
 class SAPA(nn.Module):
