@@ -427,7 +427,7 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     constexpr bool F32 = sizeof(T) == 4;
     // rows a tensor map can describe and paired stores: the TMA forms
     const bool ragged = !gath_mma_supported(W, dtype), wide = !F32 && !ragged && wide16_pays(W);
-    const char *name = ragged ? "sapa_gath_kernel" : "sapa_gath_mma_kernel";
+    const char *name = ragged ? "sapa_gath_mma_kernel<ragged>" : wide ? "sapa_gath_wide_16_kernel" : "sapa_gath_mma_kernel";
     if (F32 && ragged) {
         set_error("%s: float32 rows have to be of even length", name);
         return SAPA_ERR_UNSUPPORTED;

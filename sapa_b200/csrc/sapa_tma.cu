@@ -1203,18 +1203,17 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
                                            "sapa_tma_fused_f32_kernel<sim>", "sapa_tma_fused_f32_kernel<agg>"};
     static const char *const names16[4] = {"sapa_tma_fused_16_kernel<fwd>", "sapa_tma_fused_16_kernel<bwd>",
                                            "sapa_tma_fused_16_kernel<sim>", "sapa_tma_fused_16_kernel<agg>"};
-    const char *n32 = names32[mode & 3], *n16 = names16[mode & 3];
-    // how the ragged launches are recorded: the kernels that serve rows of any length
-    static const char *const names_ragged[4] = {"sapa_tile_kernel<fused>", "sapa_tile_kernel<bwd>", "sapa_tile_kernel<sim>", "sapa_tile_kernel<agg>"};
-    const char *nr = names_ragged[mode & 3];
+    static const char *const names_wide[4] = {"sapa_wide_16_kernel<fwd>", "sapa_wide_16_kernel<bwd>", "sapa_wide_16_kernel<sim>", "sapa_wide_16_kernel<agg>"};
+    static const char *const names_ragged[4] = {"sapa_tma_fused_16_kernel<ragged fwd>", "sapa_tma_fused_16_kernel<ragged bwd>",
+                                                "sapa_tma_fused_16_kernel<ragged sim>", "sapa_tma_fused_16_kernel<ragged agg>"};
 #define SAPA_TMA_LAUNCH32(M)                                                                                                             \
     case M:                                                                                                                              \
-        return launch_persistent(sapa_tma_fused_f32_kernel<M>, n32, NT, smem32, CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap, omap);
+        return launch_persistent(sapa_tma_fused_f32_kernel<M>, names32[M], NT, smem32, CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap, omap);
 #define SAPA_TMA_LAUNCH16(T, M)                                                                                                          \
     case M:                                                                                                                              \
-        return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, nr, h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
-               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, n16, w16::NT, w16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap, omap) \
-                      : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, n16, h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
+        return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, names_ragged[M], h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
+               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, names_wide[M], w16::NT, w16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap, omap) \
+                      : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, names16[M], h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
     if (dtype == SAPA_F32) switch (mode) { SAPA_TMA_LAUNCH32(MODE_FWD) SAPA_TMA_LAUNCH32(MODE_BWD) SAPA_TMA_LAUNCH32(MODE_SIM) SAPA_TMA_LAUNCH32(MODE_AGG) }
     if (dtype == SAPA_F16)
         switch (mode) { SAPA_TMA_LAUNCH16(__half, MODE_FWD) SAPA_TMA_LAUNCH16(__half, MODE_BWD) SAPA_TMA_LAUNCH16(__half, MODE_SIM) SAPA_TMA_LAUNCH16(__half, MODE_AGG) }

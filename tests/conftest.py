@@ -51,61 +51,58 @@ def oracle():
 
 
 # ------------------------------------------------------------------ which kernel must serve which call
-# Mirrors the dispatch rules of csrc/sapa_b.cu so that a silent fall-back to a slower kernel fails a test instead of
-# passing on the fall-back's (correct) numbers.  W = low-res width; `wide` = 16-bit element types.
+# Mirrors the dispatch rules of csrc/sapa_b.cu, csrc/sapa_tma.cu and csrc/sapa_gath_mma.cu so that a silent fall-back to a slower
+# kernel fails a test instead of passing on the fall-back's (correct) numbers.  B images of H x W low-resolution pixels.
 
-def _tensor_map_rows(W, wide):
-    """Rows of every tensor on a 16-byte boundary: what the tensor-map (TMA) kernels need."""
-    return W % (8 if wide else 4) == 0
+def _wide_columns(W):
+    """Tiles of 32 columns with at least three quarters of them inside the image, rows of 16 bytes."""
+    return W % 8 == 0 and 4 * W >= 3 * 32 * -(-W // 32)
 
 
-def expected_fused_forward(K, s, W, dtype_name):
-    wide = dtype_name in ("f16", "bf16")
+def _tensor_core(mode, W, dtype_name, B, H):
+    """The K = 5, s = 2 kernel of a mode (fwd, bwd, sim, agg); None where the FP32-pipe kernels serve (float32, W % 4 != 0)."""
+    if dtype_name == "f32":
+        return f"sapa_tma_fused_f32_kernel<{mode}>" if W % 4 == 0 else None
+    if W % 8 != 0:
+        return f"sapa_tma_fused_16_kernel<ragged {mode}>"
+    tiles = B * -(-W // 32) * -(-H // 4)
+    return f"sapa_wide_16_kernel<{mode}>" if _wide_columns(W) and tiles >= 100 else f"sapa_tma_fused_16_kernel<{mode}>"
+
+
+def expected_fused_forward(K, s, W, dtype_name, B=1, H=1):
     if s != 2 or K not in (3, 5) or dtype_name == "f64":
         return None                                   # no fused kernel: the separate ops run
-    if K == 5 and dtype_name == "f32" and W % 4 == 0:
-        return ["sapa_tma_fused_f32_kernel<fwd>"]
-    if K == 5 and wide and W % 8 == 0:
-        return ["sapa_tma_fused_16_kernel<fwd>"]
-    if K == 5 and (dtype_name == "f32" or W % 2 == 0):
+    if K == 3:
+        return ["sapa_tile_kernel<fused>"]
+    if W % (4 if dtype_name == "f32" else 8) != 0 and (dtype_name == "f32" or W % 2 == 0):
         return ["sapa_mma_fused_kernel"]
-    return ["sapa_tile_kernel<fused>"]
+    return [_tensor_core("fwd", W, dtype_name, B, H)]
 
 
-def _gath(K, s, W, dtype_name):
-    wide = dtype_name in ("f16", "bf16")
-    if K == 5 and s == 2 and dtype_name != "f64" and W % (4 if wide else 2) == 0:
-        return "sapa_gath_mma_kernel"
-    if s == 2 and K in (3, 5) and dtype_name != "f64":
+def expected_gath(K, s, W, dtype_name):
+    if s != 2 or K not in (3, 5) or dtype_name == "f64":
+        return "gath_generic_kernel"
+    if K == 3 or (dtype_name == "f32" and W % 2 != 0):
         return "sapa_gath_kernel"
-    return "gath_generic_kernel"
+    if dtype_name != "f32" and W % 4 != 0:
+        return "sapa_gath_mma_kernel<ragged>"
+    return "sapa_gath_wide_16_kernel" if dtype_name != "f32" and _wide_columns(W) else "sapa_gath_mma_kernel"
 
 
-def expected_fused_backward(K, s, W, dtype_name):
-    wide = dtype_name in ("f16", "bf16")
-    tiled = s == 2 and K in (3, 5) and dtype_name != "f64"
-    if K == 5 and s == 2 and dtype_name != "f64" and _tensor_map_rows(W, wide):
-        stage1 = ["sapa_tma_fused_16_kernel<bwd>" if wide else "sapa_tma_fused_f32_kernel<bwd>"]
-    elif tiled:
-        stage1 = ["sapa_tile_kernel<bwd>"]
-    else:
-        stage1 = ["sim_generic_kernel", "softmax_bwd_generic_kernel", "agg_generic_kernel"]
-    return stage1 + [_gath(K, s, W, dtype_name)] * 2
+def _one(mode, generic, K, s, W, dtype_name, B, H):
+    if s != 2 or K not in (3, 5) or dtype_name == "f64":
+        return generic
+    return [(_tensor_core(mode, W, dtype_name, B, H) if K == 5 else None) or f"sapa_tile_kernel<{mode}>"]
 
 
-def expected_sim(K, s, W, dtype_name):
-    wide = dtype_name in ("f16", "bf16")
-    if K == 5 and s == 2 and dtype_name != "f64" and _tensor_map_rows(W, wide):
-        return ["sapa_tma_fused_16_kernel<sim>" if wide else "sapa_tma_fused_f32_kernel<sim>"]
-    if s == 2 and K in (3, 5) and dtype_name != "f64":
-        return ["sapa_tile_kernel<sim>"]
-    return ["sim_generic_kernel"]
+def expected_fused_backward(K, s, W, dtype_name, B=1, H=1):
+    stage1 = _one("bwd", ["sim_generic_kernel", "softmax_bwd_generic_kernel", "agg_generic_kernel"], K, s, W, dtype_name, B, H)
+    return stage1 + [expected_gath(K, s, W, dtype_name)] * 2
 
 
-def expected_agg(K, s, W, dtype_name):
-    wide = dtype_name in ("f16", "bf16")
-    if K == 5 and s == 2 and dtype_name != "f64" and _tensor_map_rows(W, wide):
-        return ["sapa_tma_fused_16_kernel<agg>" if wide else "sapa_tma_fused_f32_kernel<agg>"]
-    if s == 2 and K in (3, 5) and dtype_name != "f64":
-        return ["sapa_tile_kernel<agg>"]
-    return ["agg_generic_kernel"]
+def expected_sim(K, s, W, dtype_name, B=1, H=1):
+    return _one("sim", ["sim_generic_kernel"], K, s, W, dtype_name, B, H)
+
+
+def expected_agg(K, s, W, dtype_name, B=1, H=1):
+    return _one("agg", ["agg_generic_kernel"], K, s, W, dtype_name, B, H)

@@ -46,11 +46,11 @@ def test_config2_16bit_full_size_vs_oracle(sp, oracle, dtype):
     qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
     out = sp.sapa_fused(qd, kd, vd, K, s)
     torch.cuda.synchronize()
-    assert _lib.last_kernels() == ["sapa_tma_fused_16_kernel<fwd>"]
+    assert _lib.last_kernels() == ["sapa_wide_16_kernel<fwd>"]
     assert rel_err(host64(out), want) < 1e-2
     fq, fk, fv = torch.autograd.grad(out, (qd, kd, vd), go.to(DEV))
     torch.cuda.synchronize()
-    assert _lib.last_kernels() == ["sapa_tma_fused_16_kernel<bwd>", "sapa_gath_mma_kernel", "sapa_gath_mma_kernel"]
+    assert _lib.last_kernels() == ["sapa_wide_16_kernel<bwd>", "sapa_gath_wide_16_kernel", "sapa_gath_wide_16_kernel"]
     for got, ref in ((fq, wq), (fk, wk), (fv, wv)):
         assert rel_err(host64(got), ref) < 3e-2
 

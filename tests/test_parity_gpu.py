@@ -211,7 +211,7 @@ def test_sapa_b_half_precision_fused_forward_vs_oracle(sp, oracle, shape, dtype)
     q, k, v = (torch.randn(*sh, generator=g).to(dtype) for sh in ((B, d, s * H, s * W), (B, d, H, W), (B, C, H, W)))
     want, want_p = oracle.sapa_forward(q.double().numpy(), k.double().numpy(), v.double().numpy(), K, s, return_attn=True)
     out, attn = fused_forward_raw(q.to(DEV), k.to(DEV), v.to(DEV), K, s, True)
-    assert ran() == expected_fused_forward(K, s, W, DTYPE_NAME[dtype])
+    assert ran() == expected_fused_forward(K, s, W, DTYPE_NAME[dtype], B, H)
     assert rel_err(host64(out), want) < 1e-2
     assert rel_err(host64(attn), want_p) < 1e-2
     out2, _ = fused_forward_raw(q.to(DEV), k.to(DEV), v.to(DEV), K, s, False)
@@ -222,7 +222,7 @@ def test_sapa_b_half_precision_fused_forward_vs_oracle(sp, oracle, shape, dtype)
     wq, wk, wv = oracle.sapa_backward(go.double().numpy(), q.double().numpy(), k.double().numpy(), v.double().numpy(), K, s)
     qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
     fq, fk, fv = grads(sp.sapa_fused(qd, kd, vd, K, s), (qd, kd, vd), go.to(DEV))
-    assert ran() == expected_fused_backward(K, s, W, DTYPE_NAME[dtype])
+    assert ran() == expected_fused_backward(K, s, W, DTYPE_NAME[dtype], B, H)
     for got, want_g in ((fq, wq), (fk, wk), (fv, wv)):
         assert rel_err(host64(got), want_g) < 3e-2
 

@@ -3,7 +3,7 @@ producer warps), at the widths and channel counts where its boxes, stores and wo
 import pytest
 import torch
 
-from conftest import rel_err
+from conftest import expected_fused_backward, expected_fused_forward, rel_err
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -27,8 +27,10 @@ def test_ragged_rows_vs_oracle(oracle, shape, dtype, tol, tol_grad):
     want_g = oracle.sapa_backward(go.double().numpy(), *n, 5, 2)
     t = [x.to(DEV).requires_grad_() for x in (q, k, v)]
     fused = sp.sapa_fused(*t, 5, 2)
+    name = {torch.float32: "f32", torch.bfloat16: "bf16", torch.float16: "f16"}[dtype]
+    assert _lib.last_kernels() == expected_fused_forward(5, 2, W, name, B, H)
     got = torch.autograd.grad(fused, t, go.to(DEV))
-    assert _lib.last_kernels()[0] == "sapa_tile_kernel<bwd>"
+    assert _lib.last_kernels() == expected_fused_backward(5, 2, W, name, B, H)
     sep = sp.av(torch.softmax(sp.qk(t[0], t[1], 5, 2), dim=1), t[2], 5, 2)
     got_sep = torch.autograd.grad(sep, t, go.to(DEV))
     # the separate ops round the logits and the attention map too: twice the forward's bound
