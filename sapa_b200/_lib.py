@@ -122,11 +122,15 @@ def load_host():
     global host
     if host is None:
         lib()
+        from . import build as _build
+        built, here = _build.built_host_tag(), _build.host_tag()
+        if built is not None and built != here:      # its symbols may resolve all the same
+            raise RuntimeError(f"sapa_b200/_host.so was built for {built} and this is {here}; run `python -m sapa_b200.build`")
         try:
             from . import _host
         except ImportError as exc:
             raise RuntimeError("the native host path sapa_b200/_host.so is missing or does not fit this torch; run "
-                               f"`python -m sapa_b200.build` ({exc})") from exc
+                               f"`python -m sapa_b200.build --force` ({exc})") from exc
         _host.bind(LIB_PATH)
         host = _host
     return host

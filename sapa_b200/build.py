@@ -23,6 +23,7 @@ HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "tma_util.cuh"),
            os.path.join(INCLUDE, "sapa_b200.h")]
 
 HOST = os.path.join(HERE, "_host.so")
+HOST_TAG = os.path.join(HERE, "build", "_host.tag")      # what _host.so was built for
 HOST_SOURCES = [os.path.join(CSRC, f) for f in ("host.cpp", "host_sapa.inc", "host_deform.inc", "host_module.inc")]
 
 NVCC_FLAGS = [
@@ -46,6 +47,24 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def host_tag() -> str:
+    """What a build of the host path is tied to: this torch, its C++ ABI and this Python."""
+    import sysconfig
+
+    import torch
+
+    return f"torch {torch.__version__}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, Python {sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
+def built_host_tag() -> str | None:
+    """``host_tag()`` of the build that is there, None when it is not recorded."""
+    try:
+        with open(HOST_TAG) as f:
+            return f.read()
+    except OSError:
+        return None
+
+
 def _build_host() -> None:
     import sysconfig
 
@@ -61,11 +80,14 @@ def _build_host() -> None:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for host.cpp:\n{r.stdout}\n{r.stderr}")
+    os.makedirs(os.path.dirname(HOST_TAG), exist_ok=True)
+    with open(HOST_TAG, "w") as f:
+        f.write(host_tag())
 
 
 def _host_stale() -> bool:
     deps = HOST_SOURCES + [HEADERS[-1], os.path.abspath(__file__)]
-    return not os.path.exists(HOST) or any(os.path.getmtime(d) > os.path.getmtime(HOST) for d in deps)
+    return not os.path.exists(HOST) or built_host_tag() != host_tag() or any(os.path.getmtime(d) > os.path.getmtime(HOST) for d in deps)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -125,3 +125,21 @@ def test_product_package_never_touches_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h")):
                 text = open(os.path.join(dirpath, f)).read()
                 assert not pattern.search(text), os.path.join(dirpath, f)
+
+
+def test_host_path_of_another_torch_is_stale_and_not_loaded(monkeypatch, tmp_path):
+    """The host path is tied to the torch and the Python it was built with: after an upgrade the build command rebuilds it, and
+    until then it is refused instead of loaded."""
+    from sapa_b200 import _lib, build
+    _lib.load_host()
+    assert build.built_host_tag() == build.host_tag()
+    tag = tmp_path / "_host.tag"
+    tag.write_text(build.host_tag().replace("torch ", "torch 1."))
+    monkeypatch.setattr(build, "HOST_TAG", str(tag))
+    assert build._host_stale()
+    monkeypatch.setattr(_lib, "host", None)
+    with pytest.raises(RuntimeError, match="python -m sapa_b200.build"):
+        _lib.load_host()
+    monkeypatch.setattr(build, "HOST_TAG", str(tmp_path / "none"))      # a copied file without a record is taken as it is
+    assert build._host_stale()
+    _lib.load_host()
