@@ -71,7 +71,8 @@ int sapa_abi_version(void);
  * overlap them freely).  No counterpart in the reference. */
 int sapa_wait_timeout_flags(void);
 /* Self-test of that mechanism: launches one small kernel whose bounded wait is certain to give up (it waits a few
- * dozen tries on a barrier that nothing signals, then raises the flag and returns normally; nothing hangs or faults).
+ * dozen tries on a barrier that nothing signals, goes through what a producer does then - waiting, with a limit, for the
+ * stages it has issued - raises the flag and returns normally; nothing hangs or faults).
  * Afterwards sapa_wait_timeout_flags() reports bit 0 once, and the library works as before. */
 int sapa_selftest_wait_timeout(void *stream);
 

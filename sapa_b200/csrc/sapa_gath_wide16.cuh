@@ -75,7 +75,11 @@ sapa_gath_wide_16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
                 y0 = (u % a.tiles_y) * ROWS; n = u / a.tiles_y;
             }
             for (int it = 0; it < (item < 0 ? 1 : nst); ++it) {
-                if (!mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) { atomicExch(&g_wait_timeout, 1); return; }
+                if (!mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) {
+                    atomicExch(&g_wait_timeout, 1);
+                    drain_loads<gw16::NSTAGE>(full_addr, slot, phase);
+                    return;
+                }
                 const unsigned bar = full_addr + 8 * slot, dst = ring_addr + slot * gw16::SLOT_BYTES;
                 if (it == 0) tile_ids[ti & 7] = item;
                 if (item < 0) {

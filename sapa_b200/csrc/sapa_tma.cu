@@ -637,7 +637,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 };
                 load(cur);
                 while (cur.tile < ntiles) {
-                    if (!claim()) return;
+                    if (!claim()) break;
                     const unsigned dst = ring_addr + slot * h16::SLOT_BYTES, bar = full_addr + 8 * slot;
                     if (cur.it < nk) ragged_hi_box_16<T>(dst + h16::K_BYTES, qp + (size_t)cur.n * a.d * hi_plane, cur.it * KCH, a.d, a.H, a.W, cur.y0, cur.x0, ptid);
                     box.store(dst, ptid);
@@ -649,7 +649,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 }
             } else {
                 while (cur.tile < ntiles) {
-                    if (!claim()) return;
+                    if (!claim()) break;
                     const unsigned dst = ring_addr + slot * h16::SLOT_BYTES;
                     const bool key = cur.it < nk;
                     ragged_lo_box_16<T>(dst, key ? kp + (size_t)cur.n * a.d * lo_plane : vp + (size_t)cur.n * a.C * lo_plane,
@@ -1228,14 +1228,19 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
 // One CTA waits, with a short limit, on a shared-memory barrier that nothing ever signals: the bounded wait gives up,
 // the kernel raises g_wait_timeout exactly as the production kernels would and returns normally.
 __global__ void sapa_wait_selftest_kernel(int tries) {
-    __shared__ __align__(8) unsigned long long bar;
-    const unsigned addr = (unsigned)__cvta_generic_to_shared(&bar);
+    __shared__ __align__(8) unsigned long long bars[4];
+    const unsigned addr = (unsigned)__cvta_generic_to_shared(bars), ring = addr + 8;
     if (threadIdx.x == 0) {
-        tmau::mbar_init(addr, 1);
+        for (int i = 0; i < 4; ++i) tmau::mbar_init(addr + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         bool done = false;
         for (int i = 0; i < tries && !done; ++i) done = tmau::mbar_try_wait(addr, 0);
-        if (!done) atomicExch(&tma::g_wait_timeout, 1);
+        // what a producer does then, at two positions of a ring of three stages: one stage issued and landed, then four
+        tmau::mbar_arrive(ring);
+        bool landed = tmau::drain_loads<3>(ring, 1, 0);
+        for (int i = 1; i <= 3; ++i) tmau::mbar_arrive(ring + 8 * (i % 3));
+        landed = tmau::drain_loads<3>(ring, 1, 1) && landed;
+        if (!done && landed) atomicExch(&tma::g_wait_timeout, 1);
     }
 }
 

@@ -53,6 +53,15 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap *map
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
+// A producer that gives up, with the ring position of its next stage: waits, with the same limit, for the loads that it has issued, so
+// that none lands after its CTA has left.  A barrier that was never used counts as passed.
+template <int N>
+__device__ __forceinline__ bool drain_loads(unsigned full, int slot, int phase) {
+    bool landed = true;
+#pragma unroll 1
+    for (int i = 0; i < N; ++i) landed = mbar_wait_bounded(full + 8 * i, i < slot ? phase : phase ^ 1) && landed;
+    return landed;
+}
 // shared -> global tile store; out-of-range parts of the box (tile overhang, channel tail) are clipped
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, unsigned src, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n"
