@@ -150,8 +150,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
         if (warp >= NW) {
             const int ptid = tid - NW * 32, pair = ptid & 15;       // pairs 2 .. 13 of a box row
             int slot = 0, phase = 0;
-            bool going = true;
-            for (int tile = blockIdx.x; going && tile < ntiles; tile += gridDim.x) {
+            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
                 int t_ = tile / a.csplit;
                 const int vb = tile % a.csplit * nst;
                 const int x0 = (t_ % a.tiles_x) * COLS; t_ /= a.tiles_x;
@@ -160,7 +159,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                 const int px = 2 * x0 - 8 + 2 * pair, py = 2 * (y0 - a.top - 2);
                 const bool x_ok = px >= 0 && px < sW;
                 for (int it = 0; it < nst; ++it) {
-                    if (!mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) { atomicExch(&g_wait_timeout, 1); going = false; break; }
+                    if (!mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) { atomicExch(&g_wait_timeout, 1); cp_async_wait_all(); return; }
                     const unsigned dst = ring_addr + slot * G::BOX_BYTES;
                     const int c0 = (vb + it) * NCH;
                     if (!(a.W & 1)) {             // rows start on 8 bytes: quads 1 .. 6 of a box row
@@ -188,7 +187,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                     if (++slot == NSTAGE) { slot = 0; phase ^= 1; }
                 }
             }
-            asm volatile("cp.async.wait_all;\n" ::: "memory");      // no copy outlives the thread
+            cp_async_wait_all();
             return;
         }
     }

@@ -625,6 +625,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
             const auto claim = [&]() {
                 if (mbar_wait_bounded(empty_addr + 8 * slot, phase ^ 1)) return true;
                 atomicExch(&g_wait_timeout, 1);
+                cp_async_wait_all();
                 return false;
             };
             const auto next_slot = [&]() { if (++slot == h16::NSTAGE) { slot = 0; phase ^= 1; } };
@@ -637,7 +638,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 };
                 load(cur);
                 while (cur.tile < ntiles) {
-                    if (!claim()) break;
+                    if (!claim()) return;
                     const unsigned dst = ring_addr + slot * h16::SLOT_BYTES, bar = full_addr + 8 * slot;
                     if (cur.it < nk) ragged_hi_box_16<T>(dst + h16::K_BYTES, qp + (size_t)cur.n * a.d * hi_plane, cur.it * KCH, a.d, a.H, a.W, cur.y0, cur.x0, ptid);
                     box.store(dst, ptid);
@@ -649,7 +650,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 }
             } else {
                 while (cur.tile < ntiles) {
-                    if (!claim()) break;
+                    if (!claim()) return;
                     const unsigned dst = ring_addr + slot * h16::SLOT_BYTES;
                     const bool key = cur.it < nk;
                     ragged_lo_box_16<T>(dst, key ? kp + (size_t)cur.n * a.d * lo_plane : vp + (size_t)cur.n * a.C * lo_plane,
@@ -660,7 +661,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                     advance(cur);
                 }
             }
-            asm volatile("cp.async.wait_all;\n" ::: "memory");      // no copy outlives the thread
+            cp_async_wait_all();
             return;
         }
     }
@@ -1022,14 +1023,14 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                     }
                 }
             if constexpr (RAGGED) {
-                float zero = 0.f;
+                float zero[4] = {};
 #pragma unroll
-                for (int b = 0; b < VCH / 16; ++b)
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int p = 0; p < 2; ++p)
+                    for (int b = 0; b < VCH / 16; ++b)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) zero = fmaf(acc[b][p][i], 0.f, zero);
-                if (__any_sync(0xffffffffu, !(zero == 0.f)))
+                        for (int p = 0; p < 2; ++p) zero[i] = fmaf(acc[b][p][i], 0.f, zero[i]);
+                if (__any_sync(0xffffffffu, !((zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.f)))
                     window_sums<T, TWO, MODE == MODE_FWD>(acc, pb, pl, stage + wrow * (VCH * KROW), lane);
             }
             __syncwarp();

@@ -79,6 +79,8 @@ __device__ __forceinline__ void cp_async8(unsigned dst, const void *src, bool va
 __device__ __forceinline__ void cp_async_arrive(unsigned bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
 }
+// every copy of this thread has landed: before it leaves, for none may outlive it
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 __device__ __forceinline__ void sts32(unsigned addr, unsigned v) { asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(addr), "r"(v) : "memory"); }
 // An address the compiler must take as new from here on: lds32 is a pure function of its address to the compiler, so a load
 // from a ring slot has to depend on something that follows the wait for the slot.
