@@ -35,7 +35,7 @@ struct FwdList { FwdProblem p[MAX_PROBLEMS]; int count; };
 
 // backward, first pass: by slices of the pixels, dW [d, C], r = sum_p dq [d] and, behind a norm, S1 = sum_p dy, S2 = sum_p dy x [C]
 struct MomentProblem {
-    const void *x, *g1, *g2, *weight, *gamma, *beta;     // rows of dq: the first d1 from g1 [B, d1, HW], the rest from g2
+    const void *x, *g1, *g2, *w1, *w2, *gamma, *beta;    // rows of dq (and of W): the first d1 from g1 [B, d1, HW] (w1), the rest from g2 (w2)
     const float2 *stats;
     float *dw, *rsums;
     float2 *sums;                      // [B, nsplit, C]

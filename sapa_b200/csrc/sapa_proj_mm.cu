@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(THREADS, 2) proj_moments_kernel(const __grid_c
     if (NORM) {
         for (int i = tid; i < MO_C * ((m.d + 7) & ~7); i += THREADS) {
             const int c = i & (MO_C - 1), j = i / MO_C, cc = cb * MO_C + c;
-            ws[c * MO_PITCH + j] = cc < m.C && j < m.d ? rounded<TG>(to_acc(__ldg(static_cast<const T *>(m.weight) + (size_t)j * m.C + cc))) : 0.f;
+            const T *w = j < m.d1 ? static_cast<const T *>(m.w1) + (size_t)j * m.C : static_cast<const T *>(m.w2) + (size_t)(j - m.d1) * m.C;
+            ws[c * MO_PITCH + j] = cc < m.C && j < m.d ? rounded<TG>(to_acc(__ldg(w + cc))) : 0.f;
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -682,7 +683,7 @@ static int run_backward(const sapa_projection_grad *q, int count, unsigned char 
         MomentProblem m = moment_problem(s, tiles);
         const BwdLayout l = bwd_layout(m, at);
         at = l.total;
-        m.x = s.x; m.g1 = s.grad_out; m.g2 = s.grad_out2; m.weight = s.weight; m.gamma = s.gamma; m.beta = s.beta;
+        m.x = s.x; m.g1 = s.grad_out; m.g2 = s.grad_out2; m.w1 = s.weight; m.w2 = s.weight2; m.gamma = s.gamma; m.beta = s.beta;
         m.stats = norm ? static_cast<const float2 *>(s.stats) : nullptr;
         m.dw = reinterpret_cast<float *>(ws + l.dw); m.rsums = reinterpret_cast<float *>(ws + l.rsums); m.sums = reinterpret_cast<float2 *>(ws + l.sums);
         m.vec_x = rows16(s.x, s.HW, sizeof(T));
