@@ -643,12 +643,12 @@ int run_sim_slab(const void *hi, const void *lo, void *out, int B, int Cc, int H
     });
 }
 
-// 16-bit tensors with a float32 slot tensor (K = 5, s = 2): sim writes float32 logits.  The dense-window
+// 16-bit tensors with a float32 slot tensor (K = 5, s = 2, rows of 16 bytes): sim writes float32 logits.  The dense-window
 // path of SAPA-D keeps its 25-slot similarity at full precision this way.
 int run_sim_mixed(const void *hi, const void *lo, float *out, int B, int Cc, int H, int W, int rows, int top, int dtype,
                   cudaStream_t st) {
-    if (!(all_aligned16(hi, lo, out) && (dtype == SAPA_F16 || dtype == SAPA_BF16))) {
-        set_error("run_sim_mixed: needs 16-bit tensors, 16-byte aligned");
+    if (!(all_aligned16(hi, lo, out) && (dtype == SAPA_F16 || dtype == SAPA_BF16) && fused_tma_supported(W, dtype))) {
+        set_error("run_sim_mixed: needs 16-bit tensors, 16-byte aligned, rows of 16 bytes");
         return SAPA_ERR_UNSUPPORTED;
     }
     return launch_fused_tma_slots(2, hi, lo, nullptr, nullptr, out, nullptr, B, Cc, 0, H, W, rows, top, 0, H, dtype, true, st);

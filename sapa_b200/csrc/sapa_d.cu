@@ -478,7 +478,7 @@ __device__ __forceinline__ void outlier_pixels(const OutlierTap *__restrict__ ta
     }
 }
 // A short list (learned offsets: a few hundred entries) is a chain of dependent loads per entry: a warp per entry and every channel
-// in flight at once (20 -> OUTFWD us for 600 pixels of 64 channels).  A long one is bound by its sectors, which neighbouring pixels
+// in flight at once (25 -> 7 us for 317 pixels of 64 channels in float16).  A long one is bound by its sectors, which neighbouring pixels
 // share when eight threads serve each.
 template <typename T>
 __global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const unsigned int *__restrict__ tap_count,
@@ -733,8 +733,8 @@ __global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, 
 
 // The float32 side buffers of the 16-bit gradients: zeroed before the list kernel, added to the gradients after it (one rounding per
 // element).  A short list touches a few thousand of the buffers' cells: those alone are zeroed, and taken back by an exchange that
-// gives each cell's whole sum to one of the points that share it.  A long list goes over the buffers (42 MB, 8 + 25 us, at 8 images
-// of 320 channels, 64 x 64; the short form: SHORT us).
+// gives each cell's whole sum to one of the points that share it.  A long list goes over the buffers (42 MB at 8 images of 320
+// channels, 64 x 64: 10 + 26 us; the short form, for 582 points: 5 + 10 us).
 struct Scatter { float *key, *value; size_t n_key, n_value; int gq, gc; };      // the value buffer lies behind the key buffer
 
 // f(cell index of the key buffer or of the value buffer, which) for the four corners of every listed point and all channels of its
@@ -1060,6 +1060,7 @@ int run_sim_slab(const void *hi, const void *lo, void *out, int B, int Cc, int H
 int run_agg_slab(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s, int dtype,
                  cudaStream_t st);
 int run_sim_mixed(const void *hi, const void *lo, float *out, int B, int Cc, int H, int W, int rows, int top, int dtype, cudaStream_t st);
+bool fused_tma_supported(int W, int dtype);
 }
 
 extern "C" {
@@ -1068,7 +1069,7 @@ size_t sapa_deform_fused_forward_workspace(int B, int H, int W, int P, int s, in
     if (B <= 0 || H <= 0 || W <= 0 || P <= 0 || G <= 0 || s != 2) return 0;
     // 16-bit tensors: the mixed modes of the tensor-core kernels (16-bit operands, float32 windows).  Rows that are not multiples of 16 bytes run the
     // float32 chain on widened tensors, or the gather kernels, with float32 weights
-    if (dtype != SAPA_F32 && !((dtype == SAPA_F16 || dtype == SAPA_BF16) && W % 8 == 0)) return 0;
+    if (dtype != SAPA_F32 && !((dtype == SAPA_F16 || dtype == SAPA_BF16) && fused_tma_supported(W, dtype))) return 0;
     const size_t hi = (size_t)s * H * s * W;
     if ((size_t)B * G * hi >= 0xffffffffull) return 0;       // the outlier list indexes (image, group, pixel) with 32 bits
     // dense similarity + window weights (float32 whatever the tensors' type), the outlier list (worst case: every
@@ -1232,7 +1233,7 @@ size_t sapa_deform_fused_backward_workspace(int B, int H, int W, int P, int s, i
     if (B <= 0 || H <= 0 || W <= 0 || P <= 0 || G <= 0 || s != 2) return 0;
     // 16-bit tensors: 16-bit operands in the tensor-core kernels, float32 similarities between them.  Rows that are not multiples of 16 bytes run the
     // float32 chain on widened tensors, or the gather kernels, with float32 weights
-    if (dtype != SAPA_F32 && !((dtype == SAPA_F16 || dtype == SAPA_BF16) && W % 8 == 0)) return 0;
+    if (dtype != SAPA_F32 && !((dtype == SAPA_F16 || dtype == SAPA_BF16) && fused_tma_supported(W, dtype))) return 0;
     const size_t hi = (size_t)s * H * s * W;
     if ((size_t)B * G * P >= 0xffffffffull || hi >= 0xffffffffull) return 0;
     // D, dWd (float32), dD, Wd (the tensors' type; sized for float32), the outlier list (worst case: every point) and

@@ -26,16 +26,6 @@ static_assert(SMEM_BYTES <= 227 * 1024 && A_BYTES % 1024 == 0 && SLOT_BYTES % 10
 }  // namespace gw16
 
 template <typename T>
-__device__ __forceinline__ void mma_16_k16(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-    if constexpr (std::is_same<T, __half>::value)
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-    else
-        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-template <typename T>
 __global__ void __launch_bounds__(gw16::NT, 1)
 sapa_gath_wide_16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const Args a) {
     extern __shared__ unsigned char smem_dyn[];
@@ -158,7 +148,7 @@ sapa_gath_wide_16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
                     for (int kg = 0; kg < 4; ++kg) {
                         unsigned x[4];
                         ldsm_x4(x, stage + off[kg] + j * step[kg]);
-                        mma_16_k16<T>(acc[kg], x, bw[j][kg][0], bw[j][kg][1]);
+                        mma_h16<T>(acc[kg], x[0], x[1], x[2], x[3], bw[j][kg][0], bw[j][kg][1]);
                     }
             }
             __syncwarp();

@@ -629,7 +629,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                 return false;
             };
             const auto next_slot = [&]() { if (++slot == h16::NSTAGE) { slot = 0; phase ^= 1; } };
-            if (a.W & 1) {
+            if (MODE == MODE_FWD || (a.W & 1)) {      // rows of even length have another forward kernel
                 OddBox box;
                 const auto load = [&](const Pos &p) {
                     const bool key = p.it < nk;
@@ -954,7 +954,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                         pb[p][dy][1] = pack_pair(T(), s[p][dy][2], s[p][dy][3]);
                     }
             }
-            if (it == nk - 1 && MODE == MODE_SIM && a.slots_f32 != 0) {
+            if (!RAGGED && it == nk - 1 && MODE == MODE_SIM && a.slots_f32 != 0) {
                 if (row_ok) {         // raw logits as float32 pairs (the dense similarity of the 16-bit SAPA-D path)
                     float2 *af = reinterpret_cast<float2 *>(static_cast<float *>(a.attn) + (size_t)n * 25 * hi_plane +
                                                             (size_t)(2 * y + r) * sW + 2 * x0 + 2 * t);
@@ -1122,7 +1122,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
 
 // 16-bit: tiles of 4 x 32 instead of 4 x 8 pixels where at least three quarters of their columns are inside the image (below that
 // idle warps cost what the loads save) and two thirds of the SMs get one.
-// us, 4 x 8 -> 4 x 32: bfloat16 forward 8 x 256 x 64x64 55.7 -> 40.9, 64 x 256 x 128x128 1540 -> 830, 1 x 256 x 1024x1024 2520 -> 854;
+// us, 4 x 8 -> 4 x 32: bfloat16 forward 8 x 256 x 64x64 55.7 -> 40.9, 64 x 256 x 128x128 1540 -> 930, 1 x 256 x 1024x1024 2520 -> 970;
 // float16 forward 4 x 128 x 56x56 (112 tiles) 24.6 -> 19.4; with fewer tiles the 4 x 8 ones use more SMs: module training at
 // 8 x 256 x 32x32 (64 tiles) 252 -> 264, forward of 1 x 64 x 64x64 (32 tiles) 13.2 -> 14.3.
 static bool wide16_pays(int W, int tiles_y, int B) {
@@ -1213,7 +1213,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
 #define SAPA_TMA_LAUNCH16(T, M)                                                                                                          \
     case M:                                                                                                                              \
         return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, names_ragged[M], h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
-               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, names_wide[M], w16::NT, w16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap, omap) \
+               : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, names_wide[M], w16::NT, w16::SMEM_BYTES, 1, false, a, st, qmap, kmap, vmap, omap) \
                       : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, names16[M], h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
     if (dtype == SAPA_F32) switch (mode) { SAPA_TMA_LAUNCH32(MODE_FWD) SAPA_TMA_LAUNCH32(MODE_BWD) SAPA_TMA_LAUNCH32(MODE_SIM) SAPA_TMA_LAUNCH32(MODE_AGG) }
     if (dtype == SAPA_F16)

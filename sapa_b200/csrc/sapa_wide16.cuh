@@ -8,7 +8,7 @@
 //   * outputs go through shared memory and leave as boxes with rows of 128 bytes (one lane of a spare warp issues them): a store
 //     from registers writes eight channels, 32 bytes each, which costs the load / store unit eight cycles (it was 70 % busy, and
 //     what the kernel waited for) and an address translation per channel: 64 x 256 x 128x128 1058 -> 829 us, 1 x 256 x 1024x1024,
-//     whose channels are 8 MB apart, 1666 -> 854;
+//     whose channels are 8 MB apart, 1666 -> 854 (in runs of a few launches; back to back 930 and 960);
 //   * a warp owns 8 low-res columns of one low-res row and BOTH of its high-res rows: a key or value fragment is loaded once for
 //     four products instead of twice for two each.
 // Fragments, accumulation order and roundings are those of the 4 x 8 kernel (the 24 columns that a warp reads are the same
@@ -50,6 +50,7 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     const int sW = 2 * a.W;
     const size_t hi_plane = (size_t)(2 * a.H) * sW;
     const int nk = (a.d + w16::KCH - 1) / w16::KCH, nv = a.vstages, total = nk + nv;
+    // csplit is 1 here (at least 100 tiles); the kernel compiled without it was slower: 64 x 256 x 128x128 826 -> 840 us
     const int nitems = a.B * a.tiles_x * a.tiles_y * a.csplit;
 
     if (tid == 0) {
