@@ -327,6 +327,14 @@ typedef struct sapa_projection {
     float eps;
 } sapa_projection;
 
+/* sapa_project_rows_forward for up to three projections in the same launches: one for the statistics of all that have a norm (taken
+ * once for projections of the same x), one for the folds, one for the products; what no projection of the list needs is not launched.
+ * shuffle_widths: one per projection, or NULL.  `stats` is not written.  Workspace: sapa_project_list_workspace() bytes (0: not
+ * supported) for the same records, 256-byte aligned. */
+size_t sapa_project_list_workspace(const sapa_projection *p, int count, int dtype);
+int sapa_project_list_forward(const sapa_projection *p, const int *shuffle_widths, int count, void *workspace, size_t workspace_bytes,
+                              int dtype, int out_dtype, void *stream);
+
 /* Up to three projections in two launches, for rows of any length and any d; x and parameters have `dtype`, the outputs
  * out_dtype (the same, or 16 bits of float32: then operands, product and biased sum are rounded as a 16-bit convolution of a
  * float32 GroupNorm rounds them).  Workspace: sapa_projections_workspace() bytes (0: not supported), 256-byte aligned. */

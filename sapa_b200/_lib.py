@@ -51,6 +51,7 @@ _SIGNATURES = {
     "sapa_selftest_wait_timeout": [_vp],
     "sapa_project_forward": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i, ctypes.c_float, _i, _vp],
     "sapa_project_rows_forward": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _sz, _i, _i, _i, _i, _i, ctypes.c_float, _i, _i, _vp],
+    "sapa_project_list_forward": [_vp, _vp, _i, _vp, _sz, _i, _i, _vp],
     "sapa_projections_forward": [_vp, _i, _vp, _sz, _i, _i, _vp],
     "sapa_projections_backward": [_vp, _i, _vp, _sz, _i, _i, _vp],
     "sapa_deform_fused_backward_dense": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
@@ -59,7 +60,7 @@ _SIGNATURES = {
 EXPORTS = sorted(list(_SIGNATURES) + ["sapa_last_error", "sapa_last_kernels", "sapa_abi_version", "sapa_fused_backward_workspace",
                                            "sapa_deform_fused_forward_workspace", "sapa_deform_fused_backward_workspace",
                                            "sapa_deform_fused_backward_scatter_bytes", "sapa_project_workspace",
-                                           "sapa_project_rows_workspace", "sapa_projections_workspace",
+                                           "sapa_project_rows_workspace", "sapa_project_list_workspace", "sapa_projections_workspace",
                                            "sapa_projections_backward_workspace",
                                            "sapa_fused_backward_static_capacity", "sapa_wait_timeout_flags"])
 
@@ -101,6 +102,8 @@ def lib() -> ctypes.CDLL:
     handle.sapa_project_workspace.restype = ctypes.c_size_t
     handle.sapa_project_rows_workspace.argtypes = [_i, _i, _i, _i, _i, _i]
     handle.sapa_project_rows_workspace.restype = ctypes.c_size_t
+    handle.sapa_project_list_workspace.argtypes = [_vp, _i, _i]
+    handle.sapa_project_list_workspace.restype = ctypes.c_size_t
     for name in ("sapa_projections_workspace", "sapa_projections_backward_workspace"):
         getattr(handle, name).argtypes = [_vp, _i]
         getattr(handle, name).restype = ctypes.c_size_t
