@@ -59,6 +59,13 @@ template <> __device__ __forceinline__ void store_pair<__nv_bfloat16>(__nv_bfloa
     __stcs(reinterpret_cast<unsigned int *>(p), *reinterpret_cast<const unsigned int *>(&h));
 }
 
+// First thing in a kernel that is launched with launch_next, before any access to global memory: waits until the previous kernel of
+// the stream has finished and its writes are visible, then lets the blocks of the next one be set up as this kernel's leave room.
+__device__ __forceinline__ void begin_after_previous() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 __device__ __forceinline__ void atomic_add(float *p, float v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add(double *p, double v) { atomicAdd(p, v); }
 
@@ -101,6 +108,20 @@ inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b -
     } while (0)
 
 template <typename... P> inline bool all_aligned16(const P *...p) { return (aligned16(p) && ...); }
+
+// Launch of a kernel that starts with begin_after_previous(): its blocks may be set up while the previous kernel of the stream drains
+// (programmatic dependent launch), which hides the launch latency between the kernels of a chain, about 1.5 us of 2.5: three
+// chained SAPA modules (twelve kernels) 253.6 -> 231.5 us, one SAPADeform module (six) 57.4 -> 52.4.
+template <typename... P, typename... A>
+inline void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = st;
+    config.attrs = &attribute; config.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);      // a failure is what check_launch reads
+}
 
 // Runs the lambda body with `scalar_t` bound to the element type named by the dtype code.
 // SAPA_DISPATCH_FAST: f32 / f16 / bf16 (tiled kernels).  SAPA_DISPATCH_ALL adds f64 (generic kernels).

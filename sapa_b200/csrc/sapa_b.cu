@@ -348,6 +348,7 @@ struct TileArgs {
 
 template <typename T, typename Shape, int MODE, int MINB>
 __global__ void __launch_bounds__(Shape::NT, MINB) sapa_tile_kernel(const TileArgs a) {
+    begin_after_previous();
     constexpr int K = Shape::K, S = Shape::S, KK = Shape::KK, SS = Shape::SS, CH = Shape::CH;
     __shared__ float sm[2][CH * Shape::PLANE];
 
@@ -458,6 +459,7 @@ template <typename T, typename Shape>
 __global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *__restrict__ hi, const T *__restrict__ wt,
                                                               T *__restrict__ out, int B, int Cc, int H, int W,
                                                               int tiles_x, int tiles_y) {
+    begin_after_previous();
     constexpr int K = Shape::K, S = Shape::S, KK = Shape::KK, SS = Shape::SS, R = Shape::R;
     constexpr int PH = Shape::HH, PW = Shape::HW;            // parents covered by the staged tile
     constexpr int ROWLEN = PW * S;                           // high-res columns per staged row
@@ -576,7 +578,7 @@ static int launch_tile(TileArgs a, cudaStream_t st) {
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    sapa_tile_kernel<T, Shape, MODE, 3><<<(unsigned)blocks, Shape::NT, 0, st>>>(a);
+    launch_next(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
     constexpr const char *names[4] = {"sapa_tile_kernel<sim>", "sapa_tile_kernel<agg>", "sapa_tile_kernel<fused>",
                                       "sapa_tile_kernel<bwd>"};
     return check_launch(names[MODE]);
@@ -595,7 +597,7 @@ static int launch_gath(const T *hi, const T *wt, T *out, int B, int Cc, int H, i
         using Shape = decltype(shape);
         const int tiles_x = ceil_div(W, Shape::TW), tiles_y = ceil_div(H, Shape::TH);
         const long long blocks = (long long)B * tiles_x * tiles_y;
-        sapa_gath_kernel<T, Shape><<<(unsigned)blocks, Shape::NT, 0, st>>>(hi, wt, out, B, Cc, H, W, tiles_x, tiles_y);
+        launch_next(sapa_gath_kernel<T, Shape>, (unsigned)blocks, Shape::NT, 0, st, hi, wt, out, B, Cc, H, W, tiles_x, tiles_y);
         return check_launch("sapa_gath_kernel");
     };
     if constexpr (sizeof(T) == 4)

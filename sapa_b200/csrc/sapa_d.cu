@@ -315,6 +315,7 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
                           const float *__restrict__ dense, T *__restrict__ attn, T *__restrict__ window,
                           OutlierTap *__restrict__ taps, unsigned int *__restrict__ tap_count, int B, int Cq, int H, int W,
                           int P_runtime, int G, int rows, int ytop) {
+    begin_after_previous();
     constexpr int PMAX = NP > 0 ? NP : MAXP;
     __shared__ float sd[MODE != WIN_WEIGHTS ? 25 : 1][WIN_THREADS];     // dense similarity of the thread's pixel
     __shared__ float sw[MODE != WIN_LOGITS ? 25 : 1][WIN_THREADS];      // window weights being collected
@@ -484,6 +485,7 @@ template <typename T>
 __global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const unsigned int *__restrict__ tap_count,
                                       const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ out,
                                       int C, int H, int W, int P, int G, int rows, int ytop) {
+    begin_after_previous();
     const unsigned int n = *tap_count;
     if (n <= gridDim.x * (blockDim.x / 32)) outlier_pixels<32, 2>(taps, n, value, offset, out, C, H, W, P, G, rows, ytop);
     else outlier_pixels<8, 4>(taps, n, value, offset, out, C, H, W, P, G, rows, ytop);
@@ -520,6 +522,7 @@ deform_window_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ v
                          T *__restrict__ window /* Wd, out */, T *__restrict__ grad_offset, T *__restrict__ grad_attn /* BWD_AV only */,
                          OutlierGrad *__restrict__ taps,
                          unsigned int *__restrict__ tap_count, int B, int C, int H, int W, int P_runtime, int G) {
+    begin_after_previous();
     constexpr int PMAX = NP > 0 ? NP : MAXP;
     const int P = NP > 0 ? NP : P_runtime;
     const int sH = 2 * H, sW = 2 * W, gc = C / G;
@@ -724,6 +727,7 @@ __global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, 
                                           const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ grad_query,
                                           TA *__restrict__ grad_key, TA *__restrict__ grad_value, T *__restrict__ grad_offset,
                                           int Cq, int C, int H, int W, int P, int G) {
+    begin_after_previous();
     const unsigned int n = *tap_count;
     if (n <= gridDim.x * (blockDim.x / 32))
         outlier_points_bwd<32>(taps, n, grad_out, query, key, value, offset, grad_query, grad_key, grad_value, grad_offset, Cq, C, H, W, P, G);
@@ -763,6 +767,7 @@ __device__ __forceinline__ void for_scattered(const OutlierGrad *__restrict__ ta
 template <typename T>
 __global__ void deform_zero_scatter_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count, const T *__restrict__ offset,
                                            const Scatter sc, int H, int W, int P) {
+    begin_after_previous();
     const unsigned int n = *tap_count;
     if (n <= gridDim.x * (blockDim.x / 32)) {
         for_scattered(taps, n, offset, sc, H, W, P, [&](size_t i, bool key) { (key ? sc.key : sc.value)[i] = 0.f; });
@@ -775,6 +780,7 @@ __global__ void deform_zero_scatter_kernel(const OutlierGrad *__restrict__ taps,
 template <typename T>
 __global__ void deform_add_scatter_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count, const T *__restrict__ offset,
                                           const Scatter sc, T *__restrict__ grad_key, T *__restrict__ grad_value, int H, int W, int P) {
+    begin_after_previous();
     const unsigned int n = *tap_count;
     if (n <= gridDim.x * (blockDim.x / 32)) {
         for_scattered(taps, n, offset, sc, H, W, P, [&](size_t i, bool key) {
@@ -902,6 +908,17 @@ static int check_deform(const char *fn, int B, int Cq, int C, int H, int W, int 
     return SAPA_OK;
 }
 
+
+// The counter of the outlier list.  A kernel and not a memset: a memset between kernels keeps the ones around it from being set up
+// ahead (float32 forward of 8 x 256 x 64x64 178.8 -> 174.0 us, its bfloat16 training 473 -> 455, with two such counters).
+__global__ void deform_clear_counter_kernel(unsigned int *counter) {
+    begin_after_previous();
+    *counter = 0u;
+}
+static cudaError_t clear_counter(unsigned int *counter, cudaStream_t st) {
+    launch_next(deform_clear_counter_kernel, 1, 1, 0, st, counter);
+    return cudaGetLastError();
+}
 
 static int memset_async(void *p, size_t bytes, cudaStream_t st, const char *fn) {
     const cudaError_t e = cudaMemsetAsync(p, 0, bytes, st);
@@ -1102,8 +1119,8 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     void *window = dense + (size_t)B * G * 25 * hi;
     OutlierTap *taps = reinterpret_cast<OutlierTap *>(dense + (size_t)B * G * 50 * hi);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * hi);
-    if (cudaMemsetAsync(tap_count, 0, sizeof(unsigned int), st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed: %s", fn, cudaGetErrorString(cudaGetLastError()));
+    if (clear_counter(tap_count, st) != cudaSuccess) {
+        set_error("%s: clearing the outlier counter failed", fn);
         return SAPA_ERR_LAUNCH;
     }
     // 1. dense 25-slot similarity of every group: the B x G groups are images of Cq / G channels.  16-bit tensors: the
@@ -1122,10 +1139,10 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
             const scalar_t *o = static_cast<const scalar_t *>(offset);
             scalar_t *at = static_cast<scalar_t *>(attn), *wn = static_cast<scalar_t *>(window);
             if (P == 9)          // the 3 x 3 points of the reference modules' default
-                deform_window_kernel<scalar_t, 9, WIN_FUSED><<<grid, WIN_THREADS, 0, st>>>(q, k, o, dense, at, wn, taps, tap_count, B, Cq,
+                launch_next(deform_window_kernel<scalar_t, 9, WIN_FUSED>, grid, WIN_THREADS, 0, st, q, k, o, dense, at, wn, taps, tap_count, B, Cq,
                                                                                   H, W, P, G, rows, halo_top);
             else
-                deform_window_kernel<scalar_t, 0, WIN_FUSED><<<grid, WIN_THREADS, 0, st>>>(q, k, o, dense, at, wn, taps, tap_count, B, Cq,
+                launch_next(deform_window_kernel<scalar_t, 0, WIN_FUSED>, grid, WIN_THREADS, 0, st, q, k, o, dense, at, wn, taps, tap_count, B, Cq,
                                                                                   H, W, P, G, rows, halo_top);
             return check_launch("deform_window_kernel");
         });
@@ -1135,7 +1152,7 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     if (int e = run_agg_slab(window, value, out, B * G, C / G, H, W, rows, halo_top, 5, 2, dtype, st)) return e;
     // 4. the listed points (the count is only known on the device: a fixed grid strides over the list)
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        deform_outlier_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(value),
+        launch_next(deform_outlier_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(value),
                                                                  static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(out),
                                                                  C, H, W, P, G, rows, halo_top);
         return check_launch("deform_outlier_kernel");
@@ -1174,11 +1191,11 @@ int sapa_deform_qk_forward_dense(const void *query, const void *key, const void 
     const long long total = (long long)B * G * hi;
     return SAPA_DISPATCH_FAST(dtype, [&] {
         if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-            deform_window_kernel<scalar_t, 9, WIN_LOGITS><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+            launch_next(deform_window_kernel<scalar_t, 9, WIN_LOGITS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                 static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
                 static_cast<scalar_t *>(out), nullptr, nullptr, nullptr, B, Cq, H, W, P, G, H, 0);
         else
-            deform_window_kernel<scalar_t, 0, WIN_LOGITS><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+            launch_next(deform_window_kernel<scalar_t, 0, WIN_LOGITS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                 static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
                 static_cast<scalar_t *>(out), nullptr, nullptr, nullptr, B, Cq, H, W, P, G, H, 0);
         return check_launch("deform_window_kernel<logits>");
@@ -1202,19 +1219,19 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
     float *region = static_cast<float *>(workspace) + (size_t)B * G * 25 * hi;      // the window weights (tensor type) live here
     OutlierTap *taps = reinterpret_cast<OutlierTap *>(region + (size_t)B * G * 25 * hi);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * hi);
-    if (cudaMemsetAsync(tap_count, 0, sizeof(unsigned int), st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed: %s", fn, cudaGetErrorString(cudaGetLastError()));
+    if (clear_counter(tap_count, st) != cudaSuccess) {
+        set_error("%s: clearing the outlier counter failed", fn);
         return SAPA_ERR_LAUNCH;
     }
     const long long total = (long long)B * G * hi;
     // the attention is only read in this mode
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                deform_window_kernel<scalar_t, 9, WIN_WEIGHTS><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+                launch_next(deform_window_kernel<scalar_t, 9, WIN_WEIGHTS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr, const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)),
                     reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C, H, W, P, G, H, 0);
             else
-                deform_window_kernel<scalar_t, 0, WIN_WEIGHTS><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+                launch_next(deform_window_kernel<scalar_t, 0, WIN_WEIGHTS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr, const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)),
                     reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C, H, W, P, G, H, 0);
             return check_launch("deform_window_kernel<weights>");
@@ -1222,7 +1239,7 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
         return e;
     if (int e = run_agg(region, value, out, B * G, C / G, H, W, 5, 2, dtype, st)) return e;
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        deform_outlier_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(value),
+        launch_next(deform_outlier_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(value),
                                                                  static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(out), C, H,
                                                                  W, P, G, H, 0);
         return check_launch("deform_outlier_kernel");
@@ -1273,8 +1290,8 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     void *ddense = dwin + plane, *window = dwin + 2 * plane;
     OutlierGrad *taps = reinterpret_cast<OutlierGrad *>(dense + 4 * plane);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
-    if (cudaMemsetAsync(tap_count, 0, sizeof(unsigned int), st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed: %s", fn, cudaGetErrorString(cudaGetLastError()));
+    if (clear_counter(tap_count, st) != cudaSuccess) {
+        set_error("%s: clearing the outlier counter failed", fn);
         return SAPA_ERR_LAUNCH;
     }
     // 1. D = sim(Q, Key) and dWd = sim(dOut, Value), the B x G groups as images
@@ -1294,10 +1311,10 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
             const scalar_t *o = static_cast<const scalar_t *>(offset), *a = static_cast<const scalar_t *>(attn);
             scalar_t *dd = static_cast<scalar_t *>(ddense), *wn = static_cast<scalar_t *>(window), *goff = static_cast<scalar_t *>(grad_offset);
             if (P == 9)
-                deform_window_bwd_kernel<scalar_t, 9, BWD_FUSED><<<grid, WIN_THREADS, 0, st>>>(go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
+                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
                                                                                       tap_count, B, C, H, W, P, G);
             else
-                deform_window_bwd_kernel<scalar_t, 0, BWD_FUSED><<<grid, WIN_THREADS, 0, st>>>(go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
+                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
                                                                                       tap_count, B, C, H, W, P, G);
             return check_launch("deform_window_bwd_kernel");
         });
@@ -1310,7 +1327,7 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     // 4. the listed points.  float32: atomics straight into the gradients.  16-bit: key / value contributions go to zeroed
     //    float32 side buffers behind the list and are folded into the 16-bit gradients by one more kernel.
     if (dtype == SAPA_F32) {
-        deform_outlier_bwd_kernel<float, float><<<148 * 8, 256, 0, st>>>(
+        launch_next(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const float *>(grad_out), static_cast<const float *>(query), static_cast<const float *>(key),
             static_cast<const float *>(value), static_cast<const float *>(offset), static_cast<float *>(grad_query),
             static_cast<float *>(grad_key), static_cast<float *>(grad_value), static_cast<float *>(grad_offset), Cq, C, H, W, P, G);
@@ -1320,14 +1337,14 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     float *side_k = reinterpret_cast<float *>(static_cast<char *>(workspace) + side_off), *side_v = side_k + n_k;
     const Scatter sc{side_k, side_v, n_k, n_v, Cq / G, C / G};
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        deform_zero_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
+        launch_next(deform_zero_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
         if (int e = check_launch("deform_zero_scatter_kernel")) return e;
-        deform_outlier_bwd_kernel<scalar_t, float><<<148 * 8, 256, 0, st>>>(
+        launch_next(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(query),
             static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
             static_cast<scalar_t *>(grad_query), side_k, side_v, static_cast<scalar_t *>(grad_offset), Cq, C, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
-        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(grad_key),
+        launch_next(deform_add_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(grad_key),
                                                                      static_cast<scalar_t *>(grad_value), H, W, P);
         return check_launch("deform_add_scatter_kernel");
     });
@@ -1357,8 +1374,8 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     void *window = dwin + 2 * plane;                                   // Wd, in the tensors' type
     OutlierGrad *taps = reinterpret_cast<OutlierGrad *>(static_cast<float *>(workspace) + 4 * plane);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
-    if (cudaMemsetAsync(tap_count, 0, sizeof(unsigned int), st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed: %s", fn, cudaGetErrorString(cudaGetLastError()));
+    if (clear_counter(tap_count, st) != cudaSuccess) {
+        set_error("%s: clearing the outlier counter failed", fn);
         return SAPA_ERR_LAUNCH;
     }
     if (dtype == SAPA_F32) {
@@ -1369,12 +1386,12 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     const long long total = (long long)B * G * hi;
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                deform_window_bwd_kernel<scalar_t, 9, BWD_AV><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_AV>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                     static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
                     static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
                     static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
             else
-                deform_window_bwd_kernel<scalar_t, 0, BWD_AV><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_AV>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                     static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
                     static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
                     static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
@@ -1383,7 +1400,7 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
         return e;
     if (int e = run_gath(grad_out, window, grad_value, B * G, C / G, H, W, 5, 2, dtype, st)) return e;  // dV
     if (dtype == SAPA_F32) {
-        deform_outlier_bwd_kernel<float, float><<<148 * 8, 256, 0, st>>>(
+        launch_next(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const float *>(grad_out), nullptr, nullptr, static_cast<const float *>(value),
             static_cast<const float *>(offset), nullptr, nullptr, static_cast<float *>(grad_value), static_cast<float *>(grad_offset),
             C, C, H, W, P, G);
@@ -1393,13 +1410,13 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     float *side_v = reinterpret_cast<float *>(static_cast<char *>(workspace) + side_off);
     const Scatter sc{nullptr, side_v, 0, n_v, 0, C / G};
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        deform_zero_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
+        launch_next(deform_zero_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
         if (int e = check_launch("deform_zero_scatter_kernel")) return e;
-        deform_outlier_bwd_kernel<scalar_t, float><<<148 * 8, 256, 0, st>>>(
+        launch_next(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const scalar_t *>(grad_out), nullptr, nullptr, static_cast<const scalar_t *>(value),
             static_cast<const scalar_t *>(offset), nullptr, nullptr, side_v, static_cast<scalar_t *>(grad_offset), C, C, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
-        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(nullptr),
+        launch_next(deform_add_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(nullptr),
                                                                      static_cast<scalar_t *>(grad_value), H, W, P);
         return check_launch("deform_add_scatter_kernel");
     });
@@ -1427,8 +1444,8 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     void *ddense = dense + 2 * plane;                                  // dD, in the tensors' type
     OutlierGrad *taps = reinterpret_cast<OutlierGrad *>(dense + 4 * plane);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
-    if (cudaMemsetAsync(tap_count, 0, sizeof(unsigned int), st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed: %s", fn, cudaGetErrorString(cudaGetLastError()));
+    if (clear_counter(tap_count, st) != cudaSuccess) {
+        set_error("%s: clearing the outlier counter failed", fn);
         return SAPA_ERR_LAUNCH;
     }
     if (dtype == SAPA_F32) {
@@ -1440,11 +1457,11 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     // the logit gradients enter where the fused chain reads the attention
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                deform_window_bwd_kernel<scalar_t, 9, BWD_QK><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_QK>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
                     static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
             else
-                deform_window_bwd_kernel<scalar_t, 0, BWD_QK><<<grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st>>>(
+                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_QK>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
                     static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
             return check_launch("deform_window_bwd_kernel<qk>");
@@ -1453,7 +1470,7 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     if (int e = run_agg(ddense, key, grad_query, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;       // dQ
     if (int e = run_gath(query, ddense, grad_key, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;      // dKey
     if (dtype == SAPA_F32) {
-        deform_outlier_bwd_kernel<float, float><<<148 * 8, 256, 0, st>>>(
+        launch_next(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, nullptr, static_cast<const float *>(query), static_cast<const float *>(key), nullptr,
             static_cast<const float *>(offset), static_cast<float *>(grad_query), static_cast<float *>(grad_key), nullptr,
             static_cast<float *>(grad_offset), Cq, Cq, H, W, P, G);
@@ -1463,14 +1480,14 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     float *side_k = reinterpret_cast<float *>(static_cast<char *>(workspace) + side_off);
     const Scatter sc{side_k, nullptr, n_k, 0, Cq / G, 0};
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        deform_zero_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
+        launch_next(deform_zero_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
         if (int e = check_launch("deform_zero_scatter_kernel")) return e;
-        deform_outlier_bwd_kernel<scalar_t, float><<<148 * 8, 256, 0, st>>>(
+        launch_next(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
             taps, tap_count, nullptr, static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), nullptr,
             static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(grad_query), side_k, nullptr,
             static_cast<scalar_t *>(grad_offset), Cq, Cq, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
-        deform_add_scatter_kernel<scalar_t><<<148 * 8, 256, 0, st>>>(taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(grad_key),
+        launch_next(deform_add_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, static_cast<scalar_t *>(grad_key),
                                                                      static_cast<scalar_t *>(nullptr), H, W, P);
         return check_launch("deform_add_scatter_kernel");
     });

@@ -145,6 +145,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+    begin_after_previous();
 
     if constexpr (RAGGED) {
         if (warp >= NW) {
@@ -474,11 +475,11 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
     if constexpr (!F32)
         if (ragged || wide) {
-            if (ragged) sapa_gath_mma_kernel<T, true><<<grid, f.threads, f.smem, st>>>(xmap, a);
-            else sapa_gath_wide_16_kernel<T><<<grid, f.threads, f.smem, st>>>(xmap, bmap, a);
+            if (ragged) launch_next(sapa_gath_mma_kernel<T, true>, grid, f.threads, f.smem, st, xmap, a);
+            else launch_next(sapa_gath_wide_16_kernel<T>, grid, f.threads, f.smem, st, xmap, bmap, a);
             return check_launch(name);
         }
-    sapa_gath_mma_kernel<T, false><<<grid, f.threads, f.smem, st>>>(xmap, a);
+    launch_next(sapa_gath_mma_kernel<T, false>, grid, f.threads, f.smem, st, xmap, a);
     return check_launch(name);
 }
 

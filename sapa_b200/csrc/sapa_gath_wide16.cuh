@@ -48,6 +48,7 @@ sapa_gath_wide_16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+    begin_after_previous();
 
     if (warp >= gw16::NW) {           // producer: one lane; the stages of successive items form one stream through the ring
         asm volatile("setmaxnreg.dec.sync.aligned.u32 24;\n");

@@ -207,6 +207,7 @@ constexpr int NT32 = 2 * ROWS * 32;
 
 template <int HB, int QB>
 __global__ void __launch_bounds__(NT32, 2) sapa_mma_fused_f32_kernel(const Args a) {
+    begin_after_previous();
     using T = float;
     using G = Geo<float>;
     constexpr int PLANE = G::PLANE, QPLANE = G::QPLANE, VCH = G::VCH, NBLK = VCH / 16;
@@ -390,6 +391,7 @@ __global__ void __launch_bounds__(NT32, 2) sapa_mma_fused_f32_kernel(const Args 
 // HBV / QB: bytes per cp.async of the value halo / of the query tile (the key halo always uses 4-byte copies)
 template <typename T, int HBV, int QB>
 __global__ void __launch_bounds__(NT, 3) sapa_mma_fused_16_kernel(const Args a) {
+    begin_after_previous();
     using G = Geo<T>;
     constexpr int PLANE = G::PLANE, QPLANE = G::QPLANE, VCH = G::VCH, NBLK = VCH / 16;
     constexpr int PLANE_B = PLANE * 2, QPLANE_B = QPLANE * 2;
@@ -586,7 +588,7 @@ static int launch_with_smem(Kernel kernel, int threads, int smem, const Args &a,
         set_error("sapa_mma_fused_kernel: cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
         return SAPA_ERR_LAUNCH;
     }
-    kernel<<<blocks, threads, smem, st>>>(a);
+    launch_next(kernel, blocks, threads, smem, st, a);
     return check_launch("sapa_mma_fused_kernel");
 }
 

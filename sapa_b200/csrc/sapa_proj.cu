@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
     }
     tc_fence_before();
     __syncthreads();
+    begin_after_previous();
     tc_fence_after();
     unsigned tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot) : "memory");
@@ -437,6 +438,7 @@ struct StatList { StatProblem p[MAX_PROBLEMS]; int count; };
 // partial sums of at most 32 elements, float64 beyond)
 template <typename T>
 __global__ void __launch_bounds__(STAT_THREADS) gn_partial_kernel(const __grid_constant__ StatList list) {
+    begin_after_previous();
     constexpr int VN = Vec16<T>::N;
     __shared__ double scratch[STAT_THREADS / 32];
     int i = 0;
@@ -495,6 +497,7 @@ template <typename T> __device__ __forceinline__ void fetch16(const T *p, bool v
 // d = 32, C = 256; this form 4.3.)
 template <typename T>
 __global__ void __launch_bounds__(STAT_THREADS) gn_fold_kernel(const __grid_constant__ FoldList list) {
+    begin_after_previous();
     constexpr int VN = Vec16<T>::N;
     __shared__ float s_mean[MAX_GROUPS], s_rstd[MAX_GROUPS];
     int i = 0;
@@ -683,11 +686,11 @@ static int run_parts(const Part *parts, int count, unsigned char *ws, cudaStream
         }
     }
     if (sl.count > 0) {
-        gn_partial_kernel<T><<<sblocks, STAT_THREADS, 0, st>>>(sl);
+        launch_next(gn_partial_kernel<T>, sblocks, STAT_THREADS, 0, st, sl);
         if (int e = check_launch("gn_partial_kernel")) return e;
     }
     if (fl.count > 0) {
-        gn_fold_kernel<T><<<fblocks, STAT_THREADS, 0, st>>>(fl);
+        launch_next(gn_fold_kernel<T>, fblocks, STAT_THREADS, 0, st, fl);
         if (int e = check_launch("gn_fold_kernel")) return e;
     }
 
@@ -726,7 +729,7 @@ static int run_parts(const Part *parts, int count, unsigned char *ws, cudaStream
     a.nx = l.nx; a.no = l.no; a.tmem_cols = l.tmem_cols; a.acc_cols = acc_cols;
     int sms = 0;
     if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_proj_umma_kernel<T, TO>), SMEM_LIMIT, "sapa_proj_umma_kernel", sms)) return e;
-    sapa_proj_umma_kernel<T, TO><<<std::min(a.total_tiles, sms), THREADS, l.smem, st>>>(a);
+    launch_next(sapa_proj_umma_kernel<T, TO>, std::min(a.total_tiles, sms), THREADS, l.smem, st, a);
     return check_launch("sapa_proj_umma_kernel");
 }
 

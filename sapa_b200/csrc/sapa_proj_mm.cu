@@ -76,6 +76,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // ---------------------------------------------------------------------------------- statistics
 template <typename T>
 __global__ void __launch_bounds__(THREADS) proj_stats_kernel(const __grid_constant__ StatList list) {
+    begin_after_previous();
     __shared__ double sc[2][THREADS / 32];
     int block = blockIdx.x;
     const StatProblem &q = list.p[find_problem(list, block)];
@@ -113,6 +114,7 @@ constexpr int MM_P = 128, MM_K = 32, MM_APITCH = 36, MM_XPITCH = 136;
 
 template <typename T, typename TO, int MT>
 __global__ void __launch_bounds__(THREADS, 3) proj_fwd_kernel(const __grid_constant__ FwdList list) {
+    begin_after_previous();
     constexpr bool LO = sizeof(TO) == 4;                        // float32 output: three-term products
     constexpr int WM = MT / 32, NT = 16 / (8 / WM), WPX = 8 * NT;      // warps along the rows; 8-pixel tiles / pixels of a warp
     __shared__ __align__(16) float as[MT * MM_APITCH], xs[MM_K * MM_XPITCH];
@@ -236,6 +238,7 @@ constexpr int MO_C = 64, MO_J = 64, MO_P = 64, MO_PITCH = 68;
 
 template <typename T, typename TG, bool NORM>
 __global__ void __launch_bounds__(THREADS, 2) proj_moments_kernel(const __grid_constant__ MomentList list) {
+    begin_after_previous();
     constexpr bool LO = sizeof(TG) == 4;
     extern __shared__ __align__(16) float mo_smem[];
     float *xs = mo_smem, *gs = xs + MO_C * MO_PITCH, *ws = gs + MO_J * MO_PITCH;      // ws (NORM only) = W^T: row = channel, column = row of dq
@@ -390,6 +393,7 @@ __global__ void __launch_bounds__(THREADS, 2) proj_moments_kernel(const __grid_c
 // Blocks of a problem: first the rows of W (256 channels each), then one per group of channels for gamma, beta and the tail.
 template <typename T>
 __global__ void __launch_bounds__(THREADS) proj_fold_kernel(const __grid_constant__ FoldList list) {
+    begin_after_previous();
     __shared__ float sm[2][THREADS];
     int block = blockIdx.x;
     const FoldProblem &f = list.p[find_problem(list, block)];
@@ -462,6 +466,7 @@ constexpr int DX_M = 64, DX_P = 64, DX_XPITCH = 72;
 
 template <typename T, typename TG>
 __global__ void __launch_bounds__(THREADS, sizeof(TG) == 4 ? 2 : 3) proj_dx_kernel(const __grid_constant__ DxList list) {
+    begin_after_previous();
     constexpr bool LO = sizeof(TG) == 4;
     __shared__ __align__(16) float as[DX_M * MM_APITCH], xs[MM_K * DX_XPITCH];
     int block = blockIdx.x;
@@ -621,11 +626,11 @@ static int run_forward(const sapa_projection *q, int count, unsigned char *ws, c
         f.partial = t.partial; f.nsplit = t.nsplit; f.n = t.n; f.stats = static_cast<float2 *>(s.stats);
     }
     if (sl.count > 0) {
-        proj_stats_kernel<T><<<sblocks, THREADS, 0, st>>>(sl);
+        launch_next(proj_stats_kernel<T>, sblocks, THREADS, 0, st, sl);
         if (int e = check_launch("proj_stats_kernel")) return e;
     }
-    if (mt == 32) proj_fwd_kernel<T, TO, 32><<<fblocks, THREADS, 0, st>>>(fl);
-    else proj_fwd_kernel<T, TO, 64><<<fblocks, THREADS, 0, st>>>(fl);
+    if (mt == 32) launch_next(proj_fwd_kernel<T, TO, 32>, fblocks, THREADS, 0, st, fl);
+    else launch_next(proj_fwd_kernel<T, TO, 64>, fblocks, THREADS, 0, st, fl);
     return check_launch("proj_fwd_kernel");
 }
 
@@ -712,17 +717,17 @@ static int run_backward(const sapa_projection_grad *q, int count, unsigned char 
     int sms = 0;
     if (ml[1].count > 0) {
         if (int e = prepare_launch(reinterpret_cast<const void *>(proj_moments_kernel<T, TG, true>), smem_norm, "proj_moments_kernel", sms)) return e;
-        proj_moments_kernel<T, TG, true><<<mblocks[1], THREADS, smem_norm, st>>>(ml[1]);
+        launch_next(proj_moments_kernel<T, TG, true>, mblocks[1], THREADS, smem_norm, st, ml[1]);
         if (int e = check_launch("proj_moments_kernel")) return e;
     }
     if (ml[0].count > 0) {
-        proj_moments_kernel<T, TG, false><<<mblocks[0], THREADS, smem_plain, st>>>(ml[0]);
+        launch_next(proj_moments_kernel<T, TG, false>, mblocks[0], THREADS, smem_plain, st, ml[0]);
         if (int e = check_launch("proj_moments_kernel")) return e;
     }
-    proj_fold_kernel<T><<<fblocks, THREADS, 0, st>>>(fl);
+    launch_next(proj_fold_kernel<T>, fblocks, THREADS, 0, st, fl);
     if (int e = check_launch("proj_fold_kernel")) return e;
     if (dl.count == 0) return SAPA_OK;
-    proj_dx_kernel<T, TG><<<dblocks, THREADS, 0, st>>>(dl);
+    launch_next(proj_dx_kernel<T, TG>, dblocks, THREADS, 0, st, dl);
     return check_launch("proj_dx_kernel");
 }
 

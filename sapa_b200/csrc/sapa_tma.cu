@@ -110,6 +110,7 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+    begin_after_previous();
 
     // Stages are issued in stream order (stage gs goes to slot gs % NSTAGE) by thread 0 only.  The producer keeps its
     // position incrementally: per stage it costs a handful of instructions, which matters because the other seven
@@ -599,6 +600,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
     if constexpr (RAGGED)       // box columns that are never copied must read as zero
         for (int i = tid; i < h16::NSTAGE * h16::SLOT_BYTES / 4; i += h16::NT_RAGGED) sts32(ring_addr + 4 * i, 0u);
     __syncthreads();
+    begin_after_previous();
 
     if constexpr (RAGGED) {
         if (warp >= NW) {
@@ -1102,7 +1104,7 @@ static int launch_persistent(Kernel kernel, const char *name, int threads, int s
     // persistent grid with dynamic tile claiming (static striding left SMs with 6 to 8 tiles instead of ~6.9)
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
-    kernel<<<grid, threads, smem, st>>>(maps..., a);
+    launch_next(kernel, grid, threads, smem, st, maps..., a);
     return check_launch(name);
 }
 

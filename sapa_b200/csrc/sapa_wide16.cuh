@@ -67,6 +67,7 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
+    begin_after_previous();
 
     if (warp >= w16::NW) {            // producer: one lane; the stages of successive items form one stream through the ring
         asm volatile("setmaxnreg.dec.sync.aligned.u32 24;\n");
