@@ -304,11 +304,48 @@ struct WindowTap {
 // fused op writes the attention (deform_qk); WIN_WEIGHTS = window weights from a given attention map (deform_av).
 constexpr int WIN_FUSED = 0, WIN_LOGITS = 1, WIN_WEIGHTS = 2;
 
+// The points of a pixel inside its window: fractional parts, and the place of the upper-left cell in the thread's column of a
+// [25][WIN_THREADS] array, two points to a register.  Points that are not dense have place 0 and take no part (see `dense`).
+template <int PMAX>
+struct WindowPoints {
+    float lh[PMAX], lw[PMAX];
+    unsigned place[(PMAX + 1) / 2], dense, outliers;
+    __device__ __forceinline__ int at(int p) const { return (int)(p & 1 ? place[p >> 1] >> 16 : place[p >> 1] & 0xffffu); }
+    template <typename T>
+    __device__ __forceinline__ void setup(const T *offp, size_t hi, bool live, int P, int rows, int W, int py, int px) {
+        float ow[PMAX], oh[PMAX];
+#pragma unroll
+        for (int p = 0; p < PMAX; ++p) {
+            const bool on = live && p < P;
+            ow[p] = on ? to_acc(__ldg(offp + (size_t)(2 * p) * hi)) : 0.f;
+            oh[p] = on ? to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi)) : 0.f;
+        }
+        dense = outliers = 0u;
+#pragma unroll
+        for (int p = 0; p < PMAX; ++p) {
+            WindowTap t;
+            t.setup(float(py) + oh[p], float(px) + ow[p], rows, W, py, px);
+            const bool on = live && p < P, in = on && t.dense;
+            lh[p] = t.lh; lw[p] = t.lw;
+            const unsigned c = in ? (unsigned)((t.r0 * 5 + t.c0) * WIN_THREADS) : 0u;
+            place[p >> 1] = p & 1 ? place[p >> 1] | (c << 16) : c;
+            dense |= in ? 1u << p : 0u;
+            outliers |= on && t.inside && !t.dense ? 1u << p : 0u;
+        }
+    }
+};
+template <int N> __device__ __forceinline__ void put(float (&v)[N], int p, float x) {      // at a place known at run time
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = j == p ? x : v[j];
+}
+
 // The two 25-slot windows of a thread (similarity in, window weights out) live in shared memory, column = thread, so
 // every access is conflict-free: a point touches four cells of each window, and shared memory can be indexed with the
 // cell computed at run time (a register array cannot: that form multiplies every point with all 25 cells and took
-// 82 us where this takes 56 us at B=8, 4 groups, 128 x 128 pixels).  Two passes over the points: logits and their
-// maximum, then exp and the window weights.  Six blocks per SM (80 registers; 4 and 8 measured slower).
+// 82 us at B=8, 4 groups, 128 x 128 pixels).  Two passes over the points: logits and their maximum, then exp and the window
+// weights.  Bound by latency at 24 warps per SM (80 registers; 4 and 8 blocks measured slower), so the points go side by side:
+// no branch on a point (what it must not add is multiplied by zero weights or selected away; outliers have a loop of their own), places
+// kept from pass to pass, block = pixels of one (image, group) instead of 64-bit divisions per thread: 55 -> 43 us (float32; bfloat16 59 -> 44).
 template <typename T, int NP, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 6)
 deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, const T *__restrict__ offset,
@@ -320,90 +357,81 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
     __shared__ float sd[MODE != WIN_WEIGHTS ? 25 : 1][WIN_THREADS];     // dense similarity of the thread's pixel
     __shared__ float sw[MODE != WIN_LOGITS ? 25 : 1][WIN_THREADS];      // window weights being collected
     const int P = NP > 0 ? NP : P_runtime;
-    const int sH = 2 * H, sW = 2 * W, gq = Cq / G;
-    const size_t hi = (size_t)sH * sW, lo = (size_t)rows * W;
+    const unsigned sW = 2 * W;
+    const int gq = Cq / G;
+    const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)rows * W;
     const int lane = threadIdx.x & 31, tid = threadIdx.x;
-    const long long total = (long long)B * G * hi;
-    for (long long i0 = (long long)blockIdx.x * WIN_THREADS; i0 < total; i0 += (long long)gridDim.x * WIN_THREADS) {
-        const long long i = i0 + tid;
-        const bool live = i < total;
-        const size_t pix = live ? (size_t)(i % hi) : 0;
-        const long long bg = live ? i / (long long)hi : 0;
-        const int g = (int)(bg % G), b = (int)(bg / G);
-        const int qw = (int)(pix % sW), qh = (int)(pix / sW), py = (qh >> 1) + ytop, px = qw >> 1;
+    const unsigned blocks = ((unsigned)hi + WIN_THREADS - 1) / WIN_THREADS, groups = (unsigned)(B * G);      // of an (image, group)
+    float *const dcol = &sd[0][tid], *const wcol = &sw[0][tid];
+    for (unsigned bg = blockIdx.y; bg < groups; bg += gridDim.y)
+    for (unsigned block = blockIdx.x; block < blocks; block += gridDim.x) {
+        const unsigned at_pix = block * WIN_THREADS + tid, pix = at_pix < hi ? at_pix : 0u;
+        const bool live = at_pix < hi;
+        const int qh = (int)(pix / sW), qw = (int)(pix - (unsigned)qh * sW), py = (qh >> 1) + ytop, px = qw >> 1;
+        const T *offp = offset + (size_t)bg * P * 2 * hi + pix;
+        WindowPoints<PMAX> pts;
         if (MODE != WIN_WEIGHTS) {
             const float *dp = dense + (size_t)bg * 25 * hi + pix;
 #pragma unroll
-            for (int k = 0; k < 25; ++k) sd[k][tid] = live ? __ldcs(dp + (size_t)k * hi) : 0.f;
+            for (int k = 0; k < 25; ++k) dcol[k * WIN_THREADS] = live ? __ldcs(dp + (size_t)k * hi) : 0.f;
         }
         if (MODE != WIN_LOGITS) {
 #pragma unroll
-            for (int k = 0; k < 25; ++k) sw[k][tid] = 0.f;
+            for (int k = 0; k < 25; ++k) wcol[k * WIN_THREADS] = 0.f;
         }
-        float oh[PMAX], ow[PMAX], logit[PMAX];
-        const T *offp = offset + (size_t)bg * P * 2 * hi + pix;
+        pts.setup(offp, hi, live, P, rows, W, py, px);
+        // ---- pass 1: logits (or the given attention)
+        float logit[PMAX];
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
-            const bool on = live && p < P;
-            ow[p] = on ? float(px) + to_acc(__ldg(offp + (size_t)(2 * p) * hi)) : 0.f;
-            oh[p] = on ? float(py) + to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi)) : 0.f;
+            if (MODE == WIN_WEIGHTS) {
+                logit[p] = live && p < P ? to_acc(__ldg(attn + ((size_t)bg * P + p) * hi + pix)) : 0.f;
+            } else {
+                const float *c = dcol + pts.at(p);
+                const float top = (1.f - pts.lw[p]) * c[0] + pts.lw[p] * c[WIN_THREADS];
+                const float bot = (1.f - pts.lw[p]) * c[5 * WIN_THREADS] + pts.lw[p] * c[6 * WIN_THREADS];
+                logit[p] = pts.dense >> p & 1 ? (1.f - pts.lh[p]) * top + pts.lh[p] * bot : 0.f;
+            }
         }
-        unsigned int outliers = 0;
-        float m = -INFINITY;
-        // ---- pass 1: logits (or the given attention) and which points leave the window
-#pragma unroll
-        for (int p = 0; p < PMAX; ++p) {
-            logit[p] = 0.f;
-            if (live && p < P) {
-                WindowTap t;
-                t.setup(oh[p], ow[p], rows, W, py, px);
-                if (!t.dense && t.inside) outliers |= 1u << p;
+        if (MODE != WIN_WEIGHTS)
+            for (unsigned left = pts.outliers; left != 0; left &= left - 1) {      // outliers: gather the key directly
+                const int p = __ffs(left) - 1;
+                Bilinear<float> bl;
+                bl.setup(float(py) + to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi)), float(px) + to_acc(__ldg(offp + (size_t)(2 * p) * hi)), rows, W);
+                const T *qp = query + (size_t)bg * gq * hi + pix, *kp = key + (size_t)bg * gq * lo;
                 float acc = 0.f;
-                if (MODE == WIN_WEIGHTS) {
-                    acc = to_acc(__ldg(attn + ((size_t)bg * P + p) * hi + pix));
-                } else if (t.dense) {
-                    const int c = t.r0 * 5 + t.c0;
-                    const float top = (1.f - t.lw) * sd[c][tid] + t.lw * sd[c + 1][tid];
-                    const float bot = (1.f - t.lw) * sd[c + 5][tid] + t.lw * sd[c + 6][tid];
-                    acc = (1.f - t.lh) * top + t.lh * bot;
-                } else if (t.inside) {        // outlier: gather the key directly
-                    Bilinear<float> bl;
-                    bl.setup(oh[p], ow[p], rows, W);
-                    const T *qp = query + ((size_t)b * Cq + (size_t)g * gq) * hi + pix;
-                    const T *kp = key + ((size_t)b * Cq + (size_t)g * gq) * lo;
-                    for (int ch = 0; ch < gq; ++ch) acc += bl.sample(kp + (size_t)ch * lo) * to_acc(qp[(size_t)ch * hi]);
-                }
-                logit[p] = acc;
-                m = fmaxf(m, acc);
-                if (MODE == WIN_LOGITS) attn[((size_t)bg * P + p) * hi + pix] = from_acc<T>(acc);
+                for (int ch = 0; ch < gq; ++ch) acc += bl.sample(kp + (size_t)ch * lo) * to_acc(qp[(size_t)ch * hi]);
+                put(logit, p, acc);
             }
+        if (MODE == WIN_LOGITS) {
+#pragma unroll
+            for (int p = 0; p < PMAX; ++p)
+                if (live && p < P) attn[((size_t)bg * P + p) * hi + pix] = from_acc<T>(logit[p]);
+            continue;                                       // no lane-crossing operation below was entered by any lane yet
         }
-        if (MODE == WIN_LOGITS) continue;                   // no lane-crossing operation below was entered by any lane yet
-        // ---- pass 2: exp and the window weights (the bilinear set-up is recomputed: cheaper than keeping it)
-        float z = 0.f;
+        // ---- pass 2: exp and the window weights
+        float m = -INFINITY, z = 0.f;
+#pragma unroll
+        for (int p = 0; p < PMAX; ++p)
+            if (p < P) m = fmaxf(m, logit[p]);
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
-            if (live && p < P) {
-                const float e = MODE == WIN_WEIGHTS ? logit[p] : __expf(logit[p] - m);
-                logit[p] = e;
-                z += e;
-                WindowTap t;
-                t.setup(oh[p], ow[p], rows, W, py, px);
-                if (t.dense) {
-                    const int c = t.r0 * 5 + t.c0;
-                    const float et = e * (1.f - t.lh), eb = e * t.lh;
-                    sw[c][tid] += et * (1.f - t.lw);
-                    sw[c + 1][tid] += et * t.lw;
-                    sw[c + 5][tid] += eb * (1.f - t.lw);
-                    sw[c + 6][tid] += eb * t.lw;
-                }
-            }
+            const float e = p < P ? MODE == WIN_WEIGHTS ? logit[p] : __expf(logit[p] - m) : 0.f;
+            logit[p] = e;
+            z += e;
+            const float add = pts.dense >> p & 1 ? e : 0.f, et = add * (1.f - pts.lh[p]), eb = add * pts.lh[p];
+            float *c = wcol + pts.at(p);
+            const float c00 = c[0], c01 = c[WIN_THREADS], c10 = c[5 * WIN_THREADS], c11 = c[6 * WIN_THREADS];
+            c[0] = c00 + et * (1.f - pts.lw[p]);
+            c[WIN_THREADS] = c01 + et * pts.lw[p];
+            c[5 * WIN_THREADS] = c10 + eb * (1.f - pts.lw[p]);
+            c[6 * WIN_THREADS] = c11 + eb * pts.lw[p];
         }
         const float inv = MODE == WIN_WEIGHTS ? 1.f : 1.f / z;
         if (live) {
             T *wp = window + (size_t)bg * 25 * hi + pix;
 #pragma unroll
-            for (int k = 0; k < 25; ++k) wp[(size_t)k * hi] = from_acc<T>(sw[k][tid] * inv);
+            for (int k = 0; k < 25; ++k) wp[(size_t)k * hi] = from_acc<T>(wcol[k * WIN_THREADS] * inv);
         }
         if (MODE == WIN_FUSED) {
 #pragma unroll
@@ -413,15 +441,15 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
             }
         }
         // append the pixels of this warp that have outlier points to the list: one counter update per warp
-        const unsigned int any = __ballot_sync(0xffffffffu, outliers != 0);
+        const unsigned int any = __ballot_sync(0xffffffffu, pts.outliers != 0);
         if (any != 0) {
             unsigned int base = 0;
             if (lane == 0) base = atomicAdd(tap_count, (unsigned int)__popc(any));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (outliers != 0) {
+            if (pts.outliers != 0) {
                 OutlierTap *t = taps + base + __popc(any & ((1u << lane) - 1u));
-                t->idx = (unsigned int)i;
-                t->mask = outliers;
+                t->idx = (unsigned int)(bg * hi + pix);
+                t->mask = pts.outliers;
 #pragma unroll
                 for (int p = 0; p < PMAX; ++p) t->a[p] = logit[p];
             }
@@ -897,6 +925,11 @@ static inline int grid_1d(long long total, int threads) {
     return (int)(blocks < cap ? (blocks < 1 ? 1 : blocks) : cap);
 }
 
+// blocks of the window kernels: pixels of an (image, group) along x, the (image, group)s along y
+static dim3 window_grid(int groups, size_t hi) {
+    return dim3((unsigned)((hi + WIN_THREADS - 1) / WIN_THREADS), (unsigned)(groups < 65535 ? groups : 65535), 1);
+}
+
 static int check_deform(const char *fn, int B, int Cq, int C, int H, int W, int P, int s, int G, int dtype) {
     SAPA_REQUIRE(B > 0 && Cq > 0 && C > 0 && H > 0 && W > 0, SAPA_ERR_ARGUMENT, "%s: sizes must be positive", fn);
     SAPA_REQUIRE(P >= 1, SAPA_ERR_ARGUMENT, "%s: num_point must be >= 1, got %d", fn, P);
@@ -1132,8 +1165,7 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     }
     // 2. attention over the points, dense window weights, list of the points that leave the window
     {
-        const long long total = (long long)B * G * hi;
-        const int grid = grid_1d(total, WIN_THREADS);
+        const dim3 grid = window_grid(B * G, hi);
         const int e = SAPA_DISPATCH_FAST(dtype, [&] {
             const scalar_t *q = static_cast<const scalar_t *>(query), *k = static_cast<const scalar_t *>(key);
             const scalar_t *o = static_cast<const scalar_t *>(offset);
@@ -1188,14 +1220,13 @@ int sapa_deform_qk_forward_dense(const void *query, const void *key, const void 
     } else {
         if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st)) return e;
     }
-    const long long total = (long long)B * G * hi;
     return SAPA_DISPATCH_FAST(dtype, [&] {
         if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-            launch_next(deform_window_kernel<scalar_t, 9, WIN_LOGITS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+            launch_next(deform_window_kernel<scalar_t, 9, WIN_LOGITS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
                 static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
                 static_cast<scalar_t *>(out), nullptr, nullptr, nullptr, B, Cq, H, W, P, G, H, 0);
         else
-            launch_next(deform_window_kernel<scalar_t, 0, WIN_LOGITS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+            launch_next(deform_window_kernel<scalar_t, 0, WIN_LOGITS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
                 static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
                 static_cast<scalar_t *>(out), nullptr, nullptr, nullptr, B, Cq, H, W, P, G, H, 0);
         return check_launch("deform_window_kernel<logits>");
@@ -1223,15 +1254,14 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
         set_error("%s: clearing the outlier counter failed", fn);
         return SAPA_ERR_LAUNCH;
     }
-    const long long total = (long long)B * G * hi;
     // the attention is only read in this mode
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_next(deform_window_kernel<scalar_t, 9, WIN_WEIGHTS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_next(deform_window_kernel<scalar_t, 9, WIN_WEIGHTS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr, const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)),
                     reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C, H, W, P, G, H, 0);
             else
-                launch_next(deform_window_kernel<scalar_t, 0, WIN_WEIGHTS>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_next(deform_window_kernel<scalar_t, 0, WIN_WEIGHTS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr, const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)),
                     reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C, H, W, P, G, H, 0);
             return check_launch("deform_window_kernel<weights>");
@@ -1304,8 +1334,7 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     }
     // 2. per pixel: softmax backward over the points, dD, Wd, offset gradients, list of the points outside the window
     {
-        const long long total = (long long)B * G * hi;
-        const int grid = grid_1d(total, WIN_THREADS);
+        const int grid = grid_1d((long long)B * G * hi, WIN_THREADS);
         const int e = SAPA_DISPATCH_FAST(dtype, [&] {
             const scalar_t *go = static_cast<const scalar_t *>(grad_out), *v = static_cast<const scalar_t *>(value);
             const scalar_t *o = static_cast<const scalar_t *>(offset), *a = static_cast<const scalar_t *>(attn);
@@ -1383,15 +1412,14 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     } else {
         if (int e = run_sim_mixed(grad_out, value, dwin, B * G, C / G, H, W, H, 0, dtype, st)) return e;
     }
-    const long long total = (long long)B * G * hi;
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_AV>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
                     static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
                     static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
             else
-                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_AV>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
                     static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
                     static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
@@ -1453,15 +1481,14 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     } else {
         if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st)) return e;
     }
-    const long long total = (long long)B * G * hi;
     // the logit gradients enter where the fused chain reads the attention
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_QK>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
                     static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
             else
-                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_QK>, grid_1d(total, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
                     static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
             return check_launch("deform_window_bwd_kernel<qk>");
