@@ -59,7 +59,7 @@ struct DxProblem {
     const void *x, *g1, *g2, *w1, *w2, *gamma, *add;
     const float2 *stats, *tail;        // nullptr: no norm
     void *out;
-    int B, C, d, d1, HW, groups, cpg, mblocks, pblocks, blocks, vec_g, vec;
+    int B, C, d, d1, HW, groups, cpg, mblocks, pblocks, blocks, vec_g, pair;
 };
 struct DxList { DxProblem p[MAX_PROBLEMS]; int count; };
 

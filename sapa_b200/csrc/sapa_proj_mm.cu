@@ -461,46 +461,14 @@ __global__ void __launch_bounds__(THREADS) proj_fold_kernel(const __grid_constan
 
 // ---------------------------------------------------------------------------------- backward: dx
 // Block = (problem, image, 64 channels, 64 pixels), K = the rows of dq in chunks of 32; x and the added gradient are fetched
-// before the products start.  The products go through shared memory, so that x, the added gradient and dx are read and written as
-// rows of 64 pixels, four to a thread: as fragments (32 bytes of eight channels to an instruction) the kernel took 49 us for the 90 MB
-// of 8 x 256 x 64x64 and 8 x 256 x 32x32 (d = 32, float32 under bfloat16 autocast), so it takes 36.
+// before the products start.
 constexpr int DX_M = 64, DX_P = 64, DX_XPITCH = 72;
-template <typename T> __device__ __forceinline__ float4 load4(const T *p, int valid, bool vec) {
-    if (vec && valid >= 4) {
-        if constexpr (sizeof(T) == 4) {
-            return __ldcs(reinterpret_cast<const float4 *>(p));
-        } else {
-            const uint2 u = __ldcs(reinterpret_cast<const uint2 *>(p));
-            const float2 a = unpack_pair(T(), u.x), b = unpack_pair(T(), u.y);
-            return make_float4(a.x, a.y, b.x, b.y);
-        }
-    }
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid > 0) v.x = to_acc(p[0]);
-    if (valid > 1) v.y = to_acc(p[1]);
-    if (valid > 2) v.z = to_acc(p[2]);
-    if (valid > 3) v.w = to_acc(p[3]);
-    return v;
-}
-template <typename T> __device__ __forceinline__ void store4(T *p, float4 v, int valid, bool vec) {
-    if (vec && valid >= 4) {
-        if constexpr (sizeof(T) == 4) __stcs(reinterpret_cast<float4 *>(p), v);
-        else __stcs(reinterpret_cast<uint2 *>(p), make_uint2(pack_pair(T(), v.x, v.y), pack_pair(T(), v.z, v.w)));
-        return;
-    }
-    if (valid > 0) p[0] = from_acc<T>(v.x);
-    if (valid > 1) p[1] = from_acc<T>(v.y);
-    if (valid > 2) p[2] = from_acc<T>(v.z);
-    if (valid > 3) p[3] = from_acc<T>(v.w);
-}
 
 template <typename T, typename TG>
 __global__ void __launch_bounds__(THREADS, sizeof(TG) == 4 ? 2 : 3) proj_dx_kernel(const __grid_constant__ DxList list) {
     begin_after_previous();
     constexpr bool LO = sizeof(TG) == 4;
-    static_assert(DX_M * MM_APITCH + MM_K * DX_XPITCH >= DX_M * DX_XPITCH, "the products take the place of the operands");
-    __shared__ __align__(16) float tile[DX_M * MM_APITCH + MM_K * DX_XPITCH];
-    float *const as = tile, *const xs = tile + DX_M * MM_APITCH;
+    __shared__ __align__(16) float as[DX_M * MM_APITCH], xs[MM_K * DX_XPITCH];
     int block = blockIdx.x;
     const DxProblem &m = list.p[find_problem(list, block)];
     const int pb = block % m.pblocks; block /= m.pblocks;
@@ -525,16 +493,42 @@ __global__ void __launch_bounds__(THREADS, sizeof(TG) == 4 ? 2 : 3) proj_dx_kern
     };
     fetch(0);
     const int wm = warp & 1, wp = warp >> 1;                    // warp: 32 channels, 16 pixels
-    // this thread's part of the result: channels er, er + 16, ... of the block, pixels ep .. ep + 3
-    const int er = tid >> 4, ep = p0 + (tid & 15) * 4;
-    float4 xe[4], ad[4];
+    float2 xe[2][2][2], ad[2][2][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = m0 + er + 16 * j, valid = c < m.C ? HW - ep : 0;
-        const size_t at = ((size_t)b * m.C + c) * HW + ep;
-        xe[j] = load4(static_cast<const T *>(m.x) + at, m.tail != nullptr ? valid : 0, m.vec);
-        ad[j] = load4(static_cast<const TG *>(m.add) + at, m.add != nullptr ? valid : 0, m.vec);
-    }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = m0 + 32 * wm + 16 * i + 8 * h + g;
+            const size_t row = ((size_t)b * m.C + c) * HW;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int p = p0 + 16 * wp + 8 * n + 2 * t;
+                xe[i][h][n] = ad[i][h][n] = make_float2(0.f, 0.f);
+                if (c >= m.C || p >= HW) continue;
+                const T *xp = static_cast<const T *>(m.x) + row + p;
+                const TG *ap = static_cast<const TG *>(m.add) + row + p;
+                if (m.pair) {                                   // even rows on aligned bases: pairs
+                    if (m.tail != nullptr) xe[i][h][n] = load_pair<T>(xp);
+                    if (m.add != nullptr) ad[i][h][n] = load_pair<TG>(ap);
+                } else {
+                    if (m.tail != nullptr) { xe[i][h][n].x = to_acc(xp[0]); if (p + 1 < HW) xe[i][h][n].y = to_acc(xp[1]); }
+                    if (m.add != nullptr) { ad[i][h][n].x = to_acc(ap[0]); if (p + 1 < HW) ad[i][h][n].y = to_acc(ap[1]); }
+                }
+            }
+        }
+    float scale[2][2], alpha[2][2], delta[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = m0 + 32 * wm + 16 * i + 8 * h + g;
+            scale[i][h] = 1.f; alpha[i][h] = 0.f; delta[i][h] = 0.f;
+            if (m.tail != nullptr && c < m.C) {
+                const size_t at = (size_t)b * m.groups + c / m.cpg;
+                const float2 tl = m.tail[at];
+                scale[i][h] = m.stats[at].y * to_acc(static_cast<const T *>(m.gamma)[c]); alpha[i][h] = tl.x; delta[i][h] = tl.y;
+            }
+        }
     float acc[2][2][4] = {};
     for (int k0 = 0; k0 < m.d; k0 += MM_K) {
         __syncthreads();
@@ -570,32 +564,26 @@ __global__ void __launch_bounds__(THREADS, sizeof(TG) == 4 ? 2 : 3) proj_dx_kern
             }
         }
     }
-    // D fragment: d0, d1 = (channel g, pixels 2t, 2t + 1), d2, d3 = channel g + 8
-    __syncthreads();
-    const unsigned tile_addr = (unsigned)__cvta_generic_to_shared(tile);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h) {
+            const int c = m0 + 32 * wm + 16 * i + 8 * h + g;
+            if (c >= m.C) continue;
+            T *row = static_cast<T *>(m.out) + ((size_t)b * m.C + c) * HW;
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
-                sts64(tile_addr + 4 * ((32 * wm + 16 * i + 8 * h + g) * DX_XPITCH + 16 * wp + 8 * n + 2 * t), acc[i][n][2 * h], acc[i][n][2 * h + 1]);
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int c = m0 + er + 16 * j;
-        if (c >= m.C) continue;
-        float scale = 1.f, alpha = 0.f, delta = 0.f;
-        if (m.tail != nullptr) {
-            const size_t at = (size_t)b * m.groups + c / m.cpg;
-            const float2 tl = m.tail[at];
-            scale = m.stats[at].y * to_acc(static_cast<const T *>(m.gamma)[c]); alpha = tl.x; delta = tl.y;
+            for (int n = 0; n < 2; ++n) {
+                const int p = p0 + 16 * wp + 8 * n + 2 * t;
+                if (p >= HW) continue;
+                const float o0 = fmaf(scale[i][h], rounded<TG>(acc[i][n][2 * h]), fmaf(alpha[i][h], xe[i][h][n].x, delta[i][h])) + ad[i][h][n].x;
+                const float o1 = fmaf(scale[i][h], rounded<TG>(acc[i][n][2 * h + 1]), fmaf(alpha[i][h], xe[i][h][n].y, delta[i][h])) + ad[i][h][n].y;
+                if (m.pair) store_pair<T>(row + p, o0, o1);
+                else {
+                    row[p] = from_acc<T>(o0);
+                    if (p + 1 < HW) row[p + 1] = from_acc<T>(o1);
+                }
+            }
         }
-        const float4 y = *reinterpret_cast<const float4 *>(tile + (er + 16 * j) * DX_XPITCH + (tid & 15) * 4);
-        const auto one = [&](float dy, float x, float add) { return fmaf(scale, rounded<TG>(dy), fmaf(alpha, x, delta)) + add; };
-        store4(static_cast<T *>(m.out) + ((size_t)b * m.C + c) * HW + ep,
-               make_float4(one(y.x, xe[j].x, ad[j].x), one(y.y, xe[j].y, ad[j].y), one(y.z, xe[j].z, ad[j].z), one(y.w, xe[j].w, ad[j].w)), HW - ep, m.vec);
-    }
 }
 
 // ---------------------------------------------------------------------------------- host side
@@ -722,7 +710,7 @@ static int run_backward(const sapa_projection_grad *q, int count, unsigned char 
         d.B = s.B; d.C = s.C; d.d = m.d; d.d1 = s.d; d.HW = s.HW; d.groups = m.groups; d.cpg = m.cpg;
         d.mblocks = ceil_div(s.C, DX_M); d.pblocks = ceil_div(s.HW, DX_P); d.blocks = s.B * d.mblocks * d.pblocks;
         d.vec_g = m.vec_g;
-        d.vec = s.HW % 4 == 0 && aligned16(s.x) && aligned16(s.grad_x) && (s.add == nullptr || aligned16(s.add));
+        d.pair = s.HW % 2 == 0 && aligned16(s.x) && aligned16(s.grad_x) && (s.add == nullptr || aligned16(s.add));
         dblocks += d.blocks;
     }
     constexpr int smem_norm = 3 * MO_C * MO_PITCH * 4, smem_plain = 2 * MO_C * MO_PITCH * 4;
