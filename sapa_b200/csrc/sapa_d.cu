@@ -305,7 +305,8 @@ struct WindowTap {
 constexpr int WIN_FUSED = 0, WIN_LOGITS = 1, WIN_WEIGHTS = 2;
 
 // The points of a pixel inside its window: fractional parts, and the place of the upper-left cell in the thread's column of a
-// [25][WIN_THREADS] array, two points to a register.  Points that are not dense have place 0 and take no part (see `dense`).
+// [25][WIN_THREADS] array, two points to a register.  Points that are not dense have place 0 and take no part (see `dense`); their
+// fractional parts are 0 too: those of an infinite or undefined offset are NaN, which no weight of zero keeps out of a sum.
 template <int PMAX>
 struct WindowPoints {
     float lh[PMAX], lw[PMAX];
@@ -326,7 +327,7 @@ struct WindowPoints {
             WindowTap t;
             t.setup(float(py) + oh[p], float(px) + ow[p], rows, W, py, px);
             const bool on = live && p < P, in = on && t.dense;
-            lh[p] = t.lh; lw[p] = t.lw;
+            lh[p] = in ? t.lh : 0.f; lw[p] = in ? t.lw : 0.f;
             const unsigned c = in ? (unsigned)((t.r0 * 5 + t.c0) * WIN_THREADS) : 0u;
             place[p >> 1] = p & 1 ? place[p >> 1] | (c << 16) : c;
             dense |= in ? 1u << p : 0u;
@@ -344,7 +345,7 @@ template <int N> __device__ __forceinline__ void put(float (&v)[N], int p, float
 // cell computed at run time (a register array cannot: that form multiplies every point with all 25 cells and took
 // 82 us at B=8, 4 groups, 128 x 128 pixels).  Two passes over the points: logits and their maximum, then exp and the window
 // weights.  Bound by latency at 24 warps per SM (80 registers; 4 and 8 blocks measured slower), so the points go side by side:
-// no branch on a point (what it must not add is multiplied by zero weights or selected away; outliers have a loop of their own), places
+// no branch on a point (what it must not add is selected away; outliers have a loop of their own), places
 // kept from pass to pass, block = pixels of one (image, group) instead of 64-bit divisions per thread: 55 -> 43 us (float32; bfloat16 59 -> 44).
 template <typename T, int NP, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 6)

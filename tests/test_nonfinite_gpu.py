@@ -111,3 +111,30 @@ def test_gathered_gradients(W, dtype):
         return torch.autograd.grad(sp.qk(q, t, 5, 2), t, slots)[0]
     for grad in (value_grad, key_grad):
         _same_elsewhere(grad(bad), grad(hi), reached, dtype)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 2e-2), (torch.float16, 4e-3)])
+@pytest.mark.parametrize("points", [9, 1, 4, 16])      # the unrolled form and the one for any number
+def test_sampling_offsets(points, dtype, tol):
+    """A sampling point at an infinite or undefined place lies outside the image: logit 0, nothing added to the output, no gradient.
+    tol: 2-norm against the float64 ops, as in test_outlier_lists_gpu.py."""
+    import sapa_b200 as sp
+    B, C, d, H, W, G = 2, 24, 8, 9, 16, 2
+    q, k, v, o, go = (torch.randn(*s, generator=torch.Generator().manual_seed(i)) * f for i, (s, f) in enumerate((
+        ((B, d, 2 * H, 2 * W), 0.5), ((B, d, H, W), 0.5), ((B, C, H, W), 1.0), ((B, 2 * points * G, 2 * H, 2 * W), 0.6), ((B, C, 2 * H, 2 * W), 1.0))))
+    o = (o * 64).round() / 64 + 1 / 128      # positions are exact in float32: the same cells as in float64
+    for n, (c, y, x, value) in enumerate(((0, 0, 0, INF), (1, 3, 5, NAN), (2 * points, 7, 31, -INF), (0, 4, 4, NAN), (2 * points - 1, 17, 12, INF), (1, 8, 8, -INF))):
+        o[n % B, c, y, x] = value
+    o[0, :, 11, 20] = INF      # every point of a pixel
+    t = [x.to(dtype).to(DEV).requires_grad_() for x in (q, k, v, o)]
+    r = [x.detach().double().requires_grad_() for x in t]
+    a = torch.rand(B, G, points, 2 * H, 2 * W, generator=torch.Generator().manual_seed(9)).to(dtype).to(DEV).requires_grad_()
+    ra, up = a.detach().double().requires_grad_(), go.to(dtype).to(DEV)
+
+    def results(x, attn, g):
+        fused, logits, out = sp.deform_sapa_fused(*x, points, 2, G), sp.deform_qk(x[0], x[1], x[3], points, 2, G), sp.deform_av(attn, x[2], x[3], points, 2, G)
+        return [fused, logits, out, *torch.autograd.grad(fused, x, g), *torch.autograd.grad(logits, [x[0], x[1], x[3]], attn.detach()),
+                *torch.autograd.grad(out, [attn, x[2], x[3]], g)]
+    for n, (x, y) in enumerate(zip(results(t, a, up), results(r, ra, up.double()))):
+        error, norm = float((x.detach().double() - y.detach()).norm()), float(y.detach().norm())
+        assert error <= tol * (norm or 1.0), n      # one point: its attention is 1, its logit has no gradient
