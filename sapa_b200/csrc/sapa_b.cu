@@ -195,7 +195,7 @@ struct HaloMap {
 template <typename T, typename Shape>
 struct HaloStage {
     float v[Shape::CH][Shape::PER];
-    __device__ __forceinline__ void fetch(const T *__restrict__ img, size_t plane_stride, int c0, int Cc,
+    __device__ __forceinline__ void fetch(const T *img, size_t plane_stride, int c0, int Cc,
                                           const HaloMap<Shape> &m) {
 #pragma unroll
         for (int c = 0; c < Shape::CH; ++c) {
@@ -203,7 +203,7 @@ struct HaloStage {
             const T *p = img + (size_t)(c0 + c) * plane_stride;
 #pragma unroll
             for (int j = 0; j < Shape::PER; ++j)
-                v[c][j] = (cok && m.off[j] >= 0) ? to_acc(__ldg(p + m.off[j])) : 0.f;
+                v[c][j] = (cok && m.off[j] >= 0) ? to_acc(load_current(p + m.off[j])) : 0.f;
         }
     }
     __device__ __forceinline__ void commit(float *__restrict__ sm, int tid) const {
@@ -219,7 +219,7 @@ struct HaloStage {
 
 // Loads / stores the S x S high-res values of one low-res parent for one channel plane.
 template <typename T, int S>
-__device__ __forceinline__ void load_group(const T *__restrict__ plane, int sW, int y, int x, bool active,
+__device__ __forceinline__ void load_group(const T *plane, int sW, int y, int x, bool active,
                                            float (&g)[S * S]) {
     if (!active) {
 #pragma unroll
@@ -254,7 +254,7 @@ __device__ __forceinline__ void store_group(T *__restrict__ plane, int sW, int y
 // acc[k][i] += hi_i * L(win_k) over the CH channels of one staged chunk.
 template <typename T, typename Shape>
 __device__ __forceinline__ void sim_chunk(float (&acc)[Shape::KK][Shape::SS], const float *__restrict__ sm,
-                                          const T *__restrict__ hi_img, size_t hi_plane, int sW, int c0, int Cc,
+                                          const T *hi_img, size_t hi_plane, int sW, int c0, int Cc,
                                           int y, int x, bool active, int ty, int tx) {
 #pragma unroll
     for (int c = 0; c < Shape::CH; ++c) {
@@ -316,7 +316,7 @@ __device__ __forceinline__ void softmax_regs(float (&a)[Shape::KK][Shape::SS]) {
 }
 
 template <typename T, typename Shape>
-__device__ __forceinline__ void load_slots(const T *__restrict__ img /* [KK,sH,sW] of image n */, size_t hi_plane,
+__device__ __forceinline__ void load_slots(const T *img /* [KK,sH,sW] of image n */, size_t hi_plane,
                                            int sW, int y, int x, bool active, float (&a)[Shape::KK][Shape::SS]) {
 #pragma unroll
     for (int k = 0; k < Shape::KK; ++k) load_group<T, Shape::S>(img + (size_t)k * hi_plane, sW, y, x, active, a[k]);
@@ -456,8 +456,8 @@ __global__ void __launch_bounds__(Shape::NT, MINB) sapa_tile_kernel(const TileAr
 // One thread per low-res cell u = (y, x).  Its K*K*S*S weights W_k(p) for every (parent p, slot k) that lands
 // on u stay in registers; the high-res tile of X (TH+K-1 x TW+K-1 parents) is staged per channel.
 template <typename T, typename Shape>
-__global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *__restrict__ hi, const T *__restrict__ wt,
-                                                              T *__restrict__ out, int B, int Cc, int H, int W,
+__global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *hi, const T *wt,
+                                                              T *out, int B, int Cc, int H, int W,
                                                               int tiles_x, int tiles_y) {
     begin_after_previous();
     constexpr int K = Shape::K, S = Shape::S, KK = Shape::KK, SS = Shape::SS, R = Shape::R;
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *__restric
             const int gy = py0 * S + yy, gx = px0 * S + xx;
             float v = 0.f;
             if ((c0 + c) < Cc && gy >= 0 && gy < sH && gx >= 0 && gx < sW)
-                v = to_acc(__ldg(himg + (size_t)(c0 + c) * hi_plane + (size_t)gy * sW + gx));
+                v = to_acc(load_current(himg + (size_t)(c0 + c) * hi_plane + (size_t)gy * sW + gx));
             sm[c][rem] = v;
         }
         __syncthreads();

@@ -14,8 +14,9 @@ namespace sapa {
 
 constexpr int MAXP = 16;   // largest num_point handled by the fused kernel
 
-// Bilinear footprint of one sampling point in an H x W plane.
-template <typename A>
+// Bilinear footprint of one sampling point in an H x W plane.  IN_ORDER: the kernel starts when the previous one has ended, so what it
+// reads does not change while it runs (see begin_after_previous).
+template <typename A, bool IN_ORDER = false>
 struct Bilinear {
     int i00, i01, i10, i11;   // plane offsets of the four corners, -1 when the corner is outside
     A w00, w01, w10, w11;     // corner weights
@@ -36,15 +37,19 @@ struct Bilinear {
         i10 = (inside && b && l) ? h1 * W + w0 : -1;
         i11 = (inside && b && r) ? h1 * W + w1 : -1;
     }
-    template <typename T>
-    __device__ __forceinline__ void corners(const T *__restrict__ plane, A &v00, A &v01, A &v10, A &v11) const {
-        v00 = i00 >= 0 ? to_acc(__ldg(plane + i00)) : A(0);
-        v01 = i01 >= 0 ? to_acc(__ldg(plane + i01)) : A(0);
-        v10 = i10 >= 0 ? to_acc(__ldg(plane + i10)) : A(0);
-        v11 = i11 >= 0 ? to_acc(__ldg(plane + i11)) : A(0);
+    template <typename T> static __device__ __forceinline__ T corner(const T *p) {
+        if constexpr (IN_ORDER) return __ldg(p);
+        else return *p;
     }
     template <typename T>
-    __device__ __forceinline__ A sample(const T *__restrict__ plane) const {
+    __device__ __forceinline__ void corners(const T *plane, A &v00, A &v01, A &v10, A &v11) const {
+        v00 = i00 >= 0 ? to_acc(corner(plane + i00)) : A(0);
+        v01 = i01 >= 0 ? to_acc(corner(plane + i01)) : A(0);
+        v10 = i10 >= 0 ? to_acc(corner(plane + i10)) : A(0);
+        v11 = i11 >= 0 ? to_acc(corner(plane + i11)) : A(0);
+    }
+    template <typename T>
+    __device__ __forceinline__ A sample(const T *plane) const {
         A v00, v01, v10, v11;
         corners(plane, v00, v01, v10, v11);
         return w00 * v00 + w01 * v01 + w10 * v10 + w11 * v11;
@@ -69,7 +74,7 @@ __global__ void deform_qk_fwd_kernel(const T *__restrict__ query, const T *__res
         const int b = (int)(i / (hi * AC));
         const int g = k / P;
         const T *op = offset + ((size_t)b * AC + k) * 2 * hi + pix;
-        Bilinear<A> bl;
+        Bilinear<A, true> bl;
         bl.setup(A(qh / s) + to_acc(op[hi]), A(qw / s) + to_acc(op[0]), H, W);
         A acc = 0;
         if (bl.inside) {
@@ -106,7 +111,7 @@ __global__ void deform_av_fwd_kernel(const T *__restrict__ attn, const T *__rest
         const T *vp = value + ((size_t)b * C + c0) * lo;
         for (int p = 0; p < P; ++p) {
             const size_t k = (size_t)b * AC + (size_t)g * P + p;
-            Bilinear<A> bl;
+            Bilinear<A, true> bl;
             bl.setup(A(qh / s) + to_acc(offset[k * 2 * hi + hi + pix]), A(qw / s) + to_acc(offset[k * 2 * hi + pix]), H, W);
             if (!bl.inside) continue;
             const A a = to_acc(attn[k * hi + pix]);
@@ -152,7 +157,7 @@ deform_fused_fwd_kernel(const T *__restrict__ query, const T *__restrict__ key, 
         for (int p = ty; p < P; p += FY) {
             const float w = float(qw / s) + to_acc(op[(size_t)(2 * p) * hi]);
             const float h = float(qh / s) + to_acc(op[(size_t)(2 * p + 1) * hi]);
-            Bilinear<float> bl;
+            Bilinear<float, true> bl;
             bl.setup(h, w, H, W);
             float acc = 0.f;
             if (bl.inside)
@@ -182,7 +187,7 @@ deform_fused_fwd_kernel(const T *__restrict__ query, const T *__restrict__ key, 
 #pragma unroll
         for (int j = 0; j < CPT; ++j) o[j] = 0.f;
         for (int p = 0; p < P; ++p) {
-            Bilinear<float> bl;
+            Bilinear<float, true> bl;
             bl.setup(s_h[p][tx], s_w[p][tx], H, W);
             if (!bl.inside) continue;
             const float a = expf(s_a[p][tx] - m) * inv;
@@ -220,7 +225,7 @@ __global__ void deform_bwd_kernel(const T *__restrict__ top, const T *__restrict
         const int b = (int)(i / (hi * AC));
         const int g = k / P;
         const size_t off_idx = ((size_t)b * AC + k) * 2 * hi + pix;
-        Bilinear<A> bl;
+        Bilinear<A, true> bl;
         bl.setup(A(qh / s) + to_acc(offset[off_idx + hi]), A(qw / s) + to_acc(offset[off_idx]), H, W);
         A g_w = 0, g_h = 0, g_attn = 0;
         if (bl.inside) {
@@ -318,8 +323,8 @@ struct WindowPoints {
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
             const bool on = live && p < P;
-            ow[p] = on ? to_acc(__ldg(offp + (size_t)(2 * p) * hi)) : 0.f;
-            oh[p] = on ? to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi)) : 0.f;
+            ow[p] = on ? to_acc(offp[(size_t)(2 * p) * hi]) : 0.f;
+            oh[p] = on ? to_acc(offp[(size_t)(2 * p + 1) * hi]) : 0.f;
         }
         dense = outliers = 0u;
 #pragma unroll
@@ -349,9 +354,9 @@ template <int N> __device__ __forceinline__ void put(float (&v)[N], int p, float
 // kept from pass to pass, block = pixels of one (image, group) instead of 64-bit divisions per thread: 55 -> 43 us (float32; bfloat16 59 -> 44).
 template <typename T, int NP, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 6)
-deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, const T *__restrict__ offset,
-                          const float *__restrict__ dense, T *__restrict__ attn, T *__restrict__ window,
-                          OutlierTap *__restrict__ taps, unsigned int *__restrict__ tap_count, int B, int Cq, int H, int W,
+deform_window_kernel(const T *query, const T *key, const T *offset,
+                          const float *dense, T *attn, T *window,
+                          OutlierTap *taps, unsigned int *tap_count, int B, int Cq, int H, int W,
                           int P_runtime, int G, int rows, int ytop) {
     begin_after_previous();
     constexpr int PMAX = NP > 0 ? NP : MAXP;
@@ -386,7 +391,7 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
             if (MODE == WIN_WEIGHTS) {
-                logit[p] = live && p < P ? to_acc(__ldg(attn + ((size_t)bg * P + p) * hi + pix)) : 0.f;
+                logit[p] = live && p < P ? to_acc(attn[((size_t)bg * P + p) * hi + pix]) : 0.f;
             } else {
                 const float *c = dcol + pts.at(p);
                 const float top = (1.f - pts.lw[p]) * c[0] + pts.lw[p] * c[WIN_THREADS];
@@ -398,7 +403,7 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
             for (unsigned left = pts.outliers; left != 0; left &= left - 1) {      // outliers: gather the key directly
                 const int p = __ffs(left) - 1;
                 Bilinear<float> bl;
-                bl.setup(float(py) + to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi)), float(px) + to_acc(__ldg(offp + (size_t)(2 * p) * hi)), rows, W);
+                bl.setup(float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]), float(px) + to_acc(offp[(size_t)(2 * p) * hi]), rows, W);
                 const T *qp = query + (size_t)bg * gq * hi + pix, *kp = key + (size_t)bg * gq * lo;
                 float acc = 0.f;
                 for (int ch = 0; ch < gq; ++ch) acc += bl.sample(kp + (size_t)ch * lo) * to_acc(qp[(size_t)ch * hi]);
@@ -464,8 +469,8 @@ deform_window_kernel(const T *__restrict__ query, const T *__restrict__ key, con
 // exactly one thread group, and the aggregation kernel that wrote the output has finished): the forward pass is
 // deterministic and a 16-bit output is rounded once more, not once per point.
 template <int SUB, int CH, typename T>
-__device__ __forceinline__ void outlier_pixels(const OutlierTap *__restrict__ taps, unsigned int n, const T *__restrict__ value,
-                                               const T *__restrict__ offset, T *__restrict__ out, int C, int H, int W, int P, int G, int rows, int ytop) {
+__device__ __forceinline__ void outlier_pixels(const OutlierTap *taps, unsigned int n, const T *value,
+                                               const T *offset, T *out, int C, int H, int W, int P, int G, int rows, int ytop) {
     const int sW = 2 * W, gc = C / G;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)rows * W;
     const int sub = threadIdx.x % SUB;
@@ -473,7 +478,7 @@ __device__ __forceinline__ void outlier_pixels(const OutlierTap *__restrict__ ta
     const unsigned int first = SUB == 32 ? threadIdx.x / SUB * gridDim.x + blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) / SUB;
     for (unsigned int e = first; e < n; e += gridDim.x * blockDim.x / SUB) {
         const OutlierTap *t = taps + e;
-        const unsigned int idx = __ldg(&t->idx), mask = __ldg(&t->mask);
+        const unsigned int idx = t->idx, mask = t->mask;
         const size_t bg = idx / hi, pix = idx % hi;
         const int px = (int)(pix % sW) >> 1, py = ((int)(pix / sW) >> 1) + ytop;
         const T *offp = offset + bg * P * 2 * hi + pix;
@@ -488,9 +493,9 @@ __device__ __forceinline__ void outlier_pixels(const OutlierTap *__restrict__ ta
             }
             for (unsigned int m = mask; m != 0; m &= m - 1) {
                 const int p = __ffs(m) - 1;
-                const float w = float(px) + to_acc(__ldg(offp + (size_t)(2 * p) * hi));
-                const float h = float(py) + to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi));
-                const float a = __ldg(&t->a[p]);
+                const float w = float(px) + to_acc(offp[(size_t)(2 * p) * hi]);
+                const float h = float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]);
+                const float a = t->a[p];
                 Bilinear<float> bl;
                 bl.setup(h, w, rows, W);
 #pragma unroll
@@ -511,8 +516,8 @@ __device__ __forceinline__ void outlier_pixels(const OutlierTap *__restrict__ ta
 // in flight at once (25 -> 7 us for 317 pixels of 64 channels in float16).  A long one is bound by its sectors, which neighbouring pixels
 // share when eight threads serve each.
 template <typename T>
-__global__ void deform_outlier_kernel(const OutlierTap *__restrict__ taps, const unsigned int *__restrict__ tap_count,
-                                      const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ out,
+__global__ void deform_outlier_kernel(const OutlierTap *taps, const unsigned int *tap_count,
+                                      const T *value, const T *offset, T *out,
                                       int C, int H, int W, int P, int G, int rows, int ytop) {
     begin_after_previous();
     const unsigned int n = *tap_count;
@@ -545,12 +550,12 @@ constexpr int BWD_FUSED = 0, BWD_AV = 1, BWD_QK = 2;
 
 template <typename T, int NP, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 4)
-deform_window_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ value, const T *__restrict__ offset,
-                         const T *__restrict__ attn, const float *__restrict__ dense /* D [B*G, 25, hi] */,
-                         const float *__restrict__ dwin /* dWd [B*G, 25, hi] */, T *__restrict__ ddense /* dD, out */,
-                         T *__restrict__ window /* Wd, out */, T *__restrict__ grad_offset, T *__restrict__ grad_attn /* BWD_AV only */,
-                         OutlierGrad *__restrict__ taps,
-                         unsigned int *__restrict__ tap_count, int B, int C, int H, int W, int P_runtime, int G) {
+deform_window_bwd_kernel(const T *grad_out, const T *value, const T *offset,
+                         const T *attn, const float *dense /* D [B*G, 25, hi] */,
+                         const float *dwin /* dWd [B*G, 25, hi] */, T *ddense /* dD, out */,
+                         T *window /* Wd, out */, T *grad_offset, T *grad_attn /* BWD_AV only */,
+                         OutlierGrad *taps,
+                         unsigned int *tap_count, int B, int C, int H, int W, int P_runtime, int G) {
     begin_after_previous();
     constexpr int PMAX = NP > 0 ? NP : MAXP;
     const int P = NP > 0 ? NP : P_runtime;
@@ -579,9 +584,9 @@ deform_window_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ v
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
             const bool on = live && p < P;
-            ow[p] = on ? float(px) + to_acc(__ldg(offp + (size_t)(2 * p) * hi)) : 0.f;
-            oh[p] = on ? float(py) + to_acc(__ldg(offp + (size_t)(2 * p + 1) * hi)) : 0.f;
-            at[p] = on ? to_acc(__ldg(ap + (size_t)p * hi)) : 0.f;
+            ow[p] = on ? float(px) + to_acc(offp[(size_t)(2 * p) * hi]) : 0.f;
+            oh[p] = on ? float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]) : 0.f;
+            at[p] = on ? to_acc(ap[(size_t)p * hi]) : 0.f;
         }
         // ---- pass 1: dA_p and the four bilinear forms of the offset gradients
         float da[PMAX], gh1[PMAX], gw1[PMAX], gh2[PMAX], gw2[PMAX];
@@ -691,10 +696,10 @@ deform_window_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ v
 // zeroed side buffers that deform_add_scatter_kernel folds into the 16-bit gradients afterwards (a 16-bit atomic per
 // corner and channel was 2x slower than the whole float32 pass and rounds at every addition).
 template <int SUB, typename T, typename TA>
-__device__ __forceinline__ void outlier_points_bwd(const OutlierGrad *__restrict__ taps, unsigned int n,
-                                          const T *__restrict__ grad_out, const T *__restrict__ query, const T *__restrict__ key,
-                                          const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ grad_query,
-                                          TA *__restrict__ grad_key, TA *__restrict__ grad_value, T *__restrict__ grad_offset,
+__device__ __forceinline__ void outlier_points_bwd(const OutlierGrad *taps, unsigned int n,
+                                          const T *grad_out, const T *query, const T *key,
+                                          const T *value, const T *offset, T *grad_query,
+                                          TA *grad_key, TA *grad_value, T *grad_offset,
                                           int Cq, int C, int H, int W, int P, int G) {
     const int sW = 2 * W, gq = Cq / G, gc = C / G;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)H * W;
@@ -706,8 +711,8 @@ __device__ __forceinline__ void outlier_points_bwd(const OutlierGrad *__restrict
         const OutlierGrad t = taps[e];
         const size_t pix = t.pix;
         const int px = (int)(pix % sW) >> 1, py = (int)(pix / sW) >> 1;
-        const float w = float(px) + to_acc(__ldg(offset + (size_t)t.k * 2 * hi + pix));
-        const float h = float(py) + to_acc(__ldg(offset + (size_t)t.k * 2 * hi + hi + pix));
+        const float w = float(px) + to_acc(offset[(size_t)t.k * 2 * hi + pix]);
+        const float h = float(py) + to_acc(offset[(size_t)t.k * 2 * hi + hi + pix]);
         Bilinear<float> bl;
         bl.setup(h, w, H, W);
         const float hh = 1.f - bl.lh, hw = 1.f - bl.lw;
@@ -751,10 +756,10 @@ __device__ __forceinline__ void outlier_points_bwd(const OutlierGrad *__restrict
 }
 
 template <typename T, typename TA>      // a warp per entry of a short list, as in the forward pass
-__global__ void deform_outlier_bwd_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count,
-                                          const T *__restrict__ grad_out, const T *__restrict__ query, const T *__restrict__ key,
-                                          const T *__restrict__ value, const T *__restrict__ offset, T *__restrict__ grad_query,
-                                          TA *__restrict__ grad_key, TA *__restrict__ grad_value, T *__restrict__ grad_offset,
+__global__ void deform_outlier_bwd_kernel(const OutlierGrad *taps, const unsigned int *tap_count,
+                                          const T *grad_out, const T *query, const T *key,
+                                          const T *value, const T *offset, T *grad_query,
+                                          TA *grad_key, TA *grad_value, T *grad_offset,
                                           int Cq, int C, int H, int W, int P, int G) {
     begin_after_previous();
     const unsigned int n = *tap_count;
@@ -773,7 +778,7 @@ struct Scatter { float *key, *value; size_t n_key, n_value; int gq, gc; };      
 // f(cell index of the key buffer or of the value buffer, which) for the four corners of every listed point and all channels of its
 // group; a warp per corner
 template <typename T, typename F>
-__device__ __forceinline__ void for_scattered(const OutlierGrad *__restrict__ taps, unsigned int n, const T *__restrict__ offset, const Scatter &sc, int H, int W,
+__device__ __forceinline__ void for_scattered(const OutlierGrad *taps, unsigned int n, const T *offset, const Scatter &sc, int H, int W,
                                               int P, F f) {
     const int sW = 2 * W;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)H * W;
@@ -781,7 +786,7 @@ __device__ __forceinline__ void for_scattered(const OutlierGrad *__restrict__ ta
         const OutlierGrad t = taps[e >> 2];
         const size_t pix = t.pix, bg = t.k / (unsigned int)P;
         const int px = (int)(pix % sW) >> 1, py = (int)(pix / sW) >> 1;
-        const float w = float(px) + to_acc(__ldg(offset + (size_t)t.k * 2 * hi + pix)), h = float(py) + to_acc(__ldg(offset + (size_t)t.k * 2 * hi + hi + pix));
+        const float w = float(px) + to_acc(offset[(size_t)t.k * 2 * hi + pix]), h = float(py) + to_acc(offset[(size_t)t.k * 2 * hi + hi + pix]);
         Bilinear<float> bl;
         bl.setup(h, w, H, W);
         const int at = (e & 2) != 0 ? ((e & 1) != 0 ? bl.i11 : bl.i10) : (e & 1) != 0 ? bl.i01 : bl.i00;
@@ -794,7 +799,7 @@ __device__ __forceinline__ void for_scattered(const OutlierGrad *__restrict__ ta
 }
 
 template <typename T>
-__global__ void deform_zero_scatter_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count, const T *__restrict__ offset,
+__global__ void deform_zero_scatter_kernel(const OutlierGrad *taps, const unsigned int *tap_count, const T *offset,
                                            const Scatter sc, int H, int W, int P) {
     begin_after_previous();
     const unsigned int n = *tap_count;
@@ -807,8 +812,8 @@ __global__ void deform_zero_scatter_kernel(const OutlierGrad *__restrict__ taps,
 }
 
 template <typename T>
-__global__ void deform_add_scatter_kernel(const OutlierGrad *__restrict__ taps, const unsigned int *__restrict__ tap_count, const T *__restrict__ offset,
-                                          const Scatter sc, T *__restrict__ grad_key, T *__restrict__ grad_value, int H, int W, int P) {
+__global__ void deform_add_scatter_kernel(const OutlierGrad *taps, const unsigned int *tap_count, const T *offset,
+                                          const Scatter sc, T *grad_key, T *grad_value, int H, int W, int P) {
     begin_after_previous();
     const unsigned int n = *tap_count;
     if (n <= gridDim.x * (blockDim.x / 32)) {
@@ -861,7 +866,7 @@ deform_fused_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ qu
         for (int p = 0; p < P; ++p) {
             const A w = A(qw / s) + to_acc(offset[(k0 + p) * 2 * hi + pix]);
             const A h = A(qh / s) + to_acc(offset[(k0 + p) * 2 * hi + hi + pix]);
-            Bilinear<A> bl;
+            Bilinear<A, true> bl;
             bl.setup(h, w, H, W);
             A dA = 0, g_w = 0, g_h = 0;
             if (bl.inside) {
@@ -890,7 +895,7 @@ deform_fused_bwd_kernel(const T *__restrict__ grad_out, const T *__restrict__ qu
         const size_t qch0 = (size_t)b * Cq + (size_t)g * gq;
         for (int p = 0; p < P; ++p) {
             const A dS = to_acc(ap[(size_t)p * hi]) * (s_d[p][tx] - dot);
-            Bilinear<A> bl;
+            Bilinear<A, true> bl;
             bl.setup(s_h[p][tx], s_w[p][tx], H, W);
             A g_w = s_gw[p][tx], g_h = s_gh[p][tx];
             const bool first = p == 0;

@@ -296,14 +296,14 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
                             const int b = 4 + 8 * kg + t + 4 * e, dx = g + 6 - (b >> 1), hx = 2 * x0 - 8 + b;
                             float w = 0.f;
                             if (row_in && dx >= 0 && dx <= 4 && hx >= 0 && hx < sW)
-                                w = __ldg(reinterpret_cast<const float *>(wimg) + (size_t)((4 - j) * 5 + dx) * hi_plane + (size_t)hy * sW + hx);
+                                w = reinterpret_cast<const float *>(wimg)[(size_t)((4 - j) * 5 + dx) * hi_plane + (size_t)hy * sW + hx];
                             bw[j][kg][e] = __float_as_uint(w);
                         }
                     } else {
                         const int b = 4 + 8 * kg + 2 * t, dx = g + 6 - (b >> 1), hx = 2 * x0 - 8 + b;
                         unsigned w = 0u;
                         if (row_in && dx >= 0 && dx <= 4 && hx >= 0 && hx < sW)
-                            w = __ldg(reinterpret_cast<const unsigned *>(wimg + (size_t)((4 - j) * 5 + dx) * hi_plane + (size_t)hy * sW + hx));
+                            w = *reinterpret_cast<const unsigned *>(wimg + (size_t)((4 - j) * 5 + dx) * hi_plane + (size_t)hy * sW + hx);
                         bw[j][kg][0] = w;
                     }
                 }

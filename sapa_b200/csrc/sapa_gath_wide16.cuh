@@ -132,8 +132,8 @@ sapa_gath_wide_16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
                 const int dx = g + 6 - 4 * kg - t, hx = 2 * x0 - 8 + 8 * kg + 2 * t;
                 const bool ok = row_in && dx >= 0 && dx <= 4 && hx >= 0 && hx < sW;
                 const T *p = wimg + (ok ? w0 + j * (2 * (long long)sW - 5 * plane) + kg * (8 - 4 * plane) : 0);
-                bw[j][kg][0] = ok ? __ldg(reinterpret_cast<const unsigned *>(p)) : 0u;
-                bw[j][kg][1] = ok ? __ldg(reinterpret_cast<const unsigned *>(p + sW)) : 0u;
+                bw[j][kg][0] = ok ? *reinterpret_cast<const unsigned *>(p) : 0u;
+                bw[j][kg][1] = ok ? *reinterpret_cast<const unsigned *>(p + sW) : 0u;
             }
         }
         const size_t out_plane = (size_t)a.Hout * a.W;

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
-                    v[j] = __uint_as_float(r[j]) + (folded != nullptr ? __ldg(folded + c0 + j) : given != nullptr ? to_acc(__ldg(given + c0 + j)) : 0.f);
+                    v[j] = __uint_as_float(r[j]) + (folded != nullptr ? load_current(folded + c0 + j) : given != nullptr ? to_acc(load_current(given + c0 + j)) : 0.f);
                 if (px < HW && p.shuffle_w > 0) {
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) store_pair<TO>(op + (size_t)(c0 + (j & ~3)) * HW + (j & 2) * p.shuffle_w, v[j], v[j + 1]);
@@ -488,7 +488,7 @@ template <typename T> __device__ __forceinline__ void fetch16(const T *p, bool v
         load16(p, v);
     } else {
 #pragma unroll
-        for (int i = 0; i < Vec16<T>::N; ++i) v[i] = to_acc(__ldg(p + i));
+        for (int i = 0; i < Vec16<T>::N; ++i) v[i] = to_acc(load_current(p + i));
     }
 }
 // A block of a problem writes FOLD_ROWS rows of W'[b] (split in two for float32) and of bias'[b], a warp each.  The kernel is a chain

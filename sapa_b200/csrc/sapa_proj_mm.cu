@@ -32,10 +32,10 @@ constexpr int THREADS = 256;
 template <typename T> __device__ __forceinline__ void load8(const T *p, int valid, bool vec, float (&v)[8]) {
     if (vec && valid >= 8) {
         if constexpr (sizeof(T) == 4) {
-            const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+            const float4 a = *reinterpret_cast<const float4 *>(p), b = reinterpret_cast<const float4 *>(p)[1];
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
-            const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p));
+            const uint4 u = *reinterpret_cast<const uint4 *>(p);
             const unsigned w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -49,7 +49,7 @@ template <typename T> __device__ __forceinline__ void load8(const T *p, int vali
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = i < valid ? to_acc(__ldg(p + i)) : 0.f;
+        for (int i = 0; i < 8; ++i) v[i] = i < valid ? to_acc(p[i]) : 0.f;
     }
 }
 __device__ __forceinline__ void sts8(unsigned addr, const float (&v)[8]) {
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(THREADS, 3) proj_fwd_kernel(const __grid_const
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int r = m0 + arow + 32 * i, k = k0 + acol + e;
-                av[i][e] = r < m.M && k < m.K ? rounded<TO>(to_acc(__ldg(W + (size_t)r * m.K + k))) : 0.f;
+                av[i][e] = r < m.M && k < m.K ? rounded<TO>(to_acc(W[(size_t)r * m.K + k])) : 0.f;
             }
     };
     fetch(0);
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(THREADS, 3) proj_fwd_kernel(const __grid_const
             const int k = k0 + xrow + 16 * i;
             if (m.partial != nullptr && k < m.K) {
                 const float2 st = s_st[k / m.cpg];
-                const float a = st.y * to_acc(__ldg(static_cast<const T *>(m.gamma) + k)), s = fmaf(-a, st.x, to_acc(__ldg(static_cast<const T *>(m.beta) + k)));
+                const float a = st.y * to_acc(static_cast<const T *>(m.gamma)[k]), s = fmaf(-a, st.x, to_acc(static_cast<const T *>(m.beta)[k]));
 #pragma unroll
                 for (int e = 0; e < 8; ++e) xv[i][e] = fmaf(a, xv[i][e], s);
             }
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(THREADS, 3) proj_fwd_kernel(const __grid_const
         for (int half = 0; half < 2; ++half) {
             const int r = m0 + 32 * wm + 16 * i + 8 * half + g;
             if (r >= m.M) continue;
-            const float bias = m.bias != nullptr ? rounded<TO>(to_acc(__ldg(static_cast<const T *>(m.bias) + r))) : 0.f;
+            const float bias = m.bias != nullptr ? rounded<TO>(to_acc(static_cast<const T *>(m.bias)[r])) : 0.f;
             TO *row = static_cast<TO *>(m.out) + ((size_t)b * m.M + r) * HW;
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(THREADS, 2) proj_moments_kernel(const __grid_c
         for (int i = tid; i < MO_C * ((m.d + 7) & ~7); i += THREADS) {
             const int c = i & (MO_C - 1), j = i / MO_C, cc = cb * MO_C + c;
             const T *w = j < m.d1 ? static_cast<const T *>(m.w1) + (size_t)j * m.C : static_cast<const T *>(m.w2) + (size_t)(j - m.d1) * m.C;
-            ws[c * MO_PITCH + j] = cc < m.C && j < m.d ? rounded<TG>(to_acc(__ldg(w + cc))) : 0.f;
+            ws[c * MO_PITCH + j] = cc < m.C && j < m.d ? rounded<TG>(to_acc(w[cc])) : 0.f;
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(THREADS, sizeof(TG) == 4 ? 2 : 3) proj_dx_kern
         for (int i = 0; i < 8; ++i) {
             const int k = k0 + ak + 4 * i, c = m0 + ac;
             const T *w = k < m.d1 ? static_cast<const T *>(m.w1) + (size_t)k * m.C : static_cast<const T *>(m.w2) + (size_t)(k - m.d1) * m.C;
-            av[i] = k < m.d && c < m.C ? rounded<TG>(to_acc(__ldg(w + c))) : 0.f;
+            av[i] = k < m.d && c < m.C ? rounded<TG>(to_acc(w[c])) : 0.f;
         }
     };
     fetch(0);

@@ -208,8 +208,8 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
         for (int dy = 0; dy < 5; ++dy)
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                s[dy][2 * r] = (pix_ok && ok0) ? __ldg(ap + (size_t)(dy * 5 + 2 * t - l) * hi_plane + (size_t)r * sW) : 0.f;
-                s[dy][2 * r + 1] = (pix_ok && ok1) ? __ldg(ap + (size_t)(dy * 5 + 2 * t + 1 - l) * hi_plane + (size_t)r * sW) : 0.f;
+                s[dy][2 * r] = (pix_ok && ok0) ? ap[(size_t)(dy * 5 + 2 * t - l) * hi_plane + (size_t)r * sW] : 0.f;
+                s[dy][2 * r + 1] = (pix_ok && ok1) ? ap[(size_t)(dy * 5 + 2 * t + 1 - l) * hi_plane + (size_t)r * sW] : 0.f;
             }
         realign();
     }
@@ -263,8 +263,8 @@ sapa_tma_fused_f32_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
                 for (int dy = 0; dy < 5; ++dy)
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
-                        av[dy][2 * r] = (pix_ok && ok0) ? __ldg(ap + (size_t)(dy * 5 + 2 * t - l) * hi_plane + (size_t)r * sW) : 0.f;
-                        av[dy][2 * r + 1] = (pix_ok && ok1) ? __ldg(ap + (size_t)(dy * 5 + 2 * t + 1 - l) * hi_plane + (size_t)r * sW) : 0.f;
+                        av[dy][2 * r] = (pix_ok && ok0) ? ap[(size_t)(dy * 5 + 2 * t - l) * hi_plane + (size_t)r * sW] : 0.f;
+                        av[dy][2 * r + 1] = (pix_ok && ok1) ? ap[(size_t)(dy * 5 + 2 * t + 1 - l) * hi_plane + (size_t)r * sW] : 0.f;
                     }
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
@@ -478,8 +478,8 @@ struct OddBox {
             const int rc = i * (h16::PT / 8) + (ptid >> 3), ch = rc & 31, row = rc >> 5, y = y0 - 2 + row;
             const bool ok = c0 + ch < C && y >= 0 && y < rows;
             const unsigned short *p = b16 + (size_t)(c0 + ch) * plane + (size_t)y * W + x;
-            lo[i] = ok && lo_ok ? __ldg(p) : (unsigned short)0;
-            hi[i] = ok && hi_ok ? __ldg(p + 1) : (unsigned short)0;
+            lo[i] = ok && lo_ok ? *p : (unsigned short)0;
+            hi[i] = ok && hi_ok ? p[1] : (unsigned short)0;
         }
     }
     __device__ __forceinline__ void store(unsigned dst, int ptid) const {
@@ -811,8 +811,8 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 #pragma unroll
                 for (int dy = 0; dy < 5; ++dy) {
                     unsigned ulo = 0u, uhi = 0u;
-                    if (pix && ok_lo[p]) ulo = __ldg(ap + (size_t)(dy * 5 + dx_lo[p]) * plane_w + 4 * p);
-                    if (pix && ok_hi[p]) uhi = __ldg(ap + (size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + 4 * p);
+                    if (pix && ok_lo[p]) ulo = ap[(size_t)(dy * 5 + dx_lo[p]) * plane_w + 4 * p];
+                    if (pix && ok_hi[p]) uhi = ap[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + 4 * p];
                     pb[p][dy][0] = movmatrix_trans(ulo);
                     pb[p][dy][1] = movmatrix_trans(uhi);
                 }
@@ -858,8 +858,8 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 #pragma unroll
                     for (int dy = 0; dy < 5; ++dy) {
                         unsigned ulo = 0u, uhi = 0u;
-                        if (pix && ok_lo[p]) ulo = __ldg(ap + (size_t)(dy * 5 + dx_lo[p]) * plane_w + 4 * p);
-                        if (pix && ok_hi[p]) uhi = __ldg(ap + (size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + 4 * p);
+                        if (pix && ok_lo[p]) ulo = ap[(size_t)(dy * 5 + dx_lo[p]) * plane_w + 4 * p];
+                        if (pix && ok_hi[p]) uhi = ap[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + 4 * p];
                         const float2 flo = unpack_pair(T(), ulo), fhi = unpack_pair(T(), uhi);
                         av[dy][0] = flo.x; av[dy][1] = flo.y; av[dy][2] = fhi.x; av[dy][3] = fhi.y;
                         d0 += av[dy][0] * s[p][dy][0] + av[dy][2] * s[p][dy][2];

@@ -183,8 +183,8 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         unsigned pb[2][2][5][2];                  // [group][high-res row][dy][lo, hi]: B fragments of the aggregation
         const auto load_slots = [&](const unsigned *ap, int p, int r, int dy, unsigned &lo, unsigned &hi) {
             lo = hi = 0u;
-            if (live && ok_lo[p]) lo = __ldg(ap + (size_t)(dy * 5 + dx_lo[p]) * plane_w + r * row_w + 4 * p);
-            if (live && ok_hi[p]) hi = __ldg(ap + (size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + r * row_w + 4 * p);
+            if (live && ok_lo[p]) lo = ap[(size_t)(dy * 5 + dx_lo[p]) * plane_w + r * row_w + 4 * p];
+            if (live && ok_hi[p]) hi = ap[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + r * row_w + 4 * p];
         };
         if (MODE == MODE_AGG) {                   // the weights come from memory, already in the packed pair layout
             const unsigned *ap = static_cast<const unsigned *>(a.attn) + (size_t)n * 25 * plane_w + pix_w;
