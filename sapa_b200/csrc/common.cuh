@@ -126,7 +126,7 @@ template <typename... P> inline bool all_aligned16(const P *...p) { return (alig
 
 // Launch of a kernel that starts with begin_after_previous(): its blocks may be set up while the previous kernel of the stream drains
 // (programmatic dependent launch), which hides the launch latency between the kernels of a chain, about 1.5 us of 2.5: three
-// chained SAPA modules (twelve kernels) 253.6 -> 231.5 us, one SAPADeform module (six) 57.4 -> 52.4.
+// chained SAPA modules (twelve kernels) 253.6 -> 231.5 us, one SAPADeform module (six) 57.4 -> 50.3.
 template <typename... P, typename... A>
 inline void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
     cudaLaunchAttribute attribute;
@@ -136,6 +136,29 @@ inline void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem
     config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = st;
     config.attrs = &attribute; config.numAttrs = 1;
     (void)cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);      // a failure is what check_launch reads
+}
+
+// Kernels that live on the L1 cache (gathers, neighbours' overlapping reads).  An SM divides its memory between L1 and shared memory when
+// it is empty: blocks set up beside a kernel with 200 KB of shared memory keep what that one left them.  So such a kernel is launched
+// after the previous one has ended; or ahead with all of the memory asked for as L1, which holds it back from an SM until that is empty
+// and is right only for a kernel without shared memory.  SAPA-D with sigma 1.5 (8 x 256 x 64x64, float32), its list kernels: launched as
+// above 2037 (forward) and 3270 us (backward), in order 1207 and 2820, ahead with L1 1211 and 3068; its backward window kernel 950 as
+// above, 838 in order.
+template <typename... P, typename... A>
+inline void launch_in_order(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    kernel<<<grid, block, smem, st>>>(static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline void launch_next_with_l1(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute attribute[2];
+    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    attribute[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attribute[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxL1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid; config.blockDim = block; config.stream = st;
+    config.attrs = attribute; config.numAttrs = 2;
+    (void)cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
 }
 
 // Runs the lambda body with `scalar_t` bound to the element type named by the dtype code.

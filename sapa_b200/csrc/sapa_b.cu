@@ -456,8 +456,8 @@ __global__ void __launch_bounds__(Shape::NT, MINB) sapa_tile_kernel(const TileAr
 // One thread per low-res cell u = (y, x).  Its K*K*S*S weights W_k(p) for every (parent p, slot k) that lands
 // on u stay in registers; the high-res tile of X (TH+K-1 x TW+K-1 parents) is staged per channel.
 template <typename T, typename Shape>
-__global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *hi, const T *wt,
-                                                              T *out, int B, int Cc, int H, int W,
+__global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *__restrict__ hi, const T *__restrict__ wt,
+                                                              T *__restrict__ out, int B, int Cc, int H, int W,
                                                               int tiles_x, int tiles_y) {
     begin_after_previous();
     constexpr int K = Shape::K, S = Shape::S, KK = Shape::KK, SS = Shape::SS, R = Shape::R;
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(Shape::NT) sapa_gath_kernel(const T *hi, const
             const int gy = py0 * S + yy, gx = px0 * S + xx;
             float v = 0.f;
             if ((c0 + c) < Cc && gy >= 0 && gy < sH && gx >= 0 && gx < sW)
-                v = to_acc(load_current(himg + (size_t)(c0 + c) * hi_plane + (size_t)gy * sW + gx));
+                v = to_acc(__ldg(himg + (size_t)(c0 + c) * hi_plane + (size_t)gy * sW + gx));
             sm[c][rem] = v;
         }
         __syncthreads();
@@ -578,7 +578,11 @@ static int launch_tile(TileArgs a, cudaStream_t st) {
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    launch_next(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
+    // Blocks set up ahead go where the previous kernel leaves room first, so that grids of less than a wave end up uneven; the long blocks of
+    // K = 5 and of the backward lose more by that than the launch hides (float32, 8 x 128: aggregation at 63x61, K = 5, 47 us in order, 56
+    // ahead; backward at 64x64, K = 3, 42.5 and 47.5), the short ones less (forward at 64x64, K = 3: 34.3 in order, 31.9 ahead).
+    if (Shape::K == 5 || MODE == MODE_BWD) launch_in_order(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
+    else launch_next(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
     constexpr const char *names[4] = {"sapa_tile_kernel<sim>", "sapa_tile_kernel<agg>", "sapa_tile_kernel<fused>",
                                       "sapa_tile_kernel<bwd>"};
     return check_launch(names[MODE]);
@@ -597,7 +601,7 @@ static int launch_gath(const T *hi, const T *wt, T *out, int B, int Cc, int H, i
         using Shape = decltype(shape);
         const int tiles_x = ceil_div(W, Shape::TW), tiles_y = ceil_div(H, Shape::TH);
         const long long blocks = (long long)B * tiles_x * tiles_y;
-        launch_next(sapa_gath_kernel<T, Shape>, (unsigned)blocks, Shape::NT, 0, st, hi, wt, out, B, Cc, H, W, tiles_x, tiles_y);
+        launch_in_order(sapa_gath_kernel<T, Shape>, (unsigned)blocks, Shape::NT, 0, st, hi, wt, out, B, Cc, H, W, tiles_x, tiles_y);
         return check_launch("sapa_gath_kernel");
     };
     if constexpr (sizeof(T) == 4)

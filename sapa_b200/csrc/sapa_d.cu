@@ -1190,7 +1190,7 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     if (int e = run_agg_slab(window, value, out, B * G, C / G, H, W, rows, halo_top, 5, 2, dtype, st)) return e;
     // 4. the listed points (the count is only known on the device: a fixed grid strides over the list)
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        launch_next(deform_outlier_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(value),
+        launch_next_with_l1(deform_outlier_kernel<scalar_t>, 148 * 8, 256, st, taps, tap_count, static_cast<const scalar_t *>(value),
                                                                  static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(out),
                                                                  C, H, W, P, G, rows, halo_top);
         return check_launch("deform_outlier_kernel");
@@ -1275,7 +1275,7 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
         return e;
     if (int e = run_agg(region, value, out, B * G, C / G, H, W, 5, 2, dtype, st)) return e;
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        launch_next(deform_outlier_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(value),
+        launch_next_with_l1(deform_outlier_kernel<scalar_t>, 148 * 8, 256, st, taps, tap_count, static_cast<const scalar_t *>(value),
                                                                  static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(out), C, H,
                                                                  W, P, G, H, 0);
         return check_launch("deform_outlier_kernel");
@@ -1346,10 +1346,10 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
             const scalar_t *o = static_cast<const scalar_t *>(offset), *a = static_cast<const scalar_t *>(attn);
             scalar_t *dd = static_cast<scalar_t *>(ddense), *wn = static_cast<scalar_t *>(window), *goff = static_cast<scalar_t *>(grad_offset);
             if (P == 9)
-                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
+                launch_in_order(deform_window_bwd_kernel<scalar_t, 9, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
                                                                                       tap_count, B, C, H, W, P, G);
             else
-                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
+                launch_in_order(deform_window_bwd_kernel<scalar_t, 0, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
                                                                                       tap_count, B, C, H, W, P, G);
             return check_launch("deform_window_bwd_kernel");
         });
@@ -1362,7 +1362,7 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     // 4. the listed points.  float32: atomics straight into the gradients.  16-bit: key / value contributions go to zeroed
     //    float32 side buffers behind the list and are folded into the 16-bit gradients by one more kernel.
     if (dtype == SAPA_F32) {
-        launch_next(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
+        launch_in_order(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const float *>(grad_out), static_cast<const float *>(query), static_cast<const float *>(key),
             static_cast<const float *>(value), static_cast<const float *>(offset), static_cast<float *>(grad_query),
             static_cast<float *>(grad_key), static_cast<float *>(grad_value), static_cast<float *>(grad_offset), Cq, C, H, W, P, G);
@@ -1374,7 +1374,7 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     return SAPA_DISPATCH_FAST(dtype, [&] {
         launch_next(deform_zero_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
         if (int e = check_launch("deform_zero_scatter_kernel")) return e;
-        launch_next(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
+        launch_in_order(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(query),
             static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
             static_cast<scalar_t *>(grad_query), side_k, side_v, static_cast<scalar_t *>(grad_offset), Cq, C, H, W, P, G);
@@ -1420,12 +1420,12 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     }
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_in_order(deform_window_bwd_kernel<scalar_t, 9, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
                     static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
                     static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
             else
-                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_in_order(deform_window_bwd_kernel<scalar_t, 0, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
                     static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
                     static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
@@ -1434,7 +1434,7 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
         return e;
     if (int e = run_gath(grad_out, window, grad_value, B * G, C / G, H, W, 5, 2, dtype, st)) return e;  // dV
     if (dtype == SAPA_F32) {
-        launch_next(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
+        launch_in_order(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const float *>(grad_out), nullptr, nullptr, static_cast<const float *>(value),
             static_cast<const float *>(offset), nullptr, nullptr, static_cast<float *>(grad_value), static_cast<float *>(grad_offset),
             C, C, H, W, P, G);
@@ -1446,7 +1446,7 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     return SAPA_DISPATCH_FAST(dtype, [&] {
         launch_next(deform_zero_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
         if (int e = check_launch("deform_zero_scatter_kernel")) return e;
-        launch_next(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
+        launch_in_order(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const scalar_t *>(grad_out), nullptr, nullptr, static_cast<const scalar_t *>(value),
             static_cast<const scalar_t *>(offset), nullptr, nullptr, side_v, static_cast<scalar_t *>(grad_offset), C, C, H, W, P, G);
         if (int e = check_launch("deform_outlier_bwd_kernel")) return e;
@@ -1490,11 +1490,11 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     // the logit gradients enter where the fused chain reads the attention
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_next(deform_window_bwd_kernel<scalar_t, 9, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_in_order(deform_window_bwd_kernel<scalar_t, 9, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
                     static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
             else
-                launch_next(deform_window_bwd_kernel<scalar_t, 0, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
+                launch_in_order(deform_window_bwd_kernel<scalar_t, 0, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
                     nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
                     static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
             return check_launch("deform_window_bwd_kernel<qk>");
@@ -1503,7 +1503,7 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     if (int e = run_agg(ddense, key, grad_query, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;       // dQ
     if (int e = run_gath(query, ddense, grad_key, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;      // dKey
     if (dtype == SAPA_F32) {
-        launch_next(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
+        launch_in_order(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, nullptr, static_cast<const float *>(query), static_cast<const float *>(key), nullptr,
             static_cast<const float *>(offset), static_cast<float *>(grad_query), static_cast<float *>(grad_key), nullptr,
             static_cast<float *>(grad_offset), Cq, Cq, H, W, P, G);
@@ -1515,7 +1515,7 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     return SAPA_DISPATCH_FAST(dtype, [&] {
         launch_next(deform_zero_scatter_kernel<scalar_t>, 148 * 8, 256, 0, st, taps, tap_count, static_cast<const scalar_t *>(offset), sc, H, W, P);
         if (int e = check_launch("deform_zero_scatter_kernel")) return e;
-        launch_next(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
+        launch_in_order(deform_outlier_bwd_kernel<scalar_t, float>, 148 * 8, 256, 0, st,
             taps, tap_count, nullptr, static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), nullptr,
             static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(grad_query), side_k, nullptr,
             static_cast<scalar_t *>(grad_offset), Cq, Cq, H, W, P, G);
