@@ -10,6 +10,8 @@
 // (query: P threads of a group add to one element, so it accumulates too).
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace sapa {
 
 constexpr int MAXP = 16;   // largest num_point handled by the fused kernel
@@ -304,10 +306,9 @@ struct WindowTap {
     }
 };
 
-// NP = number of points known at compile time (0: read P at run time, up to MAXP).
-// MODE: WIN_FUSED = logits -> softmax -> window weights (the fused op); WIN_LOGITS = raw logits only, written where the
-// fused op writes the attention (deform_qk); WIN_WEIGHTS = window weights from a given attention map (deform_av).
-constexpr int WIN_FUSED = 0, WIN_LOGITS = 1, WIN_WEIGHTS = 2;
+// MODE: WIN_FUSED = logits -> softmax -> window weights (the fused op); WIN_WEIGHTS = window weights from a given attention map
+// (deform_av).  Raw logits (deform_qk) have a kernel of their own.
+constexpr int WIN_FUSED = 0, WIN_WEIGHTS = 1;
 
 // The points of a pixel inside its window: fractional parts, and the place of the upper-left cell in the thread's column of a
 // [25][WIN_THREADS] array, two points to a register.  Points that are not dense have place 0 and take no part (see `dense`); their
@@ -317,9 +318,9 @@ struct WindowPoints {
     float lh[PMAX], lw[PMAX];
     unsigned place[(PMAX + 1) / 2], dense, outliers;
     __device__ __forceinline__ int at(int p) const { return (int)(p & 1 ? place[p >> 1] >> 16 : place[p >> 1] & 0xffffu); }
+    float oh[PMAX], ow[PMAX];
     template <typename T>
-    __device__ __forceinline__ void setup(const T *offp, size_t hi, bool live, int P, int rows, int W, int py, int px) {
-        float ow[PMAX], oh[PMAX];
+    __device__ __forceinline__ void load(const T *offp, size_t hi, bool live, int P) {
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
             const bool on = live && p < P;
@@ -327,69 +328,80 @@ struct WindowPoints {
             oh[p] = on ? to_acc(offp[(size_t)(2 * p + 1) * hi]) : 0.f;
         }
         dense = outliers = 0u;
-#pragma unroll
-        for (int p = 0; p < PMAX; ++p) {
-            WindowTap t;
-            t.setup(float(py) + oh[p], float(px) + ow[p], rows, W, py, px);
-            const bool on = live && p < P, in = on && t.dense;
-            lh[p] = in ? t.lh : 0.f; lw[p] = in ? t.lw : 0.f;
-            const unsigned c = in ? (unsigned)((t.r0 * 5 + t.c0) * WIN_THREADS) : 0u;
-            place[p >> 1] = p & 1 ? place[p >> 1] | (c << 16) : c;
-            dense |= in ? 1u << p : 0u;
-            outliers |= on && t.inside && !t.dense ? 1u << p : 0u;
-        }
+    }
+    __device__ __forceinline__ void set(int p, bool on, int rows, int W, int py, int px) {
+        WindowTap t;
+        t.setup(float(py) + oh[p], float(px) + ow[p], rows, W, py, px);
+        const bool in = on && t.dense;
+        lh[p] = in ? t.lh : 0.f; lw[p] = in ? t.lw : 0.f;
+        const unsigned c = in ? (unsigned)((t.r0 * 5 + t.c0) * WIN_THREADS) : 0u;
+        place[p >> 1] = p & 1 ? place[p >> 1] | (c << 16) : c;
+        dense |= in ? 1u << p : 0u;
+        outliers |= on && t.inside && !t.dense ? 1u << p : 0u;
     }
 };
 template <int N> __device__ __forceinline__ void put(float (&v)[N], int p, float x) {      // at a place known at run time
 #pragma unroll
     for (int j = 0; j < N; ++j) v[j] = j == p ? x : v[j];
 }
+// logit of a point outside the window: the key gathered directly
+template <typename T>
+__device__ __forceinline__ float far_logit(const T *query, const T *key, const T *offp, int p, size_t bg, int gq, size_t hi, size_t lo, size_t pix, int rows, int W,
+                                           int py, int px) {
+    Bilinear<float> bl;
+    bl.setup(float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]), float(px) + to_acc(offp[(size_t)(2 * p) * hi]), rows, W);
+    const T *qp = query + bg * gq * hi + pix, *kp = key + bg * gq * lo;
+    float acc = 0.f;
+    for (int ch = 0; ch < gq; ++ch) acc += bl.sample(kp + (size_t)ch * lo) * to_acc(qp[(size_t)ch * hi]);
+    return acc;
+}
 
 // The two 25-slot windows of a thread (similarity in, window weights out) live in shared memory, column = thread, so
 // every access is conflict-free: a point touches four cells of each window, and shared memory can be indexed with the
 // cell computed at run time (a register array cannot: that form multiplies every point with all 25 cells and took
 // 82 us at B=8, 4 groups, 128 x 128 pixels).  Two passes over the points: logits and their maximum, then exp and the window
-// weights.  Bound by latency at 24 warps per SM (80 registers; 4 and 8 blocks measured slower), so the points go side by side:
-// no branch on a point (what it must not add is selected away; outliers have a loop of their own), places
-// kept from pass to pass, block = pixels of one (image, group) instead of 64-bit divisions per thread: 55 -> 43 us (float32; bfloat16 59 -> 44).
-template <typename T, int NP, int MODE>
+// weights.  Bound by latency at 24 warps per SM (80 registers, of which the form for 9 points spills 20 and that for 16 points 60; 4 and
+// 8 blocks measured slower), so the points go side by side: no branch on a point (what it must not add is selected away; outliers have a
+// loop of their own), places kept from pass to pass, block = pixels of one (image, group) instead of 64-bit divisions per thread: 55 -> 43
+// us (float32; bfloat16 59 -> 44).
+//
+// PMAX = the most points of an instance (see launch_window); 9 is the 3 x 3 points of the reference modules' default, exactly.
+template <typename T, int PMAX, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 6)
 deform_window_kernel(const T *query, const T *key, const T *offset,
                           const float *dense, T *attn, T *window,
                           OutlierTap *taps, unsigned int *tap_count, int B, int Cq, int H, int W,
                           int P_runtime, int G, int rows, int ytop) {
     begin_after_previous();
-    constexpr int PMAX = NP > 0 ? NP : MAXP;
-    __shared__ float sd[MODE != WIN_WEIGHTS ? 25 : 1][WIN_THREADS];     // dense similarity of the thread's pixel
-    __shared__ float sw[MODE != WIN_LOGITS ? 25 : 1][WIN_THREADS];      // window weights being collected
-    const int P = NP > 0 ? NP : P_runtime;
+    __shared__ float sd[MODE == WIN_FUSED ? 25 : 1][WIN_THREADS];     // dense similarity of the thread's pixel
+    __shared__ float sw[25][WIN_THREADS];                               // window weights being collected
+    const int P = PMAX == 9 ? 9 : P_runtime;
     const unsigned sW = 2 * W;
     const int gq = Cq / G;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)rows * W;
     const int lane = threadIdx.x & 31, tid = threadIdx.x;
-    const unsigned blocks = ((unsigned)hi + WIN_THREADS - 1) / WIN_THREADS, groups = (unsigned)(B * G);      // of an (image, group)
+    const unsigned blocks = ((unsigned)hi + blockDim.x - 1) / blockDim.x, groups = (unsigned)(B * G);      // of an (image, group)
     float *const dcol = &sd[0][tid], *const wcol = &sw[0][tid];
     for (unsigned bg = blockIdx.y; bg < groups; bg += gridDim.y)
     for (unsigned block = blockIdx.x; block < blocks; block += gridDim.x) {
-        const unsigned at_pix = block * WIN_THREADS + tid, pix = at_pix < hi ? at_pix : 0u;
+        const unsigned at_pix = block * blockDim.x + tid, pix = at_pix < hi ? at_pix : 0u;
         const bool live = at_pix < hi;
         const int qh = (int)(pix / sW), qw = (int)(pix - (unsigned)qh * sW), py = (qh >> 1) + ytop, px = qw >> 1;
         const T *offp = offset + (size_t)bg * P * 2 * hi + pix;
-        WindowPoints<PMAX> pts;
-        if (MODE != WIN_WEIGHTS) {
+        if (MODE == WIN_FUSED) {
             const float *dp = dense + (size_t)bg * 25 * hi + pix;
 #pragma unroll
             for (int k = 0; k < 25; ++k) dcol[k * WIN_THREADS] = live ? __ldcs(dp + (size_t)k * hi) : 0.f;
         }
-        if (MODE != WIN_LOGITS) {
 #pragma unroll
-            for (int k = 0; k < 25; ++k) wcol[k * WIN_THREADS] = 0.f;
-        }
-        pts.setup(offp, hi, live, P, rows, W, py, px);
+        for (int k = 0; k < 25; ++k) wcol[k * WIN_THREADS] = 0.f;
+        WindowPoints<PMAX> pts;
+        pts.load(offp, hi, live, P);
         // ---- pass 1: logits (or the given attention)
         float logit[PMAX];
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
+            pts.set(p, live && p < P, rows, W, py, px);
             if (MODE == WIN_WEIGHTS) {
                 logit[p] = live && p < P ? to_acc(attn[((size_t)bg * P + p) * hi + pix]) : 0.f;
             } else {
@@ -399,22 +411,11 @@ deform_window_kernel(const T *query, const T *key, const T *offset,
                 logit[p] = pts.dense >> p & 1 ? (1.f - pts.lh[p]) * top + pts.lh[p] * bot : 0.f;
             }
         }
-        if (MODE != WIN_WEIGHTS)
+        if (MODE == WIN_FUSED)
             for (unsigned left = pts.outliers; left != 0; left &= left - 1) {      // outliers: gather the key directly
                 const int p = __ffs(left) - 1;
-                Bilinear<float> bl;
-                bl.setup(float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]), float(px) + to_acc(offp[(size_t)(2 * p) * hi]), rows, W);
-                const T *qp = query + (size_t)bg * gq * hi + pix, *kp = key + (size_t)bg * gq * lo;
-                float acc = 0.f;
-                for (int ch = 0; ch < gq; ++ch) acc += bl.sample(kp + (size_t)ch * lo) * to_acc(qp[(size_t)ch * hi]);
-                put(logit, p, acc);
+                put(logit, p, far_logit(query, key, offp, p, bg, gq, hi, lo, pix, rows, W, py, px));
             }
-        if (MODE == WIN_LOGITS) {
-#pragma unroll
-            for (int p = 0; p < PMAX; ++p)
-                if (live && p < P) attn[((size_t)bg * P + p) * hi + pix] = from_acc<T>(logit[p]);
-            continue;                                       // no lane-crossing operation below was entered by any lane yet
-        }
         // ---- pass 2: exp and the window weights
         float m = -INFINITY, z = 0.f;
 #pragma unroll
@@ -458,6 +459,55 @@ deform_window_kernel(const T *query, const T *key, const T *offset,
                 t->mask = pts.outliers;
 #pragma unroll
                 for (int p = 0; p < PMAX; ++p) t->a[p] = logit[p];
+            }
+        }
+    }
+}
+
+// Raw logits of the separate op: one pass, nothing kept, each logit written as it is found.  Blocks run over the pixels of all (image,
+// group)s in one row, and a point outside the window is gathered where it is met: with the blocks and the loop of far points of
+// deform_window_kernel this pass is slower (float32, 8 x 4 groups x 128x128 pixels, with the similarity: 9 points 82 us, 64 this
+// way; bfloat16 76 and 59).
+template <typename T, int PMAX>
+__global__ void __launch_bounds__(WIN_THREADS, 6)
+deform_logits_kernel(const T *query, const T *key, const T *offset, const float *dense, T *out, int groups, int gq, int H, int W, int P_runtime) {
+    begin_after_previous();
+    __shared__ float sd[25][WIN_THREADS];                   // dense similarity of the thread's pixel
+    const int P = PMAX == 9 ? 9 : P_runtime, tid = threadIdx.x;
+    const size_t sW = 2 * (size_t)W, hi = 2 * (size_t)H * sW, lo = (size_t)H * W;
+    const long long total = (long long)groups * hi;
+    for (long long i0 = (long long)blockIdx.x * WIN_THREADS; i0 < total; i0 += (long long)gridDim.x * WIN_THREADS) {
+        const long long i = i0 + tid;
+        const bool live = i < total;
+        const size_t pix = live ? (size_t)(i % hi) : 0;
+        const long long bg = live ? i / (long long)hi : 0;
+        const int py = (int)(pix / sW) >> 1, px = (int)(pix % sW) >> 1;
+        const float *dp = dense + (size_t)bg * 25 * hi + pix;
+#pragma unroll
+        for (int k = 0; k < 25; ++k) sd[k][tid] = live ? __ldcs(dp + (size_t)k * hi) : 0.f;
+        const T *offp = offset + (size_t)bg * P * 2 * hi + pix;
+        float oh[PMAX], ow[PMAX];
+#pragma unroll
+        for (int p = 0; p < PMAX; ++p) {
+            const bool on = live && p < P;
+            ow[p] = on ? float(px) + to_acc(offp[(size_t)(2 * p) * hi]) : 0.f;
+            oh[p] = on ? float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]) : 0.f;
+        }
+#pragma unroll
+        for (int p = 0; p < PMAX; ++p) {
+            if (live && p < P) {
+                WindowTap t;
+                t.setup(oh[p], ow[p], H, W, py, px);
+                float v = 0.f;
+                if (t.dense) {
+                    const int c = t.r0 * 5 + t.c0;
+                    const float top = (1.f - t.lw) * sd[c][tid] + t.lw * sd[c + 1][tid];
+                    const float bot = (1.f - t.lw) * sd[c + 5][tid] + t.lw * sd[c + 6][tid];
+                    v = (1.f - t.lh) * top + t.lh * bot;
+                } else if (t.inside) {
+                    v = far_logit(query, key, offp, p, (size_t)bg, gq, hi, lo, pix, H, W, py, px);
+                }
+                out[((size_t)bg * P + p) * hi + pix] = from_acc<T>(v);
             }
         }
     }
@@ -931,9 +981,21 @@ static inline int grid_1d(long long total, int threads) {
     return (int)(blocks < cap ? (blocks < 1 ? 1 : blocks) : cap);
 }
 
-// blocks of the window kernels: pixels of an (image, group) along x, the (image, group)s along y
-static dim3 window_grid(int groups, size_t hi) {
-    return dim3((unsigned)((hi + WIN_THREADS - 1) / WIN_THREADS), (unsigned)(groups < 65535 ? groups : 65535), 1);
+// The window kernels for up to 4, 8, 9 (exactly) or 16 points: their loops run over all points of the instance side by side, so that those
+// that are not there cost what the others do.  8 x 4 groups x 128x128 pixels, with one point, the forms of 16 and 4 points: fused op
+// float32 189 and 141 us, bfloat16 148 and 102; 16 points 223 and 176.
+template <typename F> static void for_points(int P, F launch) {
+    if (P <= 4) launch(std::integral_constant<int, 4>());
+    else if (P <= 8) launch(std::integral_constant<int, 8>());
+    else if (P == 9) launch(std::integral_constant<int, 9>());
+    else launch(std::integral_constant<int, MAXP>());
+}
+// Blocks: pixels of an (image, group) along x, the (image, group)s along y; half-sized ones where the last of a small image would be
+// half empty or more (forward of 2048 x 4 groups x 4x16 pixels, float32: 211 us with whole blocks, 197 with halves).
+template <int MODE, typename T, typename... A> static void launch_window(int P, int groups, size_t hi, cudaStream_t st, A... args) {
+    const unsigned threads = hi <= 4 * WIN_THREADS && (hi - 1) % WIN_THREADS < WIN_THREADS / 2 ? WIN_THREADS / 2 : WIN_THREADS;
+    const dim3 grid((unsigned)((hi + threads - 1) / threads), (unsigned)(groups < 65535 ? groups : 65535), 1);
+    for_points(P, [&](auto most) { launch_next(deform_window_kernel<T, decltype(most)::value, MODE>, grid, threads, 0, st, args...); });
 }
 
 static int check_deform(const char *fn, int B, int Cq, int C, int H, int W, int P, int s, int G, int dtype) {
@@ -1171,17 +1233,10 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     }
     // 2. attention over the points, dense window weights, list of the points that leave the window
     {
-        const dim3 grid = window_grid(B * G, hi);
         const int e = SAPA_DISPATCH_FAST(dtype, [&] {
-            const scalar_t *q = static_cast<const scalar_t *>(query), *k = static_cast<const scalar_t *>(key);
-            const scalar_t *o = static_cast<const scalar_t *>(offset);
-            scalar_t *at = static_cast<scalar_t *>(attn), *wn = static_cast<scalar_t *>(window);
-            if (P == 9)          // the 3 x 3 points of the reference modules' default
-                launch_next(deform_window_kernel<scalar_t, 9, WIN_FUSED>, grid, WIN_THREADS, 0, st, q, k, o, dense, at, wn, taps, tap_count, B, Cq,
-                                                                                  H, W, P, G, rows, halo_top);
-            else
-                launch_next(deform_window_kernel<scalar_t, 0, WIN_FUSED>, grid, WIN_THREADS, 0, st, q, k, o, dense, at, wn, taps, tap_count, B, Cq,
-                                                                                  H, W, P, G, rows, halo_top);
+            launch_window<WIN_FUSED, scalar_t>(P, B * G, hi, st, static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key),
+                                               static_cast<const scalar_t *>(offset), dense, static_cast<scalar_t *>(attn), static_cast<scalar_t *>(window), taps,
+                                               tap_count, B, Cq, H, W, P, G, rows, halo_top);
             return check_launch("deform_window_kernel");
         });
         if (e) return e;
@@ -1227,14 +1282,11 @@ int sapa_deform_qk_forward_dense(const void *query, const void *key, const void 
         if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st)) return e;
     }
     return SAPA_DISPATCH_FAST(dtype, [&] {
-        if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-            launch_next(deform_window_kernel<scalar_t, 9, WIN_LOGITS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
-                static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
-                static_cast<scalar_t *>(out), nullptr, nullptr, nullptr, B, Cq, H, W, P, G, H, 0);
-        else
-            launch_next(deform_window_kernel<scalar_t, 0, WIN_LOGITS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
-                static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
-                static_cast<scalar_t *>(out), nullptr, nullptr, nullptr, B, Cq, H, W, P, G, H, 0);
+        for_points(P, [&](auto most) {
+            launch_next(deform_logits_kernel<scalar_t, decltype(most)::value>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
+                        static_cast<const scalar_t *>(query), static_cast<const scalar_t *>(key), static_cast<const scalar_t *>(offset), dense,
+                        static_cast<scalar_t *>(out), B * G, Cq / G, H, W, P);
+        });
         return check_launch("deform_window_kernel<logits>");
     });
 }
@@ -1262,14 +1314,9 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
     }
     // the attention is only read in this mode
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
-            if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_next(deform_window_kernel<scalar_t, 9, WIN_WEIGHTS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
-                    nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr, const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)),
-                    reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C, H, W, P, G, H, 0);
-            else
-                launch_next(deform_window_kernel<scalar_t, 0, WIN_WEIGHTS>, window_grid(B * G, hi), WIN_THREADS, 0, st,
-                    nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr, const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)),
-                    reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C, H, W, P, G, H, 0);
+            launch_window<WIN_WEIGHTS, scalar_t>(P, B * G, hi, st, nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr,
+                                                 const_cast<scalar_t *>(static_cast<const scalar_t *>(attn)), reinterpret_cast<scalar_t *>(region), taps, tap_count, B, C,
+                                                 H, W, P, G, H, 0);
             return check_launch("deform_window_kernel<weights>");
         }))
         return e;
