@@ -1016,9 +1016,11 @@ __global__ void deform_clear_counter_kernel(unsigned int *counter) {
     begin_after_previous();
     *counter = 0u;
 }
-static cudaError_t clear_counter(unsigned int *counter, cudaStream_t st) {
+static int clear_counter(const char *fn, unsigned int *counter, cudaStream_t st) {
     launch_next(deform_clear_counter_kernel, 1, 1, 0, st, counter);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    SAPA_REQUIRE(e == cudaSuccess, SAPA_ERR_LAUNCH, "%s: clearing the outlier counter failed: %s", fn, cudaGetErrorString(e));
+    return SAPA_OK;
 }
 
 static int memset_async(void *p, size_t bytes, cudaStream_t st, const char *fn) {
@@ -1220,10 +1222,7 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     void *window = dense + (size_t)B * G * 25 * hi;
     OutlierTap *taps = reinterpret_cast<OutlierTap *>(dense + (size_t)B * G * 50 * hi);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * hi);
-    if (clear_counter(tap_count, st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed", fn);
-        return SAPA_ERR_LAUNCH;
-    }
+    if (int e = clear_counter(fn, tap_count, st)) return e;
     // 1. dense 25-slot similarity of every group: the B x G groups are images of Cq / G channels.  16-bit tensors: the
     //    logits leave the tensor-core kernel as float32 (a 16-bit logit would cost the softmax two digits)
     if (dtype == SAPA_F32) {
@@ -1308,10 +1307,7 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
     float *region = static_cast<float *>(workspace) + (size_t)B * G * 25 * hi;      // the window weights (tensor type) live here
     OutlierTap *taps = reinterpret_cast<OutlierTap *>(region + (size_t)B * G * 25 * hi);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * hi);
-    if (clear_counter(tap_count, st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed", fn);
-        return SAPA_ERR_LAUNCH;
-    }
+    if (int e = clear_counter(fn, tap_count, st)) return e;
     // the attention is only read in this mode
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             launch_window<WIN_WEIGHTS, scalar_t>(P, B * G, hi, st, nullptr, nullptr, static_cast<const scalar_t *>(offset), nullptr,
@@ -1373,10 +1369,7 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     void *ddense = dwin + plane, *window = dwin + 2 * plane;
     OutlierGrad *taps = reinterpret_cast<OutlierGrad *>(dense + 4 * plane);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
-    if (clear_counter(tap_count, st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed", fn);
-        return SAPA_ERR_LAUNCH;
-    }
+    if (int e = clear_counter(fn, tap_count, st)) return e;
     // 1. D = sim(Q, Key) and dWd = sim(dOut, Value), the B x G groups as images
     if (dtype == SAPA_F32) {
         if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;
@@ -1456,10 +1449,7 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     void *window = dwin + 2 * plane;                                   // Wd, in the tensors' type
     OutlierGrad *taps = reinterpret_cast<OutlierGrad *>(static_cast<float *>(workspace) + 4 * plane);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
-    if (clear_counter(tap_count, st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed", fn);
-        return SAPA_ERR_LAUNCH;
-    }
+    if (int e = clear_counter(fn, tap_count, st)) return e;
     if (dtype == SAPA_F32) {
         if (int e = run_sim(grad_out, value, dwin, B * G, C / G, H, W, 5, 2, dtype, st)) return e;        // dWd
     } else {
@@ -1525,10 +1515,7 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     void *ddense = dense + 2 * plane;                                  // dD, in the tensors' type
     OutlierGrad *taps = reinterpret_cast<OutlierGrad *>(dense + 4 * plane);
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
-    if (clear_counter(tap_count, st) != cudaSuccess) {
-        set_error("%s: clearing the outlier counter failed", fn);
-        return SAPA_ERR_LAUNCH;
-    }
+    if (int e = clear_counter(fn, tap_count, st)) return e;
     if (dtype == SAPA_F32) {
         if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;         // D, for the offset gradients
     } else {

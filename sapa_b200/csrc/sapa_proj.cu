@@ -745,15 +745,15 @@ static int run_list(const char *fn, const sapa_projection *p, const int *shuffle
                  "%s: needs float32 / float16 / bfloat16 (output of the same type, or 16 bits of float32), d a multiple of 16 up to 1024, rows of HW and C "
                  "elements that are multiples of 16 bytes and C divisible by groups", fn);
     for (int i = 0; i < n; ++i) {
-        const sapa_projection &q = p[i];
-        SAPA_CHECK_PTR(fn, q.x); SAPA_CHECK_PTR(fn, q.weight);
-        if (q.groups > 0) { SAPA_CHECK_PTR(fn, q.gamma); SAPA_CHECK_PTR(fn, q.beta); }
-        SAPA_REQUIRE(q.out != nullptr && all_aligned16(q.x, q.out), SAPA_ERR_ALIGNMENT, "%s: x and out must be 16-byte aligned", fn);
-        const int w = shuffle != nullptr ? shuffle[i] : 0;
-        SAPA_REQUIRE(w >= 0 && (w == 0 || q.HW % w == 0), SAPA_ERR_ARGUMENT, "%s: bad shuffle width", fn);
+        const void *x = p[i].x, *gamma = p[i].gamma, *beta = p[i].beta, *weight = p[i].weight, *out = p[i].out;
+        SAPA_CHECK_PTR(fn, x); SAPA_CHECK_PTR(fn, weight);
+        if (p[i].groups > 0) { SAPA_CHECK_PTR(fn, gamma); SAPA_CHECK_PTR(fn, beta); }
+        SAPA_REQUIRE(out != nullptr && all_aligned16(x, out), SAPA_ERR_ALIGNMENT, "%s: x and out must be 16-byte aligned", fn);
     }
     SAPA_REQUIRE(workspace != nullptr && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 256 == 0, SAPA_ERR_WORKSPACE,
                  "%s: a 256-byte aligned workspace of %zu bytes is required, got %zu", fn, need, workspace_bytes);
+    for (int i = 0; i < n && shuffle != nullptr; ++i)
+        SAPA_REQUIRE(shuffle[i] >= 0 && (shuffle[i] == 0 || p[i].HW % shuffle[i] == 0), SAPA_ERR_ARGUMENT, "%s: bad shuffle width", fn);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     for (int i = 0; i < count; i += MAX_PROBLEMS) {
         const int m = std::min(MAX_PROBLEMS, count - i);
@@ -808,6 +808,7 @@ int sapa_project_forward(const void *x, const void *gamma, const void *beta, con
     SAPA_REQUIRE(sapa_project_workspace(B, C, HW, d, groups, dtype) != 0, SAPA_ERR_UNSUPPORTED,
                  "%s: needs float32 / float16 / bfloat16, d a multiple of 16 up to 256, rows of HW and C elements that are "
                  "multiples of 16 bytes and C divisible by groups (got B=%d C=%d HW=%d d=%d groups=%d)", fn, B, C, HW, d, groups);
+    SAPA_CHECK_PTR(fn, x); SAPA_CHECK_PTR(fn, weight); SAPA_CHECK_PTR(fn, out);
     const sapa_projection q{x, gamma, beta, weight, bias, out, nullptr, B, C, HW, d, groups, eps};
     return proj::run_list(fn, &q, nullptr, 1, workspace, workspace_bytes, dtype, dtype, false, static_cast<cudaStream_t>(stream));
 }

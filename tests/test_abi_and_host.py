@@ -56,6 +56,24 @@ def test_argument_validation_needs_no_gpu():
     assert h.sapa_fused_backward_workspace(8, 64, 64, 5, 2, 0) == 8 * 25 * 128 * 128 * 4
 
 
+def test_projection_arguments_are_refused_by_name():
+    from sapa_b200 import _lib
+    h = _lib.lib()
+    null, ok = ctypes.c_void_p(0), ctypes.c_void_p(4096)
+    sizes = (2, 64, 64, 32, 8, 1e-5)                     # B, C, HW, d, groups, eps
+
+    def call(x=ok, gamma=ok, beta=ok, weight=ok, out=ok, workspace=ok, size=1 << 30):
+        return h.sapa_project_forward(x, gamma, beta, weight, null, out, workspace, size, *sizes, 0, null), h.sapa_last_error()
+    for name in ("x", "gamma", "beta", "weight", "out"):
+        assert call(**{name: null}) == (-1, f"sapa_project_forward: {name} is NULL".encode())
+    assert call(out=ctypes.c_void_p(4100))[0] == -3
+    assert call(size=16)[0] == -6
+    rows = lambda width, size, out=ok: h.sapa_project_rows_forward(ok, ok, ok, ok, null, out, width, ok, size, *sizes, 0, 0, null)
+    assert rows(5, 1 << 30) == -1 and b"shuffle" in h.sapa_last_error()
+    assert rows(5, 16) == -6                              # the workspace is looked at first
+    assert rows(0, 1 << 30, null) == -3
+
+
 def test_cpu_tensors_raise_not_implemented_like_the_reference():
     import sapa_b200 as sp
     q, k, v = torch.randn(1, 4, 4, 4), torch.randn(1, 4, 2, 2), torch.randn(1, 3, 2, 2)
