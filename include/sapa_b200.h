@@ -54,7 +54,8 @@ const char *sapa_last_error(void);
  * "sapa_tma_fused_f32_kernel<bwd>,sapa_gath_mma_kernel,sapa_gath_mma_kernel"; "" before the first call.  A host-side
  * record (no device work) meant for tests and diagnostics: they assert which kernel a shape exercised, so that a
  * silent fall-back to a slower kernel cannot pass unnoticed.  With several threads calling at once it describes
- * whichever call started last.  The returned string is valid until the calling thread asks again.
+ * whichever call started last.  The one thread that clears the counter of SAPA-D's list of far points is not named, as the memset
+ * before it was not.  The returned string is valid until the calling thread asks again.
  * No counterpart in the reference. */
 const char *sapa_last_kernels(void);
 /* ABI version of this header (bumped on any signature change). */
@@ -327,7 +328,7 @@ typedef struct sapa_projection {
     float eps;
 } sapa_projection;
 
-/* sapa_project_rows_forward for up to three projections in the same launches: one for the statistics of all that have a norm (taken
+/* sapa_project_rows_forward for up to three projections in the same launches (what the modules call at inference): one for the statistics of all that have a norm (taken
  * once for projections of the same x), one for the folds, one for the products; what no projection of the list needs is not launched.
  * shuffle_widths: one per projection, or NULL.  `stats` is not written.  Workspace: sapa_project_list_workspace() bytes (0: not
  * supported) for the same records, 256-byte aligned. */
