@@ -35,8 +35,8 @@ struct Api {
     SAPA_FN(sapa_deform_av_forward_dense) SAPA_FN(sapa_deform_av_backward_dense) SAPA_FN(sapa_deform_fused_forward_dense) \
     SAPA_FN(sapa_deform_fused_backward_dense) SAPA_FN(sapa_deform_fused_forward_workspace)                                \
     SAPA_FN(sapa_deform_fused_backward_workspace) SAPA_FN(sapa_deform_fused_backward_scatter_bytes)                       \
-    SAPA_FN(sapa_project_workspace) SAPA_FN(sapa_project_forward) SAPA_FN(sapa_project_rows_workspace)                    \
-    SAPA_FN(sapa_project_list_workspace) SAPA_FN(sapa_project_list_forward) SAPA_FN(sapa_projections_workspace) SAPA_FN(sapa_projections_forward)              \
+    SAPA_FN(sapa_project_workspace) SAPA_FN(sapa_project_forward) SAPA_FN(sapa_project_list_workspace)                    \
+    SAPA_FN(sapa_project_list_forward) SAPA_FN(sapa_projections_workspace) SAPA_FN(sapa_projections_forward)              \
     SAPA_FN(sapa_projections_backward_workspace) SAPA_FN(sapa_projections_backward)
     SAPA_FNS
 #undef SAPA_FN

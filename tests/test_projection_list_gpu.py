@@ -63,3 +63,59 @@ def test_list_equals_separate_float64(name, dtype, tol):
         if shuffle:
             ref = F.pixel_shuffle(ref, 2)
         assert float((out.double() - ref).abs().max() / ref.abs().max()) < tol
+
+
+def _reference(q, groups, shuffle):
+    y = q["x"].double()
+    if groups:
+        y = F.group_norm(y, groups, q["gamma"].double(), q["beta"].double(), 1e-5)
+    ref = F.conv2d(y, q["w"].double().view(q["w"].shape[0], -1, 1, 1), q["b"].double() if q["b"] is not None else None)
+    return F.pixel_shuffle(ref, 2) if shuffle else ref
+
+
+@pytest.mark.parametrize("out_dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 1e-2), (torch.float16, 2e-3)])
+def test_float32_lists_with_16_bit_outputs(out_dtype, tol):
+    """Mixed precision: float32 products, rounded once when they are written."""
+    from sapa_b200 import _lib
+    handle = _lib.lib()
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    inputs, problems = LISTS["shared_statistics"]
+    xs = [torch.randn(*s, generator=gen, device="cuda") for s in inputs]
+    made = [_problem(gen, xs[i], d, g, b, torch.float32, odd) for i, d, g, b, _, odd in problems]
+    records, outs = (Record * len(made))(), []
+    for r, q, (_, d, groups, _, shuffle, _) in zip(records, made, problems):
+        B, C, H, W = q["x"].shape
+        outs.append(torch.empty((B, d // 4, 2 * H, 2 * W) if shuffle else (B, d, H, W), device="cuda", dtype=out_dtype))
+        for field, t in (("x", q["x"]), ("gamma", q["gamma"]), ("beta", q["beta"]), ("weight", q["w"]), ("bias", q["b"]), ("out", outs[-1])):
+            setattr(r, field, t.data_ptr() if t is not None else None)
+        r.B, r.C, r.HW, r.d, r.groups, r.eps = B, C, H * W, d, groups, 1e-5
+    need = handle.sapa_project_list_workspace(records, len(made), 0)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    code = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[out_dtype]
+    assert handle.sapa_project_list_forward(records, (ctypes.c_int * len(made))(*[p[4] for p in problems]), len(made), ws.data_ptr(), need, 0, code,
+                                            torch.cuda.current_stream().cuda_stream) == 0, handle.sapa_last_error()
+    for q, out, (_, _, groups, _, shuffle, _) in zip(made, outs, problems):
+        ref = _reference(q, groups, shuffle)
+        assert float((out.double() - ref).abs().max() / ref.abs().max()) < tol
+
+
+@pytest.mark.parametrize("d,groups,shuffle,bias", [(32, 0, 10, True), (288, 0, 10, False), (288, 8, 0, True), (1024, 32, 10, True)])
+@pytest.mark.parametrize("dtype,out_dtype,tol", [(torch.float32, torch.float32, 1e-5), (torch.float32, torch.bfloat16, 1e-2), (torch.bfloat16, torch.bfloat16, 1e-2),
+                                                 (torch.float16, torch.float16, 2e-3)])
+def test_one_projection_of_many_rows(d, groups, shuffle, bias, dtype, out_dtype, tol):
+    """sapa_project_rows_forward: parts of up to 256 rows, sub-pixels, 16-bit outputs of float32; everything is folded."""
+    from sapa_b200 import _lib
+    handle = _lib.lib()
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    B, C, H, W = 2, 96, 8, 10
+    q = _problem(gen, torch.randn(B, C, H, W, generator=gen, device="cuda").to(dtype), d, groups, bias, dtype, False)
+    out = torch.empty((B, d // 4, 2 * H, 2 * W) if shuffle else (B, d, H, W), device="cuda", dtype=out_dtype)
+    codes = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
+    need = handle.sapa_project_rows_workspace(B, C, H * W, d, groups, codes[dtype])
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    pointer = lambda t: t.data_ptr() if t is not None else None
+    status = handle.sapa_project_rows_forward(pointer(q["x"]), pointer(q["gamma"]), pointer(q["beta"]), pointer(q["w"]), pointer(q["b"]), pointer(out), shuffle,
+                                              ws.data_ptr(), need, B, C, H * W, d, groups, 1e-5, codes[dtype], codes[out_dtype], torch.cuda.current_stream().cuda_stream)
+    assert status == 0, handle.sapa_last_error()
+    ref = _reference(q, groups, shuffle)
+    assert float((out.double() - ref).abs().max() / ref.abs().max()) < tol
