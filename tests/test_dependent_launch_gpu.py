@@ -32,9 +32,11 @@ def test_calls_back_to_back(deform, dtype, W):
         torch.cuda.synchronize()
         alone.append([t.clone() for t in one(x, go)])
         torch.cuda.synchronize()
+    # compared on the device and freed, so that the next call gets the memory and nothing waits in between
+    atomics = deform and dtype != torch.float32 and W % 8      # the gather/scatter kernels: float32 sums in any order, rounded to 16 bits
+    worst = torch.zeros((), device="cuda", dtype=torch.float64)
     for _ in range(5):
-        got = [one(x, go) for x, go in cases]
-        one(*cases[0])                                   # its buffers take the place of nothing that is still compared
-        for a, b in zip(alone, got):
-            for u, v in zip(a, b):
-                assert torch.equal(u, v) if not (deform and W % 8) else torch.allclose(u.float(), v.float(), rtol=2e-2, atol=2e-2)
+        for (x, go), want in zip(cases, alone):
+            for u, v in zip(want, one(x, go)):
+                worst = torch.maximum(worst, ((u.double() - v.double()).norm() / u.double().norm()) if atomics else (u != v).sum().double())
+    assert float(worst) <= (2.0 ** -8 if atomics else 0.0)
