@@ -604,8 +604,9 @@ static bool make_layout(Layout &l, int rows, int acc_cols, int esize) {
     return true;
 }
 
-// blocks of the statistics: at least two of the eight an SM holds for every SM, and slices of at most 32 KB, so that the last wave is
-// a small part of the whole
+// slices of a group for the statistics: as many as fill the eight blocks an SM holds on every SM, or, where that is more, of 32 KB, so that
+// the last wave is a small part of the whole; at most MAX_SPLIT, which leaves a single group on 64 blocks and gives one of 16 MB slices of
+// 256 KB
 static int stat_splits(int B, int groups, long long n, int esize) {
     const long long fill = (148 * 8 + (long long)B * groups - 1) / ((long long)B * groups), even = (n * esize + STAT_SLICE - 1) / STAT_SLICE;
     return (int)std::max<long long>(1, std::min<long long>(MAX_SPLIT, std::max(fill, even)));
