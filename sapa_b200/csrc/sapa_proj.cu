@@ -71,7 +71,7 @@ struct Problem {
     CUtensorMap x_map;              // (pixel, channel, 1, image), box = one 128-byte pixel row x (128 B / esize) channels
     CUtensorMap whi_map, wlo_map;   // (channel, output channel, 1, image), box = 128 bytes of channels x d rows
     const float *bias;              // folded bias [images or 1][d]; nullptr: `bias_as_given`
-    const void *bias_as_given;      // [d] of the activations' type, or nullptr (no bias)
+    const void *bias_as_given;      // [d] of the activations' type on a 16-byte boundary, or nullptr (no bias)
     void *out;                      // first of the d rows of image 0; images are out_rows rows of HW elements apart
     int out_rows;
     int shuffle_w;                  // > 0: the rows are sub-pixels, written as torch.pixel_shuffle(., 2) would place them (row
@@ -368,9 +368,30 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
                     mbar_arrive(tempty0 + 8 * buf);
                 }
                 float v[16];
+                if (folded != nullptr) {                // one branch for all: one per element costs more than the rest of the epilogue
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    v[j] = __uint_as_float(r[j]) + (folded != nullptr ? load_current(folded + c0 + j) : given != nullptr ? to_acc(load_current(given + c0 + j)) : 0.f);
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 t = load_current(reinterpret_cast<const float4 *>(folded + c0) + j);
+                        v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
+                    }
+                } else if (!F32 && given != nullptr) {
+                    if constexpr (!F32)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            const uint4 t = load_current(reinterpret_cast<const uint4 *>(given + c0) + j);
+                            const unsigned w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const float2 f = unpack_pair(T(), w[i]);
+                                v[8 * j + 2 * i] = f.x; v[8 * j + 2 * i + 1] = f.y;
+                            }
+                        }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
                 if (px < HW && p.shuffle_w > 0) {
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) store_pair<TO>(op + (size_t)(c0 + (j & ~3)) * HW + (j & 2) * p.shuffle_w, v[j], v[j + 1]);
@@ -640,7 +661,7 @@ static size_t make_parts(Part *parts, int &count, const sapa_projection *p, cons
             const int nimg = q.groups > 0 ? q.B : 1;
             t.nsplit = q.groups > 0 ? stat_splits(q.B, q.groups, (long long)(q.C / q.groups) * q.HW, esize) : 1;
             t.stats = q.groups > 0;
-            t.fold = q.groups > 0 || esize == 4 || !list ||
+            t.fold = q.groups > 0 || esize == 4 || !list || !aligned16(q.bias) ||
                      !aligned16(static_cast<const unsigned char *>(q.weight) + (size_t)r * q.C * esize);
             for (int j = 0; j < count - 1 && t.stats; ++j)
                 if (parts[j].stats && (parts[j].q == t.q || same_norm(*parts[j].q, q))) {
