@@ -28,14 +28,19 @@ using namespace tmau;
 
 constexpr int THREADS = 256;
 
+// IN_ORDER: the kernel starts when the previous one has ended, so what it reads does not change while it runs (see begin_after_previous)
+template <bool IN_ORDER, typename T> __device__ __forceinline__ T fetch_once(const T *p) {
+    if constexpr (IN_ORDER) return __ldg(p);
+    else return *p;
+}
 // 8 consecutive elements of a row, the ones from `valid` on as zeros
-template <typename T> __device__ __forceinline__ void load8(const T *p, int valid, bool vec, float (&v)[8]) {
+template <bool IN_ORDER = false, typename T> __device__ __forceinline__ void load8(const T *p, int valid, bool vec, float (&v)[8]) {
     if (vec && valid >= 8) {
         if constexpr (sizeof(T) == 4) {
-            const float4 a = *reinterpret_cast<const float4 *>(p), b = reinterpret_cast<const float4 *>(p)[1];
+            const float4 a = fetch_once<IN_ORDER>(reinterpret_cast<const float4 *>(p)), b = fetch_once<IN_ORDER>(reinterpret_cast<const float4 *>(p) + 1);
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
-            const uint4 u = *reinterpret_cast<const uint4 *>(p);
+            const uint4 u = fetch_once<IN_ORDER>(reinterpret_cast<const uint4 *>(p));
             const unsigned w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -49,7 +54,7 @@ template <typename T> __device__ __forceinline__ void load8(const T *p, int vali
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = i < valid ? to_acc(p[i]) : 0.f;
+        for (int i = 0; i < 8; ++i) v[i] = i < valid ? to_acc(fetch_once<IN_ORDER>(p + i)) : 0.f;
     }
 }
 __device__ __forceinline__ void sts8(unsigned addr, const float (&v)[8]) {
@@ -264,8 +269,8 @@ __global__ void __launch_bounds__(THREADS, 2) proj_moments_kernel(const __grid_c
     const auto fetch = [&](int p0) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            load8(x[i] + p0 + col, x[i] != nullptr ? p_end - p0 - col : 0, m.vec_x, xv[i]);
-            load8(gr[i] + p0 + col, gr[i] != nullptr ? p_end - p0 - col : 0, m.vec_g, gv[i]);
+            load8<LO>(x[i] + p0 + col, x[i] != nullptr ? p_end - p0 - col : 0, m.vec_x, xv[i]);
+            load8<LO>(gr[i] + p0 + col, gr[i] != nullptr ? p_end - p0 - col : 0, m.vec_g, gv[i]);
         }
     };
     fetch(split * m.slice);
@@ -276,7 +281,7 @@ __global__ void __launch_bounds__(THREADS, 2) proj_moments_kernel(const __grid_c
         for (int i = tid; i < MO_C * ((m.d + 7) & ~7); i += THREADS) {
             const int c = i & (MO_C - 1), j = i / MO_C, cc = cb * MO_C + c;
             const T *w = j < m.d1 ? static_cast<const T *>(m.w1) + (size_t)j * m.C : static_cast<const T *>(m.w2) + (size_t)(j - m.d1) * m.C;
-            ws[c * MO_PITCH + j] = cc < m.C && j < m.d ? rounded<TG>(to_acc(w[cc])) : 0.f;
+            ws[c * MO_PITCH + j] = cc < m.C && j < m.d ? rounded<TG>(to_acc(fetch_once<LO>(w + cc))) : 0.f;
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -629,8 +634,10 @@ static int run_forward(const sapa_projection *q, int count, unsigned char *ws, c
         launch_next(proj_stats_kernel<T>, sblocks, THREADS, 0, st, sl);
         if (int e = check_launch("proj_stats_kernel")) return e;
     }
-    if (mt == 32) launch_next(proj_fwd_kernel<T, TO, 32>, fblocks, THREADS, 0, st, fl);
-    else launch_next(proj_fwd_kernel<T, TO, 64>, fblocks, THREADS, 0, st, fl);
+    // The float32 forms, three products an element, have long blocks, of which a grid of less than a wave set up ahead makes an uneven
+    // load: 3 x 192 x 25x31, 64 rows: 23 us in order, 38 ahead.
+    if (sizeof(TO) == 4) launch_in_order(mt == 32 ? proj_fwd_kernel<T, TO, 32> : proj_fwd_kernel<T, TO, 64>, fblocks, THREADS, 0, st, fl);
+    else launch_next(mt == 32 ? proj_fwd_kernel<T, TO, 32> : proj_fwd_kernel<T, TO, 64>, fblocks, THREADS, 0, st, fl);
     return check_launch("proj_fwd_kernel");
 }
 
@@ -715,13 +722,16 @@ static int run_backward(const sapa_projection_grad *q, int count, unsigned char 
     }
     constexpr int smem_norm = 3 * MO_C * MO_PITCH * 4, smem_plain = 2 * MO_C * MO_PITCH * 4;
     int sms = 0;
+    // float32 in order, as above, and then with __ldg: 16 x 128 x 64x64 with a norm 192 us, ahead 200, ahead with plain loads 228
     if (ml[1].count > 0) {
         if (int e = prepare_launch(reinterpret_cast<const void *>(proj_moments_kernel<T, TG, true>), smem_norm, "proj_moments_kernel", sms)) return e;
-        launch_next(proj_moments_kernel<T, TG, true>, mblocks[1], THREADS, smem_norm, st, ml[1]);
+        if (sizeof(TG) == 4) launch_in_order(proj_moments_kernel<T, TG, true>, mblocks[1], THREADS, smem_norm, st, ml[1]);
+        else launch_next(proj_moments_kernel<T, TG, true>, mblocks[1], THREADS, smem_norm, st, ml[1]);
         if (int e = check_launch("proj_moments_kernel")) return e;
     }
     if (ml[0].count > 0) {
-        launch_next(proj_moments_kernel<T, TG, false>, mblocks[0], THREADS, smem_plain, st, ml[0]);
+        if (sizeof(TG) == 4) launch_in_order(proj_moments_kernel<T, TG, false>, mblocks[0], THREADS, smem_plain, st, ml[0]);
+        else launch_next(proj_moments_kernel<T, TG, false>, mblocks[0], THREADS, smem_plain, st, ml[0]);
         if (int e = check_launch("proj_moments_kernel")) return e;
     }
     launch_next(proj_fold_kernel<T>, fblocks, THREADS, 0, st, fl);

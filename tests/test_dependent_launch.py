@@ -27,7 +27,7 @@ def _functions(text):
 def test_dependent_kernels_read_through_the_coherent_path():
     ahead, waiting, texts = set(), set(), list(_sources())
     for _, text in texts:
-        ahead |= set(re.findall(r"\blaunch_(?:next|next_with_l1|with_smem|persistent)\(\s*(\w+)", text)) - {"void", "kernel", "Kernel"}
+        ahead |= set(re.findall(r"\blaunch_(?:next|next_with_l1|with_smem|persistent)\(\s*(?:mt == 32 \? )?(\w+)", text)) - {"void", "kernel", "Kernel"}
     for name, text in texts:
         for head, body in _functions(text):
             kernel = "__global__" in head and re.findall(r"(\w+)\s*\(\s*(?:const|unsigned|int)\b", head)[-1]
@@ -38,7 +38,7 @@ def test_dependent_kernels_read_through_the_coherent_path():
                 assert "__restrict__" not in head, (name, head)
             if kernel in ahead or (not kernel and "begin_after_previous();" in text):      # device functions of these files serve such kernels
                 body = body.replace("if constexpr (IN_ORDER) return __ldg(p);", "")
-                assert "__ldg" not in body and not re.search(r"Bilinear<\w+, true>", body), (name, head)
+                assert "__ldg" not in body and not re.search(r"Bilinear<\w+, true>|(?:fetch_once|load8)<true", body), (name, head)
                 for p in head.split(","):                 # `sm`: shared memory
                     assert not re.search(r"\bconst\b.*__restrict__ (?!sm$)", p.strip()), (name, p)
     assert ahead and ahead <= waiting, ahead - waiting
