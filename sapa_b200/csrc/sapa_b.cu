@@ -578,10 +578,12 @@ static int launch_tile(TileArgs a, cudaStream_t st) {
         set_error("too many tiles");
         return SAPA_ERR_ARGUMENT;
     }
-    // Blocks set up ahead go where the previous kernel leaves room first, so that grids of less than a wave end up uneven; the long blocks of
-    // K = 5 and of the backward lose more by that than the launch hides (float32, 8 x 128: aggregation at 63x61, K = 5, 47 us in order, 56
-    // ahead; backward at 64x64, K = 3, 42.5 and 47.5), the short ones less (forward at 64x64, K = 3: 34.3 in order, 31.9 ahead).
-    if (Shape::K == 5 || MODE == MODE_BWD) launch_in_order(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
+    // Blocks set up ahead go where the previous kernel leaves room first, so that grids of less than a wave end up uneven.  Long blocks, those
+    // of K = 5 with many channels and of the backward, lose more by that than the launch hides (float32, 8 images: aggregation of 128
+    // channels at 63x61, K = 5, 47 us in order, 56 ahead; similarity of 32 there 18.7 and 20.0; backward at 64x64, K = 3, 42.5 and 47.5),
+    // short ones less (forward at 64x64, K = 3: 34.3 and 31.9; the chain of SAPA-D with 4 and 24 channels a group, 3 x 51x37: 35.4 and 31.6).
+    const bool in_order = MODE == MODE_BWD || (Shape::K == 5 && (MODE == MODE_SIM ? a.C1 : a.C2) >= 32);
+    if (in_order) launch_in_order(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
     else launch_next(sapa_tile_kernel<T, Shape, MODE, 3>, (unsigned)blocks, Shape::NT, 0, st, a);
     constexpr const char *names[4] = {"sapa_tile_kernel<sim>", "sapa_tile_kernel<agg>", "sapa_tile_kernel<fused>",
                                       "sapa_tile_kernel<bwd>"};

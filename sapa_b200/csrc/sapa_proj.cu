@@ -12,8 +12,8 @@
 // The launches take a LIST of problems: all projections of a module share them, and what a problem does not need is left out
 // (16-bit rows without a norm are multiplied with the weight as it is: no statistics, no fold).  A launch of a small problem is
 // latency: the four GEMMs and four folds of a SAPADeform module (4 x 256 x 32x32, d = 128, 288 offset rows, float16) took 41 us and
-// the gaps between them, their one launch takes 21 (the module 91 -> 57 us); three chained SAPA modules (16 x 256, 16x16 -> 128x128,
-// bfloat16), eighteen launches before, 293 -> 254 us.
+// the gaps between them, their one launch takes 13 (the module 91 -> 42 us); three chained SAPA modules (16 x 256, 16x16 -> 128x128,
+// bfloat16), eighteen launches before, 293 -> 220 us.
 //
 // GEMM kernel (tcgen05 / TMEM; one CTA per SM, 128-pixel tiles):
 //   D[128 px x d] (+)= A[128 px x k] * B[k x d],  A = x^T, B = W' (K-major: channels contiguous)
