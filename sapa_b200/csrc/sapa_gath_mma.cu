@@ -19,8 +19,11 @@
 //     sums through shared memory (an mbarrier handshake per pair and stage), nothing is CTA-wide in the steady state;
 //   * ring protocol: full / empty mbarriers, one lane of a ninth, producer-only warp refills a slot as soon as all 8 warps released it;
 //     every wait is bounded and raises g_wait_timeout instead of spinning for ever.
-#include "tma_util.cuh"
+// Larger problems with rows of 16 bytes go to the tcgen05 kernel of sapa_gath_umma.cuh instead (umma_pays), recorded under the name of
+// the form that it stands for.
+#include "umma_util.cuh"
 
+#include <algorithm>
 #include <atomic>
 
 namespace sapa {
@@ -81,28 +84,32 @@ template <typename T> __device__ __forceinline__ int px_off(int px, int ch) {
     else                          return ((((px >> 3) ^ (ch >> 1)) & 3) << 4) | ((px & 7) << 1);             // 64-byte swizzle
 }
 
-// A lane's outputs again, columns x and x + 1 of every eighth channel, as sums over the pixels of a cell's own parents alone; for a
-// lane with a sum that is not finite.  The matrix product also takes the other pixels of its fragments, with weights of zero, and
-// 0 * inf would reach cells that no infinity reaches.
+// G[c][(y, x)] over the pixels of the cell's own parents alone.
 template <typename T>
-__device__ __forceinline__ void store_cell_sums(const Args &a, int n, int c0, int count, int y, int x0) {
+__device__ __forceinline__ float cell_sum(const Args &a, int n, int c, int y, int x) {
     const int sW = 2 * a.W;
     const size_t hi_plane = (size_t)(2 * a.H) * sW;
+    float s = 0.f;
+#pragma unroll 1
+    for (int cell = 0; cell < 25; ++cell) {       // window cell of the parent that reaches (y, x) through it
+        const int yp = y - a.top + 2 - cell / 5, xp = x + 2 - cell % 5;
+        if (yp < 0 || yp >= a.H || xp < 0 || xp >= a.W) continue;
+        const size_t at = (size_t)(2 * yp) * sW + 2 * xp;
+        const T *w = static_cast<const T *>(a.wt) + ((size_t)n * 25 + cell) * hi_plane + at, *h = static_cast<const T *>(a.hi) + ((size_t)n * a.C + c) * hi_plane + at;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s = fmaf(to_acc(w[(e >> 1) * sW + (e & 1)]), to_acc(h[(e >> 1) * sW + (e & 1)]), s);
+    }
+    return s;
+}
+// A lane's outputs again, columns x and x + 1 of every eighth channel, for a lane with a sum that is not finite.  The matrix product
+// also takes the other pixels of its fragments, with weights of zero, and 0 * inf would reach cells that no infinity reaches.
+template <typename T>
+__device__ __forceinline__ void store_cell_sums(const Args &a, int n, int c0, int count, int y, int x0) {
 #pragma unroll 1
     for (int i = 0; i < 2 * count; ++i) {
         const int c = c0 + 8 * (i >> 1), x = x0 + (i & 1);
         if (c >= a.C || x >= a.W) continue;
-        float s = 0.f;
-#pragma unroll 1
-        for (int cell = 0; cell < 25; ++cell) {       // window cell of the parent that reaches (y, x) through it
-            const int yp = y - a.top + 2 - cell / 5, xp = x + 2 - cell % 5;
-            if (yp < 0 || yp >= a.H || xp < 0 || xp >= a.W) continue;
-            const size_t at = (size_t)(2 * yp) * sW + 2 * xp;
-            const T *w = static_cast<const T *>(a.wt) + ((size_t)n * 25 + cell) * hi_plane + at, *h = static_cast<const T *>(a.hi) + ((size_t)n * a.C + c) * hi_plane + at;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s = fmaf(to_acc(w[(e >> 1) * sW + (e & 1)]), to_acc(h[(e >> 1) * sW + (e & 1)]), s);
-        }
-        static_cast<T *>(a.out)[(((size_t)n * a.C + c) * a.Hout + y) * a.W + x] = from_acc<T>(s);
+        static_cast<T *>(a.out)[(((size_t)n * a.C + c) * a.Hout + y) * a.W + x] = from_acc<T>(cell_sum<T>(a, n, c, y, x));
     }
 }
 
@@ -406,6 +413,7 @@ sapa_gath_mma_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
 }
 
 #include "sapa_gath_wide16.cuh"
+#include "sapa_gath_umma.cuh"
 
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for all element types: they share g_next_tile / g_ctas_done
@@ -422,6 +430,66 @@ static bool wide16_pays(int W) {
 // One form of the kernel: its tile, the channels of a stage and the launch.
 struct Form { int rows, cols, nch, threads, smem, ctas_per_sm; };
 
+// The tcgen05 kernel's split of a problem: rows of an item for the fewest steps (parent rows) of the busiest CTA, four of each item
+// for the parents around it and three to start and to end.
+struct UmmaPlan { gumma::UArgs u; long long items, steps; };
+template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int top, int bottom, int sms) {
+    UmmaPlan p{};
+    gumma::UArgs &u = p.u;
+    u.g.B = B; u.g.C = C; u.g.H = H; u.g.W = W; u.g.top = top; u.g.Hout = top + H + bottom;
+    u.strips = ceil_div(W, gumma::Geo<T>::CELLS);
+    u.cblocks = ceil_div(C, gumma::CH);
+    const int lines = std::min(C, gumma::CH);
+    u.x_bytes = ceil_div(lines * gumma::XROW, 128) * 128;
+    u.slot_bytes = ceil_div(u.x_bytes + gumma::L_BYTES, 128) * 128;
+    u.nx = std::min(gumma::MAX_NX, gumma::RING_BYTES / u.slot_bytes / 2 * 2);
+    const long long columns = (long long)B * u.strips * u.cblocks;
+    for (int segs = 1, most = (int)std::min<long long>(u.g.Hout, std::max<long long>(16, 4 * sms / columns)); segs <= most; ++segs) {
+        const int rows = ceil_div(u.g.Hout, segs), used = ceil_div(u.g.Hout, rows);
+        const long long n = columns * used, steps = (n + sms - 1) / sms * (rows + 4) + 3;
+        if (p.items != 0 && steps >= p.steps) continue;
+        p.items = n; p.steps = steps;
+        u.seg_rows = rows; u.segs = used;
+    }
+    return p;
+}
+
+// It serves rows of 16 bytes in and out, but for small problems and those that fill few of its lanes or columns.  A step takes about 0.95 us
+// in float32 and 0.8 in 16 bits, whatever the channels; the kernels on tiles 11.2 and 4.6 us for a million products of cells and
+// (channels + 24), and half a dozen to start.  us, tiles -> this one, float32 | bfloat16: 8 x 256 x 64x64 104 -> 45 | 43 -> 24; 8 x 64 x 64x64
+// 37 -> 27 | 18 -> 13; 1 x 32 x 512x512 170 -> 149 | 74 -> 53; 64 x 32 x 32x32 46 -> 43 | 23 -> 19; 4 x 128 x 32x32 12.7 -> 10.4 | 9.1 -> 7.6;
+// and where the line leaves them with the tiles: 8 x 32 x 32x32 9.9, 13.8 here | 8.0, 8.1; 1 x 64 x 16x16 8.7, 8.9 | 5.0, 6.4.
+template <typename T> static bool umma_pays(const UmmaPlan &p) {
+    const Args &g = p.u.g;
+    const double work = 1e-6 * g.B * g.Hout * g.W * (g.C + 24.0);
+    return g.W % (16 / (int)sizeof(T)) == 0 && (double)p.steps <= (sizeof(T) == 4 ? 4.0 + 12.0 * work : 5.0 + 5.7 * work);
+}
+
+template <typename T>
+static int launch_umma(const void *hi, const void *wt, void *out, UmmaPlan p, int sms, const char *name, cudaStream_t st) {
+    using G = gumma::Geo<T>;
+    Args &g = p.u.g;
+    const CUtensorMapDataType ty = G::F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                          : std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    constexpr int ES = (int)sizeof(T), BOX = gumma::XROW / ES;
+    CUtensorMap xmap{}, lmap{};
+    if (!make_nchw_map(&xmap, hi, 2 * g.W, 2 * g.H, g.C, g.B, BOX, std::min(g.C, gumma::CH), 1, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_nchw_map(&lmap, wt, 2 * g.W, 2 * g.H, 25, g.B, BOX, 25, 1, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE)) {
+        set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
+        return SAPA_ERR_UNSUPPORTED;
+    }
+    if (p.items > 0x7fffffffLL) {
+        set_error("too many tiles");
+        return SAPA_ERR_ARGUMENT;
+    }
+    using gumma::sapa_gath_umma_kernel;
+    int n = 0;
+    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_gath_umma_kernel<T>), G::SMEM, name, n)) return e;
+    g.hi = hi; g.wt = wt; g.out = out;
+    launch_next(sapa_gath_umma_kernel<T>, (unsigned)std::min<long long>(p.items, sms), gumma::NT, G::SMEM, st, xmap, lmap, p.u);
+    return check_launch(name);
+}
+
 template <typename T>
 static int launch(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype, cudaStream_t st) {
     using G = Geo<T>;
@@ -432,6 +500,12 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     if (F32 && ragged) {
         set_error("%s: float32 rows have to be of even length", name);
         return SAPA_ERR_UNSUPPORTED;
+    }
+    int sms = 0;
+    if (int e = device_sms(name, sms)) return e;
+    if (!ragged) {
+        const UmmaPlan p = umma_plan<T>(B, C, H, W, top, bottom, sms);
+        if (umma_pays<T>(p)) return launch_umma<T>(hi, wt, out, p, sms, name, st);
     }
     const Form f = ragged ? Form{ROWS, COLS, G::NCH, NT_RAGGED, G::SMEM_BYTES, 1}
                    : wide ? Form{ROWS, gw16::COLS, gw16::NCH, gw16::NT, gw16::SMEM_BYTES, 1}
@@ -463,7 +537,6 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     if constexpr (!F32)
         if (ragged) kernel = reinterpret_cast<const void *>(sapa_gath_mma_kernel<T, true>);
         else if (wide) kernel = reinterpret_cast<const void *>(sapa_gath_wide_16_kernel<T>);
-    int sms = 0;
     if (int e = prepare_launch(kernel, f.smem, name, sms)) return e;
     const long long resident = (long long)f.ctas_per_sm * sms;
     while (a.stages % 2 == 0 && 2 * nblocks <= resident) {      // every channel is independent: halve the items while all run at once

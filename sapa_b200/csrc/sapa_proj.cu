@@ -40,7 +40,7 @@
 // Tiles walk the images from the last to the first: the statistics pass has just read them in ascending order, so the
 // tail of x is what the L2 still holds.
 // Every mbarrier wait is bounded; a wait that gives up raises g_wait_timeout and the CTA drains and frees its TMEM.
-#include "tma_util.cuh"
+#include "umma_util.cuh"
 
 #include <algorithm>
 #include <cstdint>
@@ -51,6 +51,7 @@ namespace sapa {
 namespace proj {
 
 using namespace tmau;
+using namespace ummau;
 
 constexpr int TILE_PX = 128;
 constexpr int EPI_WARPS = 4, TMA_WARP = 4, MMA_WARP = 5, W_WARP = 6, SPLIT_WARP0 = 7, SPLIT_WARPS = 8;
@@ -98,46 +99,6 @@ __device__ __forceinline__ const Problem &find_tile(const Args &a, int tile, Til
     return p;
 }
 
-// ---------------------------------------------------------------------------------- tcgen05 wrappers
-__device__ __forceinline__ void tc_alloc(unsigned smem_slot, unsigned ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_slot), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void tc_dealloc(unsigned taddr, unsigned ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-// the mbarrier receives one arrival when every tcgen05.mma issued so far by this thread has completed
-__device__ __forceinline__ void tc_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-// One tcgen05.mma.  The 64-bit shared-memory descriptors are passed as their low words (start address and leading
-// offset; the part that changes from instruction to instruction) plus the high word all operands of this kernel share:
-// the issuing thread is a single thread whose own instruction latency bounds the MMA rate, so it must spend only a
-// handful of instructions per MMA.
-template <bool TF32>
-__device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc, unsigned accumulate) {
-    if (TF32)
-        asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
-                     " tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %4, p;\n}\n"
-                     ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
-    else
-        asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
-                     " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}\n"
-                     ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-// 16 consecutive accumulator columns of this thread's lane
-__device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-
 // Shared-memory matrix descriptor (64 bits).  Low word: start address (bits 0-13) and leading byte offset (bits 16-29),
 // both in 16-byte units.  High word: stride byte offset in 16-byte units (bits 0-13 = descriptor bits 32-45), descriptor
 // version 1 (bit 14 = bit 46), layout type 2 = 128-byte swizzle of 16-byte chunks (bits 29-31 = bits 61-63; 8-row atoms
@@ -145,15 +106,6 @@ __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sy
 // share one high word.  (Layout type 1, the 128-byte swizzle of 32-byte chunks with 4-row atoms, is what a tf32 operand
 // needs when its M / N dimension is the contiguous one; it is not used any more, see the header.)
 constexpr unsigned DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ unsigned desc_lo(unsigned addr, unsigned leading_bytes) {
-    return ((addr & 0x3ffffu) >> 4) | ((leading_bytes >> 4) << 16);
-}
-
-template <typename T> struct UmmaFormat;
-template <> struct UmmaFormat<float> { static constexpr unsigned code = 2; };            // tf32
-template <> struct UmmaFormat<__half> { static constexpr unsigned code = 0; };
-template <> struct UmmaFormat<__nv_bfloat16> { static constexpr unsigned code = 1; };
-
 __device__ __forceinline__ void store_out(float *p, float v) { __stcs(p, v); }
 __device__ __forceinline__ void store_out(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void store_out(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }

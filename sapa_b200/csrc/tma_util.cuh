@@ -182,14 +182,10 @@ inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Opts `kernel` in to `smem` bytes of dynamic shared memory on the current device (always the same number for one kernel)
-// and reports the device's SM count.  What was already done is remembered per thread: the runtime calls cost a microsecond
-// per launch otherwise.
-inline int prepare_launch(const void *kernel, int smem, const char *name, int &sms) {
-    constexpr int MAX_ENTRIES = 64, MAX_DEVICES = 64;
-    struct Entry { const void *kernel; int dev; };
-    static thread_local Entry done[MAX_ENTRIES];
-    static thread_local int used = 0, counts[MAX_DEVICES] = {};
+// The current device and its SM count (remembered per thread: the query costs a microsecond otherwise).
+inline int device_sms(const char *name, int &sms, int *device = nullptr) {
+    constexpr int MAX_DEVICES = 64;
+    static thread_local int counts[MAX_DEVICES] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES ||
         (counts[dev] == 0 && (cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || counts[dev] <= 0))) {
@@ -197,6 +193,18 @@ inline int prepare_launch(const void *kernel, int smem, const char *name, int &s
         return SAPA_ERR_LAUNCH;
     }
     sms = counts[dev];
+    if (device != nullptr) *device = dev;
+    return SAPA_OK;
+}
+// Opts `kernel` in to `smem` bytes of dynamic shared memory on the current device (always the same number for one kernel)
+// and reports the device's SM count.  What was already done is remembered per thread, as above.
+inline int prepare_launch(const void *kernel, int smem, const char *name, int &sms) {
+    constexpr int MAX_ENTRIES = 64;
+    struct Entry { const void *kernel; int dev; };
+    static thread_local Entry done[MAX_ENTRIES];
+    static thread_local int used = 0;
+    int dev = 0;
+    if (int e = device_sms(name, sms, &dev)) return e;
     for (int i = 0; i < used; ++i)
         if (done[i].kernel == kernel && done[i].dev == dev) return SAPA_OK;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
