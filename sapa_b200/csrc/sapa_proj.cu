@@ -30,11 +30,12 @@
 //     that needs the 128-byte swizzle of 32-byte chunks - CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, descriptor layout type 1,
 //     4-row atoms; with the ordinary swizzle the product is wrong.  That form is as accurate and no faster.)  W' arrives
 //     already split.
-//   * warp 5 (one lane): issues tcgen05.mma (M = 128, N = d, K = 32 bytes) into one of two TMEM accumulators, frees a
-//     stage with tcgen05.commit, signals the epilogue with another commit.  Its own instruction latency is on the
-//     critical path (one thread): ring positions and descriptors advance by additions only, and for float32 with
-//     d <= 128 the terms x_hi * W'_hi and x_hi * W'_lo are ONE instruction of N = 2d (the two W' blocks are adjacent
-//     rows of the operand; the epilogue adds the two halves of the accumulator): 8 instead of 12 MMAs per stage.
+//   * warp 5: issues tcgen05.mma (M = 128, N = d, K = 32 bytes) into one of two TMEM accumulators, frees a stage with
+//     tcgen05.commit, signals the epilogue with another commit.  The whole warp runs the loop, so that descriptors stay in uniform
+//     registers (tc_mma: an instruction from a branch of one lane took 57 clocks; q of 16 x 256 x 128x128, d = 128, bfloat16 84 -> 78 us,
+//     the three lists of the chain above 57 -> 52); for float32 with d <= 128 the terms x_hi * W'_hi and x_hi * W'_lo are ONE
+//     instruction of N = 2d (the two W' blocks are adjacent rows of the operand; the epilogue adds the two halves of the
+//     accumulator): 8 instead of 12 MMAs per stage.
 //   * warps 0-3: epilogue.  tcgen05.ld (lane = pixel, column = output channel), add bias', store: for a fixed output
 //     channel the 32 lanes of a warp write 32 consecutive pixels.  Runs under the MMAs of the next tile.
 // Tiles walk the images from the last to the first: the statistics pass has just read them in ascending order, so the
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
     const unsigned xfull0 = bars, xempty0 = bars + 8 * MAX_SLOTS, ready0 = bars + 16 * MAX_SLOTS, wfull0 = bars + 24 * MAX_SLOTS;
     const unsigned oempty0 = bars + 32 * MAX_SLOTS, tfull0 = bars + 40 * MAX_SLOTS, tempty0 = tfull0 + 16, tmem_slot = tempty0 + 16;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
     if (tid == 0) {
         for (unsigned i = 0; i < nx; ++i) {
             mbar_init(xfull0 + 8 * i, 1);
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
     tc_fence_after();
     unsigned tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot) : "memory");
+    tmem_base = warp_uniform(tmem_base);
 
     const unsigned acc_cols = (unsigned)a.acc_cols;       // accumulator columns per tile
     bool ok = true;
@@ -203,52 +205,52 @@ __global__ void __launch_bounds__(THREADS, 1) sapa_proj_umma_kernel(const __grid
                 }
             }
         }
-    } else if (warp == MMA_WARP) {
-        if (lane == 0) {
-            const unsigned idesc0 = (1u << 4) | (UmmaFormat<T>::code << 7) | (UmmaFormat<T>::code << 10) | (F32 ? 0u : (1u << 15)) | ((unsigned)(TILE_PX >> 4) << 24);
-            // low descriptor words per ring slot are base + slot * pitch; a K step adds a constant (all in 16-byte units)
-            const unsigned a_base = F32 ? desc_lo(opring, 16) : desc_lo(xring, A_BOX);
-            const unsigned a_pitch = (F32 ? op_bytes : (unsigned)Y_STAGE) >> 4, a_kstep = (F32 ? 32u : A_KSTEP) >> 4;
-            const unsigned b_base = desc_lo(opring + w_ofs, 16), b_pitch = op_bytes >> 4;
-            unsigned r = 0, rph = 0, o = 0, oph = 0, ti = 0;
-            for (int tile = blockIdx.x; tile < a.total_tiles && ok; tile += gridDim.x, ++ti) {
-                const unsigned buf = ti & 1u, tph = (ti >> 1) & 1u;
-                TileAt at;
-                const Problem &p = find_tile(a, tile, at);
-                const int kblocks = p.kblocks;
-                const unsigned w_bytes = (unsigned)p.d * 128u, wide = F32 ? (unsigned)p.wide : 0u;
-                const unsigned idesc = idesc0 | ((unsigned)(p.d >> 3) << 17), idesc_wide = idesc0 | ((unsigned)(2 * p.d >> 3) << 17);      // N = d, 2d
-                if (!mbar_wait_bounded(tempty0 + 8 * buf, tph ^ 1u)) { ok = false; break; }
+    } else if (warp == MMA_WARP) {     // the whole warp, one lane issues (tc_mma)
+        const unsigned idesc0 = (1u << 4) | (UmmaFormat<T>::code << 7) | (UmmaFormat<T>::code << 10) | (F32 ? 0u : (1u << 15)) | ((unsigned)(TILE_PX >> 4) << 24);
+        const unsigned leader = elect_leader();
+        // low descriptor words per ring slot are base + slot * pitch; a K step adds a constant (all in 16-byte units)
+        const unsigned a_base = warp_uniform(F32 ? desc_lo(opring, 16) : desc_lo(xring, A_BOX));
+        const unsigned a_pitch = (F32 ? op_bytes : (unsigned)Y_STAGE) >> 4, a_kstep = (F32 ? 32u : A_KSTEP) >> 4;
+        const unsigned b_base = warp_uniform(desc_lo(opring + w_ofs, 16)), b_pitch = op_bytes >> 4;
+        unsigned r = 0, rph = 0, o = 0, oph = 0, ti = 0;
+        for (int tile = blockIdx.x; tile < a.total_tiles && ok; tile += gridDim.x, ++ti) {
+            const unsigned buf = ti & 1u, tph = (ti >> 1) & 1u;
+            TileAt at;
+            const Problem &p = find_tile(a, tile, at);
+            const int kblocks = p.kblocks;
+            const unsigned w_bytes = (unsigned)p.d * 128u, wide = F32 ? (unsigned)p.wide : 0u;
+            const unsigned idesc = idesc0 | idesc_n((unsigned)p.d), idesc_wide = idesc0 | idesc_n(2u * (unsigned)p.d);      // N = d, 2d
+            ok = mbar_wait_warp(tempty0 + 8 * buf, tph ^ 1u);
+            if (!ok) break;
+            tc_fence_after();
+            const unsigned d_tmem = tmem_base + buf * acc_cols;
+            for (int kb = 0; kb < kblocks; ++kb) {
+                ok = mbar_wait_warp((F32 ? ready0 + 8 * o : xfull0 + 8 * r), F32 ? oph : rph) && mbar_wait_warp(wfull0 + 8 * o, oph);
+                if (!ok) break;
                 tc_fence_after();
-                const unsigned d_tmem = tmem_base + buf * acc_cols;
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!mbar_wait_bounded((F32 ? ready0 + 8 * o : xfull0 + 8 * r), F32 ? oph : rph) ||
-                        !mbar_wait_bounded(wfull0 + 8 * o, oph)) { ok = false; break; }
-                    tc_fence_after();
-                    const unsigned a0 = a_base + (F32 ? o : r) * a_pitch, b0 = b_base + o * b_pitch;
+                const unsigned a0 = a_base + (F32 ? o : r) * a_pitch, b0 = b_base + o * b_pitch;
 #pragma unroll
-                    for (int ks = 0; ks < KSTEPS; ++ks) {
-                        const unsigned first = (ks != 0 || kb != 0) ? 1u : 0u;
-                        if (F32 && wide) {
-                            // x_hi * [W'_hi ; W'_lo] as one instruction of N = 2d (columns [0, d) and [d, 2d) of the
-                            // accumulator, added by the epilogue), then x_lo * W'_hi into the first half
-                            tc_mma<F32>(d_tmem, a0 + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc_wide, first);
-                            tc_mma<F32>(d_tmem, a0 + (Y_STAGE >> 4) + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc, 1u);
-                        } else {
-                            tc_mma<F32>(d_tmem, a0 + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc, first);
-                            if (F32) {
-                                tc_mma<F32>(d_tmem, a0 + (Y_STAGE >> 4) + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc, 1u);      // lo * hi
-                                tc_mma<F32>(d_tmem, a0 + ks * a_kstep, b0 + (w_bytes >> 4) + ks * 2u, DESC_HI, idesc, 1u);      // hi * lo
-                            }
+                for (int ks = 0; ks < KSTEPS; ++ks) {
+                    const unsigned first = (ks != 0 || kb != 0) ? 1u : 0u;
+                    if (F32 && wide) {
+                        // x_hi * [W'_hi ; W'_lo] as one instruction of N = 2d (columns [0, d) and [d, 2d) of the
+                        // accumulator, added by the epilogue), then x_lo * W'_hi into the first half
+                        tc_mma<F32>(leader, d_tmem, a0 + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc_wide, first);
+                        tc_mma<F32>(leader, d_tmem, a0 + (Y_STAGE >> 4) + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc, 1u);
+                    } else {
+                        tc_mma<F32>(leader, d_tmem, a0 + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc, first);
+                        if (F32) {
+                            tc_mma<F32>(leader, d_tmem, a0 + (Y_STAGE >> 4) + ks * a_kstep, b0 + ks * 2u, DESC_HI, idesc, 1u);      // lo * hi
+                            tc_mma<F32>(leader, d_tmem, a0 + ks * a_kstep, b0 + (w_bytes >> 4) + ks * 2u, DESC_HI, idesc, 1u);      // hi * lo
                         }
                     }
-                    if (!F32) tc_commit(xempty0 + 8 * r);   // the activation slot is free once these MMAs have read it
-                    tc_commit(oempty0 + 8 * o);             // and so is the operand slot
-                    if (++r == nx) { r = 0; rph ^= 1u; }
-                    if (++o == no) { o = 0; oph ^= 1u; }
                 }
-                if (ok) tc_commit(tfull0 + 8 * buf);        // the accumulator is complete once all MMAs so far are done
+                if (!F32) tc_commit_by(leader, xempty0 + 8 * r);   // the activation slot is free once these MMAs have read it
+                tc_commit_by(leader, oempty0 + 8 * o);             // and so is the operand slot
+                if (++r == nx) { r = 0; rph ^= 1u; }
+                if (++o == no) { o = 0; oph ^= 1u; }
             }
+            if (ok) tc_commit_by(leader, tfull0 + 8 * buf);        // the accumulator is complete once all MMAs so far are done
         }
     } else if (warp >= SPLIT_WARP0) {
         if (F32) {

@@ -1,4 +1,4 @@
-// umma_util.cuh — PTX wrappers of the 5th-generation tensor core (tcgen05 and tensor memory) shared by sapa_proj.cu and sapa_gath_umma.cuh.
+// umma_util.cuh — PTX wrappers of the 5th-generation tensor core (tcgen05 and tensor memory) shared by the kernels that use it.
 #pragma once
 
 #include "tma_util.cuh"
@@ -19,41 +19,25 @@ __device__ __forceinline__ void tc_dealloc(unsigned taddr, unsigned ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-// the mbarrier receives one arrival when every tcgen05.mma issued so far by this thread has completed
-__device__ __forceinline__ void tc_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
 // Bounded wait of a whole warp, in front of instructions that all of its lanes execute together: every lane gets the same answer.
 __device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity)); }
-// One tcgen05.mma.  The 64-bit shared-memory descriptors are passed as their low words (start address and leading
-// offset; the part that changes from instruction to instruction) plus the high word all operands of this kernel share:
-// the issuing thread is a single thread whose own instruction latency bounds the MMA rate, so it must spend only a
-// handful of instructions per MMA.
+// One tcgen05.mma, for a loop that the WHOLE warp runs with values the compiler can see to be the same in all lanes (warp index and
+// addresses through warp_uniform): the operands stay in uniform registers, the lane with `leader` issues.  Measured (M = 128, tf32 and
+// bf16): N / 2 clocks an instruction and 16 at least; in a branch that one lane takes, where every operand is moved to a uniform register
+// first, 57 at least.  Shared-memory descriptors are passed as their low words (start address and leading offset; the part that changes from
+// instruction to instruction) plus the high word that a kernel's operands share.
 template <bool TF32>
-__device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc, unsigned accumulate) {
+__device__ __forceinline__ void tc_mma(unsigned leader, unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc, unsigned accumulate) {
     if (TF32)
-        asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
-                     " tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %4, p;\n}\n"
-                     ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+        asm volatile("{\n .reg .pred p, q;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
+                     " @q tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %4, p;\n}\n"
+                     ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
     else
-        asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
-                     " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}\n"
-                     ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+        asm volatile("{\n .reg .pred p, q;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
+                     " @q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}\n"
+                     ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
-// 16 consecutive accumulator columns of this thread's lane
-__device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-
-// The same with the A operand in tensor memory (lane = row of A, column = 32 bits of its K dimension: one tf32 or two 16-bit elements),
-// for a loop that the WHOLE warp runs with values the compiler can see to be the same in all lanes (warp index and addresses
-// through warp_uniform): the operands stay in uniform registers, the lane with `leader` issues.  Measured (M = 128, tf32 and bf16):
-// N / 2 clocks an instruction and 16 at least; in a branch that one lane takes, where every operand is moved to a uniform
-// register first, 57 at least.
+// The same with the A operand in tensor memory: lane = row of A, column = 32 bits of its K dimension (one tf32 or two 16-bit elements).
 template <bool TF32>
 __device__ __forceinline__ void tc_mma_ta(unsigned leader, unsigned d_tmem, unsigned a_tmem, unsigned b_lo, unsigned desc_hi, unsigned idesc, unsigned accumulate) {
     if (TF32)
@@ -65,6 +49,7 @@ __device__ __forceinline__ void tc_mma_ta(unsigned leader, unsigned d_tmem, unsi
                      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}\n"
                      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
+// the mbarrier receives one arrival when every tcgen05.mma that the leader has issued so far has completed
 __device__ __forceinline__ void tc_commit_by(unsigned leader, unsigned bar) {
     asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
                  ::"r"(bar), "r"(leader) : "memory");
@@ -76,6 +61,15 @@ __device__ __forceinline__ unsigned elect_leader() {
     return leader;
 }
 __device__ __forceinline__ unsigned warp_uniform(unsigned v) { return __shfl_sync(0xffffffffu, v, 0); }
+// 16 consecutive accumulator columns of this thread's lane
+__device__ __forceinline__ void tc_ld16(unsigned taddr, unsigned (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+
 // 8 and 16 consecutive columns of this thread's lane, from registers
 __device__ __forceinline__ void tc_st8(unsigned taddr, const unsigned *r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};\n"
