@@ -444,13 +444,7 @@ template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int 
     u.slot_bytes = ceil_div(u.x_bytes + gumma::L_BYTES, 128) * 128;
     u.nx = std::min(gumma::MAX_NX, gumma::RING_BYTES / u.slot_bytes / 2 * 2);
     const long long columns = (long long)B * u.strips * u.cblocks;
-    for (int segs = 1, most = (int)std::min<long long>(u.g.Hout, std::max<long long>(16, 4 * sms / columns)); segs <= most; ++segs) {
-        const int rows = ceil_div(u.g.Hout, segs), used = ceil_div(u.g.Hout, rows);
-        const long long n = columns * used, steps = (n + sms - 1) / sms * (rows + 4) + 3;
-        if (p.items != 0 && steps >= p.steps) continue;
-        p.items = n; p.steps = steps;
-        u.seg_rows = rows; u.segs = used;
-    }
+    ummau::split_rows(columns, u.g.Hout, sms, 4, p.items, p.steps, u.seg_rows, u.segs);
     return p;
 }
 

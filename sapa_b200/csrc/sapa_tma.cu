@@ -18,8 +18,9 @@
 //
 // float32 computes the logits on the tensor cores as well (3 x tf32, M = 16 pixels, N = 8 window cells, K = 8
 // channels): on the FP32 pipe that loop was bound by shared-memory wavefronts (12 per 10 packed FMAs).
-#include "tma_util.cuh"
+#include "umma_util.cuh"
 
+#include <algorithm>
 #include <atomic>
 
 
@@ -1076,6 +1077,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 }
 
 #include "sapa_wide16.cuh"
+#include "sapa_strip.cuh"
 
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for every kernel of this file: they all share g_next_tile / g_ctas_done, so two launches that
@@ -1105,6 +1107,58 @@ static int launch_persistent(Kernel kernel, const char *name, int threads, int s
     const unsigned grid = (unsigned)(nblocks < resident ? nblocks : resident);
     a.sched_slot = next_sched_slot(g_next_sched_slot, g_next_captured_slot, st);
     launch_next(kernel, grid, threads, smem, st, maps..., a);
+    return check_launch(name);
+}
+
+// The strip kernel's split of a problem: rows of an item for the fewest steps (low-res rows) of the busiest CTA, one more for an item's
+// halo rows and three to start.
+struct StripPlan { strip::SArgs a; long long items, steps; };
+template <typename T> static StripPlan strip_plan(int B, int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int sms) {
+    StripPlan p{};
+    strip::SArgs &a = p.a;
+    a.B = B; a.C = C; a.H = H; a.W = W; a.rows = rows; a.ytop0 = ytop0; a.y_begin = y_begin; a.y_end = y_end;
+    a.strips = ceil_div(W, strip::Geo<T>::CELLS);
+    a.cblocks = ceil_div(C, strip::CH);
+    const int band = y_end - y_begin;
+    const long long columns = (long long)B * a.strips * a.cblocks;
+    ummau::split_rows(columns, band, sms, 1, p.items, p.steps, a.seg_rows, a.segs);
+    return p;
+}
+// It serves rows of 16 bytes, but for small float32 problems and few channels in 16 bits.  A step takes about 0.75 us, whatever the channels, and
+// four to start; the kernels on tiles 3.7 (float32) and 1.5 us for a million products of cells and (channels + 99 or 136).  us, tiles -> this
+// one, float32 | bfloat16: 8 x 256 x 64x64 57 -> 38 | 32 -> 23; 32 x 64 x 64x64 79 -> 55 | 44 -> 32; 1 x 256 x 256x256 109 -> 77 | 59 -> 39;
+// 8 x 256 x 32x32 19 -> 14 | 17 -> 11; 16 x 64 x 32x32 14.8 -> 13.5 | 10.1 -> 9.6; 1 x 32 x 512x512 117 -> 93 | 64 -> 44; and where the line
+// leaves them with the tiles: 8 x 32 x 32x32 6.9, 9.7 here (bfloat16 8.9 -> 7.8); 4 x 128 x 32x32 8.7, 8.8 (9.7 -> 8.5); 32 x 16 x 64x64
+// bfloat16 35, 38 (float32 57 -> 52).
+template <typename T> static bool strip_pays(const StripPlan &p) {
+    const strip::SArgs &a = p.a;
+    const double cells = 1e-6 * a.B * (a.y_end - a.y_begin) * a.W;
+    if (sizeof(T) == 4) return (double)p.steps <= 0.7 + 5.1 * cells * (a.C + 99.0);
+    return a.C >= 32 && (double)p.steps <= 6.0 + 1.75 * cells * (a.C + 136.0);
+}
+
+template <typename T>
+static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, int sms, const char *name, cudaStream_t st) {
+    using G = strip::Geo<T>;
+    strip::SArgs &a = p.a;
+    const CUtensorMapDataType ty = G::F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                          : std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    constexpr int ES = (int)sizeof(T);
+    CUtensorMap vmap{}, wmap{}, omap{};
+    if (!make_nchw_map(&vmap, v, a.W, a.rows, a.C, a.B, strip::VROW / ES, std::min(a.C, strip::CH), 1, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_nchw_map(&wmap, wt, 2 * a.W, 2 * a.H, 25, a.B, G::PX, 25, 2, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_nchw_map(&omap, out, 2 * a.W, 2 * a.H, a.C, a.B, G::PX, 32, 1, ty, ES, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
+        return SAPA_ERR_UNSUPPORTED;
+    }
+    if (p.items > 0x7fffffffLL) {
+        set_error("too many tiles");
+        return SAPA_ERR_ARGUMENT;
+    }
+    int n = 0;
+    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_strip_kernel<T>), G::SMEM, name, n)) return e;
+    a.v = v; a.wt = wt; a.out = out;
+    launch_next(sapa_strip_kernel<T>, (unsigned)std::min<long long>(p.items, sms), strip::NT, G::SMEM, st, vmap, wmap, omap, a);
     return check_launch(name);
 }
 
@@ -1162,6 +1216,18 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         return SAPA_ERR_UNSUPPORTED;
     }
     const bool wide = !ragged && dtype != SAPA_F32 && wide16_pays(W, ceil_div(y_end - y_begin, ROWS), B);
+    if (mode == MODE_AGG && !ragged) {
+        const char *name = dtype == SAPA_F32 ? "sapa_tma_fused_f32_kernel<agg>" : wide ? "sapa_wide_16_kernel<agg>" : "sapa_tma_fused_16_kernel<agg>";
+        int sms = 0;
+        if (int e = device_sms(name, sms)) return e;
+        auto go = [&](auto one) -> int {
+            using T = decltype(one);
+            const StripPlan p = strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
+            return strip_pays<T>(p) ? launch_strip<T>(v, attn, out, p, sms, name, st) : -1000;
+        };
+        const int e = dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
+        if (e != -1000) return e;
+    }
     bool ok = true;
     if (ragged) {
     } else if (dtype == SAPA_F32) {

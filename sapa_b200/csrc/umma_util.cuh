@@ -96,5 +96,21 @@ template <> struct UmmaFormat<__nv_bfloat16> { static constexpr unsigned code = 
 template <typename T> constexpr unsigned IDESC_M128 = (1u << 4) | (UmmaFormat<T>::code << 7) | (UmmaFormat<T>::code << 10) | ((128u >> 4) << 24);
 __device__ __forceinline__ constexpr unsigned idesc_n(unsigned n) { return (n >> 3) << 17; }
 
+// ---------------------------------------------------------------------------------- host side
+// Kernels that walk `columns` (strips of all images and blocks of channels) of `rows` rows each: cuts every column into `segs` items of
+// `seg_rows` rows so that the busiest of the SMs takes the fewest steps, an item costing `extra` steps beyond its rows and the launch three.
+// The candidates are the most segments that one, two, ... rounds of items hold.
+inline void split_rows(long long columns, int rows, int sms, int extra, long long &items, long long &steps, int &seg_rows, int &segs) {
+    const int first = (int)((columns + sms - 1) / sms);
+    items = 0;
+    for (int round = first; round < first + 5; ++round) {
+        const long long most = (long long)round * sms / columns;
+        const int want = most < rows ? (int)most : rows, r = (rows + want - 1) / want, used = (rows + r - 1) / r;
+        const long long n = columns * used, total = (n + sms - 1) / sms * (r + extra) + 3;
+        if (items != 0 && total >= steps) continue;
+        items = n; steps = total; seg_rows = r; segs = used;
+    }
+}
+
 }  // namespace ummau
 }  // namespace sapa
