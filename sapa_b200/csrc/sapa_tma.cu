@@ -1078,6 +1078,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 
 #include "sapa_wide16.cuh"
 #include "sapa_strip.cuh"
+#include "sapa_strip_fwd.cuh"
 
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for every kernel of this file: they all share g_next_tile / g_ctas_done, so two launches that
@@ -1162,6 +1163,46 @@ static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, i
     return check_launch(name);
 }
 
+// The forward on strips takes up to 64 query channels, rows of 16 columns and more (a strip of 32 is less than half full below that) and at
+// least 24 value channels.  A channel of a large image is a page of memory of its own, and this kernel touches all channels of a row where
+// the tiles touch 32 of eight rows: images of more than 100 M values stay with the tiles.  The line depends on nothing but the shape of one
+// image, so that an image's result does not depend on the batch it is in.  bfloat16, us, tiles -> strips: 64 x 256 x 128x128 824 -> 687,
+// 8 x 256 x 64x64 37.3 -> 29.5 (with the attention map 41.8 -> 31.6), 16 x 128 x 64x64 47.7 -> 30.5, 8 x 256 x 32x32 (32 query channels)
+// 18.0 -> 11.2, 2 x 512 x 8x64 11.4 -> 7.7, 1 x 32 x 16x16 6.1 -> 6.3, 4 x 256 x 512x512 826 -> 755, 1 x 128 x 768x768 324 -> 273; 8 columns:
+// 64 x 256 x 16x8 19.1, 24.8 here; large images: 1 x 512 x 512x512 350, 375 here, 1 x 256 x 1024x1024 849, 1050 here.
+static bool strip_fwd_pays(int C, int d, int H, int W) { return d <= sfwd::MAX_D && W >= 16 && C >= 24 && (double)C * H * W <= 1e8; }
+
+template <typename T>
+static int launch_strip_fwd(const void *q, const void *k, const void *v, void *out, void *attn, int d, StripPlan p, int sms, const char *name, cudaStream_t st) {
+    strip::SArgs &a = p.a;
+    const CUtensorMapDataType ty = std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const int dpad = ceil_div(d, 16) * 16;
+    CUtensorMap qmap{}, kmap{}, vmap{}, omap{};
+    if (!make_nchw_map(&qmap, q, 2 * a.W, 2 * a.H, d, a.B, 64, dpad, 2, ty, 2, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_nchw_map(&kmap, k, a.W, a.rows, d, a.B, 64, dpad, 1, ty, 2, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_nchw_map(&vmap, v, a.W, a.rows, a.C, a.B, strip::VROW / 2, std::min(a.C, strip::CH), 1, ty, 2, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_nchw_map(&omap, out, 2 * a.W, 2 * a.H, a.C, a.B, 64, 32, 1, ty, 2, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
+        return SAPA_ERR_UNSUPPORTED;
+    }
+    if (p.items > 0x7fffffffLL) {
+        set_error("too many tiles");
+        return SAPA_ERR_ARGUMENT;
+    }
+    sfwd::FArgs f{};
+    a.v = v; a.out = out;
+    f.s = a; f.attn = attn;
+    auto go = [&](auto ksteps) -> int {
+        constexpr int KSTEPS = decltype(ksteps)::value, SMEM = sfwd::Lay<T, KSTEPS>::SMEM;
+        int n = 0;
+        if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_strip_fwd_kernel<T, KSTEPS>), SMEM, name, n)) return e;
+        launch_next(sapa_strip_fwd_kernel<T, KSTEPS>, (unsigned)std::min<long long>(p.items, sms), sfwd::NT, SMEM, st, qmap, kmap, vmap, omap, f);
+        return check_launch(name);
+    };
+    return dpad == 16 ? go(std::integral_constant<int, 1>{}) : dpad == 32 ? go(std::integral_constant<int, 2>{})
+           : dpad == 48 ? go(std::integral_constant<int, 3>{}) : go(std::integral_constant<int, 4>{});
+}
+
 }  // namespace tma
 
 // K = 5, s = 2 and every row of every tensor on a 16-byte boundary; other widths take the ragged form of the kernels
@@ -1227,6 +1268,17 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         };
         const int e = dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
         if (e != -1000) return e;
+    }
+    if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, H, W)) {
+        const char *name = wide ? "sapa_wide_16_kernel<fwd>" : "sapa_tma_fused_16_kernel<fwd>";
+        int sms = 0;
+        if (int e = device_sms(name, sms)) return e;
+        auto go = [&](auto one) -> int {
+            using T = decltype(one);
+            const StripPlan p = strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
+            return launch_strip_fwd<T>(q, k, v, out, attn, d, p, sms, name, st);
+        };
+        return dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
     }
     bool ok = true;
     if (ragged) {
