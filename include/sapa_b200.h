@@ -107,13 +107,19 @@ int sapa_av_backward(const void *grad_out, const void *attn, const void *value,
 
 /* ------------------------------------------------------------------ SAPA-B, fused --------------------- */
 
-/* out = atn(softmax_k(sim(query, key)), value) in one kernel: what SAPA.attention computes with three
+/* out = atn(softmax_k(sim(query, key)), value): what SAPA.attention computes with three
  * launches and two HBM round trips of the attention map (sapa_base.py:38-40).  `attn` may be NULL
  * (inference); when given, the [B,K*K,sH,sW] softmax output is also stored for the backward pass.
+ * One kernel, but for larger float32 problems with `attn` given: two, the softmax output and the aggregation.
  * Returns SAPA_ERR_UNSUPPORTED for (K, s) without a fused kernel (supported: K in {3,5}, s = 2, and
  * dtype != SAPA_F64). */
 int sapa_fused_forward(const void *query, const void *key, const void *value, void *out, void *attn,
                        int B, int d, int C, int H, int W, int K, int s, int dtype, void *stream);
+
+/* 1 when sapa_fused_forward is faster for these sizes with `attn` given than without, because it then runs as two
+ * kernels: a caller without use for the map passes a scratch buffer of its size (B*K*K*sH*sW elements).  0 otherwise. */
+int sapa_fused_forward_wants_map(int B, int d, int C, int H, int W, int K, int s, int dtype);
+
 
 /* Row-slab form of sapa_fused_forward for one spatial shard of a larger image: key and value hold
  * `halo_top` extra low-res rows above and `halo_bottom` below the H rows whose outputs are produced

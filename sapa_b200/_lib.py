@@ -26,6 +26,7 @@ _lib = None
 _vp, _i, _sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
 # name -> argument types; every function returns int except the two noted below
 _SIGNATURES = {
+    "sapa_fused_forward_wants_map": [_i] * 8,
     "sapa_qk_forward": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "sapa_qk_backward": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "sapa_av_forward": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],

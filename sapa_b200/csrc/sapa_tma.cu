@@ -1079,6 +1079,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 #include "sapa_wide16.cuh"
 #include "sapa_strip.cuh"
 #include "sapa_strip_fwd.cuh"
+#include "sapa_strip_sim.cuh"
 
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for every kernel of this file: they all share g_next_tile / g_ctas_done, so two launches that
@@ -1203,6 +1204,32 @@ static int launch_strip_fwd(const void *q, const void *k, const void *v, void *o
            : dpad == 48 ? go(std::integral_constant<int, 3>{}) : go(std::integral_constant<int, 4>{});
 }
 
+// float32 logits of hi (d channels) and lo, their softmax, or its backward with the saved map `attn`
+template <int WHAT>
+static int launch_strip_sim(const void *hi, const void *lo, const void *attn, void *out, int B, int d, int H, int W, int rows, int ytop0, int y_begin, int y_end,
+                            const char *name, cudaStream_t st) {
+    const CUtensorMapDataType ty = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+    CUtensorMap xmap{}, lmap{};
+    if (!make_nchw_map(&xmap, hi, 2 * W, 2 * H, d, B, 2 * ssim::CELLS, ssim::KCH, 4, ty, 4, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_nchw_map(&lmap, lo, W, rows, d, B, ssim::LROW / 4, ssim::KCH, ssim::ROWS6, ty, 4, CU_TENSOR_MAP_SWIZZLE_NONE)) {
+        set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
+        return SAPA_ERR_UNSUPPORTED;
+    }
+    ssim::Args a{};
+    a.attn = static_cast<const float *>(attn); a.out = static_cast<float *>(out);
+    a.B = B; a.d = d; a.H = H; a.W = W; a.ytop0 = ytop0; a.y_begin = y_begin; a.y_end = y_end;
+    a.strips = ceil_div(W, ssim::CELLS); a.pairs = ceil_div(y_end - y_begin, 2); a.stages = ceil_div(d, ssim::KCH);
+    const long long units = (long long)B * a.strips * a.pairs;
+    if (units > 0x7fffffffLL) {
+        set_error("too many tiles");
+        return SAPA_ERR_ARGUMENT;
+    }
+    int sms = 0;
+    if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_strip_sim_kernel<WHAT>), ssim::SMEM, name, sms)) return e;
+    launch_next(sapa_strip_sim_kernel<WHAT>, (unsigned)std::min<long long>(units, sms), ssim::NT, ssim::SMEM, st, xmap, lmap, a);
+    return SAPA_OK;
+}
+
 }  // namespace tma
 
 // K = 5, s = 2 and every row of every tensor on a 16-byte boundary; other widths take the ragged form of the kernels
@@ -1225,6 +1252,21 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
 static bool wide16_pays(int W, int tiles_y, int B) {
     const int tiles_x = ceil_div(W, tma::w16::COLS);
     return 4 * W >= 3 * tiles_x * tma::w16::COLS && (long long)B * tiles_x * tiles_y >= 100;
+}
+
+// float32 on strips of 16 columns, at least three quarters of them inside the image.  The similarity by itself from 12 000 low-res pixels on
+// (us, tiles -> strips: 8 images, 64 channels, 64x64 21.6 -> 16.6; 16 x 64 x 64x64 40 -> 28; 4 x 16 x 64x64 7.7 -> 7.0; 2 x 32 x 48x80
+// 6.3, 6.6 here).
+namespace tma { static bool strips_filled(int W) { return 4 * W >= 3 * ceil_div(W, ssim::CELLS) * ssim::CELLS; } }
+static bool strip_sim_pays(int B, int H, int W) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && (long long)B * H * W >= 12000;
+}
+// The forward and stage 1 of the backward as two launches, logits and what follows them per pixel, then the aggregation, from a million values
+// on (forward with its map | stage 1: 8 x 256 x 64x64 78.6 -> 53.2 | 91.4 -> 65.8; 16 x 128 x 64x64 103 -> 66 | 120 -> 80; 8 x 64 x 64x64
+// 41 -> 37 | 47 -> 38; 8 x 256 x 32x32 23.1 -> 20.9; 8 x 512 x 16x16 15.6 -> 15.3; 4 x 128 x 32x32 11.6, 14.2 here; 64 x 32 x 32x32 46.0, 47.5
+// here).
+bool fused_f32_on_strips(int B, int C, int H, int W) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)B * H * W * C >= 1e6;
 }
 
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
@@ -1268,6 +1310,20 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         };
         const int e = dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
         if (e != -1000) return e;
+    }
+    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(B, H, W) : mode == MODE_FWD ? attn != nullptr && fused_f32_on_strips(B, C, H, W)
+                                                                          : mode == MODE_BWD && fused_f32_on_strips(B, d, H, W))) {
+        static const char *const names[3] = {"sapa_tma_fused_f32_kernel<fwd>", "sapa_tma_fused_f32_kernel<bwd>", "sapa_tma_fused_f32_kernel<sim>"};
+        const char *name = names[mode];
+        void *slots = mode == MODE_BWD ? ws : attn;
+        int e = mode == MODE_SIM ? launch_strip_sim<ssim::LOGITS>(q, k, nullptr, slots, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
+                : mode == MODE_FWD ? launch_strip_sim<ssim::SOFTMAX>(q, k, nullptr, slots, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
+                                   : launch_strip_sim<ssim::SOFTMAX_BWD>(q, k, attn, slots, B, d, H, W, rows, ytop0, y_begin, y_end, name, st);
+        if (e != SAPA_OK) return e;
+        if (mode == MODE_SIM) return check_launch(name);
+        int sms = 0;
+        if ((e = device_sms(name, sms)) != SAPA_OK) return e;
+        return launch_strip<float>(v, slots, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
     }
     if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, H, W)) {
         const char *name = wide ? "sapa_wide_16_kernel<fwd>" : "sapa_tma_fused_16_kernel<fwd>";

@@ -185,10 +185,16 @@ class RowSlab:
         self._side = torch.cuda.Stream(device=device) if torch.device(device).type == "cuda" else None
         self._halo_done = torch.cuda.Event() if self._side is not None else None
         self.attn = None            # [B, K*K, s*Hl, s*W] of the last forward(keep_attn=True)
+        self._scratch = None        # of its size, where the kernels that go through the map are the faster ones
 
     def _launch(self, query, out, row_begin, row_end):
         from . import _lib
-        return _lib.call("sapa_fused_forward_slab_rows", out.device, query, self.key_padded, self.value_padded, out, self.attn,
+        attn = self.attn
+        if attn is None and _lib.lib().sapa_fused_forward_wants_map(self.B, self.d, self.C, self.Hl, self.W, self.K, self.s, _lib.dtype_code(out)):
+            if self._scratch is None:
+                self._scratch = torch.empty((self.B, self.K * self.K, self.s * self.Hl, self.s * self.W), dtype=out.dtype, device=out.device)
+            attn = self._scratch
+        return _lib.call("sapa_fused_forward_slab_rows", out.device, query, self.key_padded, self.value_padded, out, attn,
                          self.B, self.d, self.C, self.Hl, self.W, self.halo, self.halo, row_begin, row_end, self.K, self.s,
                          _lib.dtype_code(out), allow_unsupported=True)
 

@@ -1,0 +1,70 @@
+"""float32 on strips of columns: logits on the 5th-generation tensor cores with the softmax, its backward or nothing behind them, then the
+aggregation - the similarity, the fused forward with and without its map, and its backward, against float64."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# images, value channels, query channels, rows, columns: stages of channels that end early, odd rows, partial strips, many units a CTA.  A
+# million values and more, 12 000 pixels and more
+SHAPES = [(2, 300, 64, 47, 44), (9, 48, 5, 51, 60), (3, 130, 33, 71, 52), (40, 80, 16, 33, 12), (1, 520, 100, 130, 16)]
+
+
+def _rand(seed, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
+
+
+def _windows(t):
+    H, W = t.shape[2:]
+    padded = F.pad(t, (2, 2, 2, 2))
+    return [padded[:, :, i // 5:i // 5 + H, i % 5:i % 5 + W].repeat_interleave(2, 2).repeat_interleave(2, 3) for i in range(25)]
+
+
+# 2-norms: three-term tf32 products and the roundings toward zero of their sums; measured here (before, on tiles): logits of 64 channels 6.6e-7
+# (9.2e-7), output 1.1e-6 (1.5e-6), gradients up to 3.0e-6 (3.5e-6); a channel adds up to 1e-8
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "B%d_C%d_d%d_%dx%d" % s)
+def test_strips_vs_float64(shape):
+    import sapa_b200 as sp
+    from sapa_b200 import _lib
+    from sapa_b200.functions import fused_forward_raw
+    B, C, d, H, W = shape
+    assert _lib.lib().sapa_fused_forward_wants_map(B, d, C, H, W, 5, 2, 0) == 1
+    t = [_rand(1, B, d, 2 * H, 2 * W, scale=0.5).requires_grad_(), _rand(2, B, d, H, W, scale=0.5).requires_grad_(), _rand(3, B, C, H, W).requires_grad_()]
+    go = _rand(4, B, C, 2 * H, 2 * W)
+    r = [x.detach().double().requires_grad_() for x in t]
+    logits = torch.stack([(r[0] * w).sum(1) for w in _windows(r[1])], 1)
+    attn = torch.softmax(logits, 1)
+    want = sum(attn[:, i:i + 1] * w for i, w in enumerate(_windows(r[2])))
+    grads = torch.autograd.grad(want, r, go.double())
+
+    def off(a, b):
+        return float((a.detach().double() - b.detach()).norm() / b.detach().norm())
+    for _ in range(2):
+        out = sp.sapa_fused(*t, 5, 2)
+        got = torch.autograd.grad(out, t, go)
+        assert off(sp.qk(t[0].detach(), t[1].detach(), 5, 2), logits) < 5e-7 + 1e-8 * d
+        assert off(out, want) < 1.3e-6 + 1e-8 * d
+        for a, b in zip(got, grads):
+            assert off(a, b) < 2e-6 + 1e-8 * max(C, d)
+    alone, none = fused_forward_raw(*(x.detach() for x in t), 5, 2, False)
+    assert none is None and torch.equal(alone, out.detach())         # with the map as scratch
+    assert _lib.wait_timeout_flags(DEV) == 0
+
+
+def test_bands_of_a_slab_equal_the_whole_image():
+    from sapa_b200 import sharding
+    from sapa_b200.functions import fused_forward_raw
+    B, d, C, H, W, r = 2, 40, 300, 60, 48, 2
+    q, k, v = _rand(1, B, d, 2 * H, 2 * W, scale=0.5), _rand(2, B, d, H, W, scale=0.5), _rand(3, B, C, H, W)
+    whole = fused_forward_raw(q, k, v, 5, 2, False)[0]
+    lo, rows = 11, 40
+    slab = sharding.RowSlab(B, d, C, rows, W, torch.float32, torch.device(DEV), 5, 2)
+    slab.key_padded.copy_(k[:, :, lo - r:lo + rows + r])
+    slab.value_padded.copy_(v[:, :, lo - r:lo + rows + r])
+    hi = slice(2 * lo, 2 * (lo + rows))
+    ql, out = q[:, :, hi].contiguous(), torch.empty(B, C, 2 * rows, 2 * W, device=DEV)
+    for begin, end in ((0, 4), (4, rows - 3), (rows - 3, rows)):
+        slab._launch(ql, out, begin, end)
+    assert torch.equal(out, whole[:, :, hi])
