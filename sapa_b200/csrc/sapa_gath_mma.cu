@@ -452,11 +452,12 @@ template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int 
 // in float32 and 0.8 in 16 bits, whatever the channels; the kernels on tiles 11.2 and 4.6 us for a million products of cells and
 // (channels + 24), and half a dozen to start.  us, tiles -> this one, float32 | bfloat16: 8 x 256 x 64x64 104 -> 45 | 43 -> 24; 8 x 64 x 64x64
 // 37 -> 27 | 18 -> 13; 1 x 32 x 512x512 170 -> 149 | 74 -> 53; 64 x 32 x 32x32 46 -> 43 | 23 -> 19; 4 x 128 x 32x32 12.7 -> 10.4 | 9.1 -> 7.6;
-// and where the line leaves them with the tiles: 8 x 32 x 32x32 9.9, 13.8 here | 8.0, 8.1; 1 x 64 x 16x16 8.7, 8.9 | 5.0, 6.4.
+// and where the line leaves them with the tiles: 8 x 32 x 32x32 9.9, 13.8 here | 8.0, 8.1; 1 x 64 x 16x16 8.7, 8.9 | 5.0, 6.4; 4 x 32 x 64x64
+// 15.7, 16.4 here | 9.4, 9.7.
 template <typename T> static bool umma_pays(const UmmaPlan &p) {
     const Args &g = p.u.g;
     const double work = 1e-6 * g.B * g.Hout * g.W * (g.C + 24.0);
-    return g.W % (16 / (int)sizeof(T)) == 0 && (double)p.steps <= (sizeof(T) == 4 ? 4.0 + 12.0 * work : 5.0 + 5.7 * work);
+    return g.W % (16 / (int)sizeof(T)) == 0 && (double)p.steps <= (sizeof(T) == 4 ? 2.0 + 12.0 * work : 5.0 + 5.7 * work);
 }
 
 template <typename T>

@@ -68,7 +68,6 @@ struct Args {
     int csplit, vstages;   // work items per tile, each with `vstages` value stages (its own share of the channels): a problem
                            // with few tiles is spread over more CTAs, which all compute the tile's weights
     int sched_slot;        // index into g_next_tile / g_ctas_done
-    int slots_f32;         // 16-bit kernel, MODE_SIM: the logits are written as float32
 };
 
 // byte offset of element `col` of a 64-byte row under the 64-byte swizzle: the 16-byte chunk index is XORed with
@@ -957,21 +956,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
                         pb[p][dy][1] = pack_pair(T(), s[p][dy][2], s[p][dy][3]);
                     }
             }
-            if (!RAGGED && it == nk - 1 && MODE == MODE_SIM && a.slots_f32 != 0) {
-                if (row_ok) {         // raw logits as float32 pairs (the dense similarity of the 16-bit SAPA-D path)
-                    float2 *af = reinterpret_cast<float2 *>(static_cast<float *>(a.attn) + (size_t)n * 25 * hi_plane +
-                                                            (size_t)(2 * y + r) * sW + 2 * x0 + 2 * t);
-#pragma unroll
-                    for (int p = 0; p < 2; ++p)
-                        if (p == 0 ? col_ok0 : col_ok1) {
-#pragma unroll
-                            for (int dy = 0; dy < 5; ++dy) {
-                                if (ok_lo[p]) af[(size_t)(dy * 5 + dx_lo[p]) * plane_w + 4 * p] = make_float2(s[p][dy][0], s[p][dy][1]);
-                                if (ok_hi[p]) af[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w + 4 * p] = make_float2(s[p][dy][2], s[p][dy][3]);
-                            }
-                        }
-                }
-            } else if (it == nk - 1 && (MODE == MODE_FWD || MODE == MODE_SIM)) {
+            if (it == nk - 1 && (MODE == MODE_FWD || MODE == MODE_SIM)) {
                 if (a.attn != nullptr && c0 == 0 && row_ok) {
                     // the two pixels of a pair are neighbours in memory: one 32-bit store per (window slot, pair)
                     unsigned *an = reinterpret_cast<unsigned *>(static_cast<T *>(a.attn) + (size_t)n * 25 * hi_plane +
@@ -1080,6 +1065,7 @@ sapa_tma_fused_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 #include "sapa_strip.cuh"
 #include "sapa_strip_fwd.cuh"
 #include "sapa_strip_sim.cuh"
+#include "sapa_strip_sim16.cuh"
 
 // ---------------------------------------------------------------------------------- host side
 // one host-side counter for every kernel of this file: they all share g_next_tile / g_ctas_done, so two launches that
@@ -1230,6 +1216,37 @@ static int launch_strip_sim(const void *hi, const void *lo, const void *attn, vo
     return SAPA_OK;
 }
 
+// the same in 16 bits: logits (as float32 where asked for) or the softmax backward with the saved map `attn`
+template <typename T, int WHAT>
+static int launch_strip_sim_16(const void *hi, const void *lo, const void *attn, void *out, int B, int d, int H, int W, int rows, int ytop0, int y_begin, int y_end,
+                               const char *name, cudaStream_t st) {
+    const CUtensorMapDataType ty = std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const int kch = d <= 16 ? 16 : 32;
+    CUtensorMap xmap{}, lmap{};
+    if (!make_nchw_map(&xmap, hi, 2 * W, 2 * H, d, B, 2 * s16::CELLS, kch, 4, ty, 2, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_nchw_map(&lmap, lo, W, rows, d, B, 64, kch, s16::ROWS6, ty, 2, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
+        return SAPA_ERR_UNSUPPORTED;
+    }
+    s16::Args a{};
+    a.attn = attn; a.out = out;
+    a.B = B; a.d = d; a.H = H; a.W = W; a.ytop0 = ytop0; a.y_begin = y_begin; a.y_end = y_end;
+    a.strips = ceil_div(W, s16::CELLS); a.pairs = ceil_div(y_end - y_begin, 2); a.stages = ceil_div(d, kch);
+    const long long units = (long long)B * a.strips * a.pairs;
+    if (units > 0x7fffffffLL) {
+        set_error("too many tiles");
+        return SAPA_ERR_ARGUMENT;
+    }
+    auto go = [&](auto channels) -> int {
+        constexpr int KCH = decltype(channels)::value, SMEM = s16::Lay<KCH>::SMEM;
+        int sms = 0;
+        if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_strip_sim_16_kernel<T, WHAT, KCH>), SMEM, name, sms)) return e;
+        launch_next(sapa_strip_sim_16_kernel<T, WHAT, KCH>, (unsigned)std::min<long long>(units, sms), s16::NT, SMEM, st, xmap, lmap, a);
+        return SAPA_OK;
+    };
+    return kch == 16 ? go(std::integral_constant<int, 16>{}) : go(std::integral_constant<int, 32>{});
+}
+
 }  // namespace tma
 
 // K = 5, s = 2 and every row of every tensor on a 16-byte boundary; other widths take the ragged form of the kernels
@@ -1268,6 +1285,12 @@ static bool strip_sim_pays(int B, int H, int W) {
 bool fused_f32_on_strips(int B, int C, int H, int W) {
     return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)B * H * W * C >= 1e6;
 }
+
+// 16 bits: the similarity always runs on strips (us, tiles -> strips, bfloat16: 8 images, 64 channels, 64x64 15.0 -> 11.0; 1 x 32 x 16x16 6.2 ->
+// 4.3; 64 x 32 x 8x8 7.0 -> 5.4); stage 1 of the backward as two launches, logits and softmax backward, then the aggregation, with 128 value
+// channels or a million values and rows of 16 columns and more.  The whole backward, us: 8 x 256 x 64x64 85.5 -> 75.8, 16 x 128 x 64x64
+// 116 -> 91, 64 x 32 x 32x32 81 -> 69, 2 x 256 x 24x40 28.7 -> 25.9; 4 x 64 x 48x48 28.6, 30.4 on strips; 64 x 64 x 8x8 22.6, 24.5.
+static bool strip_bwd_16_pays(int B, int C, int H, int W) { return W >= 16 && (C >= 128 || (double)B * H * W * C >= 1e6); }
 
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
 // mode 0 (forward): out = atn(softmax(sim(q, k)), v), attn = optional output.
@@ -1325,6 +1348,20 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         if ((e = device_sms(name, sms)) != SAPA_OK) return e;
         return launch_strip<float>(v, slots, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
     }
+    if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(B, d, H, W)))) {
+        const char *name = mode == MODE_SIM ? (wide ? "sapa_wide_16_kernel<sim>" : "sapa_tma_fused_16_kernel<sim>") : wide ? "sapa_wide_16_kernel<bwd>" : "sapa_tma_fused_16_kernel<bwd>";
+        int sms = 0;
+        if (int e = device_sms(name, sms)) return e;
+        auto go = [&](auto one) -> int {
+            using T = decltype(one);
+            int e = mode == MODE_BWD ? launch_strip_sim_16<T, s16::SOFTMAX_BWD>(q, k, attn, ws, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
+                    : slots_f32      ? launch_strip_sim_16<T, s16::LOGITS_F32>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
+                                     : launch_strip_sim_16<T, s16::LOGITS>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, name, st);
+            if (e != SAPA_OK) return e;
+            return mode == MODE_SIM ? check_launch(name) : launch_strip<T>(v, ws, out, strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
+        };
+        return dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
+    }
     if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, H, W)) {
         const char *name = wide ? "sapa_wide_16_kernel<fwd>" : "sapa_tma_fused_16_kernel<fwd>";
         int sms = 0;
@@ -1368,7 +1405,6 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     a.q = q; a.k = k; a.v = v;
     a.out = out; a.attn = attn; a.ws = ws;
     a.B = B; a.d = d; a.C = C; a.H = H; a.W = W; a.rows = rows; a.ytop0 = ytop0;
-    a.slots_f32 = slots_f32 ? 1 : 0;
     static_assert(F_VCH == h16::VCH, "both kernels take the same number of value channels per stage");
     a.csplit = 1; a.vstages = ceil_div(C, F_VCH);
     static_assert(h16::COLS == COLS, "both kernels use the same tile");
@@ -1391,15 +1427,19 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         return ragged ? launch_persistent(sapa_tma_fused_16_kernel<T, M, true>, names_ragged[M], h16::NT_RAGGED, h16::SMEM_BYTES, 1, M != MODE_BWD, a, st, qmap, kmap, vmap) \
                : wide ? launch_persistent(sapa_wide_16_kernel<T, M>, names_wide[M], w16::NT, w16::SMEM_BYTES, 1, false, a, st, qmap, kmap, vmap, omap) \
                       : launch_persistent(sapa_tma_fused_16_kernel<T, M, false>, names16[M], h16::NT, h16::SMEM_BYTES, h16::CTAS_PER_SM, M != MODE_BWD, a, st, qmap, kmap, vmap);
+#define SAPA_TMA_LAUNCH16_SIM(T)         /* ragged rows: the others have gone to the strips */                                           \
+    case MODE_SIM:                                                                                                                       \
+        return launch_persistent(sapa_tma_fused_16_kernel<T, MODE_SIM, true>, names_ragged[MODE_SIM], h16::NT_RAGGED, h16::SMEM_BYTES, 1, true, a, st, qmap, kmap, vmap);
     if (dtype == SAPA_F32) switch (mode) { SAPA_TMA_LAUNCH32(MODE_FWD) SAPA_TMA_LAUNCH32(MODE_BWD) SAPA_TMA_LAUNCH32(MODE_SIM) SAPA_TMA_LAUNCH32(MODE_AGG) }
     if (dtype == SAPA_F16)
-        switch (mode) { SAPA_TMA_LAUNCH16(__half, MODE_FWD) SAPA_TMA_LAUNCH16(__half, MODE_BWD) SAPA_TMA_LAUNCH16(__half, MODE_SIM) SAPA_TMA_LAUNCH16(__half, MODE_AGG) }
+        switch (mode) { SAPA_TMA_LAUNCH16(__half, MODE_FWD) SAPA_TMA_LAUNCH16(__half, MODE_BWD) SAPA_TMA_LAUNCH16_SIM(__half) SAPA_TMA_LAUNCH16(__half, MODE_AGG) }
     if (dtype == SAPA_BF16)
-        switch (mode) { SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_FWD) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_BWD) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_SIM) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_AGG) }
+        switch (mode) { SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_FWD) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_BWD) SAPA_TMA_LAUNCH16_SIM(__nv_bfloat16) SAPA_TMA_LAUNCH16(__nv_bfloat16, MODE_AGG) }
     set_error("sapa_tma_fused: unknown mode %d or dtype code %d", mode, dtype);
     return SAPA_ERR_ARGUMENT;
 #undef SAPA_TMA_LAUNCH32
 #undef SAPA_TMA_LAUNCH16
+#undef SAPA_TMA_LAUNCH16_SIM
 }
 
 // One CTA waits, with a short limit, on a shared-memory barrier that nothing ever signals: the bounded wait gives up,

@@ -71,7 +71,7 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 
     if (warp >= w16::NW) {            // producer: one lane; the stages of successive items form one stream through the ring
         asm volatile("setmaxnreg.dec.sync.aligned.u32 24;\n");
-        if (MODE != MODE_SIM && tid == (w16::NW + 1) * 32) {
+        if (tid == (w16::NW + 1) * 32) {
             // output: one lane of another warp of the group stores the boxes that the consumers have written
             int buf = 0, par = 0;
             for (int ti = 0;; ++ti) {
@@ -166,10 +166,9 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         if (!mbar_wait_bounded(full_addr + 8 * slot, phase)) { atomicExch(&g_wait_timeout, 1); return; }
         int item = tile_ids[ti & 7];              // published by the producer before the barrier's phase completed
         if (item < 0) {
-            if (MODE != MODE_SIM) {               // the storing lane reads -1 and stops
-                if (!mbar_wait_bounded(free_addr + 8 * obuf, opar ^ 1)) atomicExch(&g_wait_timeout, 1);
-                else if (lane == 0) mbar_arrive(written_addr + 8 * obuf);
-            }
+            // the storing lane reads -1 and stops
+            if (!mbar_wait_bounded(free_addr + 8 * obuf, opar ^ 1)) atomicExch(&g_wait_timeout, 1);
+            else if (lane == 0) mbar_arrive(written_addr + 8 * obuf);
             break;
         }
         int c0 = item % a.csplit * nv * w16::VCH; item /= a.csplit;
@@ -311,23 +310,7 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
                             pp[dy][1] = pack_pair(T(), sp[dy][2] * i0, sp[dy][3] * i1);
                         }
                     }
-                    if (MODE == MODE_SIM && a.slots_f32 == 0) {
-#pragma unroll
-                        for (int dy = 0; dy < 5; ++dy) {
-                            pp[dy][0] = pack_pair(T(), sp[dy][0], sp[dy][1]);
-                            pp[dy][1] = pack_pair(T(), sp[dy][2], sp[dy][3]);
-                        }
-                    }
-                    if (MODE == MODE_SIM && a.slots_f32 != 0) {      // raw logits as float32 pairs
-                        if (live) {
-                            float2 *af = static_cast<float2 *>(a.attn) + at_w;
-#pragma unroll
-                            for (int dy = 0; dy < 5; ++dy) {
-                                if (ok_lo[p]) af[(size_t)(dy * 5 + dx_lo[p]) * plane_w] = make_float2(sp[dy][0], sp[dy][1]);
-                                if (ok_hi[p]) af[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w] = make_float2(sp[dy][2], sp[dy][3]);
-                            }
-                        }
-                    } else if ((MODE == MODE_FWD || MODE == MODE_SIM) && a.attn != nullptr && c0 == 0 && live) {
+                    if (MODE == MODE_FWD && a.attn != nullptr && c0 == 0 && live) {
                         unsigned *an = static_cast<unsigned *>(a.attn) + at_w;
 #pragma unroll
                         for (int dy = 0; dy < 5; ++dy) {
@@ -335,15 +318,13 @@ sapa_wide_16_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
                             if (ok_hi[p]) an[(size_t)(dy * 5 + dx_lo[p] + 8) * plane_w] = pp[dy][1];
                         }
                     }
-                    if (MODE != MODE_SIM)             // S^T accumulator fragments -> B fragments of the aggregation
 #pragma unroll
-                        for (int dy = 0; dy < 5; ++dy) {
-                            pp[dy][0] = movmatrix_trans(pp[dy][0]);
-                            pp[dy][1] = movmatrix_trans(pp[dy][1]);
-                        }
+                    for (int dy = 0; dy < 5; ++dy) {  // S^T accumulator fragments -> B fragments of the aggregation
+                        pp[dy][0] = movmatrix_trans(pp[dy][0]);
+                        pp[dy][1] = movmatrix_trans(pp[dy][1]);
+                    }
                 }
         }
-        if (MODE == MODE_SIM) continue;
         // ------------------------------------------------------------- aggregation
         for (int it = 0; it < nv; ++it) {
             if ((MODE != MODE_AGG || it > 0) && !mbar_wait_bounded(full_addr + 8 * slot, phase)) { atomicExch(&g_wait_timeout, 1); return; }
