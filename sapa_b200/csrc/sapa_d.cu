@@ -598,7 +598,14 @@ struct OutlierGrad {
 // logit gradients dS, no aggregation part).
 constexpr int BWD_FUSED = 0, BWD_AV = 1, BWD_QK = 2;
 
-template <typename T, int NP, int MODE>
+// In the form of deform_window_kernel (see there): the points of a pixel side by side, without branches, each point's place in the windows kept from
+// pass to pass, a block = pixels of one (image, group).  The two windows of a thread (D and dWd going in, dD and Wd coming out) share its two
+// columns of shared memory.  Points outside the window are few and hold up their warp, which gathers them together, a channel to a
+// lane, while they are; each thread its own where there are many (lines at 40 or none: slower).  8 x 4 groups x 128x128 pixels, 9 points, float32 |
+// bfloat16, us: sigma 0.5 118 -> 76 | 114 -> 74 (branches on each point before, in which one far point held its block), 1.0 1209 -> 418 |
+// 1183 -> 450, 1.5 855 -> 673 | 865 -> 763; 1 point 108 -> 46 | 93 -> 42, 16 points 257 -> 240 | 267 -> 201.  Bound by latency at 16 warps per SM
+// (128 registers, of which the form for 9 points spills 60).
+template <typename T, int PMAX, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 4)
 deform_window_bwd_kernel(const T *grad_out, const T *value, const T *offset,
                          const T *attn, const float *dense /* D [B*G, 25, hi] */,
@@ -607,117 +614,134 @@ deform_window_bwd_kernel(const T *grad_out, const T *value, const T *offset,
                          OutlierGrad *taps,
                          unsigned int *tap_count, int B, int C, int H, int W, int P_runtime, int G) {
     begin_after_previous();
-    constexpr int PMAX = NP > 0 ? NP : MAXP;
-    const int P = NP > 0 ? NP : P_runtime;
-    const int sH = 2 * H, sW = 2 * W, gc = C / G;
-    const size_t hi = (size_t)sH * sW, lo = (size_t)H * W;
-    // The two 25-slot windows of a thread (D and dWd going in, dD and Wd coming out) live in shared memory, column =
-    // thread (conflict-free): a point touches four cells of each, and shared memory can be indexed with the cell found
-    // at run time, where registers force a product with all 25 cells.
-    __shared__ float sd[25][WIN_THREADS], sw[25][WIN_THREADS];
+    __shared__ float sd[MODE != BWD_AV ? 25 : 1][WIN_THREADS], sw[MODE != BWD_QK ? 25 : 1][WIN_THREADS];
+    constexpr int MANY = 16;      // points outside the window of a warp's pixels
+    const int P = PMAX == 9 ? 9 : P_runtime;
+    const unsigned sW = 2 * W;
+    const int gc = C / G;
+    const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)H * W;
     const int lane = threadIdx.x & 31, tid = threadIdx.x;
-    const long long total = (long long)B * G * hi;
-    for (long long i0 = (long long)blockIdx.x * WIN_THREADS; i0 < total; i0 += (long long)gridDim.x * WIN_THREADS) {
-        const long long i = i0 + threadIdx.x;
-        const bool live = i < total;
-        const size_t pix = live ? (size_t)(i % hi) : 0;
-        const long long bg = live ? i / (long long)hi : 0;
-        const int qw = (int)(pix % sW), qh = (int)(pix / sW), py = qh >> 1, px = qw >> 1;
-        float oh[PMAX], ow[PMAX], at[PMAX];
+    const unsigned blocks = ((unsigned)hi + WIN_THREADS - 1) / WIN_THREADS, groups = (unsigned)(B * G);      // of an (image, group)
+    float *const dcol = &sd[0][tid], *const wcol = &sw[0][tid];
+    for (unsigned bg = blockIdx.y; bg < groups; bg += gridDim.y)
+    for (unsigned block = blockIdx.x; block < blocks; block += gridDim.x) {
+        const unsigned at_pix = block * WIN_THREADS + tid, pix = at_pix < hi ? at_pix : 0u;
+        const bool live = at_pix < hi;
+        const int qh = (int)(pix / sW), qw = (int)(pix - (unsigned)qh * sW), py = qh >> 1, px = qw >> 1;
+        const T *offp = offset + (size_t)bg * P * 2 * hi + pix, *ap = attn + (size_t)bg * P * hi + pix;
         const float *dp = dense + (size_t)bg * 25 * hi + pix, *wp = dwin + (size_t)bg * 25 * hi + pix;
 #pragma unroll
         for (int k = 0; k < 25; ++k) {
-            sd[k][tid] = (MODE != BWD_AV && live) ? __ldcs(dp + (size_t)k * hi) : 0.f;
-            sw[k][tid] = (MODE != BWD_QK && live) ? __ldcs(wp + (size_t)k * hi) : 0.f;
+            if (MODE != BWD_AV) dcol[k * WIN_THREADS] = live ? __ldcs(dp + (size_t)k * hi) : 0.f;
+            if (MODE != BWD_QK) wcol[k * WIN_THREADS] = live ? __ldcs(wp + (size_t)k * hi) : 0.f;
         }
-        const T *offp = offset + (size_t)bg * P * 2 * hi + pix, *ap = attn + (size_t)bg * P * hi + pix;
+        WindowPoints<PMAX> pts;
+        pts.load(offp, hi, live, P);
+        float at[PMAX];
 #pragma unroll
-        for (int p = 0; p < PMAX; ++p) {
-            const bool on = live && p < P;
-            ow[p] = on ? float(px) + to_acc(offp[(size_t)(2 * p) * hi]) : 0.f;
-            oh[p] = on ? float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]) : 0.f;
-            at[p] = on ? to_acc(ap[(size_t)p * hi]) : 0.f;
-        }
-        // ---- pass 1: dA_p and the four bilinear forms of the offset gradients
+        for (int p = 0; p < PMAX; ++p) at[p] = live && p < P ? to_acc(ap[(size_t)p * hi]) : 0.f;
+        // ---- pass 1: dA_p and the bilinear forms of the offset gradients: value (1-lh, lh) x (1-lw, lw); d/dh (-1, 1) x (1-lw, lw); d/dw (1-lh, lh) x (-1, 1)
         float da[PMAX], gh1[PMAX], gw1[PMAX], gh2[PMAX], gw2[PMAX];
-        float dot = 0.f;
-        unsigned int outliers = 0;
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
-            da[p] = 0.f; gh1[p] = 0.f; gw1[p] = 0.f; gh2[p] = 0.f; gw2[p] = 0.f;
-            if (live && p < P) {
-                WindowTap t;
-                t.setup(oh[p], ow[p], H, W, py, px);
-                if (t.dense) {
-                    // bilinear forms over the four cells: value (1-lh, lh) x (1-lw, lw); d/dh (-1, 1) x (1-lw, lw); d/dw (1-lh, lh) x (-1, 1)
-                    const int c = t.r0 * 5 + t.c0;
-                    const float hw = 1.f - t.lw, hh = 1.f - t.lh;
-                    if (MODE != BWD_QK) {
-                        const float w00 = sw[c][tid], w01 = sw[c + 1][tid], w10 = sw[c + 5][tid], w11 = sw[c + 6][tid];
-                        const float top = hw * w00 + t.lw * w01, bot = hw * w10 + t.lw * w11;
-                        da[p] = hh * top + t.lh * bot;
-                        gh1[p] = bot - top;
-                        gw1[p] = (hh * w01 + t.lh * w11) - (hh * w00 + t.lh * w10);
-                    }
-                    if (MODE != BWD_AV) {
-                        const float d00 = sd[c][tid], d01 = sd[c + 1][tid], d10 = sd[c + 5][tid], d11 = sd[c + 6][tid];
-                        gh2[p] = (hw * d10 + t.lw * d11) - (hw * d00 + t.lw * d01);
-                        gw2[p] = (hh * d01 + t.lh * d11) - (hh * d00 + t.lh * d10);
-                    }
-                } else if (t.inside) {        // outlier: dA by direct gather
-                    outliers |= 1u << p;
-                    if (MODE == BWD_QK) continue;
-                    Bilinear<float> bl;
-                    bl.setup(oh[p], ow[p], H, W);
-                    const T *gp = grad_out + (size_t)bg * gc * hi + pix, *vp = value + (size_t)bg * gc * lo;
-                    float acc = 0.f;
-                    for (int c = 0; c < gc; ++c) acc += bl.sample(vp + (size_t)c * lo) * to_acc(gp[(size_t)c * hi]);
-                    da[p] = acc;
-                }
-                dot += at[p] * da[p];
+            pts.set(p, live && p < P, H, W, py, px);
+            const bool in = pts.dense >> p & 1;
+            const float lh = pts.lh[p], lw = pts.lw[p], hh = 1.f - lh, hw = 1.f - lw;
+            da[p] = gh1[p] = gw1[p] = gh2[p] = gw2[p] = 0.f;
+            if (MODE != BWD_QK) {
+                const float *c = wcol + pts.at(p);
+                const float w00 = c[0], w01 = c[WIN_THREADS], w10 = c[5 * WIN_THREADS], w11 = c[6 * WIN_THREADS];
+                const float top = hw * w00 + lw * w01, bot = hw * w10 + lw * w11;
+                da[p] = in ? hh * top + lh * bot : 0.f;
+                gh1[p] = in ? bot - top : 0.f;
+                gw1[p] = in ? (hh * w01 + lh * w11) - (hh * w00 + lh * w10) : 0.f;
+            }
+            if (MODE != BWD_AV) {
+                const float *c = dcol + pts.at(p);
+                const float d00 = c[0], d01 = c[WIN_THREADS], d10 = c[5 * WIN_THREADS], d11 = c[6 * WIN_THREADS];
+                gh2[p] = in ? (hw * d10 + lw * d11) - (hw * d00 + lw * d01) : 0.f;
+                gw2[p] = in ? (hh * d01 + lh * d11) - (hh * d00 + lh * d10) : 0.f;
             }
         }
+        if (MODE != BWD_QK) {         // dA of the points outside the window
+            const T *gp = grad_out + (size_t)bg * gc * hi, *vp = value + (size_t)bg * gc * lo;
+            const unsigned few = __reduce_add_sync(0xffffffffu, (unsigned)__popc(pts.outliers));
+            if (few > MANY) {
+                for (unsigned left = pts.outliers; left != 0; left &= left - 1) {
+                    const int p = __ffs(left) - 1;
+                    Bilinear<float> bl;
+                    bl.setup(float(py) + to_acc(offp[(size_t)(2 * p + 1) * hi]), float(px) + to_acc(offp[(size_t)(2 * p) * hi]), H, W);
+                    float acc = 0.f;
+                    const T *v0 = vp, *g0 = gp + pix;             // pointers that advance: with products of the channel the loop takes half as long again
+#pragma unroll 4
+                    for (int c = 0; c < gc; ++c, v0 += lo, g0 += hi) acc += bl.sample(v0) * to_acc(*g0);
+                    put(da, p, acc);
+                }
+            } else {
+                for (unsigned lanes = __ballot_sync(0xffffffffu, pts.outliers != 0); lanes != 0; lanes &= lanes - 1) {
+                    const int src = __ffs(lanes) - 1;
+                    const unsigned spix = __shfl_sync(0xffffffffu, pix, src);
+                    const int sh = (int)(spix / sW), spy = sh >> 1, spx = (int)(spix - (unsigned)sh * sW) >> 1;
+                    const T *so = offset + (size_t)bg * P * 2 * hi + spix;
+                    for (unsigned left = __shfl_sync(0xffffffffu, pts.outliers, src); left != 0; left &= left - 1) {
+                        const int p = __ffs(left) - 1;
+                        Bilinear<float> bl;
+                        bl.setup(float(spy) + to_acc(so[(size_t)(2 * p + 1) * hi]), float(spx) + to_acc(so[(size_t)(2 * p) * hi]), H, W);
+                        float acc = 0.f;
+                        for (int c = lane; c < gc; c += 32) acc += bl.sample(vp + (size_t)c * lo) * to_acc(gp[(size_t)c * hi + spix]);
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                        if (lane == src) put(da, p, acc);
+                    }
+                }
+            }
+        }
+        float dot = 0.f;
+#pragma unroll
+        for (int p = 0; p < PMAX; ++p) dot += at[p] * da[p];
         // ---- pass 2: logit gradients, dD, Wd (the two shared windows become the accumulators), offset gradients
 #pragma unroll
-        for (int k = 0; k < 25; ++k) { sd[k][tid] = 0.f; sw[k][tid] = 0.f; }
+        for (int k = 0; k < 25; ++k) {
+            if (MODE != BWD_AV) dcol[k * WIN_THREADS] = 0.f;
+            if (MODE != BWD_QK) wcol[k * WIN_THREADS] = 0.f;
+        }
         T *gop = grad_offset + (size_t)bg * P * 2 * hi + pix;
 #pragma unroll
         for (int p = 0; p < PMAX; ++p) {
-            if (live && p < P) {
-                // BWD_QK: `attn` holds the logit gradients themselves; BWD_AV: no logit gradient, dA goes out as it is
-                const float a = MODE == BWD_QK ? 0.f : at[p];
-                const float ds = MODE == BWD_QK ? at[p] : MODE == BWD_AV ? 0.f : a * (da[p] - dot);
-                if (MODE == BWD_AV) grad_attn[((size_t)bg * P + p) * hi + pix] = from_acc<T>(da[p]);
-                da[p] = ds;
-                WindowTap t;
-                t.setup(oh[p], ow[p], H, W, py, px);
-                if (t.dense) {
-                    const int c = t.r0 * 5 + t.c0;
-                    const float b00 = (1.f - t.lh) * (1.f - t.lw), b01 = (1.f - t.lh) * t.lw, b10 = t.lh * (1.f - t.lw), b11 = t.lh * t.lw;
-                    if (MODE != BWD_AV) {
-                        sd[c][tid] += ds * b00; sd[c + 1][tid] += ds * b01; sd[c + 5][tid] += ds * b10; sd[c + 6][tid] += ds * b11;
-                    }
-                    if (MODE != BWD_QK) {
-                        sw[c][tid] += a * b00; sw[c + 1][tid] += a * b01; sw[c + 5][tid] += a * b10; sw[c + 6][tid] += a * b11;
-                    }
-                }
-                if (!(outliers & (1u << p))) {      // the list kernel writes the offset gradients of the outliers
-                    gop[(size_t)(2 * p) * hi] = from_acc<T>(a * gw1[p] + ds * gw2[p]);
-                    gop[(size_t)(2 * p + 1) * hi] = from_acc<T>(a * gh1[p] + ds * gh2[p]);
-                }
+            const bool on = live && p < P, in = pts.dense >> p & 1;
+            // BWD_QK: `attn` holds the logit gradients themselves; BWD_AV: no logit gradient, dA goes out as it is
+            const float a = MODE == BWD_QK ? 0.f : at[p], ds = MODE == BWD_QK ? at[p] : MODE == BWD_AV ? 0.f : a * (da[p] - dot);
+            if (MODE == BWD_AV && on) grad_attn[((size_t)bg * P + p) * hi + pix] = from_acc<T>(da[p]);
+            da[p] = ds;
+            const float lh = pts.lh[p], lw = pts.lw[p], hw = 1.f - lw;
+            if (MODE != BWD_AV) {
+                float *c = dcol + pts.at(p);
+                const float add = in ? ds : 0.f, t = add * (1.f - lh), u = add * lh;
+                const float c00 = c[0], c01 = c[WIN_THREADS], c10 = c[5 * WIN_THREADS], c11 = c[6 * WIN_THREADS];
+                c[0] = c00 + t * hw; c[WIN_THREADS] = c01 + t * lw; c[5 * WIN_THREADS] = c10 + u * hw; c[6 * WIN_THREADS] = c11 + u * lw;
+            }
+            if (MODE != BWD_QK) {
+                float *c = wcol + pts.at(p);
+                const float add = in ? a : 0.f, t = add * (1.f - lh), u = add * lh;
+                const float c00 = c[0], c01 = c[WIN_THREADS], c10 = c[5 * WIN_THREADS], c11 = c[6 * WIN_THREADS];
+                c[0] = c00 + t * hw; c[WIN_THREADS] = c01 + t * lw; c[5 * WIN_THREADS] = c10 + u * hw; c[6 * WIN_THREADS] = c11 + u * lw;
+            }
+            if (on && !(pts.outliers >> p & 1)) {      // the list kernel writes the offset gradients of the outliers
+                gop[(size_t)(2 * p) * hi] = from_acc<T>(a * gw1[p] + ds * gw2[p]);
+                gop[(size_t)(2 * p + 1) * hi] = from_acc<T>(a * gh1[p] + ds * gh2[p]);
             }
         }
         if (live) {
             T *ddp = ddense + (size_t)bg * 25 * hi + pix, *wdp = window + (size_t)bg * 25 * hi + pix;
 #pragma unroll
             for (int k = 0; k < 25; ++k) {
-                if (MODE != BWD_AV) ddp[(size_t)k * hi] = from_acc<T>(sd[k][tid]);
-                if (MODE != BWD_QK) wdp[(size_t)k * hi] = from_acc<T>(sw[k][tid]);
+                if (MODE != BWD_AV) ddp[(size_t)k * hi] = from_acc<T>(dcol[k * WIN_THREADS]);
+                if (MODE != BWD_QK) wdp[(size_t)k * hi] = from_acc<T>(wcol[k * WIN_THREADS]);
             }
         }
-        const unsigned int any = __ballot_sync(0xffffffffu, outliers != 0);
+        const unsigned int any = __ballot_sync(0xffffffffu, pts.outliers != 0);
         if (any != 0) {
-            const int mine = __popc(outliers);
+            const int mine = __popc(pts.outliers);
             int incl = mine;
 #pragma unroll
             for (int sft = 1; sft < 32; sft <<= 1) {
@@ -731,9 +755,9 @@ deform_window_bwd_kernel(const T *grad_out, const T *value, const T *offset,
             unsigned int pos = base + (unsigned int)(incl - mine);
 #pragma unroll
             for (int p = 0; p < PMAX; ++p)
-                if (outliers & (1u << p)) {
+                if (pts.outliers >> p & 1) {
                     OutlierGrad t;
-                    t.k = (unsigned int)(bg * P + p); t.pix = (unsigned int)pix; t.a = MODE == BWD_QK ? 0.f : at[p]; t.ds = da[p];
+                    t.k = (unsigned int)(bg * P + p); t.pix = pix; t.a = MODE == BWD_QK ? 0.f : at[p]; t.ds = da[p];
                     taps[pos++] = t;
                 }
         }
@@ -996,6 +1020,11 @@ template <int MODE, typename T, typename... A> static void launch_window(int P, 
     const unsigned threads = hi <= 4 * WIN_THREADS && (hi - 1) % WIN_THREADS < WIN_THREADS / 2 ? WIN_THREADS / 2 : WIN_THREADS;
     const dim3 grid((unsigned)((hi + threads - 1) / threads), (unsigned)(groups < 65535 ? groups : 65535), 1);
     for_points(P, [&](auto most) { launch_next(deform_window_kernel<T, decltype(most)::value, MODE>, grid, threads, 0, st, args...); });
+}
+
+template <int MODE, typename T, typename... A> static void launch_window_bwd(int P, int groups, size_t hi, cudaStream_t st, A... args) {
+    const dim3 grid((unsigned)((hi + WIN_THREADS - 1) / WIN_THREADS), (unsigned)(groups < 65535 ? groups : 65535), 1);
+    for_points(P, [&](auto most) { launch_in_order(deform_window_bwd_kernel<T, decltype(most)::value, MODE>, grid, WIN_THREADS, 0, st, args...); });
 }
 
 static int check_deform(const char *fn, int B, int Cq, int C, int H, int W, int P, int s, int G, int dtype) {
@@ -1380,17 +1409,12 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     }
     // 2. per pixel: softmax backward over the points, dD, Wd, offset gradients, list of the points outside the window
     {
-        const int grid = grid_1d((long long)B * G * hi, WIN_THREADS);
         const int e = SAPA_DISPATCH_FAST(dtype, [&] {
             const scalar_t *go = static_cast<const scalar_t *>(grad_out), *v = static_cast<const scalar_t *>(value);
             const scalar_t *o = static_cast<const scalar_t *>(offset), *a = static_cast<const scalar_t *>(attn);
             scalar_t *dd = static_cast<scalar_t *>(ddense), *wn = static_cast<scalar_t *>(window), *goff = static_cast<scalar_t *>(grad_offset);
-            if (P == 9)
-                launch_in_order(deform_window_bwd_kernel<scalar_t, 9, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
-                                                                                      tap_count, B, C, H, W, P, G);
-            else
-                launch_in_order(deform_window_bwd_kernel<scalar_t, 0, BWD_FUSED>, grid, WIN_THREADS, 0, st, go, v, o, a, dense, dwin, dd, wn, goff, nullptr, taps,
-                                                                                      tap_count, B, C, H, W, P, G);
+            launch_window_bwd<BWD_FUSED, scalar_t>(P, B * G, hi, st, go, v, o, a, static_cast<const float *>(dense), static_cast<const float *>(dwin), dd, wn, goff,
+                                                   static_cast<scalar_t *>(nullptr), taps, tap_count, B, C, H, W, P, G);
             return check_launch("deform_window_bwd_kernel");
         });
         if (e) return e;
@@ -1456,16 +1480,10 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
         if (int e = run_sim_mixed(grad_out, value, dwin, B * G, C / G, H, W, H, 0, dtype, st)) return e;
     }
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
-            if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_in_order(deform_window_bwd_kernel<scalar_t, 9, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
-                    static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
-                    static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
-                    static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
-            else
-                launch_in_order(deform_window_bwd_kernel<scalar_t, 0, BWD_AV>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
-                    static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value), static_cast<const scalar_t *>(offset),
-                    static_cast<const scalar_t *>(attn), nullptr, dwin, nullptr, static_cast<scalar_t *>(window),
-                    static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
+            launch_window_bwd<BWD_AV, scalar_t>(P, B * G, hi, st, static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value),
+                                                static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(attn), static_cast<const float *>(nullptr),
+                                                static_cast<const float *>(dwin), static_cast<scalar_t *>(nullptr), static_cast<scalar_t *>(window),
+                                                static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(grad_attn), taps, tap_count, B, C, H, W, P, G);
             return check_launch("deform_window_bwd_kernel<av>");
         }))
         return e;
@@ -1523,14 +1541,10 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     }
     // the logit gradients enter where the fused chain reads the attention
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
-            if (P == 9)      // the 3 x 3 points of the reference modules' default: loops unrolled for nine points
-                launch_in_order(deform_window_bwd_kernel<scalar_t, 9, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
-                    nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
-                    static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
-            else
-                launch_in_order(deform_window_bwd_kernel<scalar_t, 0, BWD_QK>, grid_1d((long long)B * G * hi, WIN_THREADS), WIN_THREADS, 0, st,
-                    nullptr, nullptr, static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), dense, nullptr,
-                    static_cast<scalar_t *>(ddense), nullptr, static_cast<scalar_t *>(grad_offset), nullptr, taps, tap_count, B, Cq, H, W, P, G);
+            launch_window_bwd<BWD_QK, scalar_t>(P, B * G, hi, st, static_cast<const scalar_t *>(nullptr), static_cast<const scalar_t *>(nullptr),
+                                                static_cast<const scalar_t *>(offset), static_cast<const scalar_t *>(grad_out), static_cast<const float *>(dense),
+                                                static_cast<const float *>(nullptr), static_cast<scalar_t *>(ddense), static_cast<scalar_t *>(nullptr),
+                                                static_cast<scalar_t *>(grad_offset), static_cast<scalar_t *>(nullptr), taps, tap_count, B, Cq, H, W, P, G);
             return check_launch("deform_window_bwd_kernel<qk>");
         }))
         return e;
