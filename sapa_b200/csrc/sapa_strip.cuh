@@ -10,7 +10,8 @@
 //   * P: the banded operand of a step, 15 tiles (window row, 32 bytes of cells) of the pixels that the cells reach: a third of the band is
 //     not zero.  Its zeros are the same in every step and are written once; two warpgroups overwrite the 25 weights per pixel.
 //     Pixels are ordered parent by parent, so that the pixels of a tile are consecutive columns of D.
-//   * one warp issues the MMAs (N = 16 to 80, N / 2 clocks each); float32 adds the small products first, because an accumulation in
+//   * one warp issues the MMAs (N = 16 to 80, N / 2 clocks each), in float32, with three times as many, one for each half of the strip: a warp issues
+//     an MMA in about 26 clocks, with one 32 x 64 x 64x64 took 58 us.  float32 adds the small products first, because an accumulation in
 //     tensor memory rounds toward zero: eight roundings of the whole sum instead of twenty-four.
 //   * epilogue: tcgen05.ld (lane = channel), zeros back into D, rows of 128 bytes through shared memory, TMA stores; a warpgroup for each of
 //     the two accumulators (with one for both it was what the kernel waited for: 32 x 64 x 64x64, bfloat16, 45 -> 32 us).
@@ -22,7 +23,7 @@ namespace strip {
 using namespace ummau;
 
 constexpr int CH = 128;                                     // channels of an item = lanes of tensor memory
-constexpr int EPI_WARPS = 8, SPLIT_WARP0 = 8, P_WARP0 = 12, P_WARPS = 8, TMA_WARP = 20, MMA_WARP = 21, NT = 22 * 32;
+constexpr int EPI_WARPS = 8, SPLIT_WARP0 = 8, P_WARP0 = 12, P_WARPS = 8, TMA_WARP = 20, MMA_WARP = 21, NT = 23 * 32;
 constexpr int VROW = 112, VCHUNKS = 7, ACOLS = 24;          // bytes and 16-byte chunks of a box row; columns of an A operand (one term)
 constexpr int V_BYTES = CH * VROW, NVL = 4;                 // landed rows of V
 constexpr int L_BYTES = 2 * 25 * 128, NWL = 4;              // landed weights: [high-res row][slot][pixel]
@@ -38,6 +39,7 @@ template <typename T> struct Geo {
     static constexpr int SHIFT = F32 ? 2 : 3;               // words from the box's start (16-byte boundary) to cell x0 - 2, the first of the product
     static constexpr int BOX0 = F32 ? 4 : 8;                // the box starts at column x0 - BOX0
     static constexpr int ABUF = TERMS * ACOLS;
+    static constexpr int ISSUERS = F32 ? 2 : 1;             // warps that issue the MMAs, each those of half of the strip's parents
     // K step j: parents [p0, p1) of the strip reach its cells (columns x0 - 2 + KS j and so on)
     __host__ __device__ static constexpr int p0(int j) { return KS * j < 4 ? 0 : KS * j - 4; }
     __host__ __device__ static constexpr int p1(int j) { return KS * j + KS < CELLS ? KS * j + KS : CELLS; }
@@ -107,9 +109,9 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
     if (tid == 0) {
         for (int i = 0; i < NVL; ++i) { mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 128); }
         for (int i = 0; i < NWL; ++i) { mbar_init(wfull + 8 * i, 1); mbar_init(wempty + 8 * i, 32 * P_WARPS); }
-        for (int i = 0; i < strip::NV; ++i) { mbar_init(aready + 8 * i, 128); mbar_init(aempty + 8 * i, 1); }
-        for (int i = 0; i < ND; ++i) { mbar_init(dfull + 8 * i, 1); mbar_init(dempty + 8 * i, 128); }
-        for (int i = 0; i < NP; ++i) { mbar_init(pready + 8 * i, 32 * P_WARPS); mbar_init(pempty + 8 * i, 1); }
+        for (int i = 0; i < strip::NV; ++i) { mbar_init(aready + 8 * i, 128); mbar_init(aempty + 8 * i, G::ISSUERS); }
+        for (int i = 0; i < ND; ++i) { mbar_init(dfull + 8 * i, G::ISSUERS); mbar_init(dempty + 8 * i, 128); }
+        for (int i = 0; i < NP; ++i) { mbar_init(pready + 8 * i, 32 * P_WARPS); mbar_init(pempty + 8 * i, G::ISSUERS); }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == MMA_WARP) {
@@ -161,43 +163,54 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                 (void)drain_loads<NWL>(wfull, ws, wph);
             }
         }
-    } else if (warp == MMA_WARP) {
+    } else if (warp >= MMA_WARP) {
         constexpr unsigned HI = (128u >> 4) | (1u << 14);             // 8-row groups 128 bytes apart, descriptor version 1, no swizzle
         const unsigned leader = elect_leader(), p_base = warp_uniform(base + G::P0);
         const unsigned b0 = desc_lo(p_base + G::tile(0), G::lbo(0)), b1 = desc_lo(p_base + G::tile(1), G::lbo(1)), b2 = desc_lo(p_base + G::tile(2), G::lbo(2));
+        // the products of a tile that reach parents [lo, hi) of the strip; nothing where there are none
+        auto part = [&](auto tile, auto lo, auto hi, unsigned d, unsigned ka, unsigned b) {
+            constexpr int J = decltype(tile)::value, LO = decltype(lo)::value, HI_P = decltype(hi)::value;
+            constexpr int P = (LO > G::p0(J)) ? LO : G::p0(J), ROWS = 4 * (((HI_P < G::p1(J)) ? HI_P : G::p1(J)) - P);
+            if constexpr (ROWS > 0) tc_mma_ta<G::F32>(leader, d + 4 * P, ka + 8 * J, b + 4 * (P - G::p0(J)), HI, IDESC_M128<T> | idesc_n(ROWS), 1u);
+        };
         int row0 = 0, db = 0, dph = 0, pb = 0, pph = 0;               // row0: rows of V of this CTA before the item
-        for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
-            const Item t = item_at<T>(a, i);
-            int known = row0;                                         // rows of V waited for
-            for (int s = 0; s < t.y1 - t.y0 && ok; ++s) {
-                for (; known < row0 + s + 5 && ok; ++known) ok = mbar_wait_warp(aready + 8 * (known % strip::NV), (known / strip::NV) & 1);
-                ok = ok && mbar_wait_warp(dempty + 8 * db, dph ^ 1) && mbar_wait_warp(pready + 8 * pb, pph);
-                if (!ok) break;
-                tc_fence_after();
-                const unsigned d = tmem + db * G::N, pofs = (unsigned)(pb * G::P_BYTES) >> 4;
-                auto product = [&](int av, int pt) {                  // terms of V and of P
+        auto run = [&](auto lo, auto hi) {
+            for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+                const Item t = item_at<T>(a, i);
+                int known = row0;                                     // rows of V waited for
+                for (int s = 0; s < t.y1 - t.y0 && ok; ++s) {
+                    for (; known < row0 + s + 5 && ok; ++known) ok = mbar_wait_warp(aready + 8 * (known % strip::NV), (known / strip::NV) & 1);
+                    ok = ok && mbar_wait_warp(dempty + 8 * db, dph ^ 1) && mbar_wait_warp(pready + 8 * pb, pph);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const unsigned d = tmem + db * G::N, pofs = (unsigned)(pb * G::P_BYTES) >> 4;
+                    auto product = [&](int av, int pt) {              // terms of V and of P
 #pragma unroll
-                    for (int dy = 0; dy < 5; ++dy) {
-                        const unsigned ka = tmem + ring + ((row0 + s + dy) % strip::NV) * G::ABUF + av * ACOLS;
-                        const unsigned kb = pofs + ((dy * G::DY_BYTES + pt * G::P_TERM) >> 4);
-                        tc_mma_ta<G::F32>(leader, d + 4 * G::p0(0), ka, b0 + kb, HI, IDESC_M128<T> | idesc_n(G::rows(0)), 1u);
-                        tc_mma_ta<G::F32>(leader, d + 4 * G::p0(1), ka + 8, b1 + kb, HI, IDESC_M128<T> | idesc_n(G::rows(1)), 1u);
-                        tc_mma_ta<G::F32>(leader, d + 4 * G::p0(2), ka + 16, b2 + kb, HI, IDESC_M128<T> | idesc_n(G::rows(2)), 1u);
-                    }
-                };
-                if (G::F32) { product(1, 0); product(0, 1); }
-                product(0, 0);
-                tc_commit_by(leader, dfull + 8 * db);
-                tc_commit_by(leader, pempty + 8 * pb);
-                tc_commit_by(leader, aempty + 8 * ((row0 + s) % strip::NV));
-                if (++db == ND) { db = 0; dph ^= 1; }
-                if (++pb == NP) { pb = 0; pph ^= 1; }
+                        for (int dy = 0; dy < 5; ++dy) {
+                            const unsigned ka = tmem + ring + ((row0 + s + dy) % strip::NV) * G::ABUF + av * ACOLS;
+                            const unsigned kb = pofs + ((dy * G::DY_BYTES + pt * G::P_TERM) >> 4);
+                            part(std::integral_constant<int, 0>{}, lo, hi, d, ka, b0 + kb);
+                            part(std::integral_constant<int, 1>{}, lo, hi, d, ka, b1 + kb);
+                            part(std::integral_constant<int, 2>{}, lo, hi, d, ka, b2 + kb);
+                        }
+                    };
+                    if (G::F32) { product(1, 0); product(0, 1); }
+                    product(0, 0);
+                    tc_commit_by(leader, dfull + 8 * db);
+                    tc_commit_by(leader, pempty + 8 * pb);
+                    tc_commit_by(leader, aempty + 8 * ((row0 + s) % strip::NV));
+                    if (++db == ND) { db = 0; dph ^= 1; }
+                    if (++pb == NP) { pb = 0; pph ^= 1; }
+                }
+                row0 += t.y1 - t.y0;
+                if (ok)
+                    for (int q = 0; q < 4; ++q) tc_commit_by(leader, aempty + 8 * ((row0 + q) % strip::NV));   // the last step's other rows
+                row0 += 4;
             }
-            row0 += t.y1 - t.y0;
-            if (ok)
-                for (int q = 0; q < 4; ++q) tc_commit_by(leader, aempty + 8 * ((row0 + q) % strip::NV));       // the last step's other rows
-            row0 += 4;
-        }
+        };
+        constexpr int HALF = G::CELLS / G::ISSUERS;
+        if (warp == MMA_WARP) run(std::integral_constant<int, 0>{}, std::integral_constant<int, HALF>{});
+        else if (G::ISSUERS == 2) run(std::integral_constant<int, HALF>{}, std::integral_constant<int, G::CELLS>{});
     } else if (warp >= SPLIT_WARP0 && warp < P_WARP0) {
         int vs = 0, vph = 0, as = 0, aph = 0;
         const unsigned line = ((warp & 3) * 32 + lane) * VROW;
