@@ -4,7 +4,7 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--dtype f32|bf16|f16] [--workload cfg2|cfg5a|cfg5b]
     python bench.py --impl reference ...      # the CPU path of the reference on the host cores
 
-A step is one fused SAPA-B forward (sim -> softmax -> atn, one kernel launch) over one batch of seeded
+A step is one fused SAPA-B forward (sim -> softmax -> atn, one kernel launch; float32 of this size: two) over one batch of seeded
 synthetic tensors.  Default workload ``cfg2``: B=8, C=256, 64x64 -> 128x128, d=64, K=5, s=2 per GPU
 (batch-sharded, weak scaling: every rank runs the same per-GPU batch, no collective on the data path).
 One pixel = one high-res output location across all C channels: Mpix = B*sH*sW / 1e6.
@@ -414,7 +414,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-extra", action="store_true", help="skip the additional (non-headline) measurements")
     ap.add_argument("--no-graph", action="store_true",
-                    help="launch every step from Python instead of replaying a CUDA graph of one launch per buffer set")
+                    help="launch every step from Python instead of replaying a CUDA graph of one step per buffer set")
     ap.add_argument("--only-path", default=None, choices=["backward", "deform"],
                     help="N = 1: run only the SAPA-B fused backward or the SAPA-D fused forward at the cfg2 shapes "
                          "(warm-up + --steps launches) and print a short JSON line; meant for profiler captures")
@@ -473,13 +473,13 @@ def main():
             def run_path():
                 sapa_b200._lib.call("sapa_fused_backward", device, g_out, t["q"], t["k"], t["v"], attn_b, gq, gk, gv, ws, nb,
                                     wl["B"], wl["d"], wl["C"], wl["H"], wl["W"], K, s, code)
-            launches = 3
+            launches = 4          # weights and aggregation of stage 1, two gathers
         else:
             off = (torch.randn(wl["B"], 4 * 9 * 2, s * wl["H"], s * wl["W"], device=device) * 0.5).to(dtype)
 
             def run_path():
                 sapa_b200.deform_sapa_fused(t["q"], t["k"], t["v"], off, 9, s, 4)
-            launches = 1
+            launches = 4          # similarity, window weights, aggregation, listed points
         for _ in range(max(3, args.warmup)):
             run_path()
         torch.cuda.synchronize()
@@ -511,12 +511,19 @@ def main():
             t["slab"].value.copy_(t["v"])
             del t["k"], t["v"]
 
+    # as the public call does: scratch of the size of the attention map where the kernels that go through it are the faster ones
+    # (a launch for the weights and one for the aggregation); the allocator hands a user's loop the same block every step
+    through_map = bool(sapa_b200._lib.lib().sapa_fused_forward_wants_map(wl["B"], wl["d"], wl["C"], wl["H"], wl["W"], K, s,
+                                                                         sapa_b200._lib.dtype_code(sets[0]["q"])))
+    map_scratch = torch.empty((wl["B"], K * K, s * wl["H"], s * wl["W"]), dtype=dtype, device=device) if through_map and not row_sharded else None
+    launches_per_step = 2 if through_map else 1
+
     def step(i):
         t = sets[i % nsets]
         if row_sharded:   # halo exchange (NCCL send/recv over NVLink) under the interior rows, then the border bands
             t["slab"].forward(t["q"], t["out"])
         else:
-            sapa_b200._lib.call("sapa_fused_forward", device, t["q"], t["k"], t["v"], t["out"], None, wl["B"], wl["d"],
+            sapa_b200._lib.call("sapa_fused_forward", device, t["q"], t["k"], t["v"], t["out"], map_scratch, wl["B"], wl["d"],
                                 wl["C"], wl["H"], wl["W"], K, s, sapa_b200._lib.dtype_code(t["q"]))
 
     def barrier():
@@ -524,7 +531,7 @@ def main():
             dist.barrier()
         torch.cuda.synchronize()
 
-    # The timed loop replays a CUDA graph that holds one launch per buffer set (the launches and their order are the
+    # The timed loop replays a CUDA graph that holds one step per buffer set (the launches and their order are the
     # same as in the eager loop; only the per-launch host work disappears).  Row-sharded steps contain an NCCL
     # exchange and stay eager; any failure to capture falls back to the eager loop.
     graph = None
@@ -607,10 +614,13 @@ def main():
                 t["out"] = torch.empty((wl["B"], wl["C"], s * wl["H"], s * wl["W"]), dtype=odt, device=device)
                 osets.append(t)
             code = sapa_b200._lib.dtype_code(osets[0]["q"])
+            omap = None
+            if sapa_b200._lib.lib().sapa_fused_forward_wants_map(wl["B"], wl["d"], wl["C"], wl["H"], wl["W"], K, s, code):
+                omap = torch.empty((wl["B"], K * K, s * wl["H"], s * wl["W"]), dtype=odt, device=device)
 
             def ostep(i):
                 t = osets[i % on]
-                sapa_b200._lib.call("sapa_fused_forward", device, t["q"], t["k"], t["v"], t["out"], None, wl["B"], wl["d"],
+                sapa_b200._lib.call("sapa_fused_forward", device, t["q"], t["k"], t["v"], t["out"], omap, wl["B"], wl["d"],
                                     wl["C"], wl["H"], wl["W"], K, s, code)
             osteps = max(3, min(args.steps, 300))
             for i in range(max(3, min(args.warmup, 20))):
@@ -626,7 +636,7 @@ def main():
             other[name] = {"value": pix_per_step_rank / (oms * 1e-3) / 1e6, "unit": "Mpix/s", "ms_per_step": oms, "steps": osteps,
                            "roofline_frac": obytes / (oms * 1e-3) / 1e9 / measured_peak()[0],
                            "algorithmic_bytes_per_launch": obytes}
-            del osets
+            del osets, omap
 
     # ---- the rest of the path at the same shapes: SAPA-B fused backward and SAPA-D fused forward (kernel time only) ----
     paths = {}
@@ -664,7 +674,7 @@ def main():
         # reads dOut, V, Q, K and the saved attention map; writes dV, dQ, dK
         bytes_b = (B_ * C_ * hi + B_ * C_ * H_ * W_ + B_ * d_ * hi + B_ * d_ * H_ * W_ + B_ * K * K * hi
                    + B_ * C_ * H_ * W_ + B_ * d_ * hi + B_ * d_ * H_ * W_) * esize
-        paths["sapa_b_fused_backward"] = {"ms": ms_b, "launches": 3, "algorithmic_bytes": bytes_b,
+        paths["sapa_b_fused_backward"] = {"ms": ms_b, "launches": 4, "algorithmic_bytes": bytes_b,
                                           "achieved_gbs": bytes_b / (ms_b * 1e-3) / 1e9, "roofline_frac": bytes_b / (ms_b * 1e-3) / 1e9 / peak_gbs,
                                           "mpix_per_s": pix_per_step_rank / (ms_b * 1e-3) / 1e6}
         del out_b, gq, gk, gv, ws
@@ -684,7 +694,7 @@ def main():
         off = (torch.randn(B_, G_ * P_ * 2, s * H_, s * W_, device=device) * 0.5).to(dtype)
         ms_d = time_path(lambda: sapa_b200.deform_sapa_fused(t["q"], t["k"], t["v"], off, P_, s, G_), 10)
         bytes_d = (B_ * d_ * hi + B_ * d_ * H_ * W_ + 2 * B_ * G_ * P_ * hi + B_ * C_ * H_ * W_ + B_ * C_ * hi) * esize
-        paths["sapa_d_fused_forward"] = {"ms": ms_d, "launches": 1, "algorithmic_bytes": bytes_d,
+        paths["sapa_d_fused_forward"] = {"ms": ms_d, "launches": 4, "algorithmic_bytes": bytes_d,
                                          "achieved_gbs": bytes_d / (ms_d * 1e-3) / 1e9, "roofline_frac": bytes_d / (ms_d * 1e-3) / 1e9 / peak_gbs,
                                          "mpix_per_s": pix_per_step_rank / (ms_d * 1e-3) / 1e6,
                                          "config": {"groups": G_, "points": P_, "offset_sigma": 0.5}}
@@ -847,14 +857,14 @@ def main():
             "data": "synthetic",
             "config": config_dict(args, w),
             "timing": {"l2": f"{nsets} rotating input/output sets ({nsets * bytes_per_launch / 1e6:.0f} MB) > 126 MB L2",
-                       "launch": (f"CUDA graph of {nsets} launches (one per buffer set), replayed" if graph is not None
+                       "launch": (f"CUDA graph of {nsets} steps (one per buffer set), replayed" if graph is not None
                                   else "one call per step from Python"),
                        "kernels_per_step": kernels_per_step},
             "clocks": clocks,
             "e2e": {"value": e2e_value, "unit": "Mpix/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "steps": e2e_steps, "how": "sapa_b200.sapa_fused on pinned host tensors, double-buffered "
                                                "H2D / kernel / D2H on three streams"},
-            "gpu_launches": args.steps,
+            "gpu_launches": launches_per_step * args.steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_source": f"of {peak_kind}",
                          "algorithmic_bytes_per_launch": bytes_per_launch,

@@ -17,7 +17,7 @@
 //     the two accumulators (with one for both it was what the kernel waited for: 32 x 64 x 64x64, bfloat16, 45 -> 32 us).
 // The kernels on tiles load (and split) a value fragment once per window row and group of pixels that it reaches; their fragment loads, splits
 // and mma.sync issue bound them.  What bounds this one: memory (8 x 256 x 64x64: float32 57 -> 38 us, 4.8 TB/s of reads and mostly writes;
-// bfloat16 32 -> 22, 4.1 TB/s), with few channels the MMAs and the epilogue, which work on 128 lanes (32 x 64 x 64x64: 79 -> 56, 44 -> 30).
+// bfloat16 32 -> 22, 4.1 TB/s), with few channels the MMAs and the epilogue, which work on 128 lanes (32 x 64 x 64x64: 79 -> 54, 44 -> 30).
 namespace strip {
 
 using namespace ummau;

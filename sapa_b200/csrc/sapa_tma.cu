@@ -1114,8 +1114,8 @@ template <typename T> static StripPlan strip_plan(int B, int C, int H, int W, in
 }
 // It serves rows of 16 bytes, but for small float32 problems and few channels in 16 bits.  A step takes about 0.75 us, whatever the channels, and
 // four to start; the kernels on tiles 3.7 (float32) and 1.5 us for a million products of cells and (channels + 99 or 136).  us, tiles -> this
-// one, float32 | bfloat16: 8 x 256 x 64x64 57 -> 38 | 32 -> 23; 32 x 64 x 64x64 79 -> 55 | 44 -> 32; 1 x 256 x 256x256 109 -> 77 | 59 -> 39;
-// 8 x 256 x 32x32 19 -> 14 | 17 -> 11; 16 x 64 x 32x32 14.8 -> 13.5 | 10.1 -> 9.6; 1 x 32 x 512x512 117 -> 93 | 64 -> 44; and where the line
+// one, float32 | bfloat16: 8 x 256 x 64x64 57 -> 38 | 32 -> 23; 32 x 64 x 64x64 79 -> 54 | 44 -> 32; 1 x 256 x 256x256 109 -> 77 | 59 -> 39;
+// 8 x 256 x 32x32 19 -> 14 | 17 -> 11; 16 x 64 x 32x32 14.8 -> 13.5 | 10.1 -> 9.6; 1 x 32 x 512x512 117 -> 92 | 64 -> 44; and where the line
 // leaves them with the tiles: 8 x 32 x 32x32 6.9, 9.7 here (bfloat16 8.9 -> 7.8); 4 x 128 x 32x32 8.7, 8.8 (9.7 -> 8.5); 32 x 16 x 64x64
 // bfloat16 35, 38 (float32 57 -> 52).
 template <typename T> static bool strip_pays(const StripPlan &p) {
