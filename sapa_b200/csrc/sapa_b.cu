@@ -541,7 +541,7 @@ static inline int grid_1d(long long total, int threads) {
 // tensor-core fused forward (sapa_mma.cu)
 bool fused_mma_supported(int W, int dtype);
 bool fused_tma_supported(int W, int dtype);
-bool fused_f32_on_strips(int B, int C, int H, int W);
+bool fused_f32_on_strips(int C, int W);
 int launch_fused_tma(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d, int C,
                      int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st);
 int launch_fused_mma(const void *q, const void *k, const void *v, void *out, void *attn, int B, int d, int C, int H, int W,
@@ -825,7 +825,7 @@ int sapa_fused_forward(const void *query, const void *key, const void *value, vo
 
 int sapa_fused_forward_wants_map(int B, int d, int C, int H, int W, int K, int s, int dtype) {
     if (B <= 0 || d <= 0 || C <= 0 || H <= 0 || W <= 0) return 0;
-    return K == 5 && s == 2 && dtype == SAPA_F32 && fused_f32_on_strips(B, C, H, W) ? 1 : 0;
+    return K == 5 && s == 2 && dtype == SAPA_F32 && fused_f32_on_strips(C, W) ? 1 : 0;
 }
 
 size_t sapa_fused_backward_workspace(int B, int H, int W, int K, int s, int dtype) {

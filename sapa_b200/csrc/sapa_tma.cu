@@ -1152,12 +1152,12 @@ static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, i
 
 // The forward on strips takes up to 64 query channels, rows of 16 columns and more (a strip of 32 is less than half full below that) and at
 // least 24 value channels.  A channel of a large image is a page of memory of its own, and this kernel touches all channels of a row where
-// the tiles touch 32 of eight rows: images of more than 100 M values stay with the tiles.  The line depends on nothing but the shape of one
-// image, so that an image's result does not depend on the batch it is in.  bfloat16, us, tiles -> strips: 64 x 256 x 128x128 824 -> 687,
+// the tiles touch 32 of eight rows: images of more than 100 M values stay with the tiles, counted as if they were square, so that
+// an image's result depends neither on the batch it is in nor on the slab of rows that a process has of it.  bfloat16, us, tiles -> strips: 64 x 256 x 128x128 824 -> 687,
 // 8 x 256 x 64x64 37.3 -> 29.5 (with the attention map 41.8 -> 31.6), 16 x 128 x 64x64 47.7 -> 30.5, 8 x 256 x 32x32 (32 query channels)
 // 18.0 -> 11.2, 2 x 512 x 8x64 11.4 -> 7.7, 1 x 32 x 16x16 6.1 -> 6.3, 4 x 256 x 512x512 826 -> 755, 1 x 128 x 768x768 324 -> 273; 8 columns:
 // 64 x 256 x 16x8 19.1, 24.8 here; large images: 1 x 512 x 512x512 350, 375 here, 1 x 256 x 1024x1024 849, 1050 here.
-static bool strip_fwd_pays(int C, int d, int H, int W) { return d <= sfwd::MAX_D && W >= 16 && C >= 24 && (double)C * H * W <= 1e8; }
+static bool strip_fwd_pays(int C, int d, int W) { return d <= sfwd::MAX_D && W >= 16 && C >= 24 && (double)C * W * W <= 1e8; }
 
 template <typename T>
 static int launch_strip_fwd(const void *q, const void *k, const void *v, void *out, void *attn, int d, StripPlan p, int sms, const char *name, cudaStream_t st) {
@@ -1278,19 +1278,27 @@ namespace tma { static bool strips_filled(int W) { return 4 * W >= 3 * ceil_div(
 static bool strip_sim_pays(int B, int H, int W) {
     return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && (long long)B * H * W >= 12000;
 }
-// The forward and stage 1 of the backward as two launches, logits and what follows them per pixel, then the aggregation, from a million values
-// on (forward with its map | stage 1: 8 x 256 x 64x64 78.6 -> 53.2 | 91.4 -> 65.8; 16 x 128 x 64x64 103 -> 66 | 120 -> 80; 8 x 64 x 64x64
-// 41 -> 37 | 47 -> 38; 8 x 256 x 32x32 23.1 -> 20.9; 8 x 512 x 16x16 15.6 -> 15.3; 4 x 128 x 32x32 11.6, 14.2 here; 64 x 32 x 32x32 46.0, 47.5
-// here).
-bool fused_f32_on_strips(int B, int C, int H, int W) {
-    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)B * H * W * C >= 1e6;
+// The forward as two launches, softmax of the logits and aggregation.  An image's result depends neither on the batch it is in nor on the slab of
+// rows that a process has of it, so the line sees channels and columns alone and lies where a single square image is no slower (us, tiles ->
+// strips: 1 x 256 x 64x64 15.6 -> 14.2; 1 x 48 x 128x128 18.3 -> 17.8; 1 x 128 x 64x64 12.2, 12.7 here; 1 x 64 x 96x96 10.5, 14.4; 1 x 256 x
+// 32x32 10.5, 11.0), although larger batches of smaller images would gain too (16 x 128 x 32x32 29.5, 21.3 here; 8 x 256 x 32x32 23.1, 18.7).
+// 8 x 256 x 64x64 78.6 -> 55.3, 16 x 128 x 64x64 103 -> 66, 4 x 128 x 64x64 29.6 -> 21.5.
+bool fused_f32_on_strips(int C, int W) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)W * W * C >= (C >= 96 ? 5e5 : 7.5e5);
+}
+// Stage 1 of the backward likewise, softmax backward of the logits and aggregation, from two million values on, counted as if the images were
+// square: a slab's query gradient equals the rows of the image's (us, tiles -> strips: 8 x 256 x 64x64 91.4 -> 62; 16 x 128 x 64x64 120 -> 80;
+// 8 x 64 x 64x64 47 -> 38).
+static bool bwd_f32_on_strips(int B, int C, int W) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)B * W * W * C >= 2e6;
 }
 
 // 16 bits: the similarity always runs on strips (us, tiles -> strips, bfloat16: 8 images, 64 channels, 64x64 15.0 -> 11.0; 1 x 32 x 16x16 6.2 ->
 // 4.3; 64 x 32 x 8x8 7.0 -> 5.4); stage 1 of the backward as two launches, logits and softmax backward, then the aggregation, with 128 value
-// channels or a million values and rows of 16 columns and more.  The whole backward, us: 8 x 256 x 64x64 85.5 -> 75.8, 16 x 128 x 64x64
-// 116 -> 91, 64 x 32 x 32x32 81 -> 69, 2 x 256 x 24x40 28.7 -> 25.9; 4 x 64 x 48x48 28.6, 30.4 on strips; 64 x 64 x 8x8 22.6, 24.5.
-static bool strip_bwd_16_pays(int B, int C, int H, int W) { return W >= 16 && (C >= 128 || (double)B * H * W * C >= 1e6); }
+// channels or two million values (of square images, as above) and rows of 16 columns and more.  The whole backward, us: 8 x 256 x 64x64
+// 85.5 -> 75.8, 16 x 128 x 64x64 116 -> 91, 64 x 32 x 32x32 81 -> 69, 2 x 256 x 24x40 28.7 -> 25.9; 4 x 64 x 48x48 28.6, 30.4 on strips;
+// 64 x 64 x 8x8 22.6, 24.5.
+static bool strip_bwd_16_pays(int B, int C, int W) { return W >= 16 && (C >= 128 || (double)B * W * W * C >= 2e6); }
 
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
 // mode 0 (forward): out = atn(softmax(sim(q, k)), v), attn = optional output.
@@ -1334,8 +1342,8 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         const int e = dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
         if (e != -1000) return e;
     }
-    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(B, H, W) : mode == MODE_FWD ? attn != nullptr && fused_f32_on_strips(B, C, H, W)
-                                                                          : mode == MODE_BWD && fused_f32_on_strips(B, d, H, W))) {
+    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(B, H, W) : mode == MODE_FWD ? attn != nullptr && fused_f32_on_strips(C, W)
+                                                                          : mode == MODE_BWD && bwd_f32_on_strips(B, d, W))) {
         static const char *const names[3] = {"sapa_tma_fused_f32_kernel<fwd>", "sapa_tma_fused_f32_kernel<bwd>", "sapa_tma_fused_f32_kernel<sim>"};
         const char *name = names[mode];
         void *slots = mode == MODE_BWD ? ws : attn;
@@ -1348,7 +1356,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         if ((e = device_sms(name, sms)) != SAPA_OK) return e;
         return launch_strip<float>(v, slots, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
     }
-    if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(B, d, H, W)))) {
+    if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(B, d, W)))) {
         const char *name = mode == MODE_SIM ? (wide ? "sapa_wide_16_kernel<sim>" : "sapa_tma_fused_16_kernel<sim>") : wide ? "sapa_wide_16_kernel<bwd>" : "sapa_tma_fused_16_kernel<bwd>";
         int sms = 0;
         if (int e = device_sms(name, sms)) return e;
@@ -1362,7 +1370,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         };
         return dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
     }
-    if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, H, W)) {
+    if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, W)) {
         const char *name = wide ? "sapa_wide_16_kernel<fwd>" : "sapa_tma_fused_16_kernel<fwd>";
         int sms = 0;
         if (int e = device_sms(name, sms)) return e;

@@ -7,9 +7,9 @@ import torch.nn.functional as F
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
-# images, value channels, query channels, rows, columns: stages of channels that end early, odd rows, partial strips, many units a CTA.  A
-# million values and more, 12 000 pixels and more
-SHAPES = [(2, 300, 64, 47, 44), (9, 48, 5, 51, 60), (3, 130, 33, 71, 52), (40, 80, 16, 33, 12), (1, 520, 100, 130, 16)]
+# images, value channels, query channels, rows, columns: stages of channels that end early, odd rows, partial strips, many units a CTA.  Two
+# million values and more, half a million an image (of square images)
+SHAPES = [(4, 300, 64, 47, 44), (3, 48, 5, 51, 128), (3, 130, 33, 71, 76), (4, 720, 16, 33, 28), (4, 520, 100, 130, 32)]
 
 
 def _rand(seed, *shape, scale=1.0):
@@ -56,7 +56,7 @@ def test_strips_vs_float64(shape):
 def test_bands_of_a_slab_equal_the_whole_image():
     from sapa_b200 import sharding
     from sapa_b200.functions import fused_forward_raw
-    B, d, C, H, W, r = 2, 40, 300, 60, 48, 2
+    B, d, C, H, W, r = 2, 40, 300, 60, 64, 2
     q, k, v = _rand(1, B, d, 2 * H, 2 * W, scale=0.5), _rand(2, B, d, H, W, scale=0.5), _rand(3, B, C, H, W)
     whole = fused_forward_raw(q, k, v, 5, 2, False)[0]
     lo, rows = 11, 40
@@ -68,3 +68,32 @@ def test_bands_of_a_slab_equal_the_whole_image():
     for begin, end in ((0, 4), (4, rows - 3), (rows - 3, rows)):
         slab._launch(ql, out, begin, end)
     assert torch.equal(out, whole[:, :, hi])
+
+
+@pytest.mark.parametrize("shape", [(1, 64, 250, 96, 96), (2, 16, 64, 40, 96), (2, 16, 140, 40, 96)], ids=lambda s: "B%d_d%d_C%d_%dx%d" % s)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_slab_goes_the_way_of_its_image(shape, dtype):
+    """The output and the query gradient of a few rows equal those of the whole image bit for bit, also where the rows alone are a small
+    problem, and the output of an image by itself that in its batch."""
+    import sapa_b200 as sp
+    from sapa_b200 import sharding
+    B, d, C, H, W = shape
+    q, k, v = (x.to(dtype) for x in (_rand(1, B, d, 2 * H, 2 * W, scale=0.5), _rand(2, B, d, H, W, scale=0.5), _rand(3, B, C, H, W)))
+    go = _rand(4, B, C, 2 * H, 2 * W).to(dtype)
+    t = [x.clone().requires_grad_() for x in (q, k, v)]
+    whole = sp.sapa_fused(*t, 5, 2)
+    gq = torch.autograd.grad(whole, t, go)[0]
+    assert torch.equal(sp.sapa_fused(*(x[-1:] for x in (q, k, v)), 5, 2)[0], whole.detach()[-1])
+    r, rows = 2, 8
+    for lo in (2, 13):
+        hi = slice(2 * lo, 2 * (lo + rows))
+        slab = sharding.RowSlab(B, d, C, rows, W, dtype, torch.device(DEV), 5, 2)
+        slab.key_padded.copy_(k[:, :, lo - r:lo + rows + r])
+        slab.value_padded.copy_(v[:, :, lo - r:lo + rows + r])
+        ql, out = q[:, :, hi].contiguous(), torch.empty(B, C, 2 * rows, 2 * W, dtype=dtype, device=DEV)
+        slab._launch(ql, out, 0, rows)
+        assert torch.equal(out, whole.detach()[:, :, hi])
+        slab.attn = torch.empty(B, 25, 2 * rows, 2 * W, dtype=dtype, device=DEV)
+        slab._launch(ql, out, 0, rows)
+        assert torch.equal(out, whole.detach()[:, :, hi])
+        assert torch.equal(slab.backward(go[:, :, hi].contiguous(), ql)[0], gq[:, :, hi])

@@ -39,7 +39,7 @@ def test_similarity(shape, dtype, tol):
 
 # the attention map, the logit gradients and the result are rounded: 2.8e-3 and 3.6e-4 measured, as on the tiles
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 4e-3), (torch.float16, 5e-4)])
-@pytest.mark.parametrize("shape", [(1, 128, 20, 9, 16), (2, 150, 32, 33, 40), (5, 300, 64, 21, 72), (24, 48, 7, 30, 32)], ids=lambda s: "B%d_C%d_d%d_%dx%d" % s)
+@pytest.mark.parametrize("shape", [(1, 128, 20, 9, 16), (2, 150, 32, 33, 40), (5, 300, 64, 21, 72), (48, 48, 7, 30, 32)], ids=lambda s: "B%d_C%d_d%d_%dx%d" % s)
 def test_backward(shape, dtype, tol):
     import sapa_b200 as sp
     from sapa_b200 import _lib
