@@ -1,6 +1,7 @@
 // sapa_tma.cu — SAPA-B for K = 5, s = 2 with TMA staging and the contractions on the tensor cores: one float32 kernel
-// and one float16 / bfloat16 kernel, each in four modes (fused forward, stage 1 of the fused backward, logits only,
-// aggregation only).
+// and one float16 / bfloat16 kernel on tiles, each in four modes (fused forward, stage 1 of the fused backward, logits only,
+// aggregation only), and the choice between them and the kernels on strips of columns (tcgen05, sapa_strip*.cuh), which take the larger
+// problems with rows of 16 bytes.
 //
 // Same mathematics as sapa_mma.cu (probabilities kept in registers between the logit MMAs and the aggregation
 // MMAs), but the key / query / value tiles are brought into shared memory by the tensor memory accelerator instead
