@@ -19,7 +19,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libsapa_b200.so")
 SOURCES = ["api.cu", "sapa_b.cu", "sapa_mma.cu", "sapa_tma.cu", "sapa_gath_mma.cu", "sapa_d.cu", "sapa_proj.cu", "sapa_proj_mm.cu",
            "sapa_nhwc.cu"]
-HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "tma_util.cuh"), os.path.join(CSRC, "umma_util.cuh"), os.path.join(CSRC, "sapa_gath_umma.cuh"), os.path.join(CSRC, "sapa_strip.cuh"), os.path.join(CSRC, "sapa_strip_fwd.cuh"), os.path.join(CSRC, "sapa_strip_sim.cuh"), os.path.join(CSRC, "sapa_strip_sim16.cuh"), os.path.join(CSRC, "proj_mm.h"), os.path.join(CSRC, "sapa_wide16.cuh"), os.path.join(CSRC, "sapa_gath_wide16.cuh"),
+HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "tma_util.cuh"), os.path.join(CSRC, "umma_util.cuh"), os.path.join(CSRC, "finite.cuh"), os.path.join(CSRC, "sapa_gath_umma.cuh"), os.path.join(CSRC, "sapa_strip.cuh"), os.path.join(CSRC, "sapa_strip_fwd.cuh"), os.path.join(CSRC, "sapa_strip_sim.cuh"), os.path.join(CSRC, "sapa_strip_sim16.cuh"), os.path.join(CSRC, "proj_mm.h"), os.path.join(CSRC, "sapa_wide16.cuh"), os.path.join(CSRC, "sapa_gath_wide16.cuh"),
            os.path.join(INCLUDE, "sapa_b200.h")]
 
 HOST = os.path.join(HERE, "_host.so")

@@ -21,6 +21,7 @@
 //     every wait is bounded and raises g_wait_timeout instead of spinning for ever.
 // Larger problems with rows of 16 bytes go to the tcgen05 kernel of sapa_gath_umma.cuh instead (umma_pays), recorded under the name of
 // the form that it stands for.
+#include "finite.cuh"
 #include "umma_util.cuh"
 
 #include <algorithm>
@@ -91,7 +92,7 @@ __device__ __forceinline__ float cell_sum(const Args &a, int n, int c, int y, in
     const size_t hi_plane = (size_t)(2 * a.H) * sW;
     float s = 0.f;
 #pragma unroll 1
-    for (int cell = 0; cell < 25; ++cell) {       // window cell of the parent that reaches (y, x) through it
+    for (int cell = 0; cell < 25 && s == s; ++cell) {       // window cell of the parent that reaches (y, x) through it; a NaN ends the sum
         const int yp = y - a.top + 2 - cell / 5, xp = x + 2 - cell % 5;
         if (yp < 0 || yp >= a.H || xp < 0 || xp >= a.W) continue;
         const size_t at = (size_t)(2 * yp) * sW + 2 * xp;

@@ -80,15 +80,60 @@ template <typename T> __device__ __forceinline__ Item item_at(const UArgs &u, in
 __device__ __forceinline__ int first_parent(const UArgs &u, const Item &t) { return max(t.y0 - u.g.top - 2, 0); }
 __device__ __forceinline__ int end_parent(const UArgs &u, const Item &t) { return min(t.y1 - u.g.top + 2, u.g.H); }
 
-template <typename T> __device__ __noinline__ float cell_alone(const Args &a, int n, int c, int y, int x) { return cell_sum<T>(a, n, c, y, x); }
+// Parents of strip columns x0 - P0 and so on that hold something not finite in high-res row h of channel c
+template <typename T> __device__ __forceinline__ finite::Marks marks_of(const Args &a, int n, int c, int h, int x0) {
+    finite::Marks m{0ull, 0ull, 0ull};
+    finite::mark_row<T, XCHUNKS, true>(static_cast<const T *>(a.hi) + (((size_t)n * a.C + c) * (2 * a.H) + h) * (2 * a.W), 2 * a.W, 2 * (x0 - Geo<T>::P0), m);
+    return m;
+}
+// The cells of a strip's output row and channel again whose sums are not finite (sums: there may be such), or that high-res rows ha .. hb - 1 reach with something not finite, which
+// the product took as zero: over their own pixels alone.
+template <typename T> __device__ __noinline__ void finish_cells(const UArgs &u, int n, int c, int y, int x0, int ha, int hb, bool sums) {
+    using G = Geo<T>;
+    const Args &a = u.g;
+    auto reached = [](unsigned long long parents) {                   // bits of cells of the strip
+        const unsigned long long m = parents >> (G::P0 - 2);
+        return (unsigned)((m | m >> 1 | m >> 2 | m >> 3 | m >> 4) & ((1ull << G::CELLS) - 1));
+    };
+    constexpr unsigned ALL = (unsigned)((1ull << G::CELLS) - 1);
+    unsigned nan = 0u, any = 0u;                                      // cells that a NaN, that something not finite reaches
+#pragma unroll 1
+    for (int h = ha; h < hb && nan != ALL; ++h) {
+        const finite::Marks m = marks_of<T>(a, n, c, h, x0);
+        nan |= reached(m.nan); any |= reached(m.any());
+    }
+    T *const o = static_cast<T *>(a.out) + (((size_t)n * a.C + c) * a.Hout + y) * a.W + x0;
+    constexpr int PER = 16 / (int)sizeof(T);
+    constexpr unsigned CHUNK = (1u << PER) - 1;
+#pragma unroll 1
+    for (int q0 = 0; q0 < G::CELLS && x0 + q0 < a.W; q0 += PER) {
+        if (!sums && (any >> q0 & CHUNK) == 0u) continue;
+        if ((nan >> q0 & CHUNK) == CHUNK) {
+            *reinterpret_cast<uint4 *>(o + q0) = finite::nan_chunk<T>();
+            continue;
+        }
+        const int yp = y - a.top;
+        if (yp >= 0 && yp < a.H) {                                    // weights of NaN of the cells' own parents
+            const T *w = static_cast<const T *>(a.wt) + (((size_t)n * 25 + 12) * (2 * a.H) + 2 * yp) * (2 * a.W) + 2 * (x0 + q0);
+            if (finite::all_nan<T>(*reinterpret_cast<const uint4 *>(w)) && finite::all_nan<T>(*reinterpret_cast<const uint4 *>(w + PER))) {
+                *reinterpret_cast<uint4 *>(o + q0) = finite::nan_chunk<T>();
+                continue;
+            }
+        }
+#pragma unroll 1
+        for (int q = q0; q < q0 + PER; ++q)
+            if ((any >> q & 1) != 0u || !isfinite(to_acc(o[q]))) o[q] = from_acc<T>(nan >> q & 1 ? finite::nan_value() : cell_sum<T>(a, n, c, y, x0 + q));
+    }
+}
 
 template <typename T>
-__global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap lmap, const UArgs u) {
+__global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap lmap, const __grid_constant__ UArgs u) {
     using G = Geo<T>;
     const Args &a = u.g;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) unsigned long long bars[2 * MAX_NX + 2 * NWB + 2 * G::NA + 2 * G::SLOTS];
     __shared__ unsigned tmem_slot;
+    __shared__ finite::Noted noted;                                   // steps, counted over the CTA's items
     const unsigned ring = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u, wbuf = ring + RING_BYTES;
     const unsigned xfull = (unsigned)__cvta_generic_to_shared(bars), xempty = xfull + 8 * MAX_NX;
     const unsigned wready = xempty + 8 * MAX_NX, wempty = wready + 8 * NWB, aready = wempty + 8 * NWB, aempty = aready + 8 * G::NA;
@@ -96,6 +141,7 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
     const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
     const int items = a.B * u.cblocks * u.segs * u.strips;
 
+    if (tid < 4) noted.clear(tid);
     if (tid == 0) {
         for (int i = 0; i < u.nx; ++i) { mbar_init(xfull + 8 * i, 1); mbar_init(xempty + 8 * i, 256); }
         for (int i = 0; i < NWB; ++i) { mbar_init(wready + 8 * i, 128); mbar_init(wempty + 8 * i, 1); }
@@ -210,7 +256,16 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
                     tc_fence_after();
                     if (t.c0 + (warp & 3) * 32 < a.C) {
                         const unsigned at = tmem + quarter + G::DCOLS + ab * G::ABUF;
-                        tc_st16(at, v); tc_st16(at + 16, v + 16); tc_st8(at + 32, v + 32);      // the tensor core reads the top 19 bits of a tf32 operand
+                        auto store = [&]() { tc_st16(at, v); tc_st16(at + 16, v + 16); tc_st8(at + 32, v + 32); };      // the tensor core reads the top 19 bits of a tf32 operand
+                        store();
+                        const bool odd = !finite::all_finite<T, ACOLS>(v);
+                        if (__any_sync(0xffffffffu, odd)) {
+                            tc_wait_st();
+#pragma unroll
+                            for (int q = 0; q < ACOLS; ++q) v[q] = finite::or_zero<T>(v[q]);
+                            store();
+                            if (odd && t.c0 + (warp & 3) * 32 + lane < a.C) noted.note(warp & 3, step);
+                        }
                         if constexpr (G::F32) {
 #pragma unroll
                             for (int q = 0; q < ACOLS; ++q) v[q] = tf32_lo(v[q]);
@@ -272,10 +327,10 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
             }
         }
     } else {
-        int cr = 0;
+        int cr = 0, step0 = 0;                                        // step0: steps of this CTA before the item
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             const Item t = item_at<T>(u, i);
-            const int c = t.c0 + (warp & 3) * 32 + lane;
+            const int c = t.c0 + (warp & 3) * 32 + lane, h0 = 2 * first_parent(u, t), h1 = 2 * end_parent(u, t);
             for (int y = t.y0; y < t.y1; ++y, ++cr) {
                 const int s = cr % G::SLOTS;
                 if (!mbar_wait_warp(dfull + 8 * s, (cr / G::SLOTS) & 1)) { ok = false; break; }
@@ -303,9 +358,10 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
                 tc_fence_before();
                 mbar_arrive(dempty + 8 * s);
                 T *o = static_cast<T *>(a.out) + (((size_t)t.n * a.C + c) * a.Hout + y) * a.W + t.x0;
-                unsigned odd = 0u;                                    // cells with a sum that is not finite
+                float zero[4] = {0.f, 0.f, 0.f, 0.f};                 // stays zero while all sums are finite
 #pragma unroll
-                for (int q = 0; q < G::CELLS; ++q) odd |= (v[q] & 0x7f800000u) == 0x7f800000u ? 1u << q : 0u;
+                for (int q = 0; q < G::CELLS; ++q) zero[q & 3] = fmaf(__uint_as_float(v[q]), 0.f, zero[q & 3]);
+                if (!((zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.f) && c < a.C) noted.note_sum(warp & 3, step0 + min(max(2 * (y - a.top), h0), h1 - 1) - h0);
                 constexpr int PER = 16 / (int)sizeof(T);
 #pragma unroll
                 for (int q = 0; q < G::CELLS; q += PER)
@@ -321,14 +377,9 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
                         }
                         *reinterpret_cast<uint4 *>(o + q) = w;
                     }
-                // a product with zero weights took in what lies outside a cell's window: such cells again, over their own pixels alone
-                while (c < a.C && odd != 0u) {
-                    const int q = __ffs(odd) - 1;
-                    odd &= odd - 1;
-                    if (t.x0 + q < a.W) o[q] = from_acc<T>(cell_alone<T>(a, t.n, c, y, t.x0 + q));
-                }
                 __syncwarp();
             }
+            step0 += h1 - h0;
         }
     }
     if (!ok) atomicExch(&g_wait_timeout, 1);
@@ -336,6 +387,21 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
     __syncthreads();
     tc_fence_after();
     if (warp == MMA_WARP) tc_dealloc(tmem, TMEM_COLS);
+    if (warp < 8 && noted.last[warp & 3] >= 0) {                      // rare: outputs with something not finite (all are stored)
+        int step0 = 0;
+        for (int i = blockIdx.x; i < items; i += gridDim.x) {
+            const Item t = item_at<T>(u, i);
+            const int c = t.c0 + (warp & 3) * 32 + lane, h0 = 2 * first_parent(u, t), h1 = 2 * end_parent(u, t);
+            for (int y = t.y0; y < t.y1; ++y) {
+                // the high-res rows that reach this one and may be noted
+                const int ha = max(2 * (y - a.top - 2), h0), hb = min(2 * (y - a.top + 3), h1);
+                const int first = noted.first[warp & 3] - step0 + h0, last = noted.last[warp & 3] - step0 + h0;
+                if ((y & 1) == warp >> 2 && c < a.C && hb > first && ha <= last)
+                    finish_cells<T>(u, t.n, c, y, t.x0, max(ha, first), min(hb, last + 1), noted.sums[warp & 3] != 0);
+            }
+            step0 += h1 - h0;
+        }
+    }
 }
 
 }  // namespace gumma

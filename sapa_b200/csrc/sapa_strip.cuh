@@ -59,7 +59,7 @@ template <typename T> struct Geo {
 };
 
 struct SArgs {
-    const void *v, *wt;    // for outputs that are not finite
+    const void *v, *wt;    // for outputs with something not finite in their windows
     void *out;
     int B, C, H, W, rows, ytop0, y_begin, y_end;
     int strips, cblocks, segs, seg_rows;
@@ -76,29 +76,121 @@ template <typename T> __device__ __forceinline__ Item item_at(const SArgs &a, in
     return t;
 }
 
-// one output over the cells of its own window alone
+// One output over the cells of its own window alone; a NaN ends the sum.
 template <typename T> __device__ __noinline__ float pixel_alone(const SArgs &a, int n, int c, int hy, int hx) {
     const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W);
     const T *w = static_cast<const T *>(a.wt) + (size_t)n * 25 * hi_plane + (size_t)hy * (2 * a.W) + hx;
     const T *v = static_cast<const T *>(a.v) + ((size_t)n * a.C + c) * a.rows * a.W;
     float s = 0.f;
 #pragma unroll 1
-    for (int k = 0; k < 25; ++k) {
+    for (int k = 0; k < 25 && s == s; ++k) {
         const int y = a.ytop0 + (hy >> 1) + k / 5 - 2, x = (hx >> 1) + k % 5 - 2;
-        if (y >= 0 && y < a.rows && x >= 0 && x < a.W) s = fmaf(to_acc(w[k * hi_plane]), to_acc(v[(size_t)y * a.W + x]), s);
+        if (y < 0 || y >= a.rows || x < 0 || x >= a.W) continue;
+        const float wk = to_acc(w[k * hi_plane]);
+        s = wk == wk ? fmaf(wk, to_acc(v[(size_t)y * a.W + x]), s) : wk;
     }
     return s;
+}
+// Moves the cells of a product from a landed row, float32 in two terms; elements that are not finite become zeros and the row is noted.
+template <typename T> __device__ __forceinline__ void move_cells(unsigned at, unsigned (&v)[4 * VCHUNKS], bool channel, finite::Noted &noted, int quarter, int row) {
+    using G = Geo<T>;
+    auto store = [&]() {
+        tc_st16(at, v + G::SHIFT); tc_st8(at + 16, v + G::SHIFT + 16);          // the tensor core reads the top 19 bits of a tf32 operand
+    };
+    store();
+    const bool odd = !finite::all_finite<T, ACOLS>(v + G::SHIFT);
+    if (__any_sync(0xffffffffu, odd)) {
+        tc_wait_st();
+#pragma unroll
+        for (int q = G::SHIFT; q < G::SHIFT + ACOLS; ++q) v[q] = finite::or_zero<T>(v[q]);
+        store();
+        if (odd && channel) noted.note(quarter, row);                           // a lane without a channel holds anything
+    }
+    if constexpr (G::F32) {
+#pragma unroll
+        for (int q = G::SHIFT; q < G::SHIFT + ACOLS; ++q) v[q] = tf32_lo(v[q]);
+        tc_st16(at + ACOLS, v + G::SHIFT); tc_st8(at + ACOLS + 16, v + G::SHIFT + 16);
+    }
+}
+// Columns x0 - BOX0 and so on of value row dy of the step of low-res row y
+template <typename T> __device__ __forceinline__ finite::Marks marks_of(const SArgs &a, int n, int c, int y, int dy, int x0) {
+    finite::Marks m{0ull, 0ull, 0ull};
+    const int row = a.ytop0 + y + dy - 2;
+    if (row >= 0 && row < a.rows)
+        finite::mark_row<T, (Geo<T>::CELLS + 2 * Geo<T>::BOX0) * (int)sizeof(T) / 16, false>(
+            static_cast<const T *>(a.v) + (((size_t)n * a.C + c) * a.rows + row) * a.W, a.W, x0 - Geo<T>::BOX0, m);
+    return m;
+}
+// Bits of parents (of the strip) whose windows hold a marked column
+template <typename T> __device__ __forceinline__ unsigned long long reached(unsigned long long columns) {
+    const unsigned long long m = columns >> (Geo<T>::BOX0 - 2);
+    return (m | m >> 1 | m >> 2 | m >> 3 | m >> 4) & ((1ull << Geo<T>::CELLS) - 1);
+}
+// The pixels of a step and channel again, once they are stored, whose sums are not finite (sums: there may be such), or that have something not finite in
+// their windows, which the product took as zero.  dy0, dy1: the window rows that may hold such elements.
+template <typename T> __device__ __noinline__ void finish_pixels(const SArgs &a, int n, int c, int y, int x0, int dy0, int dy1, bool sums) {
+    using G = Geo<T>;
+    constexpr int FIRST = G::BOX0 - 2, PER = 16 / (int)sizeof(T);     // bit of a parent's first column; elements of 16 bytes
+    constexpr unsigned long long ALL = (1ull << G::CELLS) - 1;
+    unsigned long long nan = 0ull, up[5], down[5], any = 0ull;        // nan, any: parents with such an element in their windows
+#pragma unroll 1
+    for (int dy = 0; dy < 5; ++dy) {
+        finite::Marks m{0ull, 0ull, 0ull};
+        if (dy >= dy0 && dy <= dy1 && nan != ALL) m = marks_of<T>(a, n, c, y, dy, x0);
+        nan |= reached<T>(m.nan); any |= reached<T>(m.any());
+        up[dy] = m.up; down[dy] = m.down;
+    }
+    const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W);
+#pragma unroll 1
+    for (int q = 0; q < 2 * G::PX / PER; ++q) {                       // chunks of 16 bytes of the two rows
+        const int r = q / (G::PX / PER), px0 = q % (G::PX / PER) * PER;
+        constexpr unsigned long long PARENTS = (1ull << PER / 2) - 1;
+        if (x0 + px0 / 2 >= a.W || (!sums && (any >> px0 / 2 & PARENTS) == 0ull)) continue;
+        const size_t at = (size_t)(2 * y + r) * (2 * a.W) + 2 * x0 + px0;
+        T *const o = static_cast<T *>(a.out) + ((size_t)n * a.C + c) * hi_plane + at;
+        if ((nan >> px0 / 2 & PARENTS) == PARENTS) {
+            *reinterpret_cast<uint4 *>(o) = finite::nan_chunk<T>();
+            continue;
+        }
+        const T *const wt = static_cast<const T *>(a.wt) + (size_t)n * 25 * hi_plane + at;
+        const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(o));   // stored by TMA: not from L1
+        const unsigned words[4] = {w.x, w.y, w.z, w.w};
+        if (!finite::all_finite<T, 4>(words) && finite::all_nan<T>(*reinterpret_cast<const uint4 *>(wt + 12 * hi_plane))) {
+            *reinterpret_cast<uint4 *>(o) = finite::nan_chunk<T>();   // weights of NaN for the pixels' own cells
+            continue;
+        }
+        float s[PER];                                                 // what the infinities alone come to
+#pragma unroll
+        for (int e = 0; e < PER; ++e) s[e] = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < 25; ++k) {
+            const unsigned u = (unsigned)(up[k / 5] >> (FIRST + px0 / 2 + k % 5)), d = (unsigned)(down[k / 5] >> (FIRST + px0 / 2 + k % 5));
+            if (((u | d) & (unsigned)PARENTS) == 0u) continue;
+            const uint4 wk = *reinterpret_cast<const uint4 *>(wt + k * hi_plane);
+#pragma unroll
+            for (int e = 0; e < PER; ++e)
+                if ((u | d) >> (e / 2) & 1) s[e] = fmaf(finite::element<T>(wk, e), u >> (e / 2) & 1 ? INFINITY : -INFINITY, s[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int p = px0 / 2 + e / 2;
+            if (!finite::is_finite<T>(words, e)) s[e] = pixel_alone<T>(a, n, c, 2 * y + r, 2 * x0 + px0 + e);
+            else if ((any >> p & 1) == 0ull) continue;
+            o[e] = from_acc<T>((nan >> p & 1) != 0ull ? finite::nan_value() : s[e]);
+        }
+    }
 }
 }  // namespace strip
 
 template <typename T>
 __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap wmap,
-                                                                  const __grid_constant__ CUtensorMap omap, const strip::SArgs a) {
+                                                                  const __grid_constant__ CUtensorMap omap, const __grid_constant__ strip::SArgs a) {
     using namespace strip;
     using G = strip::Geo<T>;
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) unsigned long long bars[2 * (NVL + NWL + strip::NV + ND + NP)];
     __shared__ unsigned tmem_slot;
+    __shared__ finite::Noted noted;                                   // rows of V, counted over the CTA's items
     const unsigned base = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u;
     const unsigned vfull = (unsigned)__cvta_generic_to_shared(bars), vempty = vfull + 8 * NVL, wfull = vempty + 8 * NVL, wempty = wfull + 8 * NWL;
     const unsigned aready = wempty + 8 * NWL, aempty = aready + 8 * strip::NV, dfull = aempty + 8 * strip::NV, dempty = dfull + 8 * ND;
@@ -106,6 +198,7 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
     const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
     const int items = a.B * a.cblocks * a.segs * a.strips;
 
+    if (tid < 4) noted.clear(tid);
     if (tid == 0) {
         for (int i = 0; i < NVL; ++i) { mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 128); }
         for (int i = 0; i < NWL; ++i) { mbar_init(wfull + 8 * i, 1); mbar_init(wempty + 8 * i, 32 * P_WARPS); }
@@ -212,12 +305,12 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
         if (warp == MMA_WARP) run(std::integral_constant<int, 0>{}, std::integral_constant<int, HALF>{});
         else if (G::ISSUERS == 2) run(std::integral_constant<int, HALF>{}, std::integral_constant<int, G::CELLS>{});
     } else if (warp >= SPLIT_WARP0 && warp < P_WARP0) {
-        int vs = 0, vph = 0, as = 0, aph = 0;
+        int vs = 0, vph = 0, as = 0, aph = 0, row = 0;
         const unsigned line = ((warp & 3) * 32 + lane) * VROW;
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             const Item t = item_at<T>(a, i);
             const bool used = t.c0 + (warp & 3) * 32 < a.C;           // lanes without a channel keep whatever they hold
-            for (int y = t.y0 - 2; y < t.y1 + 2; ++y) {
+            for (int y = t.y0 - 2; y < t.y1 + 2; ++y, ++row) {
                 if (!mbar_wait_warp(vfull + 8 * vs, vph)) { ok = false; break; }
                 unsigned v[4 * VCHUNKS];
                 if (used) {
@@ -228,15 +321,7 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                 }
                 if (!mbar_wait_warp(aempty + 8 * as, aph ^ 1)) { ok = false; break; }
                 tc_fence_after();
-                if (used) {
-                    const unsigned at = tmem + quarter + ring + as * G::ABUF;
-                    tc_st16(at, v + G::SHIFT); tc_st8(at + 16, v + G::SHIFT + 16);          // the tensor core reads the top 19 bits of a tf32 operand
-                    if constexpr (G::F32) {
-#pragma unroll
-                        for (int q = G::SHIFT; q < G::SHIFT + ACOLS; ++q) v[q] = tf32_lo(v[q]);
-                        tc_st16(at + ACOLS, v + G::SHIFT); tc_st8(at + ACOLS + 16, v + G::SHIFT + 16);
-                    }
-                }
+                if (used) move_cells<T>(tmem + quarter + ring + as * G::ABUF, v, t.c0 + (warp & 3) * 32 + lane < a.C, noted, warp & 3, row);
                 mbar_arrive(vempty + 8 * vs);                         // only here: an arrival does not wait for loads in flight
                 tc_wait_st();
                 tc_fence_before();
@@ -306,7 +391,7 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
     } else if (warp < EPI_WARPS) {
         const int group = warp >> 2;                                  // a warpgroup for each accumulator: every second step
         const unsigned box = base + G::OUT0 + warp * OUT_BYTES, stage = box + lane * 128, d = tmem + quarter + group * G::N;
-        int step = 0, dph = 0;
+        int step = 0, dph = 0, row0 = 0;                              // row0: rows of V of this CTA before the item
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             const Item t = item_at<T>(a, i);
             const int cw = t.c0 + (warp & 3) * 32, c = cw + lane;
@@ -317,7 +402,7 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                 tc_fence_after();
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");       // the last store has read the box
                 __syncwarp();
-                unsigned bad[G::N / 32];
+                float zero[4] = {0.f, 0.f, 0.f, 0.f};                 // stays zero while all values are finite
 #pragma unroll
                 for (int g = 0; g < G::N / 32; ++g) {                 // 8 parents at a time: 16 pixels of both high-res rows
                     unsigned v[32];
@@ -326,13 +411,8 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                     tc_wait_ld();
                     tc_st16(d + 32 * g, zeros);
                     tc_st16(d + 32 * g + 16, zeros);
-                    float zero[4] = {0.f, 0.f, 0.f, 0.f};             // stays zero while all values are finite
 #pragma unroll
                     for (int e = 0; e < 32; ++e) zero[e & 3] = fmaf(__uint_as_float(v[e]), 0.f, zero[e & 3]);
-                    bad[g] = 0u;
-                    if (!((zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.f))
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) bad[g] |= (v[e] & 0x7f800000u) == 0x7f800000u ? 1u << e : 0u;
                     constexpr int PER = 16 / (int)sizeof(T);          // pixels of a chunk
 #pragma unroll
                     for (int r = 0; r < 2; ++r)
@@ -353,22 +433,10 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                                          "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
                         }
                 }
+                if (!((zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.f) && c < a.C) noted.note_sum(warp & 3, row0 + y - t.y0);
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive(dempty + 8 * group);
-                // a product with zero weights took in cells outside a pixel's window: such pixels again, over their own cells alone
-#pragma unroll
-                for (int g = 0; g < G::N / 32; ++g)
-                    while (c < a.C && bad[g] != 0u) {
-                        const int e = __ffs(bad[g]) - 1, r = (e >> 1) & 1, px = 16 * g + 2 * (e >> 2) + (e & 1);
-                        bad[g] &= bad[g] - 1;
-                        if (t.x0 + (px >> 1) >= a.W) continue;
-                        const T s = from_acc<T>(pixel_alone<T>(a, t.n, c, 2 * y + r, 2 * t.x0 + px));
-                        constexpr int PER = 16 / (int)sizeof(T);
-                        const unsigned at = stage + r * (32 * 128) + ((((px / PER) ^ (lane & 7)) << 4) | (px % PER * (int)sizeof(T)));
-                        if constexpr (G::F32) sts32(at, __float_as_uint(s));
-                        else asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(at), "h"(*reinterpret_cast<const unsigned short *>(&s)) : "memory");
-                    }
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 __syncwarp();
                 if (lane == 0 && cw < a.C) {                          // pixels and channels beyond the tensor are cut off
@@ -377,6 +445,7 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                     asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
                 }
             }
+            row0 += t.y1 - t.y0 + 4;
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     }
@@ -385,4 +454,15 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
     __syncthreads();
     tc_fence_after();
     if (warp == MMA_WARP) tc_dealloc(tmem, TMEM_COLS);
+    if (warp < EPI_WARPS && noted.last[warp & 3] >= 0) {              // rare: outputs with something not finite (all are stored)
+        const int first = noted.first[warp & 3], last = noted.last[warp & 3];
+        int row = 0;
+        for (int i = blockIdx.x; i < items; i += gridDim.x, row += 4) {
+            const Item t = item_at<T>(a, i);
+            const int c = t.c0 + (warp & 3) * 32 + lane;
+            for (int y = t.y0; y < t.y1; ++y, ++row)
+                if ((y & 1) == warp >> 2 && c < a.C && row + 4 >= first && row <= last)
+                    finish_pixels<T>(a, t.n, c, y, t.x0, first - row, last - row, noted.sums[warp & 3] != 0);
+        }
+    }
 }

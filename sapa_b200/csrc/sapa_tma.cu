@@ -19,6 +19,7 @@
 //
 // float32 computes the logits on the tensor cores as well (3 x tf32, M = 16 pixels, N = 8 window cells, K = 8
 // channels): on the FP32 pipe that loop was bound by shared-memory wavefronts (12 per 10 packed FMAs).
+#include "finite.cuh"
 #include "umma_util.cuh"
 
 #include <algorithm>
