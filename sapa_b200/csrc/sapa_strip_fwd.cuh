@@ -40,9 +40,73 @@ template <typename T, int KSTEPS> struct Lay {
 struct FArgs {
     SArgs s;
     void *attn;            // optional output
+    const void *q, *k;     // for outputs with an infinity in their windows
+    int d;
 };
 __device__ __forceinline__ void tc_ld4(unsigned taddr, unsigned *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+// Window slots whose 16-bit weight for a pixel is zero (or NaN), formed again by a warp, a slot to a lane
+template <typename T> __device__ __forceinline__ unsigned no_weight(const FArgs &f, int n, int hy, int hx, int lane) {
+    const SArgs &a = f.s;
+    const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W), lo_plane = (size_t)a.rows * a.W;
+    const int y = a.ytop0 + (hy >> 1) + lane / 5 - 2, x = (hx >> 1) + lane % 5 - 2;
+    const bool slot = lane < 25, cell = slot && y >= 0 && y < a.rows && x >= 0 && x < a.W;
+    const T *q = static_cast<const T *>(f.q) + (size_t)n * f.d * hi_plane + (size_t)hy * (2 * a.W) + hx;
+    const T *k = static_cast<const T *>(f.k) + (size_t)n * f.d * lo_plane + (cell ? (size_t)y * a.W + x : 0);
+    float s = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < f.d; ++c) s = fmaf(to_acc(q[c * hi_plane]), cell ? to_acc(k[c * lo_plane]) : 0.f, s);
+    float m = slot ? s : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float e = slot ? expf(s - m) : 0.f;
+    float z = e;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    return __ballot_sync(0xffffffffu, slot && !(to_acc(from_acc<T>(e / z)) > 0.f));
+}
+// Outputs of half a strip's row with something not finite in their windows, which the products took as zero, once they are stored: NaN next to a NaN,
+// to infinities of both signs and to one whose weight is zero.  By a whole warp.  dy0, dy1: the window rows that may hold such elements.
+template <typename T> __device__ __noinline__ void finish_pixels(const FArgs &f, int n, int x0, int c, int y, int half, int dy0, int dy1, int lane) {
+    const SArgs &a = f.s;
+    constexpr int FIRST = strip::Geo<T>::BOX0 - 2;                    // bit of a parent's first column
+    const unsigned mine = 0xffffu << (16 * half);
+    unsigned nan = 0u;                                                // parents next to a NaN
+    unsigned long long up[5], down[5];
+#pragma unroll
+    for (int dy = 0; dy < 5; ++dy) {
+        finite::Marks m{0ull, 0ull, 0ull};
+        if (c < a.C && dy >= dy0 && dy <= dy1 && (nan & mine) != mine) m = strip::marks_of<T>(a, n, c, y, dy, x0);
+        nan |= (unsigned)strip::reached<T>(m.nan); up[dy] = m.up; down[dy] = m.down;
+    }
+    const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W);
+    T *const out = static_cast<T *>(a.out) + ((size_t)n * a.C + c) * hi_plane + (size_t)(2 * y) * (2 * a.W) + 2 * x0;
+#pragma unroll 1
+    for (int p = 16 * half; p < 16 * half + 16 && x0 + p < a.W; ++p) {
+        if ((p & 3) == 0 && __all_sync(0xffffffffu, c >= a.C || (nan >> p & 15) == 15)) {      // 16 bytes of each row
+            if (c < a.C) *reinterpret_cast<uint4 *>(out + 2 * p) = *reinterpret_cast<uint4 *>(out + 2 * a.W + 2 * p) = finite::nan_chunk<T>();
+            p += 3;
+            continue;
+        }
+        unsigned ups = 0u, downs = 0u;                                // window slots
+#pragma unroll
+        for (int dy = 0; dy < 5; ++dy) {
+            ups |= (unsigned)(up[dy] >> (FIRST + p) & 31) << (5 * dy);
+            downs |= (unsigned)(down[dy] >> (FIRST + p) & 31) << (5 * dy);
+        }
+        const bool none = (nan >> p & 1) != 0u || (ups != 0u && downs != 0u), some = (ups | downs) != 0u;
+        if (!__any_sync(0xffffffffu, none || some)) continue;
+        const bool ask = __any_sync(0xffffffffu, some && !none);
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+            const int r = e >> 1, px = 2 * p + (e & 1);
+            const unsigned gone = ask ? no_weight<T>(f, n, 2 * y + r, 2 * x0 + px, lane) : 0u;
+            if (!none && !some) continue;
+            const float s = none || ((ups | downs) & gone) != 0u ? finite::nan_value() : ups != 0u ? INFINITY : -INFINITY;
+            out[(size_t)r * (2 * a.W) + px] = from_acc<T>(s);
+        }
+    }
 }
 // the steps (rows) of a CTA's items, one after the other
 template <typename T> struct Cursor {
@@ -64,7 +128,7 @@ template <typename T> struct Cursor {
 template <typename T, int KSTEPS>
 __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                                                                      const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap omap,
-                                                                     const sfwd::FArgs f) {
+                                                                     const __grid_constant__ sfwd::FArgs f) {
     using namespace sfwd;
     using G = strip::Geo<T>;
     using L = Lay<T, KSTEPS>;
@@ -73,6 +137,7 @@ __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __gri
     extern __shared__ unsigned char smem_dyn[];
     __shared__ __align__(8) unsigned long long bars[2 * (sfwd::MAX_NVL + sfwd::NV + MAX_NKR + MAX_NQ + sfwd::NP + 2) + 6];
     __shared__ unsigned tmem_slot;
+    __shared__ finite::Noted noted;                                   // rows of V, counted over the CTA's items
     const unsigned base = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u;
     const unsigned vfull = (unsigned)__cvta_generic_to_shared(bars), vempty = vfull + 8 * NVL, aready = vempty + 8 * NVL, aempty = aready + 8 * sfwd::NV;
     const unsigned kfull = aempty + 8 * sfwd::NV, kempty = kfull + 8 * NKR, qfull = kempty + 8 * NKR, qempty = qfull + 8 * NQ;
@@ -80,6 +145,7 @@ __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __gri
     const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
     const int items = a.B * a.cblocks * a.segs * a.strips;
 
+    if (tid < 4) noted.clear(tid);
     if (tid == 0) {
         for (int i = 0; i < NVL; ++i) { mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 128); }
         for (int i = 0; i < sfwd::NV; ++i) { mbar_init(aready + 8 * i, 128); mbar_init(aempty + 8 * i, 1); }
@@ -242,12 +308,12 @@ __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __gri
             now.next(a, items);
         }
     } else if (warp >= SPLIT_WARP0 && warp < SOFT_WARP0) {
-        int vs = 0, vph = 0, as = 0, aph = 0;
+        int vs = 0, vph = 0, as = 0, aph = 0, row = 0;
         const unsigned line = ((warp & 3) * 32 + lane) * VROW;
         for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
             const Item t = strip::item_at<T>(a, i);
             const bool used = t.c0 + (warp & 3) * 32 < a.C;           // lanes without a channel keep whatever they hold
-            for (int y = t.y0 - 2; y < t.y1 + 2; ++y) {
+            for (int y = t.y0 - 2; y < t.y1 + 2; ++y, ++row) {
                 if (!mbar_wait_warp(vfull + 8 * vs, vph)) { ok = false; break; }
                 unsigned v[4 * VCHUNKS];
                 if (used) {
@@ -258,10 +324,7 @@ __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __gri
                 }
                 if (!mbar_wait_warp(aempty + 8 * as, aph ^ 1)) { ok = false; break; }
                 tc_fence_after();
-                if (used) {
-                    const unsigned at = tmem + quarter + V_COL + as * ACOLS;
-                    tc_st16(at, v + G::SHIFT); tc_st8(at + 16, v + G::SHIFT + 16);
-                }
+                if (used) strip::move_cells<T>(tmem + quarter + V_COL + as * ACOLS, v, t.c0 + (warp & 3) * 32 + lane < a.C, noted, warp & 3, row);
                 mbar_arrive(vempty + 8 * vs);                         // only here: an arrival does not wait for loads in flight
                 tc_wait_st();
                 tc_fence_before();
@@ -390,4 +453,13 @@ __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     if (warp == sfwd::MMA_WARP) tc_dealloc(tmem, sfwd::TMEM_COLS);
+    if (warp < sfwd::EPI_WARPS && noted.last[warp & 3] >= 0) {        // rare: outputs with something not finite (all are stored)
+        const int first = noted.first[warp & 3], last = noted.last[warp & 3];
+        int row = 0;
+        for (Cursor<T> c(a, items); c.more; c.next(a, items)) {
+            if (row + 4 >= first && row <= last)
+                finish_pixels<T>(f, c.t.n, c.t.x0, c.t.c0 + (warp & 3) * 32 + lane, c.y, warp >> 2, first - row, last - row, lane);
+            row += c.y == c.t.y1 - 1 ? 5 : 1;
+        }
+    }
 }

@@ -1180,7 +1180,7 @@ static int launch_strip_fwd(const void *q, const void *k, const void *v, void *o
     }
     sfwd::FArgs f{};
     a.v = v; a.out = out;
-    f.s = a; f.attn = attn;
+    f.s = a; f.attn = attn; f.q = q; f.k = k; f.d = d;
     auto go = [&](auto ksteps) -> int {
         constexpr int KSTEPS = decltype(ksteps)::value, SMEM = sfwd::Lay<T, KSTEPS>::SMEM;
         int n = 0;

@@ -6,6 +6,7 @@ import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
+INF, NAN = float("inf"), float("nan")
 
 
 def _rand(seed, *shape, dtype, scale=1.0):
@@ -63,3 +64,33 @@ def test_bands_of_a_slab(dtype):
     for begin, end in ((0, 4), (4, rows - 3), (rows - 3, rows)):
         slab._launch(ql, out, begin, end)
     assert torch.equal(out, whole[:, :, hi])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(2, 300, 24, 40, 72), (1, 40, 64, 9, 16), (2, 136, 40, 14, 40)], ids=lambda s: "B%d_C%d_d%d_%dx%d" % s)
+def test_strips_keep_infinities_to_their_windows(shape, dtype):
+    """An infinity or NaN of the value reaches the pixels whose window holds it, and those get what their weights make of it; every
+    other output has the bits that it has without it."""
+    from sapa_b200 import _lib
+    from sapa_b200.functions import fused_forward_raw
+    B, C, d, H, W = shape
+    q, k, v = _rand(1, B, d, 2 * H, 2 * W, dtype=dtype, scale=0.5), _rand(2, B, d, H, W, dtype=dtype, scale=0.5), _rand(3, B, C, H, W, dtype=dtype)
+    bad = v.clone()
+    for n, c, y, x, what in ((0, 3, 0, 0, INF), (0, C - 1, 7, 11, NAN), (B - 1, C - 1, H - 1, W - 1, -INF), (B - 1, 7, 5, 14, INF), (B - 1, 7, 6, 15, INF),
+                             (0, 20, 4, 9, INF), (0, 20, 6, 10, -INF), (0, 21, 3, 8, INF), (0, 21, 4, 8, NAN)):
+        bad[n, c, y, x] = what
+    for keep in (False, True):
+        clean, got = fused_forward_raw(q, k, v, 5, 2, keep)[0], fused_forward_raw(q, k, bad, 5, 2, keep)[0]
+        attn = fused_forward_raw(q, k, bad, 5, 2, True)[1]
+        assert torch.isfinite(attn).all()
+        reached = (F.max_pool2d((~torch.isfinite(bad)).float(), 5, 1, 2) > 0).repeat_interleave(2, 2).repeat_interleave(2, 3)
+        assert torch.equal(got[~reached], clean[~reached])
+        want = torch.zeros(B, C, 2 * H, 2 * W, dtype=torch.float64, device=DEV)
+        padded = F.pad(bad.double(), (2, 2, 2, 2))
+        for i in range(25):
+            window = padded[:, :, i // 5:i // 5 + H, i % 5:i % 5 + W].repeat_interleave(2, 2).repeat_interleave(2, 3)
+            want += attn[:, i:i + 1].double() * window
+        assert not torch.isfinite(want[reached]).any()
+        a, b = got[reached].double(), want[reached]
+        assert bool(((a == b) | (torch.isnan(a) & torch.isnan(b))).all())
+    assert _lib.wait_timeout_flags(DEV) == 0
