@@ -543,12 +543,12 @@ bool fused_mma_supported(int W, int dtype);
 bool fused_tma_supported(int W, int dtype);
 bool fused_f32_on_strips(int C, int W);
 int launch_fused_tma(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d, int C,
-                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st);
+                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st, int groups = 1);
 int launch_fused_mma(const void *q, const void *k, const void *v, void *out, void *attn, int B, int d, int C, int H, int W,
                      int rows, int ytop0, int dtype, cudaStream_t st);
 int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d,
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
-                           cudaStream_t st);
+                           cudaStream_t st, int groups);
 
 int tma_wait_timeout_flag();
 int proj_wait_timeout_flag();
@@ -557,7 +557,7 @@ int gath_wait_timeout_flag();
 // tensor-core transposed aggregation (sapa_gath_mma.cu)
 bool gath_mma_supported(int W, int dtype);
 int launch_gath_mma(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype,
-                    cudaStream_t st);
+                    cudaStream_t st, int groups = 1);
 
 // K = 5, s = 2 on the tensor-core kernels: 16-bit rows of any length, float32 where a tensor map describes the rows
 static bool tensor_core_rows(int W, int dtype) { return dtype == SAPA_F32 ? fused_tma_supported(W, dtype) : dtype != SAPA_F64; }
@@ -626,12 +626,12 @@ static int check_common(const char *fn, int B, int C, int H, int W, int K, int s
 
 // sim / agg / gath dispatchers (tiled when possible, else generic); sim and agg also serve the dense path of SAPA-D
 // Slab form: `lo` holds `rows` = top + H + bottom low-res rows per plane, of which the H rows from `top` on are the
-// ones the high-res rows of `hi` / `out` belong to (rows = H, top = 0: a whole image).
+// ones the high-res rows of `hi` / `out` belong to (rows = H, top = 0: a whole image).  groups: how many of the B belong to one image.
 int run_sim_slab(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s,
-                 int dtype, cudaStream_t st) {
+                 int dtype, cudaStream_t st, int groups = 1) {
     const bool al = all_aligned16(hi, lo, out);     // misaligned views take the scalar generic kernels
     if (al && K == 5 && s == 2 && tensor_core_rows(W, dtype)) {     // logit half of the tensor-core kernel
-        const int e = launch_fused_tma(2, hi, lo, nullptr, nullptr, out, nullptr, B, Cc, 0, H, W, rows, top, 0, H, dtype, st);
+        const int e = launch_fused_tma(2, hi, lo, nullptr, nullptr, out, nullptr, B, Cc, 0, H, W, rows, top, 0, H, dtype, st, groups);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
     if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {
@@ -655,24 +655,24 @@ int run_sim_slab(const void *hi, const void *lo, void *out, int B, int Cc, int H
 // 16-bit tensors with a float32 slot tensor (K = 5, s = 2, rows of 16 bytes): sim writes float32 logits.  The dense-window
 // path of SAPA-D keeps its 25-slot similarity at full precision this way.
 int run_sim_mixed(const void *hi, const void *lo, float *out, int B, int Cc, int H, int W, int rows, int top, int dtype,
-                  cudaStream_t st) {
+                  cudaStream_t st, int groups = 1) {
     if (!(all_aligned16(hi, lo, out) && (dtype == SAPA_F16 || dtype == SAPA_BF16) && fused_tma_supported(W, dtype))) {
         set_error("run_sim_mixed: needs 16-bit tensors, 16-byte aligned, rows of 16 bytes");
         return SAPA_ERR_UNSUPPORTED;
     }
-    return launch_fused_tma_slots(2, hi, lo, nullptr, nullptr, out, nullptr, B, Cc, 0, H, W, rows, top, 0, H, dtype, true, st);
+    return launch_fused_tma_slots(2, hi, lo, nullptr, nullptr, out, nullptr, B, Cc, 0, H, W, rows, top, 0, H, dtype, true, st, groups);
 }
 
-int run_sim(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st) {
-    return run_sim_slab(hi, lo, out, B, Cc, H, W, H, 0, K, s, dtype, st);
+int run_sim(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st, int groups = 1) {
+    return run_sim_slab(hi, lo, out, B, Cc, H, W, H, 0, K, s, dtype, st, groups);
 }
 
 int run_agg_slab(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s,
-                 int dtype, cudaStream_t st) {
+                 int dtype, cudaStream_t st, int groups = 1) {
     const bool al = all_aligned16(wt, lo, out);
     if (al && K == 5 && s == 2 && tensor_core_rows(W, dtype)) {     // aggregation half of the tensor-core kernel
         const int e = launch_fused_tma(3, nullptr, nullptr, lo, out, const_cast<void *>(wt), nullptr, B, 0, Cc, H, W, rows, top, 0, H,
-                                       dtype, st);
+                                       dtype, st, groups);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
     if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {
@@ -693,15 +693,15 @@ int run_agg_slab(const void *wt, const void *lo, void *out, int B, int Cc, int H
     });
 }
 
-int run_agg(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st) {
-    return run_agg_slab(wt, lo, out, B, Cc, H, W, H, 0, K, s, dtype, st);
+int run_agg(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st, int groups = 1) {
+    return run_agg_slab(wt, lo, out, B, Cc, H, W, H, 0, K, s, dtype, st, groups);
 }
 
 int run_gath(const void *hi, const void *wt, void *out, int B, int Cc, int H, int W, int K, int s, int dtype,
-             cudaStream_t st) {
+             cudaStream_t st, int groups = 1) {
     const bool al = all_aligned16(hi, wt, out);
     if (al && K == 5 && s == 2 && tensor_core_gath(W, dtype)) {
-        const int e = launch_gath_mma(hi, wt, out, B, Cc, H, W, 0, 0, dtype, st);
+        const int e = launch_gath_mma(hi, wt, out, B, Cc, H, W, 0, 0, dtype, st, groups);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
     if (al && tiled_supported(K, s, dtype) && (K == 3 || dtype == SAPA_F32)) {

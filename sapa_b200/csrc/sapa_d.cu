@@ -1201,14 +1201,14 @@ int sapa_deform_fused_backward(const void *grad_out, const void *query, const vo
 
 // dispatchers of the SAPA-B logit and aggregation kernels (sapa_b.cu)
 namespace sapa {
-int run_sim(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st);
-int run_agg(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st);
-int run_gath(const void *hi, const void *wt, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st);
+int run_sim(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st, int groups);
+int run_agg(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st, int groups);
+int run_gath(const void *hi, const void *wt, void *out, int B, int Cc, int H, int W, int K, int s, int dtype, cudaStream_t st, int groups);
 int run_sim_slab(const void *hi, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s, int dtype,
-                 cudaStream_t st);
+                 cudaStream_t st, int groups);
 int run_agg_slab(const void *wt, const void *lo, void *out, int B, int Cc, int H, int W, int rows, int top, int K, int s, int dtype,
-                 cudaStream_t st);
-int run_sim_mixed(const void *hi, const void *lo, float *out, int B, int Cc, int H, int W, int rows, int top, int dtype, cudaStream_t st);
+                 cudaStream_t st, int groups);
+int run_sim_mixed(const void *hi, const void *lo, float *out, int B, int Cc, int H, int W, int rows, int top, int dtype, cudaStream_t st, int groups);
 bool fused_tma_supported(int W, int dtype);
 }
 
@@ -1255,9 +1255,9 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
     // 1. dense 25-slot similarity of every group: the B x G groups are images of Cq / G channels.  16-bit tensors: the
     //    logits leave the tensor-core kernel as float32 (a 16-bit logit would cost the softmax two digits)
     if (dtype == SAPA_F32) {
-        if (int e = run_sim_slab(query, key, dense, B * G, Cq / G, H, W, rows, halo_top, 5, 2, dtype, st)) return e;
+        if (int e = run_sim_slab(query, key, dense, B * G, Cq / G, H, W, rows, halo_top, 5, 2, dtype, st, G)) return e;
     } else {
-        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, rows, halo_top, dtype, st)) return e;
+        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, rows, halo_top, dtype, st, G)) return e;
     }
     // 2. attention over the points, dense window weights, list of the points that leave the window
     {
@@ -1270,7 +1270,7 @@ int sapa_deform_fused_forward_slab(const void *query, const void *key, const voi
         if (e) return e;
     }
     // 3. aggregation of every group's channels over the window
-    if (int e = run_agg_slab(window, value, out, B * G, C / G, H, W, rows, halo_top, 5, 2, dtype, st)) return e;
+    if (int e = run_agg_slab(window, value, out, B * G, C / G, H, W, rows, halo_top, 5, 2, dtype, st, G)) return e;
     // 4. the listed points (the count is only known on the device: a fixed grid strides over the list)
     return SAPA_DISPATCH_FAST(dtype, [&] {
         launch_next_with_l1(deform_outlier_kernel<scalar_t>, 148 * 8, 256, st, taps, tap_count, static_cast<const scalar_t *>(value),
@@ -1305,9 +1305,9 @@ int sapa_deform_qk_forward_dense(const void *query, const void *key, const void 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     float *dense = static_cast<float *>(workspace);
     if (dtype == SAPA_F32) {
-        if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;
+        if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;
     } else {
-        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st)) return e;
+        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st, G)) return e;
     }
     return SAPA_DISPATCH_FAST(dtype, [&] {
         for_points(P, [&](auto most) {
@@ -1345,7 +1345,7 @@ int sapa_deform_av_forward_dense(const void *attn, const void *value, const void
             return check_launch("deform_window_kernel<weights>");
         }))
         return e;
-    if (int e = run_agg(region, value, out, B * G, C / G, H, W, 5, 2, dtype, st)) return e;
+    if (int e = run_agg(region, value, out, B * G, C / G, H, W, 5, 2, dtype, st, G)) return e;
     return SAPA_DISPATCH_FAST(dtype, [&] {
         launch_next_with_l1(deform_outlier_kernel<scalar_t>, 148 * 8, 256, st, taps, tap_count, static_cast<const scalar_t *>(value),
                                                                  static_cast<const scalar_t *>(offset), static_cast<scalar_t *>(out), C, H,
@@ -1401,11 +1401,11 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
     if (int e = clear_counter(fn, tap_count, st)) return e;
     // 1. D = sim(Q, Key) and dWd = sim(dOut, Value), the B x G groups as images
     if (dtype == SAPA_F32) {
-        if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;
-        if (int e = run_sim(grad_out, value, dwin, B * G, C / G, H, W, 5, 2, dtype, st)) return e;
+        if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;
+        if (int e = run_sim(grad_out, value, dwin, B * G, C / G, H, W, 5, 2, dtype, st, G)) return e;
     } else {
-        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st)) return e;
-        if (int e = run_sim_mixed(grad_out, value, dwin, B * G, C / G, H, W, H, 0, dtype, st)) return e;
+        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st, G)) return e;
+        if (int e = run_sim_mixed(grad_out, value, dwin, B * G, C / G, H, W, H, 0, dtype, st, G)) return e;
     }
     // 2. per pixel: softmax backward over the points, dD, Wd, offset gradients, list of the points outside the window
     {
@@ -1420,9 +1420,9 @@ int sapa_deform_fused_backward_dense(const void *grad_out, const void *query, co
         if (e) return e;
     }
     // 3. dQ = agg(dD, Key), dKey = gath(Q, dD), dV = gath(dOut, Wd): SAPA-B kernels per group, all outputs overwritten
-    if (int e = run_agg(ddense, key, grad_query, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;
-    if (int e = run_gath(query, ddense, grad_key, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;
-    if (int e = run_gath(grad_out, window, grad_value, B * G, C / G, H, W, 5, 2, dtype, st)) return e;
+    if (int e = run_agg(ddense, key, grad_query, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;
+    if (int e = run_gath(query, ddense, grad_key, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;
+    if (int e = run_gath(grad_out, window, grad_value, B * G, C / G, H, W, 5, 2, dtype, st, G)) return e;
     // 4. the listed points.  float32: atomics straight into the gradients.  16-bit: key / value contributions go to zeroed
     //    float32 side buffers behind the list and are folded into the 16-bit gradients by one more kernel.
     if (dtype == SAPA_F32) {
@@ -1475,9 +1475,9 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
     if (int e = clear_counter(fn, tap_count, st)) return e;
     if (dtype == SAPA_F32) {
-        if (int e = run_sim(grad_out, value, dwin, B * G, C / G, H, W, 5, 2, dtype, st)) return e;        // dWd
+        if (int e = run_sim(grad_out, value, dwin, B * G, C / G, H, W, 5, 2, dtype, st, G)) return e;        // dWd
     } else {
-        if (int e = run_sim_mixed(grad_out, value, dwin, B * G, C / G, H, W, H, 0, dtype, st)) return e;
+        if (int e = run_sim_mixed(grad_out, value, dwin, B * G, C / G, H, W, H, 0, dtype, st, G)) return e;
     }
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
             launch_window_bwd<BWD_AV, scalar_t>(P, B * G, hi, st, static_cast<const scalar_t *>(grad_out), static_cast<const scalar_t *>(value),
@@ -1487,7 +1487,7 @@ int sapa_deform_av_backward_dense(const void *grad_out, const void *attn, const 
             return check_launch("deform_window_bwd_kernel<av>");
         }))
         return e;
-    if (int e = run_gath(grad_out, window, grad_value, B * G, C / G, H, W, 5, 2, dtype, st)) return e;  // dV
+    if (int e = run_gath(grad_out, window, grad_value, B * G, C / G, H, W, 5, 2, dtype, st, G)) return e;  // dV
     if (dtype == SAPA_F32) {
         launch_in_order(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, static_cast<const float *>(grad_out), nullptr, nullptr, static_cast<const float *>(value),
@@ -1535,9 +1535,9 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
     unsigned int *tap_count = reinterpret_cast<unsigned int *>(taps + (size_t)B * G * P * hi);
     if (int e = clear_counter(fn, tap_count, st)) return e;
     if (dtype == SAPA_F32) {
-        if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;         // D, for the offset gradients
+        if (int e = run_sim(query, key, dense, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;         // D, for the offset gradients
     } else {
-        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st)) return e;
+        if (int e = run_sim_mixed(query, key, dense, B * G, Cq / G, H, W, H, 0, dtype, st, G)) return e;
     }
     // the logit gradients enter where the fused chain reads the attention
     if (int e = SAPA_DISPATCH_FAST(dtype, [&] {
@@ -1548,8 +1548,8 @@ int sapa_deform_qk_backward_dense(const void *grad_out, const void *query, const
             return check_launch("deform_window_bwd_kernel<qk>");
         }))
         return e;
-    if (int e = run_agg(ddense, key, grad_query, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;       // dQ
-    if (int e = run_gath(query, ddense, grad_key, B * G, Cq / G, H, W, 5, 2, dtype, st)) return e;      // dKey
+    if (int e = run_agg(ddense, key, grad_query, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;       // dQ
+    if (int e = run_gath(query, ddense, grad_key, B * G, Cq / G, H, W, 5, 2, dtype, st, G)) return e;      // dKey
     if (dtype == SAPA_F32) {
         launch_in_order(deform_outlier_bwd_kernel<float, float>, 148 * 8, 256, 0, st,
             taps, tap_count, nullptr, static_cast<const float *>(query), static_cast<const float *>(key), nullptr,

@@ -433,7 +433,7 @@ struct Form { int rows, cols, nch, threads, smem, ctas_per_sm; };
 
 // The tcgen05 kernel's split of a problem: rows of an item for the fewest steps (parent rows) of the busiest CTA, four of each item
 // for the parents around it and three to start and to end.
-struct UmmaPlan { gumma::UArgs u; long long items, steps; };
+struct UmmaPlan { gumma::UArgs u; long long items; };
 template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int top, int bottom, int sms) {
     UmmaPlan p{};
     gumma::UArgs &u = p.u;
@@ -445,20 +445,21 @@ template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int 
     u.slot_bytes = ceil_div(u.x_bytes + gumma::L_BYTES, 128) * 128;
     u.nx = std::min(gumma::MAX_NX, gumma::RING_BYTES / u.slot_bytes / 2 * 2);
     const long long columns = (long long)B * u.strips * u.cblocks;
-    ummau::split_rows(columns, u.g.Hout, sms, 4, p.items, p.steps, u.seg_rows, u.segs);
+    long long steps = 0;
+    ummau::split_rows(columns, u.g.Hout, sms, 4, p.items, steps, u.seg_rows, u.segs);
     return p;
 }
 
-// It serves rows of 16 bytes in and out, but for small problems and those that fill few of its lanes or columns.  A step takes about 0.95 us
-// in float32 and 0.8 in 16 bits, whatever the channels; the kernels on tiles 11.2 and 4.6 us for a million products of cells and
-// (channels + 24), and half a dozen to start.  us, tiles -> this one, float32 | bfloat16: 8 x 256 x 64x64 104 -> 45 | 43 -> 24; 8 x 64 x 64x64
-// 37 -> 27 | 18 -> 13; 1 x 32 x 512x512 170 -> 149 | 74 -> 53; 64 x 32 x 32x32 46 -> 43 | 23 -> 19; 4 x 128 x 32x32 12.7 -> 10.4 | 9.1 -> 7.6;
-// and where the line leaves them with the tiles: 8 x 32 x 32x32 9.9, 13.8 here | 8.0, 8.1; 1 x 64 x 16x16 8.7, 8.9 | 5.0, 6.4; 4 x 32 x 64x64
-// 15.7, 16.4 here | 9.4, 9.7.
-template <typename T> static bool umma_pays(const UmmaPlan &p) {
-    const Args &g = p.u.g;
-    const double work = 1e-6 * g.B * g.Hout * g.W * (g.C + 24.0);
-    return g.W % (16 / (int)sizeof(T)) == 0 && (double)p.steps <= (sizeof(T) == 4 ? 2.0 + 12.0 * work : 5.0 + 5.7 * work);
+// It serves rows of 16 bytes in and out, but for small images and those that fill few of its lanes or columns.  An image's result must not depend on
+// the batch that it is in, so the line sees one image (all of its groups in SAPA-D) and lies where it is about as fast alone.  us, tiles -> this one, with
+// the similarity of the same sizes in front, float32 | bfloat16: 8 x 256 x 64x64 156 -> 92 | 68 -> 45; one image of 128 x 32x32 17.1 -> 14.1 | 11.5 -> 10.3,
+// 64 x 64x64 15.5, 15.7 | 10.8 -> 10.4, 32 x 32x32 8.7, 9.8 | 9.9 -> 8.3; and where the line leaves them with the tiles: float32 64 x 32x32 11.7, 11.7 here, 16 of
+// them 33.1, 27.9; 32 x 64x64 12.2, 13.0 (16: 69, 65); bfloat16 64 x 16x16 8.1, 9.0, 128 x 64x16 10.6, 10.5 (16: 33, 27).
+template <typename T> static bool umma_pays(int groups, int C, int H, int W) {
+    const double values = (double)groups * C * H * W;
+    const int cells = gumma::Geo<T>::CELLS, columns = ceil_div(W, cells) * cells;
+    if (W % (16 / (int)sizeof(T)) != 0) return false;
+    return sizeof(T) == 4 ? C >= 64 && 2 * W >= columns && values >= 1.2e5 : C >= 32 && 4 * W >= 3 * columns && values >= 3e4;
 }
 
 template <typename T>
@@ -487,7 +488,7 @@ static int launch_umma(const void *hi, const void *wt, void *out, UmmaPlan p, in
 }
 
 template <typename T>
-static int launch(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype, cudaStream_t st) {
+static int launch(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype, cudaStream_t st, int groups) {
     using G = Geo<T>;
     constexpr bool F32 = sizeof(T) == 4;
     // rows a tensor map can describe and paired stores: the TMA forms
@@ -499,10 +500,7 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     }
     int sms = 0;
     if (int e = device_sms(name, sms)) return e;
-    if (!ragged) {
-        const UmmaPlan p = umma_plan<T>(B, C, H, W, top, bottom, sms);
-        if (umma_pays<T>(p)) return launch_umma<T>(hi, wt, out, p, sms, name, st);
-    }
+    if (!ragged && umma_pays<T>(groups, C, H, W)) return launch_umma<T>(hi, wt, out, umma_plan<T>(B, C, H, W, top, bottom, sms), sms, name, st);
     const Form f = ragged ? Form{ROWS, COLS, G::NCH, NT_RAGGED, G::SMEM_BYTES, 1}
                    : wide ? Form{ROWS, gw16::COLS, gw16::NCH, gw16::NT, gw16::SMEM_BYTES, 1}
                           : Form{ROWS, COLS, G::NCH, NT, G::SMEM_BYTES, CTAS_PER_SM};
@@ -564,11 +562,12 @@ bool gath_mma_supported(int W, int dtype) {
 
 // Returns SAPA_ERR_UNSUPPORTED when the tensor map cannot be built (the caller then uses the FP32-pipe kernel).
 // `top` / `bottom`: extra output rows above / below the H rows under the inputs (row-slab backward), 0 otherwise.
+// groups: how many of the B belong to one image (SAPA-D), for the choice of the kernel.
 int launch_gath_mma(const void *hi, const void *wt, void *out, int B, int C, int H, int W, int top, int bottom, int dtype,
-                    cudaStream_t st) {
-    if (dtype == SAPA_F32) return gmma::launch<float>(hi, wt, out, B, C, H, W, top, bottom, dtype, st);
-    if (dtype == SAPA_F16) return gmma::launch<__half>(hi, wt, out, B, C, H, W, top, bottom, dtype, st);
-    if (dtype == SAPA_BF16) return gmma::launch<__nv_bfloat16>(hi, wt, out, B, C, H, W, top, bottom, dtype, st);
+                    cudaStream_t st, int groups) {
+    if (dtype == SAPA_F32) return gmma::launch<float>(hi, wt, out, B, C, H, W, top, bottom, dtype, st, groups);
+    if (dtype == SAPA_F16) return gmma::launch<__half>(hi, wt, out, B, C, H, W, top, bottom, dtype, st, groups);
+    if (dtype == SAPA_BF16) return gmma::launch<__nv_bfloat16>(hi, wt, out, B, C, H, W, top, bottom, dtype, st, groups);
     return SAPA_ERR_UNSUPPORTED;
 }
 

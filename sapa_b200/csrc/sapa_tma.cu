@@ -1114,17 +1114,24 @@ template <typename T> static StripPlan strip_plan(int B, int C, int H, int W, in
     ummau::split_rows(columns, band, sms, 1, p.items, p.steps, a.seg_rows, a.segs);
     return p;
 }
-// It serves rows of 16 bytes, but for small float32 problems and few channels in 16 bits.  A step takes about 0.75 us, whatever the channels, and
-// four to start; the kernels on tiles 3.7 (float32) and 1.5 us for a million products of cells and (channels + 99 or 136).  us, tiles -> this
-// one, float32 | bfloat16: 8 x 256 x 64x64 57 -> 38 | 32 -> 23; 32 x 64 x 64x64 79 -> 54 | 44 -> 32; 1 x 256 x 256x256 109 -> 77 | 59 -> 39;
-// 8 x 256 x 32x32 19 -> 14 | 17 -> 11; 16 x 64 x 32x32 14.8 -> 13.5 | 10.1 -> 9.6; 1 x 32 x 512x512 117 -> 92 | 64 -> 44; and where the line
-// leaves them with the tiles: 8 x 32 x 32x32 6.9, 9.7 here (bfloat16 8.9 -> 7.8); 4 x 128 x 32x32 8.7, 8.8 (9.7 -> 8.5); 32 x 16 x 64x64
-// bfloat16 35, 38 (float32 57 -> 52).
-template <typename T> static bool strip_pays(const StripPlan &p) {
+// Which problems go to the strips.  An image's result should not depend on the batch that it is in, so the lines see one image (all of its groups in
+// SAPA-D) and lie where it is about as fast alone; batches of smaller images would gain too.  `values` of an image: channels x rows x columns.
+static double values(int groups, int C, int H, int W) { return (double)groups * C * H * W; }
+// at least part / whole of the columns of the strips lie inside the image
+static bool strips_filled(int W, int cells, int part, int whole) { return whole * W >= part * ceil_div(W, cells) * cells; }
+// The aggregation in 16 bits, us, tiles -> this one, bfloat16: 8 x 256 x 64x64 30.0 -> 17.8; one image of 64 x 64x64 6.2 -> 5.3, 32 x 32x32 4.6, 4.6, 256 x 24x24
+// 4.8, 5.6 (16 of them 13.9 -> 9.8), 256 x 16x16 4.6, 5.2 (16: 9.2 -> 7.3); left with the tiles: 64 x 16x16 4.6, 4.8 (16: 6.0, 5.7).
+static bool strip_pays_16(int groups, int C, int H, int W) {
+    return C >= 16 && W >= 16 && (strips_filled(W, 32, 3, 4) || values(groups, C, H, W) >= 6e4);
+}
+// In float32, by itself (the output of av, dQ of qk, SAPA-D), its line sees the whole problem, because alone and in a batch are too far apart: 128 x 32x32 4.3,
+// 5.7 here, 16 of them 18.4 -> 11.5; 64 x 64x64 5.4, 6.4, 16 of them 40.6 -> 28.1.  So these results may differ in rounding from those of the image alone.  A
+// step takes about 0.75 us, whatever the channels, and four to start; the kernels on tiles 3.7 us for a million products of cells and (channels + 99).  us,
+// tiles -> this one: 8 x 256 x 64x64 54 -> 37; 32 x 64 x 64x64 76 -> 51; 1 x 256 x 256x256 109 -> 77; 8 x 256 x 32x32 19 -> 14; 16 x 64 x 32x32 14.8 -> 13.5; 1 x
+// 32 x 512x512 117 -> 92; and where the line leaves them with the tiles: 8 x 32 x 32x32 6.9, 9.7 here; 4 x 128 x 32x32 8.7, 8.8.
+static bool strip_pays_f32(const StripPlan &p) {
     const strip::SArgs &a = p.a;
-    const double cells = 1e-6 * a.B * (a.y_end - a.y_begin) * a.W;
-    if (sizeof(T) == 4) return (double)p.steps <= 0.7 + 5.1 * cells * (a.C + 99.0);
-    return a.C >= 32 && (double)p.steps <= 6.0 + 1.75 * cells * (a.C + 136.0);
+    return (double)p.steps <= 0.7 + 5.1e-6 * a.B * (a.y_end - a.y_begin) * a.W * (a.C + 99.0);
 }
 
 template <typename T>
@@ -1261,7 +1268,7 @@ bool fused_tma_supported(int W, int dtype) {
 
 int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d,
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
-                           cudaStream_t st);
+                           cudaStream_t st, int groups);
 
 // 16-bit: tiles of 4 x 32 instead of 4 x 8 pixels where at least three quarters of their columns are inside the image (below that
 // idle warps cost what the loads save) and two thirds of the SMs get one.
@@ -1273,12 +1280,10 @@ static bool wide16_pays(int W, int tiles_y, int B) {
     return 4 * W >= 3 * tiles_x * tma::w16::COLS && (long long)B * tiles_x * tiles_y >= 100;
 }
 
-// float32 on strips of 16 columns, at least three quarters of them inside the image.  The similarity by itself from 12 000 low-res pixels on
-// (us, tiles -> strips: 8 images, 64 channels, 64x64 21.6 -> 16.6; 16 x 64 x 64x64 40 -> 28; 4 x 16 x 64x64 7.7 -> 7.0; 2 x 32 x 48x80
-// 6.3, 6.6 here).
-namespace tma { static bool strips_filled(int W) { return 4 * W >= 3 * ceil_div(W, ssim::CELLS) * ssim::CELLS; } }
-static bool strip_sim_pays(int B, int H, int W) {
-    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && (long long)B * H * W >= 12000;
+// float32 on strips of 16 columns, the similarity by itself (us, tiles -> strips: 8 images, 64 channels, 64x64 19.0 -> 14.5; 1 x 64 x 128x128 12.1 -> 8.8;
+// 4 x 16 x 64x64 6.7 -> 5.0; 1 x 32 x 24x24 no slower; left with the tiles: images of fewer than ten thousand values).
+static bool strip_sim_pays(int groups, int C, int H, int W) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && W >= 16 && tma::strips_filled(W, 16, 3, 4) && tma::values(groups, C, H, W) >= 1e4;
 }
 // The forward as two launches, softmax of the logits and aggregation.  An image's result depends neither on the batch it is in nor on the slab of
 // rows that a process has of it, so the line sees channels and columns alone and lies where a single square image is no slower (us, tiles ->
@@ -1286,21 +1291,21 @@ static bool strip_sim_pays(int B, int H, int W) {
 // 32x32 10.5, 11.0), although larger batches of smaller images would gain too (16 x 128 x 32x32 29.5, 21.3 here; 8 x 256 x 32x32 23.1, 18.7).
 // 8 x 256 x 64x64 78.6 -> 55.3, 16 x 128 x 64x64 103 -> 66, 4 x 128 x 64x64 29.6 -> 21.5.
 bool fused_f32_on_strips(int C, int W) {
-    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)W * W * C >= (C >= 96 ? 5e5 : 7.5e5);
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W, 16, 3, 4) && C >= 48 && (double)W * W * C >= (C >= 96 ? 5e5 : 7.5e5);
 }
-// Stage 1 of the backward likewise, softmax backward of the logits and aggregation, from two million values on, counted as if the images were
-// square: a slab's query gradient equals the rows of the image's (us, tiles -> strips: 8 x 256 x 64x64 91.4 -> 62; 16 x 128 x 64x64 120 -> 80;
-// 8 x 64 x 64x64 47 -> 38).
-static bool bwd_f32_on_strips(int B, int C, int W) {
-    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W) && C >= 48 && (double)B * W * W * C >= 2e6;
+// Stage 1 of the backward likewise, softmax backward of the logits and aggregation, from 64 value channels on and with four fifths of the strips' columns inside
+// the image.  The line sees channels and columns alone: a slab's query gradient equals the rows of the image's.  The whole backward, us, tiles -> strips
+// (gathers on tiles in both): 1 x 64 x 64x64 27.2, 27.1, 16 of them 187 -> 167; 4 x 256 x 64x64 122 -> 112, 1 x 256 x 32x32 36.7 -> 26.9, 1 x 512 x 16x16 49 -> 29;
+// 24 columns, 16 x 128 x 24x24 43, 48 on strips.
+static bool bwd_f32_on_strips(int C, int W) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && W >= 16 && C >= 64 && tma::strips_filled(W, 16, 4, 5);
 }
 
 // 16 bits: the similarity always runs on strips (us, tiles -> strips, bfloat16: 8 images, 64 channels, 64x64 15.0 -> 11.0; 1 x 32 x 16x16 6.2 ->
-// 4.3; 64 x 32 x 8x8 7.0 -> 5.4); stage 1 of the backward as two launches, logits and softmax backward, then the aggregation, with 128 value
-// channels or two million values (of square images, as above) and rows of 16 columns and more.  The whole backward, us: 8 x 256 x 64x64
-// 85.5 -> 75.8, 16 x 128 x 64x64 116 -> 91, 64 x 32 x 32x32 81 -> 69, 2 x 256 x 24x40 28.7 -> 25.9; 4 x 64 x 48x48 28.6, 30.4 on strips;
-// 64 x 64 x 8x8 22.6, 24.5.
-static bool strip_bwd_16_pays(int B, int C, int W) { return W >= 16 && (C >= 128 || (double)B * W * W * C >= 2e6); }
+// 4.3; 64 x 32 x 8x8 7.0 -> 5.4); stage 1 of the backward as two launches from 32 value channels on and with three quarters of the strips' columns inside the
+// image.  The whole backward, us: 1 x 32 x 32x32 21.9, 21.5, 64 of them 89 -> 69; 1 x 256 x 64x64 33.7 -> 29.7, 16 x 64 x 64x64 105 -> 81, 4 x 256 x 24x24 32.3 ->
+// 27.6; 16 columns, 64 x 256 x 64x16 239, 253 on strips.
+static bool strip_bwd_16_pays(int C, int W) { return W >= 24 && C >= 32 && tma::strips_filled(W, 32, 3, 4); }
 
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
 // mode 0 (forward): out = atn(softmax(sim(q, k)), v), attn = optional output.
@@ -1308,15 +1313,15 @@ static bool strip_bwd_16_pays(int B, int C, int W) { return W >= 16 && (C >= 128
 //        (C = key channels), attn = saved attention map (input), ws = logit gradients (output), out = grad_query.
 // mode 2 (sim): attn (output) = sim(q, k); v, out unused, C ignored.   mode 3 (agg): out = atn(attn (input), v); q, k unused, d ignored.
 int launch_fused_tma(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d, int C,
-                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st) {
-    return launch_fused_tma_slots(mode, q, k, v, out, attn, ws, B, d, C, H, W, rows, ytop0, y_begin, y_end, dtype, false, st);
+                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st, int groups) {
+    return launch_fused_tma_slots(mode, q, k, v, out, attn, ws, B, d, C, H, W, rows, ytop0, y_begin, y_end, dtype, false, st, groups);
 }
 
 // slots_f32 (16-bit tensors, mode 2 only): `attn` is a float32 tensor - the logits are written at full precision while
-// query and key stay 16-bit.
+// query and key stay 16-bit.  groups: how many of the B belong to one image (SAPA-D), for the choice of the kernel.
 int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d,
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
-                           cudaStream_t st) {
+                           cudaStream_t st, int groups) {
     using namespace tma;
     if (slots_f32 && (dtype == SAPA_F32 || mode != MODE_SIM)) {
         set_error("sapa_tma_fused: float32 slots are for the 16-bit logit mode");
@@ -1332,20 +1337,20 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         return SAPA_ERR_UNSUPPORTED;
     }
     const bool wide = !ragged && dtype != SAPA_F32 && wide16_pays(W, ceil_div(y_end - y_begin, ROWS), B);
-    if (mode == MODE_AGG && !ragged) {
+    if (mode == MODE_AGG && !ragged && (dtype == SAPA_F32 || strip_pays_16(groups, C, H, W))) {
         const char *name = dtype == SAPA_F32 ? "sapa_tma_fused_f32_kernel<agg>" : wide ? "sapa_wide_16_kernel<agg>" : "sapa_tma_fused_16_kernel<agg>";
         int sms = 0;
         if (int e = device_sms(name, sms)) return e;
-        auto go = [&](auto one) -> int {
-            using T = decltype(one);
-            const StripPlan p = strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
-            return strip_pays<T>(p) ? launch_strip<T>(v, attn, out, p, sms, name, st) : -1000;
-        };
-        const int e = dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
-        if (e != -1000) return e;
+        if (dtype == SAPA_F32) {
+            const StripPlan p = strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
+            if (strip_pays_f32(p)) return launch_strip<float>(v, attn, out, p, sms, name, st);
+        } else {
+            const StripPlan p = strip_plan<__half>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
+            return dtype == SAPA_F16 ? launch_strip<__half>(v, attn, out, p, sms, name, st) : launch_strip<__nv_bfloat16>(v, attn, out, p, sms, name, st);
+        }
     }
-    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(B, H, W) : mode == MODE_FWD ? attn != nullptr && fused_f32_on_strips(C, W)
-                                                                          : mode == MODE_BWD && bwd_f32_on_strips(B, d, W))) {
+    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(groups, d, H, W) : mode == MODE_FWD ? attn != nullptr && fused_f32_on_strips(C, W)
+                                                                          : mode == MODE_BWD && bwd_f32_on_strips(d, W))) {
         static const char *const names[3] = {"sapa_tma_fused_f32_kernel<fwd>", "sapa_tma_fused_f32_kernel<bwd>", "sapa_tma_fused_f32_kernel<sim>"};
         const char *name = names[mode];
         void *slots = mode == MODE_BWD ? ws : attn;
@@ -1358,7 +1363,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         if ((e = device_sms(name, sms)) != SAPA_OK) return e;
         return launch_strip<float>(v, slots, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
     }
-    if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(B, d, W)))) {
+    if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(d, W)))) {
         const char *name = mode == MODE_SIM ? (wide ? "sapa_wide_16_kernel<sim>" : "sapa_tma_fused_16_kernel<sim>") : wide ? "sapa_wide_16_kernel<bwd>" : "sapa_tma_fused_16_kernel<bwd>";
         int sms = 0;
         if (int e = device_sms(name, sms)) return e;
