@@ -117,9 +117,9 @@ int sapa_fused_forward(const void *query, const void *key, const void *value, vo
                        int B, int d, int C, int H, int W, int K, int s, int dtype, void *stream);
 
 /* 1 when sapa_fused_forward is faster for these sizes with `attn` given than without, because it then runs as two
- * kernels: a caller without use for the map passes a scratch buffer of its size (B*K*K*sH*sW elements).  0 otherwise. */
+ * kernels: a caller without use for the map passes a scratch buffer of its size (B*K*K*sH*sW elements), or a smaller one to
+ * sapa_fused_forward_part.  0 otherwise. */
 int sapa_fused_forward_wants_map(int B, int d, int C, int H, int W, int K, int s, int dtype);
-
 
 /* Row-slab form of sapa_fused_forward for one spatial shard of a larger image: key and value hold
  * `halo_top` extra low-res rows above and `halo_bottom` below the H rows whose outputs are produced
@@ -138,6 +138,17 @@ int sapa_fused_forward_slab(const void *query, const void *key, const void *valu
 int sapa_fused_forward_slab_rows(const void *query, const void *key, const void *value, void *out, void *attn,
                                  int B, int d, int C, int H, int W, int halo_top, int halo_bottom,
                                  int row_begin, int row_end, int K, int s, int dtype, void *stream);
+
+/* The general form of the four above: `image_rows` is the height of the whole image of which these H rows are a slab, so that a slab
+ * takes the kernels of its image and has its bits (0: not known; H is meant where there are no halos, a square image otherwise), and
+ * `scratch`, used where `attn` is NULL and the form in two kernels is the faster one, is in place of the map: the image is then
+ * computed in as many parts as fit it, with the same result.  Bytes that are worth it (256 MiB at most): sapa_fused_forward_scratch, 0
+ * where none are; without scratch (NULL, or less than two rows of the map) one kernel runs that needs none.  The scratch may be used again
+ * as soon as the work queued on `stream` is done. */
+int sapa_fused_forward_part(const void *query, const void *key, const void *value, void *out, void *attn,
+                            void *scratch, size_t scratch_bytes, int B, int d, int C, int H, int W, int halo_top, int halo_bottom,
+                            int row_begin, int row_end, int image_rows, int K, int s, int dtype, void *stream);
+size_t sapa_fused_forward_scratch(int B, int d, int C, int H, int W, int image_rows, int K, int s, int dtype);
 
 /* Bytes of scratch sapa_fused_backward needs (grad of the logits, [B,K*K,sH,sW] elements of dtype). */
 size_t sapa_fused_backward_workspace(int B, int H, int W, int K, int s, int dtype);

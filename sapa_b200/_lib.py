@@ -27,6 +27,8 @@ _vp, _i, _sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
 # name -> argument types; every function returns int except the two noted below
 _SIGNATURES = {
     "sapa_fused_forward_wants_map": [_i] * 8,
+    "sapa_fused_forward_scratch": [_i] * 9,
+    "sapa_fused_forward_part": [_vp] * 6 + [_sz] + [_i] * 13 + [_vp],
     "sapa_qk_forward": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "sapa_qk_backward": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "sapa_av_forward": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
@@ -93,6 +95,7 @@ def lib() -> ctypes.CDLL:
     handle.sapa_abi_version.restype = ctypes.c_int
     handle.sapa_fused_backward_workspace.argtypes = [_i, _i, _i, _i, _i, _i]
     handle.sapa_fused_backward_workspace.restype = ctypes.c_size_t
+    handle.sapa_fused_forward_scratch.restype = ctypes.c_size_t
     handle.sapa_deform_fused_backward_scatter_bytes.argtypes = [_i, _i, _i, _i, _i, _i]
     handle.sapa_deform_fused_backward_scatter_bytes.restype = ctypes.c_size_t
     handle.sapa_deform_fused_forward_workspace.argtypes = [_i, _i, _i, _i, _i, _i, _i]

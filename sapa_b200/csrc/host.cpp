@@ -29,7 +29,7 @@ struct Api {
 #define SAPA_FNS                                                                                                          \
     SAPA_FN(sapa_last_error) SAPA_FN(sapa_qk_forward) SAPA_FN(sapa_qk_backward) SAPA_FN(sapa_av_forward)                  \
     SAPA_FN(sapa_av_backward) SAPA_FN(sapa_fused_forward_slab) SAPA_FN(sapa_fused_backward_workspace)                     \
-    SAPA_FN(sapa_fused_forward_wants_map)                                                                                 \
+    SAPA_FN(sapa_fused_forward_part) SAPA_FN(sapa_fused_forward_scratch)                                                                                 \
     SAPA_FN(sapa_fused_backward) SAPA_FN(sapa_deform_qk_forward) SAPA_FN(sapa_deform_qk_backward)                         \
     SAPA_FN(sapa_deform_av_forward) SAPA_FN(sapa_deform_av_backward) SAPA_FN(sapa_deform_fused_forward)                   \
     SAPA_FN(sapa_deform_fused_backward) SAPA_FN(sapa_deform_qk_forward_dense) SAPA_FN(sapa_deform_qk_backward_dense)      \

@@ -541,14 +541,17 @@ static inline int grid_1d(long long total, int threads) {
 // tensor-core fused forward (sapa_mma.cu)
 bool fused_mma_supported(int W, int dtype);
 bool fused_tma_supported(int W, int dtype);
-bool fused_f32_on_strips(int C, int W);
+bool fused_f32_on_strips(int C, int W, int image_rows);
+size_t fused_scratch(int B, int H, int W);
+size_t fused_scratch_row(int W);
 int launch_fused_tma(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d, int C,
-                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st, int groups = 1);
+                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st, int groups = 1, int image_rows = 0,
+                     void *scratch = nullptr, size_t scratch_bytes = 0);
 int launch_fused_mma(const void *q, const void *k, const void *v, void *out, void *attn, int B, int d, int C, int H, int W,
                      int rows, int ytop0, int dtype, cudaStream_t st);
 int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d,
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
-                           cudaStream_t st, int groups);
+                           cudaStream_t st, int groups, int image_rows = 0, void *scratch = nullptr, size_t scratch_bytes = 0);
 
 int tma_wait_timeout_flag();
 int proj_wait_timeout_flag();
@@ -777,9 +780,14 @@ int sapa_av_backward(const void *grad_out, const void *attn, const void *value, 
     return run_gath(grad_out, attn, grad_value, B, C, H, W, K, s, dtype, st);                // dV = gath(dOut, A)
 }
 
-int sapa_fused_forward_slab_rows(const void *query, const void *key, const void *value, void *out, void *attn, int B, int d,
-                                 int C, int H, int W, int halo_top, int halo_bottom, int row_begin, int row_end, int K, int s,
-                                 int dtype, void *stream) {
+size_t sapa_fused_forward_scratch(int B, int d, int C, int H, int W, int image_rows, int K, int s, int dtype) {
+    if (B <= 0 || d <= 0 || C <= 0 || H <= 0 || W <= 0) return 0;
+    return K == 5 && s == 2 && dtype == SAPA_F32 && fused_f32_on_strips(C, W, image_rows > 0 ? image_rows : W) ? fused_scratch(B, H, W) : 0;
+}
+
+int sapa_fused_forward_part(const void *query, const void *key, const void *value, void *out, void *attn, void *scratch, size_t scratch_bytes, int B, int d,
+                            int C, int H, int W, int halo_top, int halo_bottom, int row_begin, int row_end, int image_rows, int K, int s,
+                            int dtype, void *stream) {
     const char *fn = "sapa_fused_forward";
     trace_reset();
     if (int e = check_common(fn, B, d, H, W, K, s, dtype)) return e;
@@ -788,7 +796,7 @@ int sapa_fused_forward_slab_rows(const void *query, const void *key, const void 
     SAPA_REQUIRE(0 <= row_begin && row_begin <= row_end && row_end <= H, SAPA_ERR_ARGUMENT,
                  "%s: row band [%d, %d) is not inside [0, %d)", fn, row_begin, row_end, H);
     SAPA_CHECK_PTR(fn, query); SAPA_CHECK_PTR(fn, key); SAPA_CHECK_PTR(fn, value); SAPA_CHECK_PTR(fn, out);
-    SAPA_REQUIRE(all_aligned16(query, key, value, out) && (attn == nullptr || aligned16(attn)), SAPA_ERR_ALIGNMENT,
+    SAPA_REQUIRE(all_aligned16(query, key, value, out) && (attn == nullptr || aligned16(attn)) && aligned16(scratch), SAPA_ERR_ALIGNMENT,
                  "%s: the fused kernels need 16-byte aligned tensors (copy the misaligned view, or use the separate ops)", fn);
     SAPA_REQUIRE(tiled_supported(K, s, dtype), SAPA_ERR_UNSUPPORTED,
                  "%s: no fused kernel for K=%d s=%d dtype=%d (use the separate ops)", fn, K, s, dtype);
@@ -797,9 +805,12 @@ int sapa_fused_forward_slab_rows(const void *query, const void *key, const void 
     a.hi = query; a.lo1 = key; a.lo2 = value; a.out_hi = out; a.out_slots = attn;
     a.B = B; a.C1 = d; a.C2 = C; a.H = H; a.W = W; a.rows = halo_top + H + halo_bottom; a.ytop0 = halo_top;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // a slab of an image whose height is not known goes the way of a square one
+    const int image = image_rows > 0 ? image_rows : halo_top == 0 && halo_bottom == 0 ? H : W;
+    if (scratch == nullptr || scratch_bytes < 2 * fused_scratch_row(W)) scratch_bytes = 0;      // two rows of an image at least
     if (K == 5 && fused_tma_supported(W, dtype)) {
         const int e = launch_fused_tma(0, query, key, value, out, attn, nullptr, B, d, C, H, W, a.rows, a.ytop0, row_begin, row_end,
-                                       dtype, st);
+                                       dtype, st, 1, image, scratch, scratch_bytes);
         if (e != SAPA_ERR_UNSUPPORTED) return e;
     }
     // the remaining kernels (rows that are not 16-byte aligned, K = 3) always produce the whole slab
@@ -810,6 +821,12 @@ int sapa_fused_forward_slab_rows(const void *query, const void *key, const void 
     if (K == 5)      // 16-bit rows of odd length
         return launch_fused_tma(0, query, key, value, out, attn, nullptr, B, d, C, H, W, a.rows, a.ytop0, 0, H, dtype, st);
     return SAPA_DISPATCH_FAST(dtype, [&] { return launch_tile_ks<scalar_t, MODE_FUSED>(a, K, st); });
+}
+
+int sapa_fused_forward_slab_rows(const void *query, const void *key, const void *value, void *out, void *attn, int B, int d,
+                                 int C, int H, int W, int halo_top, int halo_bottom, int row_begin, int row_end, int K, int s,
+                                 int dtype, void *stream) {
+    return sapa_fused_forward_part(query, key, value, out, attn, nullptr, 0, B, d, C, H, W, halo_top, halo_bottom, row_begin, row_end, 0, K, s, dtype, stream);
 }
 
 int sapa_fused_forward_slab(const void *query, const void *key, const void *value, void *out, void *attn, int B, int d,
@@ -824,8 +841,7 @@ int sapa_fused_forward(const void *query, const void *key, const void *value, vo
 }
 
 int sapa_fused_forward_wants_map(int B, int d, int C, int H, int W, int K, int s, int dtype) {
-    if (B <= 0 || d <= 0 || C <= 0 || H <= 0 || W <= 0) return 0;
-    return K == 5 && s == 2 && dtype == SAPA_F32 && fused_f32_on_strips(C, W) ? 1 : 0;
+    return sapa_fused_forward_scratch(B, d, C, H, W, H, K, s, dtype) != 0 ? 1 : 0;
 }
 
 size_t sapa_fused_backward_workspace(int B, int H, int W, int K, int s, int dtype) {

@@ -62,6 +62,7 @@ struct SArgs {
     const void *v, *wt;    // for outputs with something not finite in their windows
     void *out;
     int B, C, H, W, rows, ytop0, y_begin, y_end;
+    int wrows, wy0;        // low-res rows of the weights, the first of them
     int strips, cblocks, segs, seg_rows;
 };
 // Work item: rows y0 .. y1 - 1 of a strip for one block of channels of one image; neighbouring strips run side by side.
@@ -78,15 +79,15 @@ template <typename T> __device__ __forceinline__ Item item_at(const SArgs &a, in
 
 // One output over the cells of its own window alone; a NaN ends the sum.
 template <typename T> __device__ __noinline__ float pixel_alone(const SArgs &a, int n, int c, int hy, int hx) {
-    const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W);
-    const T *w = static_cast<const T *>(a.wt) + (size_t)n * 25 * hi_plane + (size_t)hy * (2 * a.W) + hx;
+    const size_t w_plane = (size_t)(2 * a.wrows) * (2 * a.W);
+    const T *w = static_cast<const T *>(a.wt) + (size_t)n * 25 * w_plane + (size_t)(hy - 2 * a.wy0) * (2 * a.W) + hx;
     const T *v = static_cast<const T *>(a.v) + ((size_t)n * a.C + c) * a.rows * a.W;
     float s = 0.f;
 #pragma unroll 1
     for (int k = 0; k < 25 && s == s; ++k) {
         const int y = a.ytop0 + (hy >> 1) + k / 5 - 2, x = (hx >> 1) + k % 5 - 2;
         if (y < 0 || y >= a.rows || x < 0 || x >= a.W) continue;
-        const float wk = to_acc(w[k * hi_plane]);
+        const float wk = to_acc(w[k * w_plane]);
         s = wk == wk ? fmaf(wk, to_acc(v[(size_t)y * a.W + x]), s) : wk;
     }
     return s;
@@ -140,7 +141,7 @@ template <typename T> __device__ __noinline__ void finish_pixels(const SArgs &a,
         nan |= reached<T>(m.nan); any |= reached<T>(m.any());
         up[dy] = m.up; down[dy] = m.down;
     }
-    const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W);
+    const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W), w_plane = (size_t)(2 * a.wrows) * (2 * a.W);
 #pragma unroll 1
     for (int q = 0; q < 2 * G::PX / PER; ++q) {                       // chunks of 16 bytes of the two rows
         const int r = q / (G::PX / PER), px0 = q % (G::PX / PER) * PER;
@@ -152,10 +153,10 @@ template <typename T> __device__ __noinline__ void finish_pixels(const SArgs &a,
             *reinterpret_cast<uint4 *>(o) = finite::nan_chunk<T>();
             continue;
         }
-        const T *const wt = static_cast<const T *>(a.wt) + (size_t)n * 25 * hi_plane + at;
+        const T *const wt = static_cast<const T *>(a.wt) + (size_t)n * 25 * w_plane + at - (size_t)(2 * a.wy0) * (2 * a.W);
         const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(o));   // stored by TMA: not from L1
         const unsigned words[4] = {w.x, w.y, w.z, w.w};
-        if (!finite::all_finite<T, 4>(words) && finite::all_nan<T>(*reinterpret_cast<const uint4 *>(wt + 12 * hi_plane))) {
+        if (!finite::all_finite<T, 4>(words) && finite::all_nan<T>(*reinterpret_cast<const uint4 *>(wt + 12 * w_plane))) {
             *reinterpret_cast<uint4 *>(o) = finite::nan_chunk<T>();   // weights of NaN for the pixels' own cells
             continue;
         }
@@ -166,7 +167,7 @@ template <typename T> __device__ __noinline__ void finish_pixels(const SArgs &a,
         for (int k = 0; k < 25; ++k) {
             const unsigned u = (unsigned)(up[k / 5] >> (FIRST + px0 / 2 + k % 5)), d = (unsigned)(down[k / 5] >> (FIRST + px0 / 2 + k % 5));
             if (((u | d) & (unsigned)PARENTS) == 0u) continue;
-            const uint4 wk = *reinterpret_cast<const uint4 *>(wt + k * hi_plane);
+            const uint4 wk = *reinterpret_cast<const uint4 *>(wt + k * w_plane);
 #pragma unroll
             for (int e = 0; e < PER; ++e)
                 if ((u | d) >> (e / 2) & 1) s[e] = fmaf(finite::element<T>(wk, e), u >> (e / 2) & 1 ? INFINITY : -INFINITY, s[e]);
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                     if (y < t.y0 + 2) continue;
                     if (!mbar_wait_bounded(wempty + 8 * ws, wph ^ 1)) { ok = false; break; }
                     mbar_expect_tx(wfull + 8 * ws, L_BYTES);
-                    tma_load_4d(base + G::L0 + ws * L_BYTES, &wmap, wfull + 8 * ws, 2 * t.x0, 0, 2 * (y - 2), t.n);
+                    tma_load_4d(base + G::L0 + ws * L_BYTES, &wmap, wfull + 8 * ws, 2 * t.x0, 0, 2 * (y - 2 - a.wy0), t.n);
                     if (++ws == NWL) { ws = 0; wph ^= 1; }
                 }
             }

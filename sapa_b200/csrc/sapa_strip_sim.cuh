@@ -25,7 +25,8 @@ constexpr int LOGITS = 0, SOFTMAX = 1, SOFTMAX_BWD = 2;
 
 struct Args {
     const float *attn;     // SOFTMAX_BWD: the saved map
-    float *out;            // [B, 25, 2H, 2W]: logits, attention map or logit gradients
+    float *out;            // [B, 25, 2 map_rows, 2W], from low-res row map_y0 on: logits, attention map or logit gradients
+    int map_rows, map_y0;
     int B, d, H, W, ytop0, y_begin, y_end;
     int strips, pairs, stages;
 };
@@ -178,13 +179,13 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
         // thread = lane of S: pixel `lane` of high-res row (warp & 3) of the unit, whose low-res row is (warp & 3) / 2
         const int group = warp >> 2, row = warp & 3, shift = lane >> 1;
         const unsigned from = tmem + quarter + group * Z::N + (row >> 1) * Z::SPAN;
-        const size_t hi_plane = (size_t)(2 * a.H) * (2 * a.W);
+        const size_t hi_plane = (size_t)(2 * a.map_rows) * (2 * a.W);
         int step = 0, ph = 0;
         for (int i = blockIdx.x; i < units && ok; i += gridDim.x, ++step) {
             if ((step & 1) != group) continue;
             const Z::Unit u = Z::unit_at(a, i);
             const bool inside = u.y + (row >> 1) < a.y_end && u.x0 + shift < a.W;
-            const size_t at = (size_t)u.n * 25 * hi_plane + (size_t)(2 * u.y + row) * (2 * a.W) + 2 * u.x0 + lane;
+            const size_t at = (size_t)u.n * 25 * hi_plane + (size_t)(2 * (u.y - a.map_y0) + row) * (2 * a.W) + 2 * u.x0 + lane;
             float w[WHAT == Z::SOFTMAX_BWD ? 25 : 1];
             if (WHAT == Z::SOFTMAX_BWD)
 #pragma unroll

@@ -1107,6 +1107,7 @@ template <typename T> static StripPlan strip_plan(int B, int C, int H, int W, in
     StripPlan p{};
     strip::SArgs &a = p.a;
     a.B = B; a.C = C; a.H = H; a.W = W; a.rows = rows; a.ytop0 = ytop0; a.y_begin = y_begin; a.y_end = y_end;
+    a.wrows = H; a.wy0 = 0;
     a.strips = ceil_div(W, strip::Geo<T>::CELLS);
     a.cblocks = ceil_div(C, strip::CH);
     const int band = y_end - y_begin;
@@ -1143,7 +1144,7 @@ static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, i
     constexpr int ES = (int)sizeof(T);
     CUtensorMap vmap{}, wmap{}, omap{};
     if (!make_nchw_map(&vmap, v, a.W, a.rows, a.C, a.B, strip::VROW / ES, std::min(a.C, strip::CH), 1, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE) ||
-        !make_nchw_map(&wmap, wt, 2 * a.W, 2 * a.H, 25, a.B, G::PX, 25, 2, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !make_nchw_map(&wmap, wt, 2 * a.W, 2 * a.wrows, 25, a.B, G::PX, 25, 2, ty, ES, CU_TENSOR_MAP_SWIZZLE_NONE) ||
         !make_nchw_map(&omap, out, 2 * a.W, 2 * a.H, a.C, a.B, G::PX, 32, 1, ty, ES, CU_TENSOR_MAP_SWIZZLE_128B)) {
         set_error("%s: cuTensorMapEncodeTiled rejected the tensor layout", name);
         return SAPA_ERR_UNSUPPORTED;
@@ -1202,7 +1203,7 @@ static int launch_strip_fwd(const void *q, const void *k, const void *v, void *o
 // float32 logits of hi (d channels) and lo, their softmax, or its backward with the saved map `attn`
 template <int WHAT>
 static int launch_strip_sim(const void *hi, const void *lo, const void *attn, void *out, int B, int d, int H, int W, int rows, int ytop0, int y_begin, int y_end,
-                            const char *name, cudaStream_t st) {
+                            int map_rows, int map_y0, const char *name, cudaStream_t st) {
     const CUtensorMapDataType ty = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     CUtensorMap xmap{}, lmap{};
     if (!make_nchw_map(&xmap, hi, 2 * W, 2 * H, d, B, 2 * ssim::CELLS, ssim::KCH, 4, ty, 4, CU_TENSOR_MAP_SWIZZLE_NONE) ||
@@ -1212,6 +1213,7 @@ static int launch_strip_sim(const void *hi, const void *lo, const void *attn, vo
     }
     ssim::Args a{};
     a.attn = static_cast<const float *>(attn); a.out = static_cast<float *>(out);
+    a.map_rows = map_rows; a.map_y0 = map_y0;
     a.B = B; a.d = d; a.H = H; a.W = W; a.ytop0 = ytop0; a.y_begin = y_begin; a.y_end = y_end;
     a.strips = ceil_div(W, ssim::CELLS); a.pairs = ceil_div(y_end - y_begin, 2); a.stages = ceil_div(d, ssim::KCH);
     const long long units = (long long)B * a.strips * a.pairs;
@@ -1268,7 +1270,7 @@ bool fused_tma_supported(int W, int dtype) {
 
 int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d,
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
-                           cudaStream_t st, int groups);
+                           cudaStream_t st, int groups, int image_rows, void *scratch, size_t scratch_bytes);
 
 // 16-bit: tiles of 4 x 32 instead of 4 x 8 pixels where at least three quarters of their columns are inside the image (below that
 // idle warps cost what the loads save) and two thirds of the SMs get one.
@@ -1290,8 +1292,15 @@ static bool strip_sim_pays(int groups, int C, int H, int W) {
 // strips: 1 x 256 x 64x64 15.6 -> 14.2; 1 x 48 x 128x128 18.3 -> 17.8; 1 x 128 x 64x64 12.2, 12.7 here; 1 x 64 x 96x96 10.5, 14.4; 1 x 256 x
 // 32x32 10.5, 11.0), although larger batches of smaller images would gain too (16 x 128 x 32x32 29.5, 21.3 here; 8 x 256 x 32x32 23.1, 18.7).
 // 8 x 256 x 64x64 78.6 -> 55.3, 16 x 128 x 64x64 103 -> 66, 4 x 128 x 64x64 29.6 -> 21.5.
-bool fused_f32_on_strips(int C, int W) {
+bool fused_f32_on_strips(int C, int W, int) {
     return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W, 16, 3, 4) && C >= 48 && (double)W * W * C >= (C >= 96 ? 5e5 : 7.5e5);
+}
+// Bytes of the map of one low-res row of an image; the scratch in place of the whole map, which may be half of the output's size: 256 MiB at most (as many images
+// or rows as that holds at a time: 64 x 64 x 128x128, whose map has 419 MB, 614 us through one piece, 628 through two, 695 through seven of 64 MiB).
+size_t fused_scratch_row(int W) { return (size_t)25 * 4 * W * sizeof(float); }
+size_t fused_scratch(int B, int H, int W) {
+    const size_t row = fused_scratch_row(W), limit = (size_t)256 << 20, image = row * H, all = image * B;
+    return all <= limit ? all : image <= limit ? limit / image * image : std::max<size_t>(limit / row & ~(size_t)1, 2) * row;
 }
 // Stage 1 of the backward likewise, softmax backward of the logits and aggregation, from 64 value channels on and with four fifths of the strips' columns inside
 // the image.  The line sees channels and columns alone: a slab's query gradient equals the rows of the image's.  The whole backward, us, tiles -> strips
@@ -1313,15 +1322,17 @@ static bool strip_bwd_16_pays(int C, int W) { return W >= 24 && C >= 32 && tma::
 //        (C = key channels), attn = saved attention map (input), ws = logit gradients (output), out = grad_query.
 // mode 2 (sim): attn (output) = sim(q, k); v, out unused, C ignored.   mode 3 (agg): out = atn(attn (input), v); q, k unused, d ignored.
 int launch_fused_tma(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d, int C,
-                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st, int groups) {
-    return launch_fused_tma_slots(mode, q, k, v, out, attn, ws, B, d, C, H, W, rows, ytop0, y_begin, y_end, dtype, false, st, groups);
+                     int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, cudaStream_t st, int groups, int image_rows,
+                     void *scratch, size_t scratch_bytes) {
+    return launch_fused_tma_slots(mode, q, k, v, out, attn, ws, B, d, C, H, W, rows, ytop0, y_begin, y_end, dtype, false, st, groups, image_rows, scratch, scratch_bytes);
 }
 
 // slots_f32 (16-bit tensors, mode 2 only): `attn` is a float32 tensor - the logits are written at full precision while
-// query and key stay 16-bit.  groups: how many of the B belong to one image (SAPA-D), for the choice of the kernel.
+// query and key stay 16-bit.  groups: how many of the B belong to one image (SAPA-D), image_rows: rows of the image of which a slab is a part, for the choice
+// of the kernel.  scratch: in place of `attn` where the forward goes through a map (fused_scratch).
 int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v, void *out, void *attn, void *ws, int B, int d,
                            int C, int H, int W, int rows, int ytop0, int y_begin, int y_end, int dtype, bool slots_f32,
-                           cudaStream_t st, int groups) {
+                           cudaStream_t st, int groups, int image_rows, void *scratch, size_t scratch_bytes) {
     using namespace tma;
     if (slots_f32 && (dtype == SAPA_F32 || mode != MODE_SIM)) {
         set_error("sapa_tma_fused: float32 slots are for the 16-bit logit mode");
@@ -1349,19 +1360,38 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
             return dtype == SAPA_F16 ? launch_strip<__half>(v, attn, out, p, sms, name, st) : launch_strip<__nv_bfloat16>(v, attn, out, p, sms, name, st);
         }
     }
-    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(groups, d, H, W) : mode == MODE_FWD ? attn != nullptr && fused_f32_on_strips(C, W)
-                                                                          : mode == MODE_BWD && bwd_f32_on_strips(d, W))) {
-        static const char *const names[3] = {"sapa_tma_fused_f32_kernel<fwd>", "sapa_tma_fused_f32_kernel<bwd>", "sapa_tma_fused_f32_kernel<sim>"};
-        const char *name = names[mode];
-        void *slots = mode == MODE_BWD ? ws : attn;
-        int e = mode == MODE_SIM ? launch_strip_sim<ssim::LOGITS>(q, k, nullptr, slots, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
-                : mode == MODE_FWD ? launch_strip_sim<ssim::SOFTMAX>(q, k, nullptr, slots, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
-                                   : launch_strip_sim<ssim::SOFTMAX_BWD>(q, k, attn, slots, B, d, H, W, rows, ytop0, y_begin, y_end, name, st);
+    if (dtype == SAPA_F32 && mode == MODE_FWD && (attn != nullptr || scratch_bytes > 0) && fused_f32_on_strips(C, W, image_rows)) {
+        const char *name = "sapa_tma_fused_f32_kernel<fwd>";
+        int sms = 0;
+        if (int e = device_sms(name, sms)) return e;
+        // images n0 .., rows y0 .. y1 - 1 through a map that holds low-res rows map_y0 and on of each image
+        auto part = [&](int n0, int images, int y0, int y1, void *map, int map_rows, int map_y0) -> int {
+            const size_t hi = (size_t)(2 * H) * (2 * W), lo = (size_t)rows * W;
+            const float *qn = static_cast<const float *>(q) + (size_t)n0 * d * hi, *kn = static_cast<const float *>(k) + (size_t)n0 * d * lo, *vn = static_cast<const float *>(v) + (size_t)n0 * C * lo;
+            if (int e = launch_strip_sim<ssim::SOFTMAX>(qn, kn, nullptr, map, images, d, H, W, rows, ytop0, y0, y1, map_rows, map_y0, name, st)) return e;
+            StripPlan p = strip_plan<float>(images, C, H, W, rows, ytop0, y0, y1, sms);
+            p.a.wrows = map_rows; p.a.wy0 = map_y0;
+            return launch_strip<float>(vn, map, static_cast<float *>(out) + (size_t)n0 * C * hi, p, sms, name, st);
+        };
+        if (attn != nullptr) return part(0, B, y_begin, y_end, attn, H, 0);
+        // scratch: as many images at a time as it holds the rows of, or bands of rows of an image
+        const size_t row_bytes = fused_scratch_row(W), band = (size_t)(y_end - y_begin);
+        const int images = (int)std::min<size_t>((size_t)B, scratch_bytes / (row_bytes * band));
+        const int step = images > 0 ? (int)band : (int)(scratch_bytes / row_bytes) & ~1;
+        for (int n0 = 0; n0 < B; n0 += std::max(images, 1))
+            for (int y0 = y_begin; y0 < y_end; y0 += step)
+                if (int e = part(n0, std::min(std::max(images, 1), B - n0), y0, std::min(y0 + step, y_end), scratch, std::min(step, y_end - y0), y0)) return e;
+        return SAPA_OK;
+    }
+    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(groups, d, H, W) : mode == MODE_BWD && bwd_f32_on_strips(d, W))) {
+        const char *name = mode == MODE_BWD ? "sapa_tma_fused_f32_kernel<bwd>" : "sapa_tma_fused_f32_kernel<sim>";
+        int e = mode == MODE_SIM ? launch_strip_sim<ssim::LOGITS>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, H, 0, name, st)
+                                 : launch_strip_sim<ssim::SOFTMAX_BWD>(q, k, attn, ws, B, d, H, W, rows, ytop0, y_begin, y_end, H, 0, name, st);
         if (e != SAPA_OK) return e;
         if (mode == MODE_SIM) return check_launch(name);
         int sms = 0;
         if ((e = device_sms(name, sms)) != SAPA_OK) return e;
-        return launch_strip<float>(v, slots, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
+        return launch_strip<float>(v, ws, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
     }
     if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(d, W)))) {
         const char *name = mode == MODE_SIM ? (wide ? "sapa_wide_16_kernel<sim>" : "sapa_tma_fused_16_kernel<sim>") : wide ? "sapa_wide_16_kernel<bwd>" : "sapa_tma_fused_16_kernel<bwd>";

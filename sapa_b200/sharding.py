@@ -30,20 +30,21 @@ def row_slice(rows: int, world_size: int, rank: int) -> slice:
     return batch_slice(rows, world_size, rank)
 
 
-def check_row_split(local_rows: int, halo: int, group=None) -> None:
-    """Every rank must own at least ``halo`` rows (a halo comes from the direct neighbour only).  The decision is
+def check_row_split(local_rows: int, halo: int, group=None) -> int:
+    """The rows of the whole image, 0 where there is one process.  Every rank must own at least ``halo`` rows (a halo comes from the direct neighbour only).  The decision is
     taken from the shares of ALL ranks, so that either every rank raises or none does: a rank that raised alone
     would leave its neighbour waiting in a receive."""
     if not dist.is_initialized():
-        return
+        return 0
     world = dist.get_world_size(group)
     if world == 1 or halo == 0:
-        return
+        return 0
     shares = [None] * world
     dist.all_gather_object(shares, int(local_rows), group=group)
     if min(shares) < halo:
         raise ValueError(f"row-slab sharding with a halo of {halo} rows needs at least {halo} rows on every rank, "
                          f"got shares {shares}")
+    return sum(shares)
 
 
 def _exchange_into(padded, halo: int, group=None) -> None:
@@ -176,7 +177,7 @@ class RowSlab:
         self.K, self.s, self.group = kernel_size, scale_factor, group
         self.halo = (kernel_size - 1) // 2
         self.B, self.d, self.C, self.Hl, self.W = batch, channels_qk, channels_v, local_rows, width
-        check_row_split(local_rows, self.halo, group)
+        self.image_rows = check_row_split(local_rows, self.halo, group)      # 0: not known
         rows = local_rows + 2 * self.halo
         self.key_padded = torch.zeros((batch, channels_qk, rows, width), dtype=dtype, device=device)
         self.value_padded = torch.zeros((batch, channels_v, rows, width), dtype=dtype, device=device)
@@ -185,17 +186,20 @@ class RowSlab:
         self._side = torch.cuda.Stream(device=device) if torch.device(device).type == "cuda" else None
         self._halo_done = torch.cuda.Event() if self._side is not None else None
         self.attn = None            # [B, K*K, s*Hl, s*W] of the last forward(keep_attn=True)
-        self._scratch = None        # of its size, where the kernels that go through the map are the faster ones
 
     def _launch(self, query, out, row_begin, row_end):
         from . import _lib
-        attn = self.attn
-        if attn is None and _lib.lib().sapa_fused_forward_wants_map(self.B, self.d, self.C, self.Hl, self.W, self.K, self.s, _lib.dtype_code(out)):
-            if self._scratch is None:
-                self._scratch = torch.empty((self.B, self.K * self.K, self.s * self.Hl, self.s * self.W), dtype=out.dtype, device=out.device)
-            attn = self._scratch
-        return _lib.call("sapa_fused_forward_slab_rows", out.device, query, self.key_padded, self.value_padded, out, attn,
-                         self.B, self.d, self.C, self.Hl, self.W, self.halo, self.halo, row_begin, row_end, self.K, self.s,
+        sizes = (self.B, self.d, self.C, self.Hl, self.W)
+        scratch = None              # where the kernels that go through the attention map are the faster ones
+        if self.attn is None:
+            nbytes = _lib.lib().sapa_fused_forward_scratch(*sizes, self.image_rows, self.K, self.s, _lib.dtype_code(out))
+            if nbytes:
+                try:
+                    scratch = torch.empty(nbytes, dtype=torch.uint8, device=out.device)
+                except torch.OutOfMemoryError:
+                    pass            # the kernel that needs none
+        return _lib.call("sapa_fused_forward_part", out.device, query, self.key_padded, self.value_padded, out, self.attn, scratch,
+                         0 if scratch is None else scratch.numel(), *sizes, self.halo, self.halo, row_begin, row_end, self.image_rows, self.K, self.s,
                          _lib.dtype_code(out), allow_unsupported=True)
 
     def forward(self, query, out=None, keep_attn=False):
