@@ -621,11 +621,11 @@ deform_window_bwd_kernel(const T *grad_out, const T *value, const T *offset,
     const int gc = C / G;
     const size_t hi = (size_t)(2 * H) * sW, lo = (size_t)H * W;
     const int lane = threadIdx.x & 31, tid = threadIdx.x;
-    const unsigned blocks = ((unsigned)hi + WIN_THREADS - 1) / WIN_THREADS, groups = (unsigned)(B * G);      // of an (image, group)
+    const unsigned blocks = ((unsigned)hi + blockDim.x - 1) / blockDim.x, groups = (unsigned)(B * G);      // of an (image, group)
     float *const dcol = &sd[0][tid], *const wcol = &sw[0][tid];
     for (unsigned bg = blockIdx.y; bg < groups; bg += gridDim.y)
     for (unsigned block = blockIdx.x; block < blocks; block += gridDim.x) {
-        const unsigned at_pix = block * WIN_THREADS + tid, pix = at_pix < hi ? at_pix : 0u;
+        const unsigned at_pix = block * blockDim.x + tid, pix = at_pix < hi ? at_pix : 0u;
         const bool live = at_pix < hi;
         const int qh = (int)(pix / sW), qw = (int)(pix - (unsigned)qh * sW), py = qh >> 1, px = qw >> 1;
         const T *offp = offset + (size_t)bg * P * 2 * hi + pix, *ap = attn + (size_t)bg * P * hi + pix;
@@ -1015,16 +1015,18 @@ template <typename F> static void for_points(int P, F launch) {
     else launch(std::integral_constant<int, MAXP>());
 }
 // Blocks: pixels of an (image, group) along x, the (image, group)s along y; half-sized ones where the last of a small image would be
-// half empty or more (forward of 2048 x 4 groups x 4x16 pixels, float32: 211 us with whole blocks, 197 with halves).
+// half empty or more (2048 x 4 groups of 4x16 pixels, float32: forward 211 us with whole blocks, 197 with halves; forward and backward 738 and 719,
+// bfloat16 605 and 576).
+static unsigned window_threads(size_t hi) { return hi <= 4 * WIN_THREADS && (hi - 1) % WIN_THREADS < WIN_THREADS / 2 ? WIN_THREADS / 2 : WIN_THREADS; }
+static dim3 window_grid(size_t hi, unsigned threads, int groups) { return dim3((unsigned)((hi + threads - 1) / threads), (unsigned)(groups < 65535 ? groups : 65535), 1); }
 template <int MODE, typename T, typename... A> static void launch_window(int P, int groups, size_t hi, cudaStream_t st, A... args) {
-    const unsigned threads = hi <= 4 * WIN_THREADS && (hi - 1) % WIN_THREADS < WIN_THREADS / 2 ? WIN_THREADS / 2 : WIN_THREADS;
-    const dim3 grid((unsigned)((hi + threads - 1) / threads), (unsigned)(groups < 65535 ? groups : 65535), 1);
-    for_points(P, [&](auto most) { launch_next(deform_window_kernel<T, decltype(most)::value, MODE>, grid, threads, 0, st, args...); });
+    const unsigned threads = window_threads(hi);
+    for_points(P, [&](auto most) { launch_next(deform_window_kernel<T, decltype(most)::value, MODE>, window_grid(hi, threads, groups), threads, 0, st, args...); });
 }
 
 template <int MODE, typename T, typename... A> static void launch_window_bwd(int P, int groups, size_t hi, cudaStream_t st, A... args) {
-    const dim3 grid((unsigned)((hi + WIN_THREADS - 1) / WIN_THREADS), (unsigned)(groups < 65535 ? groups : 65535), 1);
-    for_points(P, [&](auto most) { launch_in_order(deform_window_bwd_kernel<T, decltype(most)::value, MODE>, grid, WIN_THREADS, 0, st, args...); });
+    const unsigned threads = window_threads(hi);
+    for_points(P, [&](auto most) { launch_in_order(deform_window_bwd_kernel<T, decltype(most)::value, MODE>, window_grid(hi, threads, groups), threads, 0, st, args...); });
 }
 
 static int check_deform(const char *fn, int B, int Cq, int C, int H, int W, int P, int s, int G, int dtype) {
