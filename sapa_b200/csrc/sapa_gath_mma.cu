@@ -452,14 +452,15 @@ template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int 
 
 // It serves rows of 16 bytes in and out, but for small images and those that fill few of its lanes or columns.  An image's result must not depend on
 // the batch that it is in, so the line sees one image (all of its groups in SAPA-D) and lies where it is about as fast alone.  us, tiles -> this one, with
-// the similarity of the same sizes in front, float32 | bfloat16: 8 x 256 x 64x64 156 -> 92 | 68 -> 45; one image of 128 x 32x32 17.1 -> 14.1 | 11.5 -> 10.3,
-// 64 x 64x64 15.5, 15.7 | 10.8 -> 10.4, 32 x 32x32 8.7, 9.8 | 9.9 -> 8.3; and where the line leaves them with the tiles: float32 64 x 32x32 11.7, 11.7 here, 16 of
-// them 33.1, 27.9; 32 x 64x64 12.2, 13.0 (16: 69, 65); bfloat16 64 x 16x16 8.1, 9.0, 128 x 64x16 10.6, 10.5 (16: 33, 27).
+// the similarity of the same sizes in front, float32 | bfloat16: 8 x 256 x 64x64 156 -> 91 | 68 -> 45; one image of 128 x 32x32 17.1 -> 14.1 | 11.5 -> 10.3,
+// 64 x 32x32 11.7, 11.7 (16 of them 33.1 -> 27.9) | 10.4 -> 9.1; float32 256 x 16x16 15.9, 18.3 (16: 35.7 -> 28.3); bfloat16 32 x 32x32 9.9 -> 8.3; and where
+// the line leaves them with the tiles: float32 64 x 16x16 9.3, 11.3 here (64: 32.9, 26.7), 32 x 64x64 12.2, 13.0 (16: 69, 65); bfloat16 256 x 16x16 11.4,
+// 12.6 (64: 58, 43).
 template <typename T> static bool umma_pays(int groups, int C, int H, int W) {
     const double values = (double)groups * C * H * W;
     const int cells = gumma::Geo<T>::CELLS, columns = ceil_div(W, cells) * cells;
     if (W % (16 / (int)sizeof(T)) != 0) return false;
-    return sizeof(T) == 4 ? C >= 64 && 2 * W >= columns && values >= 1.2e5 : C >= 32 && 4 * W >= 3 * columns && values >= 3e4;
+    return 4 * W >= 3 * columns && (sizeof(T) == 4 ? C >= 64 && values >= 6e4 : C >= 32 && values >= 3e4);
 }
 
 template <typename T>

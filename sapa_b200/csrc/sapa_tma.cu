@@ -1161,13 +1161,16 @@ static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, i
 }
 
 // The forward on strips takes up to 64 query channels, rows of 16 columns and more (a strip of 32 is less than half full below that) and at
-// least 24 value channels.  A channel of a large image is a page of memory of its own, and this kernel touches all channels of a row where
-// the tiles touch 32 of eight rows: images of more than 100 M values stay with the tiles, counted as if they were square, so that
-// an image's result depends neither on the batch it is in nor on the slab of rows that a process has of it.  bfloat16, us, tiles -> strips: 64 x 256 x 128x128 824 -> 687,
-// 8 x 256 x 64x64 37.3 -> 29.5 (with the attention map 41.8 -> 31.6), 16 x 128 x 64x64 47.7 -> 30.5, 8 x 256 x 32x32 (32 query channels)
-// 18.0 -> 11.2, 2 x 512 x 8x64 11.4 -> 7.7, 1 x 32 x 16x16 6.1 -> 6.3, 4 x 256 x 512x512 826 -> 755, 1 x 128 x 768x768 324 -> 273; 8 columns:
-// 64 x 256 x 16x8 19.1, 24.8 here; large images: 1 x 512 x 512x512 350, 375 here, 1 x 256 x 1024x1024 849, 1050 here.
-static bool strip_fwd_pays(int C, int d, int W) { return d <= sfwd::MAX_D && W >= 16 && C >= 24 && (double)C * W * W <= 1e8; }
+// least 24 value channels, of images of twenty thousand values and more.  A channel of a large image is a page of memory of its own, and this kernel touches
+// all channels of a row where the tiles touch 32 of eight rows: images of more than 100 M values in more than 64 channels stay with the tiles.  A slab
+// goes the way of its image (image_rows).  bfloat16, us, tiles -> strips: 64 x 256 x 128x128 824 -> 700, 8 x 256 x 64x64 35.4 -> 27.2, 16 x 64 x 64x64 30 -> 19 (32
+// query channels), 8 x 256 x 32x32 18.0 -> 11.2, 4 x 256 x 512x512 826 -> 755, 1 x 64 x 2048x1024 865 -> 777; an image alone 256 x 1024x64 64 -> 47, 64 x 64x64 8.1
+// -> 6.3, 256 x 16x16 5.6, 6.0 here (16 of them 11.8 -> 10.6), 128 x 24x24 5.6, 6.6 (16: 12.1 -> 10.1); 8 columns: 64 x 256 x 16x8 19.1, 24.8; smaller images: 64 x
+// 16x16 4.8, 5.2 (16: 7.0, 7.1); large ones: 1 x 256 x 1024x512 420, 458, 8192x128 865, 1014, 4096x512 1748, 2273.
+static bool strip_fwd_pays(int C, int d, int W, int image_rows) {
+    const double n = values(1, C, image_rows, W);
+    return d <= sfwd::MAX_D && W >= 16 && C >= 24 && n >= 2e4 && (n <= 1e8 || C <= 64);
+}
 
 template <typename T>
 static int launch_strip_fwd(const void *q, const void *k, const void *v, void *out, void *attn, int d, StripPlan p, int sms, const char *name, cudaStream_t st) {
@@ -1288,12 +1291,13 @@ static bool strip_sim_pays(int groups, int C, int H, int W) {
     return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && W >= 16 && tma::strips_filled(W, 16, 3, 4) && tma::values(groups, C, H, W) >= 1e4;
 }
 // The forward as two launches, softmax of the logits and aggregation.  An image's result depends neither on the batch it is in nor on the slab of
-// rows that a process has of it, so the line sees channels and columns alone and lies where a single square image is no slower (us, tiles ->
-// strips: 1 x 256 x 64x64 15.6 -> 14.2; 1 x 48 x 128x128 18.3 -> 17.8; 1 x 128 x 64x64 12.2, 12.7 here; 1 x 64 x 96x96 10.5, 14.4; 1 x 256 x
-// 32x32 10.5, 11.0), although larger batches of smaller images would gain too (16 x 128 x 32x32 29.5, 21.3 here; 8 x 256 x 32x32 23.1, 18.7).
-// 8 x 256 x 64x64 78.6 -> 55.3, 16 x 128 x 64x64 103 -> 66, 4 x 128 x 64x64 29.6 -> 21.5.
-bool fused_f32_on_strips(int C, int W, int) {
-    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W, 16, 3, 4) && C >= 48 && (double)W * W * C >= (C >= 96 ? 5e5 : 7.5e5);
+// rows that a process has of it (image_rows), so the line sees one image.  It gives up to two microseconds of a single image of its smallest for a
+// third of a batch of them (us, tiles -> strips, 64 query channels: 128 x 64x64 12.1, 12.3 here, 4 of them 29.6 -> 21, 16 95 -> 65; with 32 query channels 10.3, 11.6, 4
+// 25.5 -> 20.6; 256 x 48x48 12.1 -> 11.9; 256 x 64x64 15.6 -> 13.9; 48 x 128x128 22 -> 20; 8 x 256 x 64x64 72 -> 51) and leaves with the tiles: 64 x 64x64 10.5, 13.7 (16:
+// 75, 57), 256 x 32x32 10.4, 11.1 (16: 44, 30), and flat images, 48 x 8x256 6.3, 9.7, 256 x 4x64 8.0, 9.7, 256 x 16x64 10.4, 11.0.
+bool fused_f32_on_strips(int C, int W, int image_rows) {
+    return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && tma::strips_filled(W, 16, 3, 4) && C >= 48 && (double)W * W * C >= (C >= 96 ? 5e5 : 7.5e5) &&
+           tma::values(1, C, image_rows, W) >= 3e5;
 }
 // Bytes of the map of one low-res row of an image; the scratch in place of the whole map, which may be half of the output's size: 256 MiB at most (as many images
 // or rows as that holds at a time: 64 x 64 x 128x128, whose map has 419 MB, 614 us through one piece, 628 through two, 695 through seven of 64 MiB).
@@ -1311,10 +1315,10 @@ static bool bwd_f32_on_strips(int C, int W) {
 }
 
 // 16 bits: the similarity always runs on strips (us, tiles -> strips, bfloat16: 8 images, 64 channels, 64x64 15.0 -> 11.0; 1 x 32 x 16x16 6.2 ->
-// 4.3; 64 x 32 x 8x8 7.0 -> 5.4); stage 1 of the backward as two launches from 32 value channels on and with three quarters of the strips' columns inside the
+// 4.3; 64 x 32 x 8x8 7.0 -> 5.4); stage 1 of the backward as two launches from 32 value channels on and with five eighths of the strips' columns inside the
 // image.  The whole backward, us: 1 x 32 x 32x32 21.9, 21.5, 64 of them 89 -> 69; 1 x 256 x 64x64 33.7 -> 29.7, 16 x 64 x 64x64 105 -> 81, 4 x 256 x 24x24 32.3 ->
-// 27.6; 16 columns, 64 x 256 x 64x16 239, 253 on strips.
-static bool strip_bwd_16_pays(int C, int W) { return W >= 24 && C >= 32 && tma::strips_filled(W, 32, 3, 4); }
+// 27.6, 2 x 256 x 24x40 28.8 -> 25.7; 16 columns, 64 x 256 x 64x16 239, 253 on strips.
+static bool strip_bwd_16_pays(int C, int W) { return W >= 24 && C >= 32 && tma::strips_filled(W, 32, 5, 8); }
 
 // Returns SAPA_ERR_UNSUPPORTED when a tensor map cannot be built (the caller then uses another kernel).
 // mode 0 (forward): out = atn(softmax(sim(q, k)), v), attn = optional output.
@@ -1407,7 +1411,7 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         };
         return dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
     }
-    if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, W)) {
+    if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, W, image_rows)) {
         const char *name = wide ? "sapa_wide_16_kernel<fwd>" : "sapa_tma_fused_16_kernel<fwd>";
         int sms = 0;
         if (int e = device_sms(name, sms)) return e;

@@ -73,3 +73,25 @@ def test_a_call_that_just_fits():
         finally:
             torch.cuda.set_per_process_memory_fraction(1.0)
     assert float((out.cpu().double() - want.double()).norm() / want.double().norm()) < 4e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(64, 8, 8, 512), (96, 8, 200, 64), (72, 8, 2800, 512)], ids=lambda s: "C%d_d%d_%dx%d" % s)
+def test_a_slab_goes_the_way_of_its_image(shape, dtype):
+    """Flat and tall images, which a slab by itself would take for square ones: told the image's height, its bits are the image's."""
+    from sapa_b200 import _lib
+    from sapa_b200.functions import fused_forward_raw
+    C, d, H, W = shape
+    if dtype == torch.float32:
+        flat = H * 4 < W                  # two launches do not pay for a few rows
+        assert _lib.lib().sapa_fused_forward_wants_map(1, d, C, H, W, 5, 2, 0) == (0 if flat else 1 if W * W * C >= 5e5 else 0)
+    q, k, v = _rand(1, 1, d, 2 * H, 2 * W, scale=0.5, dtype=dtype), _rand(2, 1, d, H, W, scale=0.5, dtype=dtype), _rand(3, 1, C, H, W, dtype=dtype)
+    whole = fused_forward_raw(q, k, v, 5, 2, False)[0]
+    rows = min(16, H - 4)
+    for lo in (2, H - 2 - rows):
+        hi, pad = slice(2 * lo, 2 * (lo + rows)), slice(lo - 2, lo + rows + 2)
+        out = torch.empty(1, C, 2 * rows, 2 * W, dtype=dtype, device=DEV)
+        nbytes = int(_lib.lib().sapa_fused_forward_scratch(1, d, C, rows, W, H, 5, 2, _lib.dtype_code(out)))
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=DEV) if nbytes else None
+        _part(q[:, :, hi].contiguous(), k[:, :, pad].contiguous(), v[:, :, pad].contiguous(), out, scratch, 1, d, C, rows, W, 0, rows, halo=2, image_rows=H)
+        assert torch.equal(out, whole[:, :, hi])
