@@ -51,7 +51,7 @@ extern "C" {
 const char *sapa_last_error(void);
 /* Names of the kernels the most recent entry-point call of the process launched (on whichever thread: PyTorch runs
  * the backward of an autograd Function on a worker thread), comma separated and in launch order, e.g.
- * "sapa_tma_fused_f32_kernel<bwd>,sapa_gath_mma_kernel,sapa_gath_mma_kernel"; "" before the first call.  A host-side
+ * "sapa_strip_sim_kernel<softmax_bwd>,sapa_strip_kernel,sapa_gath_umma_kernel,sapa_gath_umma_kernel"; "" before the first call.  A host-side
  * record (no device work) meant for tests and diagnostics: they assert which kernel a shape exercised, so that a
  * silent fall-back to a slower kernel cannot pass unnoticed.  With several threads calling at once it describes
  * whichever call started last.  The one thread that clears the counter of SAPA-D's list of far points is not named, as the memset

@@ -19,8 +19,7 @@
 //     sums through shared memory (an mbarrier handshake per pair and stage), nothing is CTA-wide in the steady state;
 //   * ring protocol: full / empty mbarriers, one lane of a ninth, producer-only warp refills a slot as soon as all 8 warps released it;
 //     every wait is bounded and raises g_wait_timeout instead of spinning for ever.
-// Larger problems with rows of 16 bytes go to the tcgen05 kernel of sapa_gath_umma.cuh instead (umma_pays), recorded under the name of
-// the form that it stands for.
+// Larger images with rows of 16 bytes go to the tcgen05 kernel of sapa_gath_umma.cuh instead (umma_pays).
 #include "finite.cuh"
 #include "umma_util.cuh"
 
@@ -455,16 +454,17 @@ template <typename T> static UmmaPlan umma_plan(int B, int C, int H, int W, int 
 // the similarity of the same sizes in front, float32 | bfloat16: 8 x 256 x 64x64 156 -> 91 | 68 -> 45; one image of 128 x 32x32 17.1 -> 14.1 | 11.5 -> 10.3,
 // 64 x 32x32 11.7, 11.7 (16 of them 33.1 -> 27.9) | 10.4 -> 9.1; float32 256 x 16x16 15.9, 18.3 (16: 35.7 -> 28.3); bfloat16 32 x 32x32 9.9 -> 8.3; and where
 // the line leaves them with the tiles: float32 64 x 16x16 9.3, 11.3 here (64: 32.9, 26.7), 32 x 64x64 12.2, 13.0 (16: 69, 65); bfloat16 256 x 16x16 11.4,
-// 12.6 (64: 58, 43).
+// 12.6 (64: 58, 43), rows of 40 columns 64 x 24x40 8.2, 9.1 (on strips 256 x 24x40 18.2 -> 12.8).
 template <typename T> static bool umma_pays(int groups, int C, int H, int W) {
     const double values = (double)groups * C * H * W;
     const int cells = gumma::Geo<T>::CELLS, columns = ceil_div(W, cells) * cells;
     if (W % (16 / (int)sizeof(T)) != 0) return false;
-    return 4 * W >= 3 * columns && (sizeof(T) == 4 ? C >= 64 && values >= 6e4 : C >= 32 && values >= 3e4);
+    return C >= (sizeof(T) == 4 ? 64 : 32) && (4 * W >= 3 * columns ? values >= (sizeof(T) == 4 ? 6e4 : 3e4) : sizeof(T) == 2 && 8 * W >= 5 * columns && values >= 1e5);
 }
 
 template <typename T>
-static int launch_umma(const void *hi, const void *wt, void *out, UmmaPlan p, int sms, const char *name, cudaStream_t st) {
+static int launch_umma(const void *hi, const void *wt, void *out, UmmaPlan p, int sms, cudaStream_t st) {
+    static const char *const name = "sapa_gath_umma_kernel";
     using G = gumma::Geo<T>;
     Args &g = p.u.g;
     const CUtensorMapDataType ty = G::F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
@@ -501,7 +501,7 @@ static int launch(const void *hi, const void *wt, void *out, int B, int C, int H
     }
     int sms = 0;
     if (int e = device_sms(name, sms)) return e;
-    if (!ragged && umma_pays<T>(groups, C, H, W)) return launch_umma<T>(hi, wt, out, umma_plan<T>(B, C, H, W, top, bottom, sms), sms, name, st);
+    if (!ragged && umma_pays<T>(groups, C, H, W)) return launch_umma<T>(hi, wt, out, umma_plan<T>(B, C, H, W, top, bottom, sms), sms, st);
     const Form f = ragged ? Form{ROWS, COLS, G::NCH, NT_RAGGED, G::SMEM_BYTES, 1}
                    : wide ? Form{ROWS, gw16::COLS, gw16::NCH, gw16::NT, gw16::SMEM_BYTES, 1}
                           : Form{ROWS, COLS, G::NCH, NT, G::SMEM_BYTES, CTAS_PER_SM};

@@ -1136,8 +1136,9 @@ static bool strip_pays_f32(const StripPlan &p) {
 }
 
 template <typename T>
-static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, int sms, const char *name, cudaStream_t st) {
+static int launch_strip(const void *v, const void *wt, void *out, StripPlan p, int sms, cudaStream_t st) {
     using G = strip::Geo<T>;
+    static const char *const name = "sapa_strip_kernel";
     strip::SArgs &a = p.a;
     const CUtensorMapDataType ty = G::F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                           : std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -1173,7 +1174,8 @@ static bool strip_fwd_pays(int C, int d, int W, int image_rows) {
 }
 
 template <typename T>
-static int launch_strip_fwd(const void *q, const void *k, const void *v, void *out, void *attn, int d, StripPlan p, int sms, const char *name, cudaStream_t st) {
+static int launch_strip_fwd(const void *q, const void *k, const void *v, void *out, void *attn, int d, StripPlan p, int sms, cudaStream_t st) {
+    static const char *const name = "sapa_strip_fwd_kernel";
     strip::SArgs &a = p.a;
     const CUtensorMapDataType ty = std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int dpad = ceil_div(d, 16) * 16;
@@ -1206,7 +1208,8 @@ static int launch_strip_fwd(const void *q, const void *k, const void *v, void *o
 // float32 logits of hi (d channels) and lo, their softmax, or its backward with the saved map `attn`
 template <int WHAT>
 static int launch_strip_sim(const void *hi, const void *lo, const void *attn, void *out, int B, int d, int H, int W, int rows, int ytop0, int y_begin, int y_end,
-                            int map_rows, int map_y0, const char *name, cudaStream_t st) {
+                            int map_rows, int map_y0, cudaStream_t st) {
+    static const char *const names[3] = {"sapa_strip_sim_kernel<logits>", "sapa_strip_sim_kernel<softmax>", "sapa_strip_sim_kernel<softmax_bwd>"}, *const name = names[WHAT];
     const CUtensorMapDataType ty = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     CUtensorMap xmap{}, lmap{};
     if (!make_nchw_map(&xmap, hi, 2 * W, 2 * H, d, B, 2 * ssim::CELLS, ssim::KCH, 4, ty, 4, CU_TENSOR_MAP_SWIZZLE_NONE) ||
@@ -1227,13 +1230,15 @@ static int launch_strip_sim(const void *hi, const void *lo, const void *attn, vo
     int sms = 0;
     if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_strip_sim_kernel<WHAT>), ssim::SMEM, name, sms)) return e;
     launch_next(sapa_strip_sim_kernel<WHAT>, (unsigned)std::min<long long>(units, sms), ssim::NT, ssim::SMEM, st, xmap, lmap, a);
-    return SAPA_OK;
+    return check_launch(name);
 }
 
 // the same in 16 bits: logits (as float32 where asked for) or the softmax backward with the saved map `attn`
 template <typename T, int WHAT>
 static int launch_strip_sim_16(const void *hi, const void *lo, const void *attn, void *out, int B, int d, int H, int W, int rows, int ytop0, int y_begin, int y_end,
-                               const char *name, cudaStream_t st) {
+                               cudaStream_t st) {
+    static const char *const names[3] = {"sapa_strip_sim_16_kernel<logits>", "sapa_strip_sim_16_kernel<logits_f32>", "sapa_strip_sim_16_kernel<softmax_bwd>"},
+                *const name = names[WHAT];
     const CUtensorMapDataType ty = std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int kch = d <= 16 ? 16 : 32;
     CUtensorMap xmap{}, lmap{};
@@ -1256,7 +1261,7 @@ static int launch_strip_sim_16(const void *hi, const void *lo, const void *attn,
         int sms = 0;
         if (int e = prepare_launch(reinterpret_cast<const void *>(sapa_strip_sim_16_kernel<T, WHAT, KCH>), SMEM, name, sms)) return e;
         launch_next(sapa_strip_sim_16_kernel<T, WHAT, KCH>, (unsigned)std::min<long long>(units, sms), s16::NT, SMEM, st, xmap, lmap, a);
-        return SAPA_OK;
+        return check_launch(name);
     };
     return kch == 16 ? go(std::integral_constant<int, 16>{}) : go(std::integral_constant<int, 32>{});
 }
@@ -1352,30 +1357,27 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
         return SAPA_ERR_UNSUPPORTED;
     }
     const bool wide = !ragged && dtype != SAPA_F32 && wide16_pays(W, ceil_div(y_end - y_begin, ROWS), B);
-    if (mode == MODE_AGG && !ragged && (dtype == SAPA_F32 || strip_pays_16(groups, C, H, W))) {
-        const char *name = dtype == SAPA_F32 ? "sapa_tma_fused_f32_kernel<agg>" : wide ? "sapa_wide_16_kernel<agg>" : "sapa_tma_fused_16_kernel<agg>";
-        int sms = 0;
-        if (int e = device_sms(name, sms)) return e;
-        if (dtype == SAPA_F32) {
-            const StripPlan p = strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
-            if (strip_pays_f32(p)) return launch_strip<float>(v, attn, out, p, sms, name, st);
-        } else {
-            const StripPlan p = strip_plan<__half>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
-            return dtype == SAPA_F16 ? launch_strip<__half>(v, attn, out, p, sms, name, st) : launch_strip<__nv_bfloat16>(v, attn, out, p, sms, name, st);
-        }
-    }
+    int sms = 0;
+    if (int e = device_sms("sapa_tma_fused", sms)) return e;
+    auto in_type = [&](auto go) { return dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{}); };
+    // the aggregation on strips, of all rows of the launch
+    auto aggregate = [&](const void *wt) {
+        return in_type([&](auto one) {
+            using T = decltype(one);
+            return launch_strip<T>(v, wt, out, strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, st);
+        });
+    };
+    if (mode == MODE_AGG && !ragged && (dtype == SAPA_F32 ? strip_pays_f32(strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms)) : strip_pays_16(groups, C, H, W)))
+        return aggregate(attn);
     if (dtype == SAPA_F32 && mode == MODE_FWD && (attn != nullptr || scratch_bytes > 0) && fused_f32_on_strips(C, W, image_rows)) {
-        const char *name = "sapa_tma_fused_f32_kernel<fwd>";
-        int sms = 0;
-        if (int e = device_sms(name, sms)) return e;
         // images n0 .., rows y0 .. y1 - 1 through a map that holds low-res rows map_y0 and on of each image
         auto part = [&](int n0, int images, int y0, int y1, void *map, int map_rows, int map_y0) -> int {
             const size_t hi = (size_t)(2 * H) * (2 * W), lo = (size_t)rows * W;
             const float *qn = static_cast<const float *>(q) + (size_t)n0 * d * hi, *kn = static_cast<const float *>(k) + (size_t)n0 * d * lo, *vn = static_cast<const float *>(v) + (size_t)n0 * C * lo;
-            if (int e = launch_strip_sim<ssim::SOFTMAX>(qn, kn, nullptr, map, images, d, H, W, rows, ytop0, y0, y1, map_rows, map_y0, name, st)) return e;
+            if (int e = launch_strip_sim<ssim::SOFTMAX>(qn, kn, nullptr, map, images, d, H, W, rows, ytop0, y0, y1, map_rows, map_y0, st)) return e;
             StripPlan p = strip_plan<float>(images, C, H, W, rows, ytop0, y0, y1, sms);
             p.a.wrows = map_rows; p.a.wy0 = map_y0;
-            return launch_strip<float>(vn, map, static_cast<float *>(out) + (size_t)n0 * C * hi, p, sms, name, st);
+            return launch_strip<float>(vn, map, static_cast<float *>(out) + (size_t)n0 * C * hi, p, sms, st);
         };
         if (attn != nullptr) return part(0, B, y_begin, y_end, attn, H, 0);
         // scratch: as many images at a time as it holds the rows of, or bands of rows of an image
@@ -1387,38 +1389,26 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
                 if (int e = part(n0, std::min(std::max(images, 1), B - n0), y0, std::min(y0 + step, y_end), scratch, std::min(step, y_end - y0), y0)) return e;
         return SAPA_OK;
     }
-    if (dtype == SAPA_F32 && (mode == MODE_SIM ? strip_sim_pays(groups, d, H, W) : mode == MODE_BWD && bwd_f32_on_strips(d, W))) {
-        const char *name = mode == MODE_BWD ? "sapa_tma_fused_f32_kernel<bwd>" : "sapa_tma_fused_f32_kernel<sim>";
-        int e = mode == MODE_SIM ? launch_strip_sim<ssim::LOGITS>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, H, 0, name, st)
-                                 : launch_strip_sim<ssim::SOFTMAX_BWD>(q, k, attn, ws, B, d, H, W, rows, ytop0, y_begin, y_end, H, 0, name, st);
-        if (e != SAPA_OK) return e;
-        if (mode == MODE_SIM) return check_launch(name);
-        int sms = 0;
-        if ((e = device_sms(name, sms)) != SAPA_OK) return e;
-        return launch_strip<float>(v, ws, out, strip_plan<float>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
+    if (dtype == SAPA_F32 && mode == MODE_SIM && strip_sim_pays(groups, d, H, W))
+        return launch_strip_sim<ssim::LOGITS>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, H, 0, st);
+    if (dtype == SAPA_F32 && mode == MODE_BWD && bwd_f32_on_strips(d, W)) {
+        const int e = launch_strip_sim<ssim::SOFTMAX_BWD>(q, k, attn, ws, B, d, H, W, rows, ytop0, y_begin, y_end, H, 0, st);
+        return e != SAPA_OK ? e : aggregate(ws);
     }
     if (dtype != SAPA_F32 && !ragged && (mode == MODE_SIM || (mode == MODE_BWD && strip_bwd_16_pays(d, W)))) {
-        const char *name = mode == MODE_SIM ? (wide ? "sapa_wide_16_kernel<sim>" : "sapa_tma_fused_16_kernel<sim>") : wide ? "sapa_wide_16_kernel<bwd>" : "sapa_tma_fused_16_kernel<bwd>";
-        int sms = 0;
-        if (int e = device_sms(name, sms)) return e;
         auto go = [&](auto one) -> int {
             using T = decltype(one);
-            int e = mode == MODE_BWD ? launch_strip_sim_16<T, s16::SOFTMAX_BWD>(q, k, attn, ws, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
-                    : slots_f32      ? launch_strip_sim_16<T, s16::LOGITS_F32>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, name, st)
-                                     : launch_strip_sim_16<T, s16::LOGITS>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, name, st);
-            if (e != SAPA_OK) return e;
-            return mode == MODE_SIM ? check_launch(name) : launch_strip<T>(v, ws, out, strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, name, st);
+            return mode == MODE_BWD ? launch_strip_sim_16<T, s16::SOFTMAX_BWD>(q, k, attn, ws, B, d, H, W, rows, ytop0, y_begin, y_end, st)
+                   : slots_f32      ? launch_strip_sim_16<T, s16::LOGITS_F32>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, st)
+                                    : launch_strip_sim_16<T, s16::LOGITS>(q, k, nullptr, attn, B, d, H, W, rows, ytop0, y_begin, y_end, st);
         };
-        return dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
+        const int e = dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
+        return e != SAPA_OK || mode == MODE_SIM ? e : aggregate(ws);
     }
     if (mode == MODE_FWD && !ragged && dtype != SAPA_F32 && strip_fwd_pays(C, d, W, image_rows)) {
-        const char *name = wide ? "sapa_wide_16_kernel<fwd>" : "sapa_tma_fused_16_kernel<fwd>";
-        int sms = 0;
-        if (int e = device_sms(name, sms)) return e;
         auto go = [&](auto one) -> int {
             using T = decltype(one);
-            const StripPlan p = strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms);
-            return launch_strip_fwd<T>(q, k, v, out, attn, d, p, sms, name, st);
+            return launch_strip_fwd<T>(q, k, v, out, attn, d, strip_plan<T>(B, C, H, W, rows, ytop0, y_begin, y_end, sms), sms, st);
         };
         return dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{});
     }

@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import rel_err
+from conftest import expected_agg, expected_fused_backward, rel_err
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -46,11 +46,11 @@ def test_config2_16bit_full_size_vs_oracle(sp, oracle, dtype):
     qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
     out = sp.sapa_fused(qd, kd, vd, K, s)
     torch.cuda.synchronize()
-    assert _lib.last_kernels() == ["sapa_wide_16_kernel<fwd>"]
+    assert _lib.last_kernels() == ["sapa_strip_fwd_kernel"]
     assert rel_err(host64(out), want) < 1e-2
     fq, fk, fv = torch.autograd.grad(out, (qd, kd, vd), go.to(DEV))
     torch.cuda.synchronize()
-    assert _lib.last_kernels() == ["sapa_wide_16_kernel<bwd>", "sapa_gath_wide_16_kernel", "sapa_gath_wide_16_kernel"]
+    assert _lib.last_kernels() == ["sapa_strip_sim_16_kernel<softmax_bwd>", "sapa_strip_kernel", "sapa_gath_umma_kernel", "sapa_gath_umma_kernel"]
     for got, ref in ((fq, wq), (fk, wk), (fv, wv)):
         assert rel_err(host64(got), ref) < 3e-2
 
@@ -158,8 +158,7 @@ def test_row_slab_backward_of_two_slabs_sums_to_the_unsharded_gradients(dtype, t
         ws = torch.empty(nb, dtype=torch.uint8, device=dev)
         _lib.call("sapa_fused_backward_slab", dev, go[:, :, hi].contiguous(), ql, slab.key_padded, slab.value_padded, slab.attn,
                   mq, mk, mv, ws, nb, B, d, C, hl, W, r, r, K, s, code)
-        assert _lib.last_kernels() == [f"sapa_tma_fused_{'f32' if dtype == torch.float32 else '16'}_kernel<bwd>",
-                                       "sapa_gath_mma_kernel", "sapa_gath_mma_kernel"]
+        assert _lib.last_kernels() == expected_fused_backward(K, s, W, "f32" if dtype == torch.float32 else "bf16", B, hl, C, d)
         assert torch.equal(mq, gq[:, :, hi])
         sum_k[:, :, half * hl:half * hl + hl + 2 * r] += mk.float()
         sum_v[:, :, half * hl:half * hl + hl + 2 * r] += mv.float()
@@ -219,10 +218,10 @@ def test_deform_16bit_dense_window_forward_and_backward(sp, dtype, tol, sigma):
     t32 = [t.detach().float().requires_grad_() for t in t16]
     go16 = go.to(dtype)
     out = sp.deform_sapa_fused(*t16, P, s, G)
-    assert _lib.last_kernels()[0] == "sapa_tma_fused_16_kernel<sim>"
+    assert _lib.last_kernels()[0] == "sapa_strip_sim_16_kernel<logits_f32>"
     got = torch.autograd.grad(out, t16, go16)
     kernels = _lib.last_kernels()
-    assert kernels[:2] == ["sapa_tma_fused_16_kernel<sim>"] * 2 and kernels[-1] == "deform_add_scatter_kernel"
+    assert kernels[:2] == ["sapa_strip_sim_16_kernel<logits_f32>"] * 2 and kernels[-1] == "deform_add_scatter_kernel"
     ref_out = sp.deform_sapa_fused(*t32, P, s, G)
     ref = torch.autograd.grad(ref_out, t32, go16.float())
     for a, b in [(out, ref_out)] + list(zip(got, ref)):
@@ -245,7 +244,7 @@ def test_deform_16bit_separate_ops_through_the_window(sp, dtype, tol):
     q16, k16, v16, o16 = (t.to(dtype).requires_grad_() for t in (q, k, v, off))
     q32, k32, v32, o32 = (t.detach().float().requires_grad_() for t in (q16, k16, v16, o16))
     sim = sp.deform_qk(q16, k16, o16, P, s, G)
-    assert _lib.last_kernels() == ["sapa_tma_fused_16_kernel<sim>", "deform_window_kernel<logits>"]
+    assert _lib.last_kernels() == ["sapa_strip_sim_16_kernel<logits_f32>", "deform_window_kernel<logits>"]
     got = torch.autograd.grad(sim, (q16, k16, o16), gs.to(dtype))
     assert _lib.last_kernels()[-1] == "deform_add_scatter_kernel"
     sim32 = sp.deform_qk(q32, k32, o32, P, s, G)
@@ -255,7 +254,7 @@ def test_deform_16bit_separate_ops_through_the_window(sp, dtype, tol):
     a16 = torch.softmax(sim32.detach(), dim=2).to(dtype).requires_grad_()
     a32 = a16.detach().float().requires_grad_()
     out = sp.deform_av(a16, v16, o16, P, s, G)
-    assert _lib.last_kernels()[:2] == ["deform_window_kernel<weights>", "sapa_tma_fused_16_kernel<agg>"]
+    assert _lib.last_kernels()[:2] == ["deform_window_kernel<weights>"] + expected_agg(5, 2, W, "bf16", B * G, H, C // G, G)
     got = torch.autograd.grad(out, (a16, v16, o16), go.to(dtype))
     assert _lib.last_kernels()[-1] == "deform_add_scatter_kernel"
     out32 = sp.deform_av(a32, v32, o32, P, s, G)

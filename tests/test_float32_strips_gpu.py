@@ -2,6 +2,7 @@
 aggregation - the similarity, the fused forward with and without its map, and its backward, against float64."""
 import pytest
 import torch
+from conftest import expected_fused_backward
 import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
@@ -43,8 +44,11 @@ def test_strips_vs_float64(shape):
         return float((a.detach().double() - b.detach()).norm() / b.detach().norm())
     for _ in range(2):
         out = sp.sapa_fused(*t, 5, 2)
+        assert _lib.last_kernels() == ["sapa_strip_sim_kernel<softmax>", "sapa_strip_kernel"]
         got = torch.autograd.grad(out, t, go)
+        assert _lib.last_kernels() == expected_fused_backward(5, 2, W, "f32", B, H, C, d)
         assert off(sp.qk(t[0].detach(), t[1].detach(), 5, 2), logits) < 5e-7 + 1e-8 * d
+        assert _lib.last_kernels() == ["sapa_strip_sim_kernel<logits>"]
         assert off(out, want) < 1.3e-6 + 1e-8 * d
         for a, b in zip(got, grads):
             assert off(a, b) < 2e-6 + 1e-8 * max(C, d)

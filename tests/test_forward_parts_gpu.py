@@ -87,6 +87,9 @@ def test_a_slab_goes_the_way_of_its_image(shape, dtype):
         assert _lib.lib().sapa_fused_forward_wants_map(1, d, C, H, W, 5, 2, 0) == (0 if flat else 1 if W * W * C >= 5e5 else 0)
     q, k, v = _rand(1, 1, d, 2 * H, 2 * W, scale=0.5, dtype=dtype), _rand(2, 1, d, H, W, scale=0.5, dtype=dtype), _rand(3, 1, C, H, W, dtype=dtype)
     whole = fused_forward_raw(q, k, v, 5, 2, False)[0]
+    ran = set(_lib.last_kernels())
+    if dtype == torch.bfloat16 and H * W * C > 1e8:
+        assert ran == {"sapa_wide_16_kernel<fwd>"}
     rows = min(16, H - 4)
     for lo in (2, H - 2 - rows):
         hi, pad = slice(2 * lo, 2 * (lo + rows)), slice(lo - 2, lo + rows + 2)
@@ -94,4 +97,4 @@ def test_a_slab_goes_the_way_of_its_image(shape, dtype):
         nbytes = int(_lib.lib().sapa_fused_forward_scratch(1, d, C, rows, W, H, 5, 2, _lib.dtype_code(out)))
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=DEV) if nbytes else None
         _part(q[:, :, hi].contiguous(), k[:, :, pad].contiguous(), v[:, :, pad].contiguous(), out, scratch, 1, d, C, rows, W, 0, rows, halo=2, image_rows=H)
-        assert torch.equal(out, whole[:, :, hi])
+        assert torch.equal(out, whole[:, :, hi]) and (set(_lib.last_kernels()) == ran or "strip" not in _lib.last_kernels()[0])

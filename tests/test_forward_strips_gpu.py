@@ -26,7 +26,7 @@ def _forward(q, k, v):
 # 2-norms.  The attention map is rounded once (half an ulp at most, 0.3 of one in the mean: 1.7e-3 in bfloat16, 2.1e-4 in float16), the
 # output is a sum of products with rounded weights, rounded again (1.4 of that)
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2.1e-3), (torch.float16, 2.6e-4)])
-@pytest.mark.parametrize("shape", [(1, 24, 8, 3, 16), (2, 130, 16, 7, 40), (3, 300, 24, 41, 72), (40, 48, 33, 20, 24), (2, 256, 48, 150, 104), (5, 200, 64, 70, 136),
+@pytest.mark.parametrize("shape", [(1, 24, 8, 3, 16), (1, 24, 8, 53, 16), (2, 130, 16, 7, 40), (3, 300, 24, 41, 72), (40, 48, 33, 20, 24), (2, 256, 48, 150, 104), (5, 200, 64, 70, 136),
                                    (1, 64, 65, 9, 32), (2, 64, 1, 12, 48)], ids=lambda s: "B%d_C%d_d%d_%dx%d" % s)
 def test_strips_vs_float64(shape, dtype, tol):
     from sapa_b200 import _lib
@@ -37,6 +37,8 @@ def test_strips_vs_float64(shape, dtype, tol):
     first = None
     for keep in (False, True, True):
         out, attn = fused_forward_raw(q, k, v, 5, 2, keep)
+        # the smallest image, and more than 64 query channels, are left to the tiles
+        assert _lib.last_kernels() == ["sapa_strip_fwd_kernel"] or d > 64 or C * H * W < 2e4
         assert float((out.double() - want).norm() / want.norm()) < 1.4 * tol
         assert float((out.double() - want).abs().max() / want.abs().max()) < 4 * tol
         assert first is None or torch.equal(out, first)
@@ -82,6 +84,7 @@ def test_strips_keep_infinities_to_their_windows(shape, dtype):
     for keep in (False, True):
         clean, got = fused_forward_raw(q, k, v, 5, 2, keep)[0], fused_forward_raw(q, k, bad, 5, 2, keep)[0]
         attn = fused_forward_raw(q, k, bad, 5, 2, True)[1]
+        assert _lib.last_kernels() == ["sapa_strip_fwd_kernel"]
         assert torch.isfinite(attn).all()
         reached = (F.max_pool2d((~torch.isfinite(bad)).float(), 5, 1, 2) > 0).repeat_interleave(2, 2).repeat_interleave(2, 3)
         assert torch.equal(got[~reached], clean[~reached])

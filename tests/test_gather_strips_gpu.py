@@ -34,7 +34,7 @@ TOLERANCE = [(torch.float32, 6e-7), (torch.bfloat16, 2e-3), (torch.float16, 2.5e
 
 
 @pytest.mark.parametrize("dtype,tol", TOLERANCE)
-@pytest.mark.parametrize("shape", [(1, 600, 28, 72), (6, 129, 70, 40), (40, 128, 20, 16), (2, 256, 150, 104)], ids=lambda s: "B%d_C%d_%dx%d" % s)
+@pytest.mark.parametrize("shape", [(1, 600, 28, 72), (6, 129, 70, 40), (40, 128, 20, 16), (2, 256, 150, 104), (40, 128, 24, 32)], ids=lambda s: "B%d_C%d_%dx%d" % s)
 def test_strips_vs_float64(shape, dtype, tol):
     from sapa_b200 import _lib
     B, C, H, W = shape
@@ -43,6 +43,7 @@ def test_strips_vs_float64(shape, dtype, tol):
     want = _gather(go, wt)
     for _ in range(3):
         got = _value_grad(go, wt, C, H, W)
+        assert _lib.last_kernels()[-1] == "sapa_gath_umma_kernel" or W == 16      # the smallest images are left to the tiles
         assert float((got.double() - want).norm() / want.norm()) < tol
         assert float((got.double() - want).abs().max() / want.abs().max()) < 4 * tol
     assert _lib.wait_timeout_flags(DEV) == 0
@@ -64,6 +65,7 @@ def test_strips_of_a_slab(dtype, tol):
     ws = torch.empty(nb, dtype=torch.uint8, device=DEV)
     _lib.call("sapa_fused_backward_slab", torch.device(DEV), go, q, slab.key_padded, slab.value_padded, slab.attn, mq, mk, mv, ws, nb,
               B, d, C, H, W, r, r, 5, 2, code)
+    assert _lib.last_kernels()[-2:] == ["sapa_gath_umma_kernel"] * 2
     ds = ws[:B * 25 * 4 * H * W * q.element_size()].view(dtype).view(B, 25, 2 * H, 2 * W)
     for got, want in ((mv, _gather(go, slab.attn, r)), (mk, _gather(q, ds, r))):
         assert got.shape == want.shape and float((got.double() - want).norm() / want.norm()) < tol
@@ -72,6 +74,7 @@ def test_strips_of_a_slab(dtype, tol):
 
 @pytest.mark.parametrize("dtype,tol", TOLERANCE)
 def test_strips_keep_infinities_to_their_cells(dtype, tol):
+    from sapa_b200 import _lib
     B, C, H, W = 2, 300, 40, 72
     wt = (torch.rand(B, 25, 2 * H, 2 * W, generator=torch.Generator().manual_seed(1)) + 0.1).to(dtype).to(DEV)
     go = _rand(2, B, C, 2 * H, 2 * W, dtype=dtype)
@@ -81,6 +84,7 @@ def test_strips_keep_infinities_to_their_cells(dtype, tol):
     marked = F.max_pool2d((~torch.isfinite(bad)).float(), 2) > 0
     reached = F.max_pool2d(marked.float(), 5, 1, 2) > 0
     clean, got = _value_grad(go, wt, C, H, W), _value_grad(bad, wt, C, H, W)
+    assert _lib.last_kernels()[-1] == "sapa_gath_umma_kernel"
     assert not torch.isfinite(got[reached]).any()
     a, b = got[~reached].double(), clean[~reached].double()
     assert float((a - b).abs().max() / b.abs().max()) < 4 * tol      # cells of the marked rows: sums in another order

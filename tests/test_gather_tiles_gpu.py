@@ -32,6 +32,6 @@ def test_gather_vs_float64(shape, dtype, tol):
     attn, go, v = (torch.randn(*s, generator=g).to(dtype) for s in ((B, 25, 2 * H, 2 * W), (B, C, 2 * H, 2 * W), (B, C, H, W)))
     t = v.to(DEV).requires_grad_()
     got = torch.autograd.grad(sp.av(attn.to(DEV), t, 5, 2), t, go.to(DEV))[0]
-    assert _lib.last_kernels()[-1] == expected_gath(5, 2, W, {torch.float32: "f32", torch.bfloat16: "bf16", torch.float16: "f16"}[dtype])
+    assert _lib.last_kernels()[-1] == expected_gath(5, 2, W, {torch.float32: "f32", torch.bfloat16: "bf16", torch.float16: "f16"}[dtype], H, C)
     assert rel_err(got.double().cpu().numpy(), _want(go, attn, v)) < tol
     assert _lib.wait_timeout_flags(DEV) == 0

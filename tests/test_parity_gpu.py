@@ -184,18 +184,18 @@ def test_sapa_b_seeded_vs_oracle(sp, oracle, shape, K):
     wq, wk, wv = oracle.sapa_backward(go.double().numpy(), q.double().numpy(), k.double().numpy(), v.double().numpy(), K, s)
     qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
     out = sp.sapa_fused(qd, kd, vd, K, s)
-    assert ran() == expected_fused_forward(K, s, W, "f32")          # no silent fall-back to a slower kernel
+    assert ran() == expected_fused_forward(K, s, W, "f32", B, H, C, d)          # no silent fall-back to a slower kernel
     assert rel_err(host64(out), want) < 1e-5
     fq, fk, fv = grads(out, (qd, kd, vd), go.to(DEV))
-    assert ran() == expected_fused_backward(K, s, W, "f32")
+    assert ran() == expected_fused_backward(K, s, W, "f32", B, H, C, d)
     assert rel_err(host64(fq), wq) < 2e-5 and rel_err(host64(fk), wk) < 2e-5 and rel_err(host64(fv), wv) < 2e-5
     # separate path: same numbers from three launches, attention rows sum to one
     sim = sp.qk(qd.detach(), kd.detach(), K, s)
-    assert ran() == expected_sim(K, s, W, "f32")
+    assert ran() == expected_sim(K, s, W, "f32", B, H, d)
     prob = torch.softmax(sim, dim=1)
     assert rel_err(host64(prob), want_p) < 1e-5
     sep = sp.av(prob, vd.detach(), K, s)
-    assert ran() == expected_agg(K, s, W, "f32")
+    assert ran() == expected_agg(K, s, W, "f32", B, H, C)
     assert rel_err(host64(sep), want) < 1e-5
 
 
@@ -211,7 +211,7 @@ def test_sapa_b_half_precision_fused_forward_vs_oracle(sp, oracle, shape, dtype)
     q, k, v = (torch.randn(*sh, generator=g).to(dtype) for sh in ((B, d, s * H, s * W), (B, d, H, W), (B, C, H, W)))
     want, want_p = oracle.sapa_forward(q.double().numpy(), k.double().numpy(), v.double().numpy(), K, s, return_attn=True)
     out, attn = fused_forward_raw(q.to(DEV), k.to(DEV), v.to(DEV), K, s, True)
-    assert ran() == expected_fused_forward(K, s, W, DTYPE_NAME[dtype], B, H)
+    assert ran() == expected_fused_forward(K, s, W, DTYPE_NAME[dtype], B, H, C, d)
     assert rel_err(host64(out), want) < 1e-2
     assert rel_err(host64(attn), want_p) < 1e-2
     out2, _ = fused_forward_raw(q.to(DEV), k.to(DEV), v.to(DEV), K, s, False)
@@ -222,7 +222,7 @@ def test_sapa_b_half_precision_fused_forward_vs_oracle(sp, oracle, shape, dtype)
     wq, wk, wv = oracle.sapa_backward(go.double().numpy(), q.double().numpy(), k.double().numpy(), v.double().numpy(), K, s)
     qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
     fq, fk, fv = grads(sp.sapa_fused(qd, kd, vd, K, s), (qd, kd, vd), go.to(DEV))
-    assert ran() == expected_fused_backward(K, s, W, DTYPE_NAME[dtype], B, H)
+    assert ran() == expected_fused_backward(K, s, W, DTYPE_NAME[dtype], B, H, C, d)
     for got, want_g in ((fq, wq), (fk, wk), (fv, wv)):
         assert rel_err(host64(got), want_g) < 3e-2
 
@@ -239,10 +239,10 @@ def test_sapa_b_config2_full_size_vs_oracle_float32(sp, oracle):
     wq, wk, wv = oracle.sapa_backward(go.numpy(), q.numpy(), k.numpy(), v.numpy(), K, s)
     qd, kd, vd = (t.to(DEV).requires_grad_() for t in (q, k, v))
     out = sp.sapa_fused(qd, kd, vd, K, s)
-    assert ran() == ["sapa_tma_fused_f32_kernel<fwd>"]
+    assert ran() == expected_fused_forward(K, s, W, "f32", B, H, C, d) == ["sapa_strip_sim_kernel<softmax>", "sapa_strip_kernel"]
     assert rel_err(host64(out), want) < 1e-5
     fq, fk, fv = grads(out, (qd, kd, vd), go.to(DEV))
-    assert ran() == ["sapa_tma_fused_f32_kernel<bwd>", "sapa_gath_mma_kernel", "sapa_gath_mma_kernel"]
+    assert ran() == ["sapa_strip_sim_kernel<softmax_bwd>", "sapa_strip_kernel", "sapa_gath_umma_kernel", "sapa_gath_umma_kernel"]
     assert rel_err(host64(fq), wq) < 2e-5 and rel_err(host64(fk), wk) < 2e-5 and rel_err(host64(fv), wv) < 2e-5
     # size-independent properties
     sep = sp.av(torch.softmax(sp.qk(qd.detach(), kd.detach(), K, s), dim=1), vd.detach(), K, s)

@@ -28,9 +28,9 @@ def test_ragged_rows_vs_oracle(oracle, shape, dtype, tol, tol_grad):
     t = [x.to(DEV).requires_grad_() for x in (q, k, v)]
     fused = sp.sapa_fused(*t, 5, 2)
     name = {torch.float32: "f32", torch.bfloat16: "bf16", torch.float16: "f16"}[dtype]
-    assert _lib.last_kernels() == expected_fused_forward(5, 2, W, name, B, H)
+    assert _lib.last_kernels() == expected_fused_forward(5, 2, W, name, B, H, C, d)
     got = torch.autograd.grad(fused, t, go.to(DEV))
-    assert _lib.last_kernels() == expected_fused_backward(5, 2, W, name, B, H)
+    assert _lib.last_kernels() == expected_fused_backward(5, 2, W, name, B, H, C, d)
     sep = sp.av(torch.softmax(sp.qk(t[0], t[1], 5, 2), dim=1), t[2], 5, 2)
     got_sep = torch.autograd.grad(sep, t, go.to(DEV))
     # the separate ops round the logits and the attention map too: twice the forward's bound

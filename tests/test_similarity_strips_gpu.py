@@ -33,6 +33,7 @@ def test_similarity(shape, dtype, tol):
     want = torch.stack([(q.double() * w).sum(1) for w in _windows(k.double())], 1)
     for _ in range(2):
         got = sp.qk(q, k, 5, 2)
+        assert _lib.last_kernels() == ["sapa_strip_sim_16_kernel<logits>"]
         assert _off(got, want) < tol and float((got.double() - want).abs().max() / want.abs().max()) < 4 * tol
     assert _lib.wait_timeout_flags(DEV) == 0
 
@@ -53,4 +54,6 @@ def test_backward(shape, dtype, tol):
     for _ in range(2):
         for a, b in zip(torch.autograd.grad(sp.sapa_fused(*t, 5, 2), t, go), grads):
             assert _off(a, b) < tol
+        # rows of 16 columns are left to the tiles
+        assert _lib.last_kernels()[:2] == ["sapa_strip_sim_16_kernel<softmax_bwd>", "sapa_strip_kernel"] or W == 16
     assert _lib.wait_timeout_flags(DEV) == 0
