@@ -4,17 +4,19 @@
 //
 // A unit is two low-res rows of a strip of 16 columns: its four high-res rows of 32 pixels are the 128 lanes of ONE product
 //     S[128 px x 120 cells] += X^T[128 px x 32 ch] * L[32 ch x 120 cells],       cells = six rows of the 20 columns that the windows reach
-// per 32 channels, three terms of tf32 (small products first: an accumulation in tensor memory rounds toward zero).
+// per 32 channels, three terms of tf32, the small products of a stage first.  An accumulation in tensor memory rounds toward zero, twelve times a
+// stage, which numbers of one sign feel most: a product is of 64 channels at most, and the sums of those are added in registers (features of one sign,
+// logits of 256 channels 4.7e-6 from float64 in one product, 9.6e-7 in four, of 720 1.6e-5 and 9.5e-7; on tiles 5.2e-6, 1.6e-5; times the same).
 //   * X: a warpgroup reads the landed box (lane = pixel, a channel at a time) and writes both terms to tensor memory as the A operand.
 //   * L: eight warps turn the landed box into rows of channels (unswizzled 8 x 16 byte core matrices) and split it.
 //   * per pixel: a thread reads the 20 cells that its row of pixels reaches of each of its five window rows, shifts its own five to the
-//     front and holds its 25 logits: no shuffles.  Two warpgroups take turns, with an accumulator each.
+//     front and holds its 25 logits: no shuffles.  Two warpgroups take turns.
 namespace ssim {
 
 using namespace ummau;
 
 constexpr int CELLS = 16, SPAN = 20, ROWS6 = 6, N = 128;    // columns of a strip; cells of a row, rows; operand rows (120, rounded up)
-constexpr int KCH = 32;                                     // channels of a stage
+constexpr int KCH = 32, PART = 2;                           // channels of a stage, stages of a product
 constexpr int PIX_WARPS = 8, X_WARP0 = 8, L_WARP0 = 12, L_WARPS = 8, TMA_WARP = 20, MMA_WARP = 21, NT = 22 * 32;
 constexpr int LROW = 112, X_BYTES = 4 * KCH * 128, L_BYTES = ROWS6 * KCH * LROW, SLOT = X_BYTES + L_BYTES, NL = 4;
 constexpr int B_LBO = N * 16, B_TERM = KCH / 4 * B_LBO, B_BYTES = 2 * B_TERM, NB = 2;              // a buffer for each of the two warpgroups that write L
@@ -45,11 +47,11 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
     using namespace ummau;
     namespace Z = ssim;
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ __align__(8) unsigned long long bars[2 * (Z::NL + Z::NA + Z::NB + 2)];
+    __shared__ __align__(8) unsigned long long bars[2 * (Z::NL + Z::NA + Z::NB) + 6];
     __shared__ unsigned tmem_slot;
     const unsigned ring = ((unsigned)__cvta_generic_to_shared(smem_dyn) + 1023u) & ~1023u, bop = ring + Z::NL * Z::SLOT;
     const unsigned full = (unsigned)__cvta_generic_to_shared(bars), empty = full + 8 * Z::NL, aready = empty + 8 * Z::NL, aempty = aready + 8 * Z::NA;
-    const unsigned bready = aempty + 8 * Z::NA, bempty = bready + 8 * Z::NB, sfull = bempty + 8 * Z::NB, sempty = sfull + 16;
+    const unsigned bready = aempty + 8 * Z::NA, bempty = bready + 8 * Z::NB, sfull = bempty + 8 * Z::NB, sempty = sfull + 32;      // sfull: [warpgroup that takes the unit][accumulator]
     const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
     const int units = a.B * a.pairs * a.strips;
 
@@ -57,7 +59,8 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
         for (int i = 0; i < Z::NL; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, 128 + 128); }
         for (int i = 0; i < Z::NA; ++i) { mbar_init(aready + 8 * i, 128); mbar_init(aempty + 8 * i, 1); }
         for (int i = 0; i < Z::NB; ++i) { mbar_init(bready + 8 * i, 128); mbar_init(bempty + 8 * i, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(sfull + 8 * i, 1); mbar_init(sempty + 8 * i, 128); }
+        for (int i = 0; i < 4; ++i) mbar_init(sfull + 8 * i, 1);
+        for (int i = 0; i < 2; ++i) mbar_init(sempty + 8 * i, 128);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == Z::MMA_WARP) {
@@ -92,21 +95,21 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
     } else if (warp == Z::MMA_WARP) {
         constexpr unsigned HI = (128u >> 4) | (1u << 14), IDESC = IDESC_M128<float> | idesc_n(Z::N);
         const unsigned leader = elect_leader(), b_base = warp_uniform(desc_lo(bop, Z::B_LBO));
-        int ab = 0, aph = 0, bb = 0, bph = 0, step = 0;
-        for (int i = blockIdx.x; i < units && ok; i += gridDim.x, ++step) {
-            const int buf = step & 1;
-            ok = mbar_wait_warp(sempty + 8 * buf, ((step >> 1) & 1) ^ 1);
-            const unsigned d = tmem + buf * Z::N;
+        int ab = 0, aph = 0, bb = 0, bph = 0, part = 0, group = 0;
+        for (int i = blockIdx.x; i < units && ok; i += gridDim.x, group ^= 1)
             for (int s = 0; s < a.stages && ok; ++s) {
-                ok = mbar_wait_warp(aready + 8 * ab, aph) && mbar_wait_warp(bready + 8 * bb, bph);
+                const int buf = part & 1, in = s % Z::PART;           // stage of its product
+                if (in == 0) ok = mbar_wait_warp(sempty + 8 * buf, ((part >> 1) & 1) ^ 1);
+                ok = ok && mbar_wait_warp(aready + 8 * ab, aph) && mbar_wait_warp(bready + 8 * bb, bph);
                 if (!ok) break;
+                const unsigned d = tmem + buf * Z::N;
                 tc_fence_after();
                 const unsigned at = tmem + Z::A_COL + ab * 2 * Z::KCH, b = b_base + ((bb * Z::B_BYTES) >> 4);
                 constexpr unsigned KB = 2 * Z::B_LBO >> 4;            // 8 channels further
                 auto product = [&](auto steps) {
                     constexpr int KS = decltype(steps)::value;
 #pragma unroll
-                    for (int ks = 0; ks < KS; ++ks) tc_mma_ta<true>(leader, d, at + Z::KCH + 8 * ks, b + ks * KB, HI, IDESC, s > 0 || ks > 0 ? 1u : 0u);
+                    for (int ks = 0; ks < KS; ++ks) tc_mma_ta<true>(leader, d, at + Z::KCH + 8 * ks, b + ks * KB, HI, IDESC, in > 0 || ks > 0 ? 1u : 0u);
 #pragma unroll
                     for (int ks = 0; ks < KS; ++ks) tc_mma_ta<true>(leader, d, at + 8 * ks, b + (Z::B_TERM >> 4) + ks * KB, HI, IDESC, 1u);
 #pragma unroll
@@ -118,9 +121,11 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
                 tc_commit_by(leader, bempty + 8 * bb);
                 if (++ab == Z::NA) { ab = 0; aph ^= 1; }
                 if (++bb == Z::NB) { bb = 0; bph ^= 1; }
+                if (in == Z::PART - 1 || s == a.stages - 1) {
+                    tc_commit_by(leader, sfull + 16 * group + 8 * buf);
+                    ++part;
+                }
             }
-            if (ok) tc_commit_by(leader, sfull + 8 * buf);
-        }
     } else if (warp >= Z::X_WARP0 && warp < Z::L_WARP0) {
         int slot = 0, phase = 0, ab = 0, aph = 0;
         for (int i = blockIdx.x; i < units && ok; i += gridDim.x)
@@ -178,9 +183,10 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
     } else if (warp < Z::PIX_WARPS) {
         // thread = lane of S: pixel `lane` of high-res row (warp & 3) of the unit, whose low-res row is (warp & 3) / 2
         const int group = warp >> 2, row = warp & 3, shift = lane >> 1;
-        const unsigned from = tmem + quarter + group * Z::N + (row >> 1) * Z::SPAN;
+        const unsigned from0 = tmem + quarter + (row >> 1) * Z::SPAN;
+        const int parts = (a.stages + Z::PART - 1) / Z::PART;
         const size_t hi_plane = (size_t)(2 * a.map_rows) * (2 * a.W);
-        int step = 0, ph = 0;
+        int step = 0, ph = 0;                                         // bit b of ph: the phase of accumulator b
         for (int i = blockIdx.x; i < units && ok; i += gridDim.x, ++step) {
             if ((step & 1) != group) continue;
             const Z::Unit u = Z::unit_at(a, i);
@@ -190,27 +196,35 @@ __global__ void __launch_bounds__(ssim::NT, 1) sapa_strip_sim_kernel(const __gri
             if (WHAT == Z::SOFTMAX_BWD)
 #pragma unroll
                 for (int k = 0; k < 25; ++k) w[WHAT == Z::SOFTMAX_BWD ? k : 0] = inside ? a.attn[at + k * hi_plane] : 0.f;
-            if (!mbar_wait_warp(sfull + 8 * group, ph)) { ok = false; break; }
-            ph ^= 1;
-            tc_fence_after();
             float s[25];
+            for (int p = 0; p < parts; ++p) {
+                const int buf = (step * parts + p) & 1;
+                const unsigned from = from0 + buf * Z::N;
+                if (!mbar_wait_warp(sfull + 16 * group + 8 * buf, ph >> buf & 1)) { ok = false; break; }
+                ph ^= 1 << buf;
+                tc_fence_after();
 #pragma unroll
-            for (int dy = 0; dy < 5; ++dy) {
-                unsigned t[20];
-                tc_ld16(from + dy * Z::SPAN, *reinterpret_cast<unsigned (*)[16]>(&t[0]));
-                sfwd::tc_ld4(from + dy * Z::SPAN + 16, &t[16]);
-                tc_wait_ld();
+                for (int dy = 0; dy < 5; ++dy) {
+                    unsigned t[20];
+                    tc_ld16(from + dy * Z::SPAN, *reinterpret_cast<unsigned (*)[16]>(&t[0]));
+                    sfwd::tc_ld4(from + dy * Z::SPAN + 16, &t[16]);
+                    tc_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 12; ++e) t[e] = shift & 8 ? t[e + 8] : t[e];
+                    for (int e = 0; e < 12; ++e) t[e] = shift & 8 ? t[e + 8] : t[e];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) t[e] = shift & 4 ? t[e + 4] : t[e];
+                    for (int e = 0; e < 8; ++e) t[e] = shift & 4 ? t[e + 4] : t[e];
 #pragma unroll
-                for (int e = 0; e < 6; ++e) t[e] = shift & 2 ? t[e + 2] : t[e];
+                    for (int e = 0; e < 6; ++e) t[e] = shift & 2 ? t[e + 2] : t[e];
 #pragma unroll
-                for (int e = 0; e < 5; ++e) s[5 * dy + e] = __uint_as_float(shift & 1 ? t[e + 1] : t[e]);
+                    for (int e = 0; e < 5; ++e) {
+                        const float x = __uint_as_float(shift & 1 ? t[e + 1] : t[e]);
+                        s[5 * dy + e] = p > 0 ? s[5 * dy + e] + x : x;
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive(sempty + 8 * buf);
             }
-            tc_fence_before();
-            mbar_arrive(sempty + 8 * group);
+            if (!ok) break;
             if (WHAT == Z::SOFTMAX) {
                 float m = s[0], z = 0.f;
 #pragma unroll
