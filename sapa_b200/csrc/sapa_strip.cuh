@@ -11,13 +11,16 @@
 //     not zero.  Its zeros are the same in every step and are written once; two warpgroups overwrite the 25 weights per pixel.
 //     Pixels are ordered parent by parent, so that the pixels of a tile are consecutive columns of D.
 //   * one warp issues the MMAs (N = 16 to 80, N / 2 clocks each), in float32, with three times as many, one for each half of the strip: a warp issues
-//     an MMA in about 26 clocks, with one 32 x 64 x 64x64 took 58 us.  float32 adds the small products first, because an accumulation in
+//     an MMA in about 26 clocks (32 x 64 x 64x64 58 us with one, 54 with two).  float32 adds the small products first, because an accumulation in
 //     tensor memory rounds toward zero: eight roundings of the whole sum instead of twenty-four.
 //   * epilogue: tcgen05.ld (lane = channel), zeros back into D, rows of 128 bytes through shared memory, TMA stores; a warpgroup for each of
 //     the two accumulators (with one for both it was what the kernel waited for: 32 x 64 x 64x64, bfloat16, 45 -> 32 us).
+//   * what is not finite stays out of the products (finite.cuh); a second pass over the rows in question forms the outputs that it reaches.  Formed in
+//     the epilogue, output by output, they took one NaN in the values from 19 to 640 us and a tensor of NaN to 6.8 ms; now 58 and 125 (8 x 256 x
+//     64x64, bfloat16).
 // The kernels on tiles load (and split) a value fragment once per window row and group of pixels that it reaches; their fragment loads, splits
-// and mma.sync issue bound them.  What bounds this one: memory (8 x 256 x 64x64: float32 57 -> 38 us, 4.8 TB/s of reads and mostly writes;
-// bfloat16 32 -> 22, 4.1 TB/s), with few channels the MMAs and the epilogue, which work on 128 lanes (32 x 64 x 64x64: 79 -> 54, 44 -> 30).
+// and mma.sync issue bound them.  What bounds this one: memory (8 x 256 x 64x64: float32 54 -> 37 us, 4.9 TB/s of reads and mostly writes;
+// bfloat16 30 -> 18, 5.1 TB/s), with few channels the MMAs and the epilogue, which work on 128 lanes (32 x 64 x 64x64: 76 -> 51, 42 -> 26).
 namespace strip {
 
 using namespace ummau;

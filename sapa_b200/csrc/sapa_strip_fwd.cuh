@@ -13,7 +13,9 @@
 //   * the aggregation's accumulator is two halves (16 parents each), drained by a warpgroup each while the other half is computed.
 // The logits of a step are computed while the step before is aggregated; a warp each issues the two kinds of MMAs (one for both could not
 // issue them fast enough: 64 x 32 x 32x32 27.8 us, 18.4 with two).  Blocks of 128 value channels compute their logits anew.
-// What bounds it: loads in flight, and memory (64 x 256 x 128x128, bfloat16: 687 us, 4.9 TB/s; 824 on tiles, whose ldmatrix wavefronts and MMA
+// Values that are not finite stay out of the product (finite.cuh) and reach the pixels whose windows hold them; an infinity comes to what its 16-bit weight
+// makes of it.
+// What bounds it: loads in flight, and memory (64 x 256 x 128x128, bfloat16: 700 us, 4.8 TB/s; 824 on tiles, whose ldmatrix wavefronts and MMA
 // issue bound them).  Prefetches of the next rows into L2 make it slower (830).
 namespace sfwd {
 
@@ -31,7 +33,7 @@ static_assert(V_COL + NV * ACOLS <= TMEM_COLS, "tensor memory");
 template <typename T, int KSTEPS> struct Lay {
     using G = strip::Geo<T>;
     // five rows of keys and one step of queries are in use, the others on their way, as shared memory allows: 64 x 256 x 128x128, 64 query channels:
-    // 6 rows, 2 steps and 3 rows of values 739 us, 7, 2 and 3 737, 7, 3 and 2 687
+    // 6 rows, 2 steps and 3 rows of values 739 us, 7, 2 and 3 737, 7, 3 and 2 687 to 700
     static constexpr int KROW = KSTEPS * 16 * 128, NKR = KSTEPS == 4 ? 7 : KSTEPS == 3 ? 8 : 10, NQ = KSTEPS == 4 ? 3 : 4, NVL = KSTEPS == 4 ? 2 : KSTEPS == 3 ? 3 : 4;
     static constexpr int OUT0 = 0, K0 = 4 * OUT_BYTES, Q0 = K0 + NKR * KROW, V0 = Q0 + NQ * 2 * KROW, P0 = V0 + NVL * V_BYTES;
     static constexpr int SMEM = P0 + NP * G::P_BYTES + 1024;

@@ -1358,7 +1358,8 @@ int launch_fused_tma_slots(int mode, const void *q, const void *k, const void *v
     }
     const bool wide = !ragged && dtype != SAPA_F32 && wide16_pays(W, ceil_div(y_end - y_begin, ROWS), B);
     int sms = 0;
-    if (int e = device_sms("sapa_tma_fused", sms)) return e;
+    if (!ragged)
+        if (int e = device_sms("sapa_tma_fused", sms)) return e;
     auto in_type = [&](auto go) { return dtype == SAPA_F32 ? go(float{}) : dtype == SAPA_F16 ? go(__half{}) : go(__nv_bfloat16{}); };
     // the aggregation on strips, of all rows of the launch
     auto aggregate = [&](const void *wt) {
