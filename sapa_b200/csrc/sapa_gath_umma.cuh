@@ -79,7 +79,8 @@ template <typename T> __device__ __forceinline__ Item item_at(const UArgs &u, in
 }
 // the parent rows (of the frame of the high-res rows) that reach an item, clipped to the image
 __device__ __forceinline__ int first_parent(const UArgs &u, const Item &t) { return max(t.y0 - u.g.top - 2, 0); }
-__device__ __forceinline__ int end_parent(const UArgs &u, const Item &t) { return min(t.y1 - u.g.top + 2, u.g.H); }
+// (none for an item of rows that the slab's pixels do not reach)
+__device__ __forceinline__ int end_parent(const UArgs &u, const Item &t) { return max(min(t.y1 - u.g.top + 2, u.g.H), first_parent(u, t)); }
 
 // Parents of strip columns x0 - P0 and so on that hold something not finite in high-res row h of channel c
 template <typename T> __device__ __forceinline__ finite::Marks marks_of(const Args &a, int n, int c, int h, int x0) {

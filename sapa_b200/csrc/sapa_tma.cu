@@ -1291,7 +1291,8 @@ static bool wide16_pays(int W, int tiles_y, int B) {
 }
 
 // float32 on strips of 16 columns, the similarity by itself (us, tiles -> strips: 8 images, 64 channels, 64x64 19.0 -> 14.5; 1 x 64 x 128x128 12.1 -> 8.8;
-// 4 x 16 x 64x64 6.7 -> 5.0; 1 x 32 x 24x24 no slower; left with the tiles: images of fewer than ten thousand values).
+// 4 x 16 x 64x64 6.7 -> 5.0; 1 x 64 x 16x64 5.1 -> 4.4; 1 x 32 x 24x24 4.2 -> 3.7; 4 x 16 x 16x64 3.5, 3.8; left with the tiles: images of fewer than ten
+// thousand values).
 static bool strip_sim_pays(int groups, int C, int H, int W) {
     return tma::encode_tiled_fn() != nullptr && W % 4 == 0 && W >= 16 && tma::strips_filled(W, 16, 3, 4) && tma::values(groups, C, H, W) >= 1e4;
 }

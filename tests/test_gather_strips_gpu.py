@@ -91,3 +91,31 @@ def test_strips_keep_infinities_to_their_cells(dtype, tol):
     only = F.max_pool2d(F.max_pool2d((bad == INF).float(), 2), 5, 1, 2) > 0
     only &= ~(F.max_pool2d(F.max_pool2d(((bad != bad) | (bad == -INF)).float(), 2), 5, 1, 2) > 0)
     assert bool((got[only] == INF).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("top,bottom", [(40, 2), (3, 45)])
+def test_rows_that_no_pixel_reaches(top, bottom, dtype):
+    """A slab's gradients in a frame with more rows around it than its pixels reach: some items of a CTA have none, others have a NaN."""
+    from sapa_b200 import _lib
+    B, C, H, W = 75, 64, 30, 32
+    code = _lib.dtype_code(torch.empty(0, dtype=dtype))
+    q, k = _rand(1, B, C, 2 * H, 2 * W, dtype=dtype), _rand(2, B, C, top + H + bottom, W, dtype=dtype)
+    go, v = _rand(3, B, C, 2 * H, 2 * W, dtype=dtype), _rand(4, B, C, top + H + bottom, W, dtype=dtype)
+    attn = torch.softmax(_rand(5, B, 25, 2 * H, 2 * W, dtype=torch.float32), 1).to(dtype)
+    marked = torch.zeros(B, C, top + H + bottom, W, device=DEV)
+    for n in range(0, B, 4):
+        for c, y, x in ((n % C, 0, 2 * (n % W)), (7, 2 * H - 1, 5), (9, 31, 40)):
+            go[n, c, y, x] = NAN
+            marked[n, c, top + y // 2, x // 2] = 1
+    reached = F.max_pool2d(marked, 5, 1, 2) > 0
+    gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    nb = _lib.fused_backward_workspace(B, H, W, 5, 2, code)
+    _lib.call("sapa_fused_backward_slab", torch.device(DEV), go, q, k, v, attn, gq, gk, gv, torch.empty(nb, dtype=torch.uint8, device=DEV), nb, B, C, C, H, W,
+              top, bottom, 5, 2, code)
+    assert _lib.last_kernels()[-1] == "sapa_gath_umma_kernel"
+    assert torch.equal(~torch.isfinite(gv), reached)
+    outside = torch.ones(top + H + bottom, dtype=torch.bool, device=DEV)
+    outside[top - 2:top + H + 2] = False
+    assert not gv[:, :, outside].any()
+    assert _lib.wait_timeout_flags(DEV) == 0
