@@ -139,11 +139,11 @@ int sapa_fused_forward_slab_rows(const void *query, const void *key, const void 
                                  int B, int d, int C, int H, int W, int halo_top, int halo_bottom,
                                  int row_begin, int row_end, int K, int s, int dtype, void *stream);
 
-/* The general form of the four above: `image_rows` is the height of the whole image of which these H rows are a slab, so that a slab
+/* The general form of the three above: `image_rows` is the height of the whole image of which these H rows are a slab, so that a slab
  * takes the kernels of its image and has its bits (0: not known; H is meant where there are no halos, a square image otherwise), and
  * `scratch`, used where `attn` is NULL and the form in two kernels is the faster one, is in place of the map: the image is then
  * computed in as many parts as fit it, with the same result.  Bytes that are worth it (256 MiB at most): sapa_fused_forward_scratch, 0
- * where none are; without scratch (NULL, or less than two rows of the map) one kernel runs that needs none.  The scratch may be used again
+ * where none are; without scratch (NULL, or less than two rows of the map, or the one that there is) one kernel runs that needs none.  The scratch may be used again
  * as soon as the work queued on `stream` is done. */
 int sapa_fused_forward_part(const void *query, const void *key, const void *value, void *out, void *attn,
                             void *scratch, size_t scratch_bytes, int B, int d, int C, int H, int W, int halo_top, int halo_bottom,

@@ -807,7 +807,8 @@ int sapa_fused_forward_part(const void *query, const void *key, const void *valu
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // a slab of an image whose height is not known goes the way of a square one
     const int image = image_rows > 0 ? image_rows : halo_top == 0 && halo_bottom == 0 ? H : W;
-    if (scratch == nullptr || scratch_bytes < 2 * fused_scratch_row(W)) scratch_bytes = 0;      // two rows of an image at least
+    // two rows of an image at least, or the one that there is
+    if (scratch == nullptr || scratch_bytes < (row_end - row_begin > 1 ? 2 : 1) * fused_scratch_row(W)) scratch_bytes = 0;
     if (K == 5 && fused_tma_supported(W, dtype)) {
         const int e = launch_fused_tma(0, query, key, value, out, attn, nullptr, B, d, C, H, W, a.rows, a.ytop0, row_begin, row_end,
                                        dtype, st, 1, image, scratch, scratch_bytes);

@@ -90,8 +90,7 @@ def test_a_slab_goes_the_way_of_its_image(shape, dtype):
     ran = set(_lib.last_kernels())
     if dtype == torch.bfloat16 and H * W * C > 1e8:
         assert ran == {"sapa_wide_16_kernel<fwd>"}
-    rows = min(16, H - 4)
-    for lo in (2, H - 2 - rows):
+    for lo, rows in ((2, min(16, H - 4)), (H - 2 - min(16, H - 4), min(16, H - 4)), (3, 1), (4, 2)):
         hi, pad = slice(2 * lo, 2 * (lo + rows)), slice(lo - 2, lo + rows + 2)
         out = torch.empty(1, C, 2 * rows, 2 * W, dtype=dtype, device=DEV)
         nbytes = int(_lib.lib().sapa_fused_forward_scratch(1, d, C, rows, W, H, 5, 2, _lib.dtype_code(out)))
