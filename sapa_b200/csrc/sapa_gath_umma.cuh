@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
                         const unsigned at = tmem + quarter + G::DCOLS + ab * G::ABUF;
                         auto store = [&]() { tc_st16(at, v); tc_st16(at + 16, v + 16); tc_st8(at + 32, v + 32); };      // the tensor core reads the top 19 bits of a tf32 operand
                         store();
+                        mbar_arrive(xempty + 8 * slot);               // only here: an arrival does not wait for loads in flight
                         const bool odd = !finite::all_finite<T, ACOLS>(v);
                         if (__any_sync(0xffffffffu, odd)) {
                             tc_wait_st();
@@ -273,8 +274,9 @@ __global__ void __launch_bounds__(NT, 1) sapa_gath_umma_kernel(const __grid_cons
                             for (int q = 0; q < ACOLS; ++q) v[q] = tf32_lo(v[q]);
                             tc_st16(at + ACOLS, v); tc_st16(at + ACOLS + 16, v + 16); tc_st8(at + ACOLS + 32, v + 32);
                         }
+                    } else {
+                        mbar_arrive(xempty + 8 * slot);
                     }
-                    mbar_arrive(xempty + 8 * slot);                   // only here: an arrival does not wait for loads in flight
                     tc_wait_st();
                     tc_fence_before();
                     mbar_arrive(aready + 8 * ab);

@@ -42,6 +42,9 @@ template <typename T> struct Geo {
     static constexpr int SHIFT = F32 ? 2 : 3;               // words from the box's start (16-byte boundary) to cell x0 - 2, the first of the product
     static constexpr int BOX0 = F32 ? 4 : 8;                // the box starts at column x0 - BOX0
     static constexpr int ABUF = TERMS * ACOLS;
+    // words of a row that windows reach (float32: all, zeros for the last four cost 32 x 64 x 64x64 51.7 -> 53.0 us), and the landed chunks that hold them
+    static constexpr int WORDS = F32 ? ACOLS : (CELLS + 4) * (int)sizeof(T) / 4;
+    static constexpr int LOADS = (SHIFT + WORDS + 3) / 4;
     static constexpr int ISSUERS = F32 ? 2 : 1;             // warps that issue the MMAs, each those of half of the strip's parents
     // K step j: parents [p0, p1) of the strip reach its cells (columns x0 - 2 + KS j and so on)
     __host__ __device__ static constexpr int p0(int j) { return KS * j < 4 ? 0 : KS * j - 4; }
@@ -95,18 +98,23 @@ template <typename T> __device__ __noinline__ float pixel_alone(const SArgs &a, 
     }
     return s;
 }
-// Moves the cells of a product from a landed row, float32 in two terms; elements that are not finite become zeros and the row is noted.
-template <typename T> __device__ __forceinline__ void move_cells(unsigned at, unsigned (&v)[4 * VCHUNKS], bool channel, finite::Noted &noted, int quarter, int row) {
+// Moves the cells of a product from a landed row, float32 in two terms; elements that are not finite become zeros and the row is noted.  The landed row is
+// given back (`landed`) as soon as its values have been used: an arrival does not wait for loads in flight.
+template <typename T>
+__device__ __forceinline__ void move_cells(unsigned at, unsigned (&v)[4 * VCHUNKS], bool channel, finite::Noted &noted, int quarter, int row, unsigned landed) {
     using G = Geo<T>;
+#pragma unroll
+    for (int q = G::SHIFT + G::WORDS; q < G::SHIFT + ACOLS; ++q) v[q] = 0u;     // their weights are zero
     auto store = [&]() {
         tc_st16(at, v + G::SHIFT); tc_st8(at + 16, v + G::SHIFT + 16);          // the tensor core reads the top 19 bits of a tf32 operand
     };
     store();
-    const bool odd = !finite::all_finite<T, ACOLS>(v + G::SHIFT);
+    mbar_arrive(landed);
+    const bool odd = !finite::all_finite<T, G::WORDS>(v + G::SHIFT);
     if (__any_sync(0xffffffffu, odd)) {
         tc_wait_st();
 #pragma unroll
-        for (int q = G::SHIFT; q < G::SHIFT + ACOLS; ++q) v[q] = finite::or_zero<T>(v[q]);
+        for (int q = G::SHIFT; q < G::SHIFT + G::WORDS; ++q) v[q] = finite::or_zero<T>(v[q]);
         store();
         if (odd && channel) noted.note(quarter, row);                           // a lane without a channel holds anything
     }
@@ -319,14 +327,14 @@ __global__ void __launch_bounds__(strip::NT, 1) sapa_strip_kernel(const __grid_c
                 unsigned v[4 * VCHUNKS];
                 if (used) {
 #pragma unroll
-                    for (int q = 0; q < VCHUNKS; ++q)
+                    for (int q = 0; q < G::LOADS; ++q)
                         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v[4 * q]), "=r"(v[4 * q + 1]), "=r"(v[4 * q + 2]), "=r"(v[4 * q + 3])
                                      : "r"(base + G::V0 + vs * strip::V_BYTES + line + 16 * q) : "memory");
                 }
                 if (!mbar_wait_warp(aempty + 8 * as, aph ^ 1)) { ok = false; break; }
                 tc_fence_after();
-                if (used) move_cells<T>(tmem + quarter + ring + as * G::ABUF, v, t.c0 + (warp & 3) * 32 + lane < a.C, noted, warp & 3, row);
-                mbar_arrive(vempty + 8 * vs);                         // only here: an arrival does not wait for loads in flight
+                if (used) move_cells<T>(tmem + quarter + ring + as * G::ABUF, v, t.c0 + (warp & 3) * 32 + lane < a.C, noted, warp & 3, row, vempty + 8 * vs);
+                else mbar_arrive(vempty + 8 * vs);
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive(aready + 8 * as);

@@ -320,14 +320,14 @@ __global__ void __launch_bounds__(sfwd::NT, 1) sapa_strip_fwd_kernel(const __gri
                 unsigned v[4 * VCHUNKS];
                 if (used) {
 #pragma unroll
-                    for (int q = 0; q < VCHUNKS; ++q)
+                    for (int q = 0; q < G::LOADS; ++q)
                         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v[4 * q]), "=r"(v[4 * q + 1]), "=r"(v[4 * q + 2]), "=r"(v[4 * q + 3])
                                      : "r"(base + L::V0 + vs * sfwd::V_BYTES + line + 16 * q) : "memory");
                 }
                 if (!mbar_wait_warp(aempty + 8 * as, aph ^ 1)) { ok = false; break; }
                 tc_fence_after();
-                if (used) strip::move_cells<T>(tmem + quarter + V_COL + as * ACOLS, v, t.c0 + (warp & 3) * 32 + lane < a.C, noted, warp & 3, row);
-                mbar_arrive(vempty + 8 * vs);                         // only here: an arrival does not wait for loads in flight
+                if (used) strip::move_cells<T>(tmem + quarter + V_COL + as * ACOLS, v, t.c0 + (warp & 3) * 32 + lane < a.C, noted, warp & 3, row, vempty + 8 * vs);
+                else mbar_arrive(vempty + 8 * vs);
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive(aready + 8 * as);
